@@ -217,10 +217,21 @@ int gemm_entry(int order, int transA, int transB, int64_t m, int64_t n, int64_t 
     Stored da = sa, db = sb, dc = sc;
     bool c_staged = false;
     if (!done) {
+    // float: the split forms run on double copies at the float target (device_product_float); small
+    // products under `auto` stay on the native kernel, as for double
+    const bool split_path = product && method != GB300_METHOD_NATIVE &&
+                            (is_double || !(method == GB300_METHOD_AUTO && split_auto_uses_native(g)));
+    const NativePlan plan = native_plan(g.m, g.n, g.k, int(sizeof(T)), r.num_sms, ctl.inject_stall != 0);
     if (product) {
-        if (!devA || !aligned_for_tma<T>(sa))
+        // device operands are used in place where they are aligned for their elements; the native
+        // kernel's TMA tiles need 16-byte bases and pitches (device_product realigns its own)
+        const bool tma = !split_path && plan.tile == 0;
+        auto in_place = [&](const Stored& x) {
+            return tma ? aligned_for_tma<T>(x) : reinterpret_cast<uintptr_t>(x.ptr) % sizeof(T) == 0;
+        };
+        if (!devA || !in_place(sa))
             if (!stage_in<T>(sa, kSlotA, !devA, s, &da, &err)) return fail(GB300_ERR_NO_MEMORY, err);
-        if (!devB || !aligned_for_tma<T>(sb))
+        if (!devB || !in_place(sb))
             if (!stage_in<T>(sb, kSlotB, !devB, s, &db, &err)) return fail(GB300_ERR_NO_MEMORY, err);
     }
     if (!devC) {
@@ -240,10 +251,6 @@ int gemm_entry(int order, int transA, int transB, int64_t m, int64_t n, int64_t 
     g.C = const_cast<void*>(dc.ptr); g.ldc = dc.ld;
 
     // ---- run ----
-    // float: the split forms run on double copies at the float target (device_product_float); small
-    // products under `auto` stay on the native kernel, as for double
-    const bool split_path = product && method != GB300_METHOD_NATIVE &&
-                            (is_double || !(method == GB300_METHOD_AUTO && split_auto_uses_native(g)));
     if (split_path) {
         SplitRequest req;
         req.method = method;
@@ -261,16 +268,12 @@ int gemm_entry(int order, int transA, int transB, int64_t m, int64_t n, int64_t 
         }
     } else {
         used = GB300_METHOD_NATIVE;
-        int splits = 1;
         T* ws = nullptr;
-        if (g.k > 0) {
-            splits = native_choose_splits(g.m, g.n, g.k, int(sizeof(T)), r.num_sms);
-            if (splits > 1) {
-                ws = static_cast<T*>(pool_get(kSlotWork, size_t(splits) * size_t(g.m) * size_t(g.n) * sizeof(T), &err));
-                if (!ws) return fail(GB300_ERR_NO_MEMORY, err);
-            }
+        if (plan.splits > 1) {
+            ws = static_cast<T*>(pool_get(kSlotWork, size_t(plan.splits) * size_t(g.m) * size_t(g.n) * sizeof(T), &err));
+            if (!ws) return fail(GB300_ERR_NO_MEMORY, err);
         }
-        e = native_gemm<T>(g, splits, ws, ctl, s, &err);
+        e = native_gemm<T>(g, plan, ws, ctl, s, &err);
         if (e != cudaSuccess) return fail(GB300_ERR_CUDA, err.empty() ? cudaGetErrorString(e) : err);
         if (opts) opts->error_bound = double(g.k) * (is_double ? 0x1p-53 : 0x1p-24);
     }

@@ -130,19 +130,16 @@ int real_product(const Gemm& g, const LaunchCtl& ctl, cudaStream_t st, std::stri
         ld = ldp;
         return true;
     };
-    if (g.k > 0 && (!realign(gn.A, gn.lda, g.ta ? g.k : g.m, g.ta ? g.m : g.k, kSlotA) ||
+    const NativePlan plan = native_plan(g.m, g.n, g.k, int(sizeof(T)), r.num_sms, ctl.inject_stall != 0);
+    if (g.k > 0 && plan.tile == 0 && (!realign(gn.A, gn.lda, g.ta ? g.k : g.m, g.ta ? g.m : g.k, kSlotA) ||
                     !realign(gn.B, gn.ldb, g.tb ? g.n : g.k, g.tb ? g.k : g.n, kSlotB)))
         return GB300_ERR_NO_MEMORY;
-    int splits = 1;
     T* w = nullptr;
-    if (g.k > 0) {
-        splits = native_choose_splits(g.m, g.n, g.k, int(sizeof(T)), r.num_sms);
-        if (splits > 1) {
-            w = static_cast<T*>(r.ws.get(kSlotWork, size_t(splits) * size_t(g.m) * size_t(g.n) * sizeof(T), err));
-            if (!w) return GB300_ERR_NO_MEMORY;
-        }
+    if (plan.splits > 1) {
+        w = static_cast<T*>(r.ws.get(kSlotWork, size_t(plan.splits) * size_t(g.m) * size_t(g.n) * sizeof(T), err));
+        if (!w) return GB300_ERR_NO_MEMORY;
     }
-    const cudaError_t e = native_gemm<T>(gn, splits, w, ctl, st, err);
+    const cudaError_t e = native_gemm<T>(gn, plan, w, ctl, st, err);
     return e == cudaSuccess ? GB300_OK : GB300_ERR_CUDA;
 }
 

@@ -63,13 +63,22 @@ bool encode_tmap_3d(CUtensorMap* map, CUtensorMapDataType dtype, size_t elem_byt
                     uint32_t box_rows, uint32_t box_cols, CUtensorMapSwizzle swizzle, std::string* err);
 
 // ---- native (DFMA / FFMA) GEMM --------------------------------------------------------------
-// Launches the TMA-staged SIMT kernel.  `splits` > 1 partitions k; the partial products then go
-// through `workspace` (splits * m * n elements of T) and a fixed-order reduction.
+// How the native kernels run a product: `tile` = 0 for the TMA-staged tiles of 16384 outputs (A and B
+// then need 16-byte aligned bases and pitches), else square tiles of 8, 16 or 32 (any operand aligned
+// for its elements); `splits` > 1 partitions k.
+struct NativePlan {
+    int tile = 0;
+    int splits = 1;
+};
+NativePlan native_plan(int64_t m, int64_t n, int64_t k, int elem_bytes, int num_sms, bool tma_only);
+
+// Runs a plan.  The partial products of a split k go through `workspace` (splits * m * n elements of
+// T) and a fixed-order reduction.
 template <typename T>
-cudaError_t native_gemm(const Gemm& g, int splits, T* workspace, const LaunchCtl& ctl, cudaStream_t s,
+cudaError_t native_gemm(const Gemm& g, const NativePlan& plan, T* workspace, const LaunchCtl& ctl, cudaStream_t s,
                         std::string* err);
 
-// Split count the native kernel uses for a shape on `num_sms` SMs (1 = no split).
+// Split count of the TMA-staged tiles for a shape on `num_sms` SMs (1 = no split).
 int native_choose_splits(int64_t m, int64_t n, int64_t k, int elem_bytes, int num_sms);
 // The shared implementation behind cblas_?gemm and gb300_?gemm_ex (CBLAS argument conventions).
 // The method cblas_?gemm uses (GB300_DGEMM_METHOD / gb300_set_default_method).

@@ -22,6 +22,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <mutex>
 #include <string>
 
@@ -337,6 +338,16 @@ __global__ void splitk_reduce_kernel(const T* __restrict__ ws, int splits, int64
     }
 }
 
+template <typename T>
+cudaError_t launch_splitk_reduce(const Gemm& g, const T* workspace, int splits, cudaStream_t s) {
+    const int64_t total = g.m * g.n;
+    const int blocks = int(std::min<int64_t>((total + 255) / 256, 152 * 16));
+    splitk_reduce_kernel<T><<<blocks, 256, 0, s>>>(workspace, splits, g.m, g.n, T(g.alpha), T(g.beta),
+                                                   static_cast<T*>(g.C), g.ldc);
+    count_launches(1);
+    return cudaGetLastError();
+}
+
 // C = beta * C (k == 0); beta == 0 writes zeros without reading C.
 template <typename T>
 __global__ void scale_c_kernel(int64_t m, int64_t n, T beta, T* __restrict__ C, int64_t ldc) {
@@ -347,6 +358,157 @@ __global__ void scale_c_kernel(int64_t m, int64_t n, T beta, T* __restrict__ C, 
         T* c = C + i * ldc + j;
         *c = (beta == T(0)) ? T(0) : beta * *c;
     }
+}
+
+// ---- small tiles -------------------------------------------------------------------------------
+// The same product in tiles of TM x TN outputs, RM x RN of them per thread, for products whose
+// 128 x 128 tiles would leave most SMs idle: a 96 x 80 x 112 product is a single such tile, whose
+// multiply-adds one SM's FP64 pipe takes 450 us for (2 multiply-adds a clock and SM); in 120 tiles
+// of 8 x 8 it takes a few microseconds.  What bounds it is the FP64 pipe (each multiply-add of a
+// warp holds it for 16 clocks), so one output a thread and two 8-byte shared loads per
+// multiply-add cost nothing; float takes 2 x 2 outputs a thread, which halves the shared loads that
+// bound it.  Operands come in by cp.async of one element a thread, SM_KC k-steps at a time through
+// SM_STAGES buffers: any base and any leading dimension that the element type allows, no tensor map
+// and no realigned copy.  Each output sums its k range in order, as in the tiles above.
+constexpr int SM_KC = 32;
+constexpr int SM_STAGES = 4;
+
+template <typename T>
+struct SmallParams {
+    const T* A;
+    const T* B;
+    T* C;
+    T* ws;                   // split-k partials (splits x m x n) or nullptr
+    int64_t lda, ldb, ldc;
+    int64_t m, n, k, k_per_split;
+    int64_t tiles_n;
+    T alpha, beta;
+};
+
+template <typename T>
+__device__ __forceinline__ void cp_async_elem(uint32_t dst, const T* src, bool valid) {
+    if constexpr (sizeof(T) == 8) cp_async8(dst, src, valid);
+    else cp_async4(dst, src, valid);
+}
+
+template <typename T, int TM, int TN, int RM, int RN, bool TRANS_A, bool TRANS_B>
+__global__ void __launch_bounds__((TM / RM) * (TN / RN)) small_gemm_kernel(const SmallParams<T> p) {
+    constexpr int TX = TN / RN, TY = TM / RM, NT = TX * TY;
+    constexpr int PA = SM_KC + 1, PB = TN + 1;  // odd pitches: transposed writes spread over the banks
+    __shared__ T As[SM_STAGES][TM * PA];
+    __shared__ T Bs[SM_STAGES][SM_KC * PB];
+    const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
+    const int64_t m0 = int64_t(blockIdx.x / p.tiles_n) * TM, n0 = int64_t(blockIdx.x % p.tiles_n) * TN;
+    const int64_t kbeg = int64_t(blockIdx.z) * p.k_per_split, kend = min(p.k, kbeg + p.k_per_split);
+    const int chunks = int((kend - kbeg + SM_KC - 1) / SM_KC);
+
+    // chunk c of the operands into buffer c % SM_STAGES, zeros outside the matrices
+    auto issue = [&](int c) {
+        if (c < chunks) {
+            const int64_t k0 = kbeg + int64_t(c) * SM_KC;
+            const uint32_t sa = smem_u32(As[c % SM_STAGES]), sb = smem_u32(Bs[c % SM_STAGES]);
+#pragma unroll
+            for (int e = tid; e < TM * SM_KC; e += NT) {
+                const int i = TRANS_A ? e % TM : e / SM_KC, kk = TRANS_A ? e / TM : e % SM_KC;
+                const bool ok = m0 + i < p.m && k0 + kk < kend;
+                const T* src = p.A + (TRANS_A ? (k0 + kk) * p.lda + m0 + i : (m0 + i) * p.lda + k0 + kk);
+                cp_async_elem<T>(sa + uint32_t(i * PA + kk) * sizeof(T), ok ? src : p.A, ok);
+            }
+#pragma unroll
+            for (int e = tid; e < TN * SM_KC; e += NT) {
+                const int j = TRANS_B ? e / SM_KC : e % TN, kk = TRANS_B ? e % SM_KC : e / TN;
+                const bool ok = n0 + j < p.n && k0 + kk < kend;
+                const T* src = p.B + (TRANS_B ? (n0 + j) * p.ldb + k0 + kk : (k0 + kk) * p.ldb + n0 + j);
+                cp_async_elem<T>(sb + uint32_t(kk * PB + j) * sizeof(T), ok ? src : p.B, ok);
+            }
+        }
+        cp_async_commit();  // an empty group keeps the wait count uniform
+    };
+
+    T acc[RM][RN];
+#pragma unroll
+    for (int r = 0; r < RM; ++r)
+#pragma unroll
+        for (int c = 0; c < RN; ++c) acc[r][c] = T(0);
+#pragma unroll
+    for (int c = 0; c < SM_STAGES - 1; ++c) issue(c);
+    for (int c = 0; c < chunks; ++c) {
+        cp_async_wait<SM_STAGES - 2>();
+        __syncthreads();  // chunk c is in, and every thread is done with chunk c - 1's buffer
+        issue(c + SM_STAGES - 1);
+        const T* a0 = As[c % SM_STAGES] + ty * PA;
+        const T* b0 = Bs[c % SM_STAGES] + tx;
+        const int kc = int(min(int64_t(SM_KC), kend - kbeg - int64_t(c) * SM_KC));
+#pragma unroll 8
+        for (int kk = 0; kk < kc; ++kk) {
+            T a[RM], b[RN];
+#pragma unroll
+            for (int r = 0; r < RM; ++r) a[r] = a0[r * TY * PA + kk];
+#pragma unroll
+            for (int q = 0; q < RN; ++q) b[q] = b0[kk * PB + q * TX];
+#pragma unroll
+            for (int r = 0; r < RM; ++r)
+#pragma unroll
+                for (int q = 0; q < RN; ++q) acc[r][q] = fma(a[r], b[q], acc[r][q]);
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < RM; ++r) {
+        const int64_t i = m0 + ty + TY * r;
+        if (i >= p.m) continue;
+#pragma unroll
+        for (int q = 0; q < RN; ++q) {
+            const int64_t j = n0 + tx + TX * q;
+            if (j >= p.n) continue;
+            if (p.ws != nullptr) {
+                p.ws[(int64_t(blockIdx.z) * p.m + i) * p.n + j] = acc[r][q];
+                continue;
+            }
+            T* c = p.C + i * p.ldc + j;
+            const T v = p.alpha * acc[r][q];
+            *c = (p.beta == T(0)) ? v : fma(p.beta, *c, v);
+        }
+    }
+}
+
+template <typename T, int TM, int TN, int RM, int RN>
+void launch_small(const Gemm& g, const SmallParams<T>& p, dim3 grid, cudaStream_t s) {
+    constexpr int NT = (TM / RM) * (TN / RN);
+    KernelTimer timer("native_gemm", s);
+    if (!g.ta && !g.tb) small_gemm_kernel<T, TM, TN, RM, RN, false, false><<<grid, NT, 0, s>>>(p);
+    else if (!g.ta) small_gemm_kernel<T, TM, TN, RM, RN, false, true><<<grid, NT, 0, s>>>(p);
+    else if (!g.tb) small_gemm_kernel<T, TM, TN, RM, RN, true, false><<<grid, NT, 0, s>>>(p);
+    else small_gemm_kernel<T, TM, TN, RM, RN, true, true><<<grid, NT, 0, s>>>(p);
+}
+
+template <typename T>
+cudaError_t native_gemm_small(const Gemm& g, const NativePlan& plan, T* workspace, cudaStream_t s, std::string* err) {
+    if (plan.splits > 1 && workspace == nullptr) {
+        if (err) *err = "split-k needs a workspace";
+        return cudaErrorInvalidValue;
+    }
+    SmallParams<T> p;
+    p.A = static_cast<const T*>(g.A); p.B = static_cast<const T*>(g.B); p.C = static_cast<T*>(g.C);
+    p.lda = g.lda; p.ldb = g.ldb; p.ldc = g.ldc;
+    p.m = g.m; p.n = g.n; p.k = g.k;
+    p.k_per_split = (g.k + plan.splits - 1) / plan.splits;
+    const int splits = int((g.k + p.k_per_split - 1) / p.k_per_split);
+    p.ws = splits > 1 ? workspace : nullptr;
+    p.tiles_n = (g.n + plan.tile - 1) / plan.tile;
+    p.alpha = T(g.alpha); p.beta = T(g.beta);
+    const dim3 grid(unsigned(((g.m + plan.tile - 1) / plan.tile) * p.tiles_n), 1, unsigned(splits));
+    switch (plan.tile) {
+        case 8: launch_small<T, 8, 8, 1, 1>(g, p, grid, s); break;
+        case 16: launch_small<T, 16, 16, 1, 1>(g, p, grid, s); break;
+        default:
+            if constexpr (sizeof(T) == 4) launch_small<T, 32, 32, 2, 2>(g, p, grid, s);
+            else return cudaErrorInvalidValue;
+            break;
+    }
+    count_launches(1);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess || splits == 1) return e;
+    return launch_splitk_reduce<T>(g, workspace, splits, s);
 }
 
 template <typename T>
@@ -421,12 +583,7 @@ cudaError_t native_gemm_tiled(const Gemm& g, int splits, T* workspace, const Lau
     else if (g.ta && !g.tb) e = launch_variant<T, true, false, BN_>(ta, tb, p, grid, s);
     else e = launch_variant<T, true, true, BN_>(ta, tb, p, grid, s);
     if (e != cudaSuccess || splits == 1) return e;
-    const int64_t total = g.m * g.n;
-    const int blocks = int(std::min<int64_t>((total + 255) / 256, 152 * 16));
-    splitk_reduce_kernel<T><<<blocks, 256, 0, s>>>(workspace, splits, g.m, g.n, T(g.alpha), T(g.beta),
-                                                   static_cast<T*>(g.C), g.ldc);
-    count_launches(1);
-    return cudaGetLastError();
+    return launch_splitk_reduce<T>(g, workspace, splits, s);
 }
 
 }  // namespace
@@ -444,9 +601,60 @@ int native_choose_splits(int64_t m, int64_t n, int64_t k, int elem_bytes, int nu
     return int(std::max<int64_t>(splits, 1));
 }
 
+// Tile and split count of a product: the smaller of the clocks that each form takes, from the
+// multiply-adds of the busiest SM and the pipe's rate (FP64: 2 a clock and SM in every tile; float:
+// what the shared loads of each tile let through).  See the figures at small_gemm_kernel and in the
+// constants below; a second kernel for the split sums costs about kReduceClk.
+NativePlan native_plan(int64_t m, int64_t n, int64_t k, int elem_bytes, int num_sms, bool tma_only) {
+    NativePlan best;
+    best.splits = native_choose_splits(m, n, k, elem_bytes, num_sms);
+    if (tma_only || m <= 0 || n <= 0 || k <= 0) return best;
+    constexpr double kReduceClk = 6000.0;
+    auto waves = [&](double tiles) { return std::ceil(tiles / double(num_sms)); };
+    auto ceil_div = [](int64_t a, int64_t b) { return double((a + b - 1) / b); };
+    const int64_t bn = native_tile_n(m, n), bm = 16384 / bn;
+    // the 16384-output tile: one CTA per SM, its pipeline fill and epilogue about 4000 clocks
+    double best_clk = waves(ceil_div(m, bm) * ceil_div(n, bn) * best.splits) *
+                          (16384.0 * ceil_div(k, best.splits) / (elem_bytes == 8 ? 2.0 : 75.0) + 4000.0) +
+                      (best.splits > 1 ? kReduceClk : 0.0);
+    struct Small {
+        int tile;
+        double rate, latency;  // multiply-adds a clock and SM; clocks of one k step of a lone CTA
+    };
+    // FP64: 16 x 16 tiles reach 1.24 TFLOP/s at 1024^3 and 2048^3, 0.99 of the FP64 peak, as the large
+    // tiles do on a full last wave; 8 x 8 tiles (two warps a CTA) leave a little more of the pipe idle,
+    // and a lone one waits 48 clocks a step for its own chain.  Measured, large tiles -> this rule:
+    // 96^3 393 -> 10.5 us (about 7 of them the launches), 256^3 1030 -> 36, 512^3 1032 -> 233,
+    // 1024^3 2055 -> 1733, 2048^3 16362 -> 13776.
+    // Float: 128^3 25.8 -> 7.6 us, 256^3 38.5 -> 12.2, 512^3 64.7 -> 27.6, 768^3 94.3 -> 70.5; from
+    // 1024^3 on the large tiles stay ahead (28.7 TFLOP/s there, 36.6 at 2048^3).
+    const Small f64[] = {{16, 1.97, 128.0}, {8, 1.7, 48.0}};
+    const Small f32[] = {{32, 40.0, 32.0}, {16, 18.0, 24.0}, {8, 10.0, 24.0}};
+    const Small* forms = elem_bytes == 8 ? f64 : f32;
+    for (int f = 0; f < (elem_bytes == 8 ? 2 : 3); ++f) {
+        const Small& t = forms[f];
+        const double tiles = ceil_div(m, t.tile) * ceil_div(n, t.tile);
+        if (tiles > 2147483647.0) continue;  // gridDim.x
+        const int max_splits = int(std::min<double>(double(num_sms) / tiles, double(k / 128)));
+        for (int splits : {1, max_splits}) {
+            if (splits < 1) continue;
+            const double per_sm = waves(tiles * splits);
+            const double step = std::max(per_sm * t.tile * t.tile / t.rate, t.latency);
+            const double clk = ceil_div(k, splits) * step + 3000.0 + (splits > 1 ? kReduceClk : 0.0);
+            if (clk < best_clk) {
+                best_clk = clk;
+                best.tile = t.tile;
+                best.splits = splits;
+            }
+        }
+    }
+    return best;
+}
+
 template <typename T>
-cudaError_t native_gemm(const Gemm& g, int splits, T* workspace, const LaunchCtl& ctl, cudaStream_t s,
+cudaError_t native_gemm(const Gemm& g, const NativePlan& plan, T* workspace, const LaunchCtl& ctl, cudaStream_t s,
                         std::string* err) {
+    const int splits = plan.splits;
     if (g.m <= 0 || g.n <= 0) return cudaSuccess;
     if (g.k == 0) {
         const int64_t total = g.m * g.n;
@@ -455,6 +663,7 @@ cudaError_t native_gemm(const Gemm& g, int splits, T* workspace, const LaunchCtl
         count_launches(1);
         return cudaGetLastError();
     }
+    if (plan.tile != 0) return native_gemm_small<T>(g, plan, workspace, s, err);
     switch (native_tile_n(g.m, g.n)) {
         case 64: return native_gemm_tiled<T, 64>(g, splits, workspace, ctl, s, err);
         case 256: return native_gemm_tiled<T, 256>(g, splits, workspace, ctl, s, err);
@@ -462,8 +671,10 @@ cudaError_t native_gemm(const Gemm& g, int splits, T* workspace, const LaunchCtl
     }
 }
 
-template cudaError_t native_gemm<double>(const Gemm&, int, double*, const LaunchCtl&, cudaStream_t, std::string*);
-template cudaError_t native_gemm<float>(const Gemm&, int, float*, const LaunchCtl&, cudaStream_t, std::string*);
+template cudaError_t native_gemm<double>(const Gemm&, const NativePlan&, double*, const LaunchCtl&, cudaStream_t,
+                                         std::string*);
+template cudaError_t native_gemm<float>(const Gemm&, const NativePlan&, float*, const LaunchCtl&, cudaStream_t,
+                                        std::string*);
 
 }  // namespace gb
 
@@ -602,8 +813,14 @@ extern "C" int gb300_dgemm_native_noalloc(int order, int transA, int transB, int
         cudaGetLastError();
         return fail(GB300_ERR_NO_DEVICE, "cannot query the SM count");
     }
-    int splits = g.k > 0 ? native_choose_splits(g.m, g.n, g.k, 8, sms) : 1;
-    const size_t need = splits > 1 ? size_t(splits) * size_t(g.m) * size_t(g.n) * sizeof(double) : 0;
+    // the scratch rule is that of the 16384-output tiles, whatever tile the product then runs in; a
+    // plan whose own partials do not fit runs in those tiles
+    NativePlan plan;
+    plan.splits = g.k > 0 ? native_choose_splits(g.m, g.n, g.k, 8, sms) : 1;
+    auto partials = [&](int splits) {
+        return splits > 1 ? size_t(splits) * size_t(g.m) * size_t(g.n) * sizeof(double) : size_t(0);
+    };
+    const size_t need = partials(plan.splits);
     if (need > kNoAllocScratchBytes - kNoAllocStatusBytes)
         return fail(GB300_ERR_INVALID_ARG,
                     "the product needs " + std::to_string(need) + " bytes of split-k scratch; the allocation-free "
@@ -627,6 +844,10 @@ extern "C" int gb300_dgemm_native_noalloc(int order, int transA, int transB, int
             ctl.wait_limit_ns = r.inject_limit_ns;
         }
     }
+    if (g.k > 0) {
+        const NativePlan fit = native_plan(g.m, g.n, g.k, 8, sms, ctl.inject_stall != 0);
+        if (partials(fit.splits) <= kNoAllocScratchBytes - kNoAllocStatusBytes) plan = fit;
+    }
     // from here on work may be queued: every return waits for the stream first, so that no kernel
     // of this call still touches the shared array once the lock is released
     auto fail_after_queue = [&](int st_, const std::string& msg) {
@@ -636,7 +857,7 @@ extern "C" int gb300_dgemm_native_noalloc(int order, int transA, int transB, int
     };
     cudaError_t e = cudaMemsetAsync(status, 0, sizeof(int), s);
     if (e != cudaSuccess) return fail_after_queue(GB300_ERR_CUDA, std::string("status reset: ") + cudaGetErrorString(e));
-    e = native_gemm<double>(g, splits, splits > 1 ? ws : nullptr, ctl, s, &err);
+    e = native_gemm<double>(g, plan, plan.splits > 1 ? ws : nullptr, ctl, s, &err);
     if (e != cudaSuccess) return fail_after_queue(GB300_ERR_CUDA, err.empty() ? cudaGetErrorString(e) : err);
     int h = 0;
     e = cudaMemcpyAsync(&h, status, sizeof(int), cudaMemcpyDeviceToHost, s);

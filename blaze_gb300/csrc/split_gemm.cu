@@ -1642,13 +1642,13 @@ namespace {
 int native_product(const Gemm& g, const LaunchCtl& ctl, cudaStream_t st, Workspace& ws, SplitResult* out,
                    std::string* err) {
     Runtime& r = runtime();
-    const int splits = g.k > 0 ? native_choose_splits(g.m, g.n, g.k, 8, r.num_sms) : 1;
+    const NativePlan plan = native_plan(g.m, g.n, g.k, 8, r.num_sms, ctl.inject_stall != 0);
     double* w = nullptr;
-    if (splits > 1) {
-        w = static_cast<double*>(ws.get(kSlotWork, size_t(splits) * size_t(g.m) * size_t(g.n) * 8, err));
+    if (plan.splits > 1) {
+        w = static_cast<double*>(ws.get(kSlotWork, size_t(plan.splits) * size_t(g.m) * size_t(g.n) * 8, err));
         if (!w) return GB300_ERR_NO_MEMORY;
     }
-    cudaError_t e = native_gemm<double>(g, splits, w, ctl, st, err);
+    cudaError_t e = native_gemm<double>(g, plan, w, ctl, st, err);
     if (e != cudaSuccess) {
         if (err && err->empty()) *err = cudaGetErrorString(e);
         return GB300_ERR_CUDA;
@@ -1750,13 +1750,28 @@ void stored_a(const Gemm& g, int64_t* rows, int64_t* cols) { *rows = g.ta ? g.k 
 void stored_b(const Gemm& g, int64_t* rows, int64_t* cols) { *rows = g.tb ? g.n : g.k; *cols = g.tb ? g.k : g.n; }
 bool tma_ready(const void* p, int64_t ld) { return reinterpret_cast<uintptr_t>(p) % 16 == 0 && (ld * 8) % 16 == 0; }
 
-// Copy operands whose base or pitch TMA cannot address (16-byte alignment) into the workspace.
-int realign_operands(Gemm& g, Workspace& ws, cudaStream_t st, std::string* err) {
+// Whether a product runs on the native kernel, and whether there in the tiles that read their
+// operands through TMA.
+bool runs_native(const Gemm& g, const SplitRequest& req) {
+    return g.k == 0 || req.method == GB300_METHOD_NATIVE || (req.method == GB300_METHOD_AUTO && auto_uses_native(g));
+}
+bool runs_tma_tiles(const Gemm& g, const SplitRequest& req, bool stall) {
+    return runs_native(g, req) && native_plan(g.m, g.n, g.k, 8, runtime().num_sms, stall).tile == 0;
+}
+
+// An operand read in place: by TMA when it is 16-byte aligned in base and pitch, by every other
+// kernel (single-element loads) when its base is aligned for a double.
+bool read_in_place(const void* p, int64_t ld, bool tma) {
+    return tma ? tma_ready(p, ld) : reinterpret_cast<uintptr_t>(p) % 8 == 0;
+}
+
+// Copy operands that cannot be read in place into the workspace.
+int realign_operands(Gemm& g, bool tma, Workspace& ws, cudaStream_t st, std::string* err) {
     if (g.k == 0) return GB300_OK;
     for (int which = 0; which < 2; ++which) {
         const void*& p = which == 0 ? g.A : g.B;
         int64_t& ld = which == 0 ? g.lda : g.ldb;
-        if (tma_ready(p, ld)) continue;
+        if (read_in_place(p, ld, tma)) continue;
         int64_t rows, cols;
         if (which == 0) stored_a(g, &rows, &cols);
         else stored_b(g, &rows, &cols);
@@ -1782,12 +1797,13 @@ void device_product_slot_needs(const Gemm& g, const SplitRequest& req, size_t ne
     for (int i = 0; i < kSlotCount; ++i) need[i] = 0;
     auto rounded = [](size_t b) { return b == 0 ? size_t(0) : (b + (size_t(2) << 20) - 1) & ~((size_t(2) << 20) - 1); };
     if (g.k > 0) {
+        const bool tma = runs_tma_tiles(g, req, false);
         int64_t rr, cc;
-        if (!tma_ready(g.A, g.lda)) { stored_a(g, &rr, &cc); need[kSlotA] = rounded(size_t(rr) * size_t((cc + 1) / 2 * 2) * 8); }
-        if (!tma_ready(g.B, g.ldb)) { stored_b(g, &rr, &cc); need[kSlotB] = rounded(size_t(rr) * size_t((cc + 1) / 2 * 2) * 8); }
+        if (!read_in_place(g.A, g.lda, tma)) { stored_a(g, &rr, &cc); need[kSlotA] = rounded(size_t(rr) * size_t((cc + 1) / 2 * 2) * 8); }
+        if (!read_in_place(g.B, g.ldb, tma)) { stored_b(g, &rr, &cc); need[kSlotB] = rounded(size_t(rr) * size_t((cc + 1) / 2 * 2) * 8); }
     }
-    if (g.k == 0 || req.method == GB300_METHOD_NATIVE || (req.method == GB300_METHOD_AUTO && auto_uses_native(g))) {
-        const int splits = g.k > 0 ? native_choose_splits(g.m, g.n, g.k, 8, r.num_sms) : 1;
+    if (runs_native(g, req)) {
+        const int splits = native_plan(g.m, g.n, g.k, 8, r.num_sms, false).splits;
         if (splits > 1) need[kSlotWork] = rounded(size_t(splits) * size_t(g.m) * size_t(g.n) * 8);
         return;
     }
@@ -1890,11 +1906,10 @@ int device_product(const Gemm& g_in, const SplitRequest& req, const LaunchCtl& c
     Runtime& r = runtime();
     Gemm g = g_in;
     {
-        const int rst = realign_operands(g, ws, st, err);
+        const int rst = realign_operands(g, runs_tma_tiles(g, req, ctl.inject_stall != 0), ws, st, err);
         if (rst != GB300_OK) return rst;
     }
-    if (g.k == 0 || req.method == GB300_METHOD_NATIVE || (req.method == GB300_METHOD_AUTO && auto_uses_native(g)))
-        return native_product(g, ctl, st, ws, out, err);
+    if (runs_native(g, req)) return native_product(g, ctl, st, ws, out, err);
 
     const SplitGeometry G = split_geometry(g, req, r.num_sms);
     const int mode = G.mode;
