@@ -185,7 +185,7 @@ int gemm_entry(int order, int transA, int transB, int64_t m, int64_t n, int64_t 
         ctl.inject_stall = 1;
         ctl.wait_limit_ns = r.inject_limit_ns;
     }
-    cudaMemsetAsync(r.d_status, 0, sizeof(int), s);
+    status_begin(s, sync);
     int used = method;
     const void* info_dev = nullptr;
     cudaError_t e = cudaSuccess;
@@ -289,8 +289,7 @@ int gemm_entry(int order, int transA, int transB, int64_t m, int64_t n, int64_t 
     if (sync) {
         e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) return fail(GB300_ERR_CUDA, std::string("kernel failed: ") + cudaGetErrorString(e));
-        int status = 0;
-        cudaMemcpy(&status, r.d_status, sizeof(int), cudaMemcpyDeviceToHost);
+        const int status = status_end();
         if (status != kDevOk)
             return fail(GB300_ERR_DEVICE_TIMEOUT, std::string("a device-side wait ran out (code ") +
                                                       std::to_string(status) + ", method " + method_name(used) +

@@ -94,8 +94,7 @@ int finish(cudaStream_t st, std::string* err) {
         if (err) *err = std::string("kernel failed: ") + cudaGetErrorString(e);
         return GB300_ERR_CUDA;
     }
-    int status = 0;
-    cudaMemcpy(&status, runtime().d_status, sizeof(int), cudaMemcpyDeviceToHost);
+    const int status = status_end();
     if (status != kDevOk) {
         if (err) *err = "a device-side wait ran out (code " + std::to_string(status) + "); the result is incomplete";
         return GB300_ERR_DEVICE_TIMEOUT;
@@ -147,7 +146,7 @@ LaunchCtl fresh_ctl(cudaStream_t st) {
     Runtime& r = runtime();
     LaunchCtl ctl;
     ctl.status = r.d_status;
-    cudaMemsetAsync(r.d_status, 0, sizeof(int), st);
+    status_begin(st, true);
     return ctl;
 }
 

@@ -66,6 +66,18 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
     return ok != 0;
 }
 
+// Record `code` in the status word unless an error is there already.  The 64-bit word 8 bytes behind
+// the status word, when not zero, is the device address of a page-locked host word that takes the
+// code too, so that a host that waited for the launch sees a failure without a copy.
+__device__ __forceinline__ void record_status(int* status, int code) {
+    if (atomicCAS(status, 0, code) != 0) return;
+    volatile int* host = *reinterpret_cast<int* const*>(status + 2);
+    if (host != nullptr) {
+        *host = code;
+        __threadfence_system();
+    }
+}
+
 // Bounded wait for phase `parity` of barrier `bar`.  Returns false (after recording `code` in
 // *status unless another thread already recorded an error) when the limit runs out or when
 // another thread of the launch has already failed.
@@ -78,7 +90,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* st
         if ((it & 63u) == 0) {
             if (*reinterpret_cast<volatile int*>(status) != 0) return false;
             if (globaltimer_ns() - t0 > limit_ns) {
-                atomicCAS(status, 0, code);
+                record_status(status, code);
                 return false;
             }
         }

@@ -131,7 +131,15 @@ int ensure_init(std::string* err) {
         return GB300_ERR_NO_DEVICE;
     }
     if ((e = cudaStreamCreateWithFlags(&r.stream, cudaStreamNonBlocking)) != cudaSuccess ||
-        (e = cudaMalloc(&r.d_status, 64)) != cudaSuccess || (e = cudaMemset(r.d_status, 0, 64)) != cudaSuccess) {
+        (e = cudaMalloc(&r.d_status, 64)) != cudaSuccess || (e = cudaMemset(r.d_status, 0, 64)) != cudaSuccess ||
+        (e = cudaHostAlloc(&r.h_status, 64, cudaHostAllocMapped)) != cudaSuccess) {
+        if (err) *err = std::string("device set-up: ") + cudaGetErrorString(e);
+        return GB300_ERR_CUDA;
+    }
+    std::memset(r.h_status, 0, 64);
+    void* h_dev = nullptr;
+    if ((e = cudaHostGetDevicePointer(&h_dev, r.h_status, 0)) != cudaSuccess ||
+        (e = cudaMemcpy(r.d_status + 2, &h_dev, sizeof(h_dev), cudaMemcpyHostToDevice)) != cudaSuccess) {
         if (err) *err = std::string("device set-up: ") + cudaGetErrorString(e);
         return GB300_ERR_CUDA;
     }
@@ -147,6 +155,25 @@ int ensure_init(std::string* err) {
     r.aux.d_status = r.d_status;
     r.inited = true;
     return GB300_OK;
+}
+
+void status_begin(cudaStream_t s, bool synchronous) {
+    Runtime& r = runtime();
+    if (!synchronous) r.async_seen = true;
+    if (r.async_seen || !r.status_clean) {
+        *static_cast<volatile int*>(r.h_status) = 0;
+        cudaMemsetAsync(r.d_status, 0, sizeof(int), s);
+    }
+    r.status_clean = false;
+}
+
+int status_end() {
+    Runtime& r = runtime();
+    int status = 0;
+    if (r.async_seen) cudaMemcpy(&status, r.d_status, sizeof(int), cudaMemcpyDeviceToHost);
+    else status = *static_cast<volatile int*>(r.h_status);
+    r.status_clean = status == 0;
+    return status;
 }
 
 std::atomic<int64_t> g_pool_bytes{0};

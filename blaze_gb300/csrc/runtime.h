@@ -55,6 +55,9 @@ struct Runtime {
     int num_sms = 0;
     cudaStream_t stream = nullptr;
     int* d_status = nullptr;       // device status word of the default context
+    int* h_status = nullptr;       // page-locked word that a failing wait sets too (record_status)
+    bool status_clean = true;      // both words are known to be zero
+    bool async_seen = false;       // an asynchronous call was made: work may be running between calls
     Workspace ws;                  // default context (stream = `stream`)
     Workspace aux;                 // operands and intermediates of ?gemv, complex ?gemm, ?trmm
                                    // (their real products use `ws`)
@@ -84,6 +87,16 @@ int ensure_init(std::string* err);
 // Device buffer of at least `bytes` in slot `s` of the default context (caller holds
 // runtime().mu).  nullptr on failure.
 void* pool_get(int s, size_t bytes, std::string* err);
+
+// The default context's status word around a call on stream `s` (caller holds runtime().mu):
+// status_begin clears it for the call, status_end returns what the call's kernels left in it, once
+// the stream has been waited for.  While every call was synchronous, a call that succeeded leaves
+// both words zero and the host reads its own copy, so neither costs the stream anything (clearing
+// and copying back took about 15 us of every call, more than a small product's kernel).  After the
+// first asynchronous call the word is cleared on the stream and copied back in each call: a kernel
+// of an earlier call may still write it.
+void status_begin(cudaStream_t s, bool synchronous);
+int status_end();
 
 // Thread-local last error.
 void set_error(int status, const std::string& msg);
