@@ -67,8 +67,7 @@ cudaError_t launch_dot(int64_t n, const T* x, int64_t incx, const T* y, int64_t 
 
 // ---- trsm.cu -----------------------------------------------------------------------------------
 // Rows of the diagonal blocks that a triangular solve inverts (its recursion's leaves) for elements
-// of `elem` bytes: 512 for every element type; the inverse kernel's shared memory, (9 nb + 64)
-// elements, stays below 75 KB even for complex double.  Larger leaves mean fewer, larger products
+// of `elem` bytes: 512 for every element type.  Larger leaves mean fewer, larger products
 // for the same work: 512 rows instead of 256 made ztrsm 4096 5 % faster and halved its error.
 constexpr int solve_block(size_t /*elem*/) { return 512; }
 
@@ -76,7 +75,7 @@ constexpr int solve_block(size_t /*elem*/) { return 512; }
 template <typename T, bool CPLX>
 cudaError_t launch_scale(int64_t rows, int64_t cols, const T* alpha, T* X, int64_t ld, cudaStream_t st);
 
-// Dense inverses of the diagonal blocks (nb x nb, nb a multiple of 32 up to solve_block(); the last
+// Dense inverses of the diagonal blocks (nb x nb, nb a power of two from 32 to solve_block(); the last
 // block may be smaller) of the triangular op(SA): SA ka x ka in row-major storage, op = transpose
 // (trans) and conjugation (conj), `upper` when op(SA) is upper triangular, `unit` for a unit
 // diagonal (not read).  Block b's inverse goes to inv + b nb nb (pitch nb).

@@ -35,92 +35,151 @@ __global__ void scale_kernel(int64_t rows, int64_t cols, V alpha, V* __restrict_
 
 // Inverse of every diagonal block of the triangular matrix op(SA).  SA is ka x ka in row-major
 // storage with pitch lda, and op transposes it (trans) and conjugates it (conj).  Block b covers
-// rows and columns [b nb, min(ka, (b + 1) nb)).  Its inverse is written densely to inv + b nb nb
+// rows and columns [b nb, min(ka, (b + 1) nb)).  Its inverse Y is written densely to inv + b nb nb
 // with pitch nb, zeros outside the triangle included.
 //
 // Each block is brought to lower-triangular form L'.  L' is the block itself when op(SA) is lower;
-// when it is upper (`upper`), L' is the block with its rows and columns reversed.  L' is inverted
-// by forward substitution, Y[r][c] = (delta_rc - sum_{j<r} L'[r][j] Y[j][c]) / L'[r][r].
-//
-// The work is FP64 FMAs and column c needs about (nb - c)^2 / 2 of them, so the first columns set
-// the kernel's time: on GB300 one SM retires about two FP64 FMAs per clock.  A block of the grid
-// therefore takes only kInvCols columns (blockIdx.x picks the group, blockIdx.y the diagonal block)
-// and spreads each column's sums over kInvChains chains: lane = column + kInvCols * slice, and warp
-// w with slice s takes j = r0 + kInvSlices w + s, then every kInvChains-th.  The shuffles and then
-// warp 0 add the chains in a fixed order.  Those adds cost FP64 instructions every row: with 8
-// warps (32 chains) they were 40 % of the kernel's 18.9 M FP64 instructions at 8192 rows (1.71 ms,
-// FP64 pipe 80 % active).  4 warps (16 chains) measured 1.44-1.53 ms and 2 warps 1.79-1.84 ms;
-// 16-column groups measured 1.77-1.87 ms (the heaviest group then does twice the FMAs on one SM).  Warp 0 scales by the diagonal's reciprocal (computed for all rows up front, so the
-// serial step per row is a multiply) and publishes Y[r] in shared memory before the next row.
-// Y[j][c] = 0 for j < c comes out of the recurrence itself, so the loops are the same for every
-// column of a group, which starts at its first column r0.  A unit diagonal is not read.
-constexpr int kInvWarps = 4;
-constexpr int kInvCols = 8;                      // columns per grid block
-constexpr int kInvSlices = 32 / kInvCols;        // lanes per column in a warp
-constexpr int kInvChains = kInvWarps * kInvSlices;  // FMA chains per column
-
+// when it is upper (`upper`), L' is the block with its rows and columns reversed.  The inverse is
+// built from the diagonal up: tri_base_kernel inverts the 16 x 16 blocks on the diagonal, and each
+// level joins two neighbours of s rows into one of 2 s by two products,
+//     T = L21 Y11,   Y21 = -Y22 T                              (s = 16, 32, ... nb / 2),
+// T being kept where the zeros above the diagonal go in the end (tri_zero_kernel).  The products skip
+// the zeros of Y11 and Y22, so the levels together take the nb^3 / 6 multiply-adds of a substitution,
+// and what bounds them is the FP64 pipe.  Substituting column by column was bound by its chain of
+// rows instead: 512 steps of a block-wide sum and two barriers, 1120 us for the four 512-row blocks of
+// a 2048-row triangle whatever the rest of the chip did; base and levels take 264 us there, against 143 us for their multiply-adds at the full FP64 rate.
 template <typename V>
-__global__ void __launch_bounds__(32 * kInvWarps) tri_inverse_kernel(int64_t ka, int nb, const V* __restrict__ SA,
-                                                                     int64_t lda, int trans, int conj, int upper,
-                                                                     int unit, V* __restrict__ inv) {
-    extern __shared__ __align__(16) unsigned char tri_smem[];
-    V* ycol = reinterpret_cast<V*>(tri_smem);              // [nb][kInvCols]
-    V* rdiag = ycol + int64_t(nb) * kInvCols;                // [nb]
-    V* part = rdiag + nb;                                    // [kInvWarps][kInvCols]
-    using A = Ar<V>;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int cl = lane % kInvCols, slice = lane / kInvCols;
-    const int64_t b0 = int64_t(blockIdx.y) * nb;
-    const int nbk = int(min(int64_t(nb), ka - b0));
-    const int r0 = int(blockIdx.x) * kInvCols;
-    if (r0 >= nbk) return;
-    const int c = r0 + cl;
-    // L'[r][j] sits at P + r * sr + j * sj
-    int64_t sr = trans ? 1 : lda, sj = trans ? lda : 1;
-    const V* P = SA + b0 * lda + b0;
-    if (upper) {
-        P += int64_t(nbk - 1) * (lda + 1);
-        sr = -sr;
-        sj = -sj;
-    }
-    V* out = inv + int64_t(blockIdx.y) * nb * nb;
-    // Y[r][c] lands at out[r][c], or at out[nbk-1-r][nbk-1-c] for a reversed (upper) block
-    const int64_t o0 = upper ? int64_t(nbk - 1) * (nb + 1) : 0, orow = upper ? -int64_t(nb) : int64_t(nb),
-                  ocol = upper ? -1 : 1;
-    for (int r = r0 + threadIdx.x; r < nbk; r += blockDim.x) {
-        const V d = unit ? A::one() : (conj ? A::conj(P[r * (sr + sj)]) : P[r * (sr + sj)]);
-        rdiag[r - r0] = A::div(A::one(), d);
-    }
-    // rows above the group: zero (the inverse of a lower triangle is lower)
-    for (int i = threadIdx.x; i < r0 * kInvCols; i += blockDim.x) {
-        const int r = i / kInvCols, cc = r0 + i % kInvCols;
-        if (cc < nbk) out[o0 + r * orow + cc * ocol] = A::zero();
-    }
-    __syncthreads();
-    const int chain = warp * kInvSlices + slice;
-    const int64_t lstep = kInvChains * sj;
-    for (int r = r0; r < nbk; ++r) {
-        V s = A::zero();
-        int j = r0 + chain;
-        const V* lp = P + r * sr + j * sj;
-        const V* yp = ycol + (j - r0) * kInvCols + cl;
-        for (; j < r; j += kInvChains, lp += lstep, yp += kInvChains * kInvCols)
-            s = A::fmadd(conj ? A::conj(*lp) : *lp, *yp, s);
-        // the slices of this warp (lanes cl, cl + kInvCols, ...), then the warps
-#pragma unroll
-        for (int o = kInvCols; o < 32; o *= 2) s = A::add(s, A::shfl_xor(s, o));
-        if (slice == 0) part[warp * kInvCols + cl] = s;
-        __syncthreads();
-        if (warp == 0 && slice == 0) {
-            V sum = part[cl];
-#pragma unroll
-            for (int w = 1; w < kInvWarps; ++w) sum = A::add(sum, part[w * kInvCols + cl]);
-            const V acc = A::mul(A::fnmadd(A::one(), sum, (r == c) ? A::one() : A::zero()), rdiag[r - r0]);
-            ycol[(r - r0) * kInvCols + cl] = acc;
-            if (c < nbk) out[o0 + r * orow + c * ocol] = acc;
+struct TriArgs {
+    const V* SA;
+    V* inv;
+    int64_t ka, lda;
+    int nb, trans, conj, upper, unit;
+};
+
+// One block in lower-triangular form: L'[r][j] at P + r sr + j sj, Y[r][c] at out + r orow + c ocol.
+template <typename V>
+struct TriBlock {
+    const V* P;
+    V* out;
+    int64_t sr, sj, orow, ocol;
+    int rows;
+    __device__ __forceinline__ TriBlock(const TriArgs<V>& a, int64_t b) {
+        const int64_t b0 = b * a.nb;
+        rows = int(min(int64_t(a.nb), a.ka - b0));
+        sr = a.trans ? 1 : a.lda;
+        sj = a.trans ? a.lda : 1;
+        orow = a.nb;
+        ocol = 1;
+        P = a.SA + b0 * a.lda + b0;
+        out = a.inv + b * a.nb * a.nb;
+        if (a.upper) {
+            P += int64_t(rows - 1) * (a.lda + 1);
+            out += int64_t(rows - 1) * (a.nb + 1);
+            sr = -sr; sj = -sj; orow = -orow; ocol = -ocol;
         }
-        __syncthreads();
     }
+};
+
+constexpr int kTriBase = 16;
+
+// The inverses of two 16 x 16 diagonal blocks per warp, one in each half: lane c of a half carries
+// column c of Y in registers and subtracts each finished row from all the rows below it, so that the
+// multiply-adds of a row are independent of one another (a sum per row would wait for its own chain).
+// A lone warp has a quarter of its SM's FP64 pipe, 64 clocks per multiply-add: 32 x 32 blocks, four
+// times the instructions, took 36 us at 2048 rows, these 16 with one more level of products.
+template <typename V>
+__global__ void __launch_bounds__(32) tri_base_kernel(const TriArgs<V> a) {
+    using A = Ar<V>;
+    __shared__ V Ls[2][kTriBase][kTriBase + 1];
+    const int per = a.nb / kTriBase, c = threadIdx.x % kTriBase, h = threadIdx.x / kTriBase;
+    V (&L)[kTriBase][kTriBase + 1] = Ls[h];
+    const int g = int(blockIdx.x) * 2 + h;
+    const TriBlock<V> t(a, g / per);
+    const int r0 = (g % per) * kTriBase;
+    const int n = min(kTriBase, t.rows - r0);  // below 1 past the end of the last block
+    const V* P = t.P + r0 * (t.sr + t.sj);
+    const bool by_row = t.sj == 1 || t.sj == -1;  // lanes along the contiguous index
+#pragma unroll
+    for (int i = 0; i < kTriBase; ++i) {
+        const int r = by_row ? i : c, j = by_row ? c : i;
+        if (j < r) L[r][j] = r < n ? (a.conj ? A::conj(P[r * t.sr + j * t.sj]) : P[r * t.sr + j * t.sj]) : A::zero();
+    }
+    V d = A::one();
+    if (c < n && !a.unit) d = a.conj ? A::conj(P[c * (t.sr + t.sj)]) : P[c * (t.sr + t.sj)];
+    L[c][c] = A::div(A::one(), d);
+    __syncwarp();
+    V y[kTriBase];
+#pragma unroll
+    for (int r = 0; r < kTriBase; ++r) y[r] = r == c ? A::one() : A::zero();
+#pragma unroll
+    for (int r = 0; r < kTriBase; ++r) {
+        y[r] = r >= c ? A::mul(y[r], L[r][r]) : A::zero();  // a zero diagonal stays in its own columns
+#pragma unroll
+        for (int i = r + 1; i < kTriBase; ++i) y[i] = A::fnmadd(L[i][r], y[r], y[i]);
+    }
+    V* out = t.out + r0 * (t.orow + t.ocol) + c * t.ocol;
+#pragma unroll
+    for (int r = 0; r < kTriBase; ++r)
+        if (r < n && r >= c) out[r * t.orow] = y[r];
+}
+
+// One 16 x 16 tile of T = L21 Y11 (SECOND == false; k from the tile's first column on) or of
+// Y21 = -Y22 T (SECOND == true; k up to the tile's last row) for the pair of s-row halves that
+// blockIdx.y picks.  A thread holds one output: on the FP64 pipe a warp's multiply-add takes 16
+// clocks, far more than its two shared loads, and the next 16 k steps are in registers meanwhile.
+template <typename V, bool SECOND>
+__global__ void __launch_bounds__(256) tri_join_kernel(const TriArgs<V> a, int s) {
+    using A = Ar<V>;
+    __shared__ V As[16][17], Bs[16][17];
+    const int pairs = a.nb / (2 * s);
+    const TriBlock<V> t(a, blockIdx.y / pairs);
+    const int q0 = int(blockIdx.y % pairs) * 2 * s;   // first row of the upper half
+    const int n2 = min(s, t.rows - (q0 + s));         // rows of the lower half
+    const int tiles = s / 16;
+    // longest k ranges first
+    const int ti = SECOND ? tiles - 1 - int(blockIdx.x) / tiles : int(blockIdx.x) % tiles;
+    const int tj = SECOND ? int(blockIdx.x) % tiles : int(blockIdx.x) / tiles;
+    const int i0 = ti * 16, j0 = tj * 16;
+    if (i0 >= n2) return;
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    // left operand (i, k) and right operand (k, j), T in place of the block above the diagonal
+    V* const T = t.out + q0 * t.orow + (q0 + s) * t.ocol;
+    const V* left = SECOND ? t.out + (q0 + s) * (t.orow + t.ocol) : t.P + (q0 + s) * t.sr + q0 * t.sj;
+    const int64_t li = SECOND ? t.orow : t.sr, lk = SECOND ? t.ocol : t.sj;
+    const V* right = SECOND ? T : t.out + q0 * (t.orow + t.ocol);
+    const int k0 = SECOND ? 0 : j0, k1 = SECOND ? min(n2, i0 + 16) : s;
+    const bool by_row = lk == 1 || lk == -1;
+    const int ai = by_row ? ty : tx, ak = by_row ? tx : ty;
+    V va = A::zero(), vb = A::zero();
+    auto fetch = [&](int k) {
+        const bool oka = i0 + ai < n2 && k + ak < k1 && (!SECOND || k + ak <= i0 + ai);
+        va = oka ? left[(i0 + ai) * li + (k + ak) * lk] : A::zero();
+        if (!SECOND && a.conj) va = A::conj(va);
+        const bool okb = k + ty < k1 && (SECOND || k + ty >= j0 + tx);
+        vb = okb ? right[(k + ty) * t.orow + (j0 + tx) * t.ocol] : A::zero();
+    };
+    fetch(k0);
+    V acc = A::zero();
+    for (int k = k0; k < k1; k += 16) {
+        __syncthreads();
+        As[ai][ak] = va;
+        Bs[ty][tx] = vb;
+        __syncthreads();
+        if (k + 16 < k1) fetch(k + 16);
+#pragma unroll
+        for (int kk = 0; kk < 16; ++kk) acc = A::fmadd(As[ty][kk], Bs[kk][tx], acc);
+    }
+    if (i0 + ty >= n2) return;
+    if (SECOND) t.out[(q0 + s + i0 + ty) * t.orow + (q0 + j0 + tx) * t.ocol] = A::fnmadd(A::one(), acc, A::zero());
+    else T[(i0 + ty) * t.orow + (j0 + tx) * t.ocol] = acc;
+}
+
+// Zeros above the diagonal of every inverted block.
+template <typename V>
+__global__ void __launch_bounds__(256) tri_zero_kernel(const TriArgs<V> a) {
+    const TriBlock<V> t(a, blockIdx.y);
+    for (int r = blockIdx.x; r < t.rows; r += gridDim.x)
+        for (int c = r + 1 + threadIdx.x; c < t.rows; c += blockDim.x) t.out[r * t.orow + c * t.ocol] = Ar<V>::zero();
 }
 
 }  // namespace
@@ -141,19 +200,28 @@ template <typename T, bool CPLX>
 cudaError_t launch_tri_inverse(int64_t ka, int nb, const T* SA, int64_t lda, bool trans, bool conj, bool upper,
                                bool unit, T* inv, cudaStream_t st) {
     using V = typename std::conditional<CPLX, Cx<T>, T>::type;
-    // Y's columns, the diagonal's reciprocals and the partial sums
-    auto smem_for = [](int rows) { return (size_t(rows) * (kInvCols + 1) + kInvWarps * kInvCols) * sizeof(V); };
-    constexpr int nb_max = solve_block(sizeof(V));
-    static const cudaError_t attr = cudaFuncSetAttribute(tri_inverse_kernel<V>,
-                                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                         int(smem_for(nb_max)));
-    if (attr != cudaSuccess) return attr;
-    if (nb > nb_max || nb % 32 != 0) return cudaErrorInvalidValue;
-    const int64_t blocks = (ka + nb - 1) / nb;
-    tri_inverse_kernel<V><<<dim3(unsigned(nb / kInvCols), unsigned(blocks)), 32 * kInvWarps, smem_for(nb), st>>>(
-        ka, nb, reinterpret_cast<const V*>(SA), lda, trans ? 1 : 0, conj ? 1 : 0, upper ? 1 : 0, unit ? 1 : 0,
-        reinterpret_cast<V*>(inv));
-    count_launches(1);
+    if (nb > solve_block(sizeof(V)) || nb < 2 * kTriBase || (nb & (nb - 1)) != 0) return cudaErrorInvalidValue;
+    TriArgs<V> a;
+    a.SA = reinterpret_cast<const V*>(SA);
+    a.inv = reinterpret_cast<V*>(inv);
+    a.ka = ka;
+    a.lda = lda;
+    a.nb = nb;
+    a.trans = trans ? 1 : 0;
+    a.conj = conj ? 1 : 0;
+    a.upper = upper ? 1 : 0;
+    a.unit = unit ? 1 : 0;
+    const int64_t blocks = (ka + nb - 1) / nb, rows = std::min<int64_t>(ka, nb);
+    int launches = 2;
+    tri_base_kernel<V><<<unsigned(blocks * (nb / (2 * kTriBase))), 32, 0, st>>>(a);
+    for (int s = kTriBase; s < rows; s *= 2, launches += 2) {
+        // gridDim.y holds at most 65535 pairs: ka / 32 of them on the first level
+        const dim3 grid(unsigned((s / 16) * (s / 16)), unsigned(blocks * (nb / (2 * s))));
+        tri_join_kernel<V, false><<<grid, 256, 0, st>>>(a, s);
+        tri_join_kernel<V, true><<<grid, 256, 0, st>>>(a, s);
+    }
+    tri_zero_kernel<V><<<dim3(unsigned(std::min<int64_t>(rows, 64)), unsigned(blocks)), 256, 0, st>>>(a);
+    count_launches(launches);
     return cudaGetLastError();
 }
 
