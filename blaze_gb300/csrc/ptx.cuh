@@ -174,6 +174,27 @@ __device__ __forceinline__ uint32_t swz128(uint32_t off) {
     return off ^ (((off >> 7) & 7u) << 4);
 }
 
+// ---- packed FP32 pairs -----------------------------------------------------------------------------
+__device__ __forceinline__ uint64_t f32x2_bits(uint32_t lo, uint32_t hi) {
+    uint64_t d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"(hi));
+    return d;
+}
+__device__ __forceinline__ uint64_t f32x2(float lo, float hi) {
+    return f32x2_bits(__float_as_uint(lo), __float_as_uint(hi));
+}
+// Each half rounded on its own, as the scalar instruction rounds it.
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+
 // ---- tcgen05 -----------------------------------------------------------------------------------
 // Allocate `ncols` TMEM columns (power of two >= 32); the base address is written to smem at
 // `dst`.  Must be executed by one full warp.

@@ -98,10 +98,6 @@ enum Mode : int { kExact = 0, kBf16 = 1, kBf16x3 = 2, kCrt = 3 };
 // 239; 233; 229; 227; 223; 7,31; 211; 199.  Product of all 15: about 2^118.2.
 constexpr int MAX_MODULI = 15;
 __constant__ uint32_t c_mod[MAX_MODULI] = {257, 256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 217, 211, 199};
-// floor(2^32 / p) for the reduction of 32-bit values.
-__constant__ uint32_t c_mod_inv32[MAX_MODULI] = {
-    16711935u, 16777216u, 16843009u, 16976155u, 17111423u, 17388531u, 17821441u, 17970574u,
-    18433336u, 18755315u, 18920560u, 19259943u, 19792476u, 20355295u, 21582750u};
 // log2 of each modulus (device copy: the plan kernels sum these instead of calling log2).
 __constant__ double c_mod_log2[MAX_MODULI] = {
     8.005624549193879, 8.0, 7.994353436858858, 7.98299357469431, 7.971543553950772, 7.948367231584678,
@@ -1031,6 +1027,20 @@ __device__ __forceinline__ void unit_coords(const TcParams& p, int u, int& tm, i
     tn = p.tn0 + r / rows_in_band;
 }
 
+// Residues of two FP32 integers |x| <= 2^24 modulo p: q = rint(x fl(1/p)) is within one of x / p's
+// nearest integer (fl(1/p) is off by at most 2^-24 relative, x / p by at most 1 / p, so only an x
+// next to a half multiple of p can round the other way), and r = x - p q, an integer of at most
+// (p + 1) / 2 in magnitude, is exact.  For |x| < 2^23, r is the symmetric residue, |r| <= p / 2.  Four
+// packed instructions for two outputs; converting each group sum to an integer and reducing the
+// total modulo p in integers took about twelve an output, which paced every unit of few k steps
+// (65536 x 256 x 256: 222 us in this kernel, now 140; 8192 x 8192 x 8192:
+// 7.20 -> 6.59 ms, 2.0 PFLOP/s).
+__device__ __forceinline__ uint64_t residue2(uint64_t x, uint64_t pinv2, uint64_t pneg2) {
+    const uint64_t magic = f32x2(MAGIC, MAGIC), nmagic = f32x2(-MAGIC, -MAGIC);
+    const uint64_t q = add2(fma2(x, pinv2, magic), nmagic);
+    return fma2(pneg2, q, x);
+}
+
 template <int MODE>
 __global__ void __cluster_dims__(2, 1, 1) __maxnreg__(168)
 tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
@@ -1046,10 +1056,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     const bool leader = rank == 0;
     const int pair = int(blockIdx.x >> 1), npairs = int(gridDim.x >> 1);
 
-    // the epilogue's arithmetic is fixed at compile time (exact integer sums or FP32 tiles); the
-    // digit and residue schedules share the exact instantiation and differ only in the plane pairs
-    constexpr int emode = MODE;
-    const int mode = (MODE == kExact) ? p.mode : MODE;
+    // the epilogue's arithmetic is fixed at compile time: residues, exact integer sums or FP32 tiles
+    constexpr int mode = MODE;
     const int S = (mode == kExact || mode == kCrt) ? p.info->slices : 1;
     const int nlev = num_levels(mode, S);
     const int units = p.m_tiles * p.n_tiles * p.nseg * nlev;
@@ -1057,7 +1065,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     if (threadIdx.x == 0) {
         tma_prefetch_desc(&tmA);
         tma_prefetch_desc(&tmB);
-        if (p.mode == kCrt) tma_prefetch_desc(&tmC);
+        if (mode == kCrt) tma_prefetch_desc(&tmC);
         // full: the even CTA's arm plus both CTAs' bytes; empty / acc_full: one pair-MMA commit
         // (multicast to both CTAs); acc_empty (even CTA): every epilogue warp of both CTAs
         for (int s = 0; s < STAGES; ++s) {
@@ -1203,9 +1211,18 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 const int np = pairs_in_level(mode, L);
                 const int items = np * kbn;
                 const int gsize = (mode == kExact || mode == kCrt) ? GROUP_ITEMS : items;
-                uint32_t acc[128];
+                // kCrt: FP32 pairs, sums of the groups' residues; kExact: int32 sums; else FP32 values
+                uint64_t rsum[mode == kCrt ? 64 : 1];
+                uint32_t acc[mode == kCrt ? 1 : 128];
+                const float pf = c_modf[mode == kCrt ? L : 0], pinv = c_modf_inv[mode == kCrt ? L : 0];
+                const uint64_t pneg2 = f32x2(-pf, -pf), pinv2 = f32x2(pinv, pinv);
+                if constexpr (mode == kCrt) {
 #pragma unroll
-                for (int c = 0; c < 128; ++c) acc[c] = 0u;
+                    for (int c = 0; c < 64; ++c) rsum[c] = 0ull;
+                } else {
+#pragma unroll
+                    for (int c = 0; c < 128; ++c) acc[c] = 0u;
+                }
                 for (int g0 = 0; g0 < items; g0 += gsize, ++grp) {
                     const int buf = grp & 1;
                     if (!mbar_wait(smem_u32(&bars->acc_full[buf]), (grp >> 1) & 1, p.status, kDevTimeoutMma,
@@ -1220,10 +1237,16 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         uint32_t v[16];
                         tmem_ld_32x32b_x16(base + uint32_t(c4 * 16), v);
                         tc_wait_ld();
-                        if (emode == kExact) {
-                            // the group sum is an integer of at most 2^24 in magnitude: exact in
-                            // FP32 and exactly converted (adding 1.5 * 2^23 would be exact only
-                            // below 2^22, i.e. for groups of 256 products)
+                        if constexpr (mode == kCrt) {
+                            // the group sum is an integer of at most 2^24 in magnitude, exact in
+                            // FP32: its residue (below 130 in magnitude, see residue2) is added up
+#pragma unroll
+                            for (int c = 0; c < 8; ++c)
+                                rsum[c4 * 8 + c] = add2(rsum[c4 * 8 + c],
+                                                        residue2(f32x2_bits(v[2 * c], v[2 * c + 1]), pinv2, pneg2));
+                        } else if constexpr (mode == kExact) {
+                            // exactly converted (adding 1.5 * 2^23 would be exact only below 2^22,
+                            // i.e. for groups of 256 products)
 #pragma unroll
                             for (int c = 0; c < 16; ++c)
                                 acc[c4 * 16 + c] += uint32_t(__float2int_rn(__uint_as_float(v[c])));
@@ -1241,11 +1264,16 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 // schedule the sum is reduced modulo the level's modulus and stored as 16 bits
                 const int64_t plane_off = ((int64_t(seg) * p.max_levels + L) * p.mpad + row) * p.npad +
                                           int64_t(tn) * TN + h * 128;
-                if (emode == kExact && mode == kCrt) {
-                    // residues in [0, p) as 16-bit values; two 64-column halves per warp go out
-                    // through the warp's staging tile (row = lane, 16-byte chunk j of a row at
+                if constexpr (mode == kCrt) {
+                    // residues as 16-bit values r + p in (0, 2 p); two 64-column halves per warp go
+                    // out through the warp's staging tile (row = lane, 16-byte chunk j of a row at
                     // j ^ (lane % 8): the TMA 128-byte swizzle) and a TMA store
-                    const uint32_t pm = c_mod[L], inv = c_mod_inv32[L];
+                    if (items > gsize) {
+#pragma unroll
+                        for (int c = 0; c < 64; ++c) rsum[c] = residue2(rsum[c], pinv2, pneg2);
+                    }
+                    // r + p + 2^23 holds r + p in its low bits
+                    const uint64_t bias2 = f32x2(pf + 8388608.f, pf + 8388608.f);
                     uint8_t* stg = out_stage + (warp - 2) * OUT_WARP_BYTES;
                     const int32_t ytile = int32_t((int64_t(seg) * p.max_levels + L) * p.mpad + int64_t(tm) * TMP +
                                                   int64_t(rank) * TM + 32 * q);
@@ -1255,18 +1283,14 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         __syncwarp();
 #pragma unroll
                         for (int j = 0; j < 8; ++j) {
-                            const int c = ch * 64 + j * 8;
-                            __align__(16) uint16_t rr[8];
+                            uint32_t w[4];
 #pragma unroll
-                            for (int e = 0; e < 8; ++e) {
-                                const int32_t t = int32_t(acc[c + e]);
-                                const uint32_t mag = t < 0 ? uint32_t(-int64_t(t)) : uint32_t(t);
-                                uint32_t rsd = mod_small(mag, pm, inv);
-                                if (t < 0 && rsd) rsd = pm - rsd;
-                                rr[e] = uint16_t(rsd);
+                            for (int e = 0; e < 4; ++e) {
+                                const uint64_t t = add2(rsum[ch * 32 + j * 4 + e], bias2);
+                                w[e] = __byte_perm(uint32_t(t), uint32_t(t >> 32), 0x5410);
                             }
                             *reinterpret_cast<uint4*>(stg + lane * 128 + ((j ^ (lane & 7)) << 4)) =
-                                *reinterpret_cast<const uint4*>(rr);
+                                make_uint4(w[0], w[1], w[2], w[3]);
                         }
                         fence_proxy_async_smem();
                         __syncwarp();
@@ -2020,8 +2044,9 @@ int device_product(const Gemm& g_in, const SplitRequest& req, const LaunchCtl& c
     // units: one level of one pair tile and k-segment (the device picks the level count, at most
     // max_levels); CTA pairs (clusters of two): at most one pair per unit, at least one pair
     const int sms = req.max_sms > 0 ? std::min(req.max_sms, r.num_sms) : r.num_sms;
-    auto kern = (mode == kExact || mode == kCrt) ? tc_gemm_kernel<kExact>
-                                                 : (mode == kBf16 ? tc_gemm_kernel<kBf16> : tc_gemm_kernel<kBf16x3>);
+    auto kern = mode == kCrt ? tc_gemm_kernel<kCrt>
+                             : mode == kExact ? tc_gemm_kernel<kExact>
+                                              : (mode == kBf16 ? tc_gemm_kernel<kBf16> : tc_gemm_kernel<kBf16x3>);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTcSmem));
     if (e != cudaSuccess) {
         if (err) *err = std::string("tc_gemm_kernel smem attribute: ") + cudaGetErrorString(e);
@@ -2320,7 +2345,7 @@ int device_product_host_panels(const Gemm& g, const SplitRequest& req, const Lau
         if (!encode_tmap_2d(&tC[b], CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, lv + b * lv_elems,
                             uint64_t(nseg) * max_levels * mpad, npb, npb, 32, 64, CU_TENSOR_MAP_SWIZZLE_128B, err))
             return GB300_ERR_CUDA;
-    e = cudaFuncSetAttribute(tc_gemm_kernel<kExact>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTcSmem));
+    e = cudaFuncSetAttribute(tc_gemm_kernel<kCrt>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTcSmem));
     if (e != cudaSuccess) return cuda_fail("tc_gemm_kernel smem attribute", e);
 
     // ---- operands in, blocks as their operands arrive, C back ----
@@ -2401,7 +2426,7 @@ int device_product_host_panels(const Gemm& g, const SplitRequest& req, const Lau
         const int grid = 2 * std::max(1, std::min(units, r.num_sms / 2));
         {
             KernelTimer timer("tc_gemm", st);
-            tc_gemm_kernel<kExact><<<grid, THREADS, kTcSmem, st>>>(tA, tB, tC[buf], tp);
+            tc_gemm_kernel<kCrt><<<grid, THREADS, kTcSmem, st>>>(tA, tB, tC[buf], tp);
         }
         cudaEventRecord(tc_done_ev(l), st);
         cudaStreamWaitEvent(aux, tc_done_ev(l), 0);
