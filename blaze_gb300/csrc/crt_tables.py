@@ -56,6 +56,10 @@ def table(n):
         else:
             s["A"] = ys % Ps
             s["B"] = 0
+        # the residues come as b = r + 128 (r symmetric, b in [0, 256]): x = b_p A + b_q B + K, K taking
+        # the 128s out again
+        s["K"] = -128 * (s["A"] + s["B"]) % Ps
+        assert 256 * (s["A"] + s["B"]) + s["K"] < 1 << 26
         s["Psinv32"] = (1 << 32) // Ps
         s["pinv32"] = (1 << 32) // p
         s["qinv32"] = (1 << 32) // q if q > 1 else 0
@@ -67,7 +71,7 @@ def table(n):
         assert (p - 1) * s["A"] + (q - 1) * s["B"] < 1 << 26
     fbias = sum((1 << 23) / s["Ps"] for s in sups)
     limbs = (P.bit_length() + 1 + 31) // 32  # signed result |W| < P / 2
-    return dict(n=n, P=P, sups=sups, fbias=fbias, limbs=limbs)
+    return dict(n=n, P=P, sups=sups, fbias=fbias, limbs=limbs, negP=(1 << (32 * limbs)) - P)
 
 
 def emit(path):
@@ -81,8 +85,9 @@ def emit(path):
         "struct CrtSuper {",
         "    int ia, ib;                 // residue planes (ib < 0: single modulus)",
         "    uint32_t p, q;              // q = 1 for a single modulus",
-        "    uint32_t A, B;              // u = (c_p A + c_q B) mod P_s",
-        "    uint32_t Ps, Psinv32;       // P_s and floor(2^32 / P_s)",
+        "    uint32_t A, B;              // c_p A + c_q B is congruent to the super residue mod P_s",
+        "    uint32_t K;                 // -128 (A + B) mod P_s",
+        "    uint32_t Ps;                // p q",
         "    uint32_t pinv32, qinv32;    // floor(2^32 / p), floor(2^32 / q)",
         "    uint32_t M[4];              // P / P_s, 32-bit limbs",
         "    float finv;                 // 1 / P_s rounded to FP32",
@@ -90,8 +95,7 @@ def emit(path):
         "",
         "struct CrtTable {",
         "    int nsup, limbs;            // super moduli; 32-bit limbs of the signed result",
-        "    uint32_t P[4];              // product of the moduli, 32-bit limbs",
-        "    float fbias;                // sum_s 2^23 / P_s rounded to FP32",
+        "    uint32_t negP[4];           // 2^(32 limbs) - product of the moduli, 32-bit limbs",
         f"    CrtSuper sup[{MAX_SUP}];",
         "};",
         "",
@@ -100,14 +104,14 @@ def emit(path):
     ]
     for n in range(2, 16):
         t = table(n)
-        P32 = ", ".join(f"{(t['P'] >> (32 * l)) & 0xFFFFFFFF}u" for l in range(4))
-        lines.append(f"    {{{len(t['sups'])}, {t['limbs']}, {{{P32}}}, {f32hex(t['fbias'])}f, {{  // N = {n}")
+        P32 = ", ".join(f"{(t['negP'] >> (32 * l)) & 0xFFFFFFFF}u" for l in range(4))
+        lines.append(f"    {{{len(t['sups'])}, {t['limbs']}, {{{P32}}}, {{  // N = {n}")
         for s in t["sups"]:
             M = ", ".join(f"{m}u" for m in s["M"])
             finv = f32hex(1.0 / s["Ps"])
             lines.append(
-                f"        {{{s['ia']}, {s['ib']}, {s['p']}u, {s['q']}u, {s['A']}u, {s['B']}u, {s['Ps']}u, "
-                f"{s['Psinv32']}u, {s['pinv32']}u, {s['qinv32']}u, {{{M}}}, {finv}f}},"
+                f"        {{{s['ia']}, {s['ib']}, {s['p']}u, {s['q']}u, {s['A']}u, {s['B']}u, {s['K']}u, {s['Ps']}u, "
+                f"{s['pinv32']}u, {s['qinv32']}u, {{{M}}}, {finv}f}},"
             )
         lines.append("    }},")
     lines += ["};", "", "}  // namespace gb", ""]

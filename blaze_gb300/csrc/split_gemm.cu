@@ -971,7 +971,8 @@ struct TcParams {
     int kb_per_seg;          // 64-wide k-blocks per segment
     int kb_total;            // 64-wide k-blocks in the padded K
     int64_t mpad, npad;      // padded rows of the A / B planes
-    int32_t* levels;         // [nseg][nlevels][mpad][npad] int32 (float modes: fp32 bits)
+    int32_t* levels;         // [nseg][nlevels][mpad][npad] int32 (float modes: fp32 bits); kCrt: the
+                             // residue planes described at crt_plane
     int max_levels;          // level dimension of `levels`
     int band = 8;            // m-tiles per band of the unit order (2..32 measured alike at 8192^3)
     int tn0 = 0;             // first n-tile of this launch (a product launched in column parts)
@@ -1044,7 +1045,7 @@ __device__ __forceinline__ uint64_t residue2(uint64_t x, uint64_t pinv2, uint64_
 template <int MODE>
 __global__ void __cluster_dims__(2, 1, 1) __maxnreg__(168)
 tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-               const __grid_constant__ CUtensorMap tmC, const TcParams p) {
+               const __grid_constant__ CUtensorMap tmC0, const __grid_constant__ CUtensorMap tmC, const TcParams p) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* out_stage = smem + STAGES * STAGE_BYTES;
@@ -1065,7 +1066,10 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     if (threadIdx.x == 0) {
         tma_prefetch_desc(&tmA);
         tma_prefetch_desc(&tmB);
-        if (mode == kCrt) tma_prefetch_desc(&tmC);
+        if (mode == kCrt) {
+            tma_prefetch_desc(&tmC0);
+            tma_prefetch_desc(&tmC);
+        }
         // full: the even CTA's arm plus both CTAs' bytes; empty / acc_full: one pair-MMA commit
         // (multicast to both CTAs); acc_empty (even CTA): every epilogue warp of both CTAs
         for (int s = 0; s < STAGES; ++s) {
@@ -1260,25 +1264,26 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     if (lane == 0) mbar_arrive_cluster(buf ? acc_empty1 : acc_empty0);
                 }
                 if (!ok) break;
-                // level sums -> global level plane (row-major, pitch npad); in the residue (CRT)
-                // schedule the sum is reduced modulo the level's modulus and stored as 16 bits
+                // level sums -> global level plane (row-major, pitch npad)
                 const int64_t plane_off = ((int64_t(seg) * p.max_levels + L) * p.mpad + row) * p.npad +
                                           int64_t(tn) * TN + h * 128;
                 if constexpr (mode == kCrt) {
-                    // residues as 16-bit values r + p in (0, 2 p); two 64-column halves per warp go
-                    // out through the warp's staging tile (row = lane, 16-byte chunk j of a row at
-                    // j ^ (lane % 8): the TMA 128-byte swizzle) and a TMA store
-                    if (items > gsize) {
+                    // residues as r + 128: one byte each, 16 bits for the first modulus (257, whose
+                    // 129 values a side do not fit a byte).  A single group's residue may be one past
+                    // the symmetric range, which matters for 257 and 255 (253 and below stay within
+                    // 127, and modulo 256 the byte wraps to the same residue).
+                    if (items > gsize || L == 0 || L == 2) {
 #pragma unroll
                         for (int c = 0; c < 64; ++c) rsum[c] = residue2(rsum[c], pinv2, pneg2);
                     }
-                    // r + p + 2^23 holds r + p in its low bits
-                    const uint64_t bias2 = f32x2(pf + 8388608.f, pf + 8388608.f);
+                    // r + 128 + 2^23 holds r + 128 in its low bits
+                    const uint64_t bias2 = f32x2(128.f + 8388608.f, 128.f + 8388608.f);
+                    // out through the warp's staging tile (32 rows of 128 bytes, row = lane, 16-byte
+                    // chunk j of a row at j ^ (lane % 8): the TMA 128-byte swizzle) and a TMA store
                     uint8_t* stg = out_stage + (warp - 2) * OUT_WARP_BYTES;
-                    const int32_t ytile = int32_t((int64_t(seg) * p.max_levels + L) * p.mpad + int64_t(tm) * TMP +
-                                                  int64_t(rank) * TM + 32 * q);
-#pragma unroll
-                    for (int ch = 0; ch < 2; ++ch) {
+                    const int32_t trow = int32_t(int64_t(tm) * TMP + int64_t(rank) * TM + 32 * q);
+                    const int64_t seg_rows = int64_t(seg) * (p.max_levels + 1) * p.mpad;
+                    if (L != 0) {
                         if (lane == 0) bulk_wait_read0();  // the previous store has read the tile
                         __syncwarp();
 #pragma unroll
@@ -1286,8 +1291,10 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                             uint32_t w[4];
 #pragma unroll
                             for (int e = 0; e < 4; ++e) {
-                                const uint64_t t = add2(rsum[ch * 32 + j * 4 + e], bias2);
-                                w[e] = __byte_perm(uint32_t(t), uint32_t(t >> 32), 0x5410);
+                                const uint64_t t = add2(rsum[j * 8 + 2 * e], bias2);
+                                const uint64_t v = add2(rsum[j * 8 + 2 * e + 1], bias2);
+                                w[e] = __byte_perm(__byte_perm(uint32_t(t), uint32_t(t >> 32), 0x0040),
+                                                   __byte_perm(uint32_t(v), uint32_t(v >> 32), 0x0040), 0x5410);
                             }
                             *reinterpret_cast<uint4*>(stg + lane * 128 + ((j ^ (lane & 7)) << 4)) =
                                 make_uint4(w[0], w[1], w[2], w[3]);
@@ -1295,8 +1302,33 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         fence_proxy_async_smem();
                         __syncwarp();
                         if (lane == 0) {
-                            tma_store_2d(&tmC, int32_t(tn * TN + h * 128 + ch * 64), ytile, smem_u32(stg));
+                            tma_store_2d(&tmC, int32_t(tn * TN + h * 128),
+                                         int32_t(seg_rows + int64_t(L + 1) * p.mpad) + trow, smem_u32(stg));
                             bulk_commit();
+                        }
+                    } else {
+#pragma unroll
+                        for (int ch = 0; ch < 2; ++ch) {
+                            if (lane == 0) bulk_wait_read0();
+                            __syncwarp();
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) {
+                                uint32_t w[4];
+#pragma unroll
+                                for (int e = 0; e < 4; ++e) {
+                                    const uint64_t t = add2(rsum[ch * 32 + j * 4 + e], bias2);
+                                    w[e] = __byte_perm(uint32_t(t), uint32_t(t >> 32), 0x5410);
+                                }
+                                *reinterpret_cast<uint4*>(stg + lane * 128 + ((j ^ (lane & 7)) << 4)) =
+                                    make_uint4(w[0], w[1], w[2], w[3]);
+                            }
+                            fence_proxy_async_smem();
+                            __syncwarp();
+                            if (lane == 0) {
+                                tma_store_2d(&tmC0, int32_t(tn * TN + h * 128 + ch * 64),
+                                             int32_t(seg_rows / 2) + trow, smem_u32(stg));
+                                bulk_commit();
+                            }
                         }
                     }
                 } else {
@@ -1364,42 +1396,6 @@ __device__ __forceinline__ double int128_to_double_scaled(__int128 W, int x) {
     return neg ? -v : v;
 }
 
-// The same for W given as two's-complement 64-bit halves, on 64-bit integer operations: normalize
-// the magnitude so that its top bit is bit 127, keep 53 bits, round to nearest even, and write the
-// exponent field by adding (be - 1) << 52 to the 53-bit mantissa (a rounding carry into 2^53 then
-// moves the exponent up by itself).
-__device__ __forceinline__ double i128_to_double_scaled(unsigned long long hi, unsigned long long lo, int x) {
-    const bool neg = (long long)hi < 0;
-    if (neg) {
-        lo = ~lo + 1ull;
-        hi = ~hi + (lo == 0ull ? 1ull : 0ull);
-    }
-    if ((hi | lo) == 0ull) return 0.0;
-    int lz;
-    unsigned long long t, sticky;
-    if (hi) {
-        lz = __clzll((long long)hi);
-        t = lz ? (hi << lz) | (lo >> (64 - lz)) : hi;
-        sticky = lo << lz;
-    } else {
-        const int l2 = __clzll((long long)lo);
-        lz = 64 + l2;
-        t = lo << l2;
-        sticky = 0ull;
-    }
-    // |W| = (t + sticky 2^-64) 2^(64 - lz); mantissa bits 63..11 of t, bit 10 the rounding bit
-    unsigned long long mant = t >> 11;
-    if ((t & 0x400ull) && ((t & 0x3ffull) || sticky || (mant & 1ull))) ++mant;
-    // |W| 2^x ~= mant 2^(75 - lz + x), leading bit 2^(127 - lz + x)
-    const int be = 127 - lz + x + 1023;
-    if (be >= 1 && be + int(mant >> 53) <= 2046) {
-        const unsigned long long bits = ((unsigned long long)(be - 1) << 52) + mant;
-        return __longlong_as_double((long long)(bits | (neg ? (1ull << 63) : 0ull)));
-    }
-    const double v = ldexp(double(mant), 75 - lz + x);
-    return neg ? -v : v;
-}
-
 // C = alpha * 2^(e_i + f_j) * sum_L 2^(-14-8L) * sum_seg T[seg][L] + beta * C   (exact mode)
 // C = alpha * sum_seg P[seg] + beta * C                                         (float modes)
 // Exact mode forms W = sum_L T_L * 2^(8(S-1-L)) exactly in 128-bit integers, so the only roundings
@@ -1407,154 +1403,262 @@ __device__ __forceinline__ double i128_to_double_scaled(unsigned long long hi, u
 // Grid: x over groups of 4 consecutive columns (one 16-byte load per level plane), y over rows.
 constexpr int COMBINE_COLS = 4;
 
-// Residue (CRT) reconstruction of CC consecutive outputs of one row for N moduli, all constants
-// compile-time (crt_tables.h).  u_s = (c_p A_s + c_q B_s) mod P_s per super modulus (< 2^26 before
-// the reduction), W = sum_s u_s (P / P_s) in signed 64-bit sums of 32-bit limb products (each below
-// 2^48, at most 8 per limb), and the symmetric residue W - round(W / P) P with the quotient from an
-// FP32 estimate of sum_s u_s / P_s: the product of the scaled integers has |value| < P / 2.125, so
-// W / P lies at least 0.029 from a half integer and an estimate off by less than 0.01 picks the
-// right multiple of P.
-// Residues of CC consecutive columns (CC / 2 words of two 16-bit residues).
-template <int CC>
-__device__ __forceinline__ void load_res(const uint16_t* __restrict__ p, uint32_t (&w)[CC / 2]) {
-    if constexpr (CC == 4) {
-        const uint2 v = *reinterpret_cast<const uint2*>(p);
-        w[0] = v.x;
-        w[1] = v.y;
-    } else {
-        w[0] = *reinterpret_cast<const uint32_t*>(p);
-    }
+// Residue planes of a residue (CRT) product, S = mpad npad elements each, row-major: per k-segment the
+// plane of the first modulus in 16 bits, then one byte per element for every other modulus, all
+// holding r + 128 for the symmetric residue r.  Byte offset of plane t of segment g.
+__host__ __device__ __forceinline__ int64_t crt_plane(int64_t S, int max_levels, int g, int t) {
+    return S * (int64_t(g) * (max_levels + 1) + (t == 0 ? 0 : t + 1));
 }
 
-template <int N, int CC>
-__device__ __forceinline__ void crt_cols(const uint16_t* __restrict__ res16, int64_t plane, int64_t off, int nseg,
-                                         int max_levels, int scale, int ei, const int (&fj)[CC], double (&v)[CC]) {
-    constexpr CrtTable T = kCrtTables[N - 2];
-    constexpr int NS = T.nsup, LB = T.limbs;
-    uint32_t rq[2 * NS][CC / 2];
+// The residues of four consecutive outputs of one row: words[t] holds four bytes (the first modulus:
+// two words of two 16-bit values).
+template <int N>
+struct CrtWords {
+    uint32_t w0[2];
+    uint32_t w[N];  // w[0] unused
+};
+
+template <int N>
+__device__ __forceinline__ CrtWords<N> crt_load(const uint8_t* __restrict__ res, int64_t S, int max_levels, int64_t off) {
+    CrtWords<N> r;
+    const uint2 z = *reinterpret_cast<const uint2*>(res + 2 * off);
+    r.w0[0] = z.x;
+    r.w0[1] = z.y;
 #pragma unroll
-    for (int s = 0; s < NS; ++s) {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int t = h ? T.sup[s].ib : T.sup[s].ia;
-            if (t < 0) continue;
-            load_res<CC>(res16 + int64_t(t) * plane + off, rq[2 * s + h]);
-            for (int g = 1; g < nseg; ++g) {
-                // segment residues add up: each < p, words hold two 16-bit residues and no carry
-                // crosses for nseg < 256
-                uint32_t b[CC / 2];
-                load_res<CC>(res16 + (int64_t(g) * max_levels + t) * plane + off, b);
-#pragma unroll
-                for (int w = 0; w < CC / 2; ++w) rq[2 * s + h][w] += b[w];
-            }
+    for (int t = 1; t < N; ++t) r.w[t] = *reinterpret_cast<const uint32_t*>(res + crt_plane(S, max_levels, 0, t) + off);
+    return r;
+}
+
+// With k in segments: the sum of the residues b = r + 128 of column cc over the segments, reduced to
+// [0, p) and congruent to (sum of r) + 128, as the single segment's b is.
+template <int N>
+__device__ __forceinline__ uint32_t crt_seg_sum(const uint8_t* __restrict__ res, int64_t S, int max_levels, int64_t off,
+                                                int nseg, int t, int cc, uint32_t p, uint32_t pinv32) {
+    uint32_t sum = 0;
+    for (int g = 0; g < nseg; ++g) {
+        const uint8_t* q = res + crt_plane(S, max_levels, g, t);
+        sum += t == 0 ? uint32_t(reinterpret_cast<const uint16_t*>(q)[off + cc]) : uint32_t(q[off + cc]);
+    }
+    return mod_small(sum + 128u * (p - 1u) * uint32_t(nseg - 1), p, pinv32);
+}
+
+// sign |W| 2^x for the two's-complement integer W of LB 32-bit words (low word first), rounded to nearest
+// even.  Straight-line code: the magnitude's words move up until the top one is not zero, a funnel
+// shift brings the leading bit to the top, and the 53-bit mantissa is rounded on integers; adding
+// (be - 1) << 52 to it writes the exponent, a rounding carry into 2^53 moving it up by itself.  Results
+// that are not normal numbers take the FP64 path (ldexp), rows or columns with Inf / NaN (whose
+// exponent kNonFinite lands there too) give NaN.
+template <int LB>
+__device__ __forceinline__ double words_to_double(const uint32_t (&w)[4], int ei, int fj, int scale) {
+    const uint32_t sgn = uint32_t(int32_t(w[LB - 1]) >> 31);
+    uint32_t z[4] = {0u, 0u, 0u, 0u};  // the magnitude, top word first
+    if constexpr (LB == 1) {
+        z[0] = (w[0] ^ sgn) - sgn;
+    } else {
+        unsigned long long lo = (unsigned long long)w[0] | ((unsigned long long)w[1] << 32);
+        lo = (lo ^ (unsigned long long)(long long)int32_t(sgn)) - (unsigned long long)(long long)int32_t(sgn);
+        z[LB - 1] = uint32_t(lo);
+        z[LB - 2] = uint32_t(lo >> 32);
+        if constexpr (LB > 2) {
+            const unsigned long long carry = (sgn != 0u && lo == 0ull) ? 1ull : 0ull;
+            unsigned long long hi = (unsigned long long)w[2] | (LB > 3 ? (unsigned long long)w[LB - 1] << 32 : 0ull);
+            hi = (hi ^ (unsigned long long)(long long)int32_t(sgn)) + carry;
+            z[LB - 3] = uint32_t(hi);
+            if constexpr (LB > 3) z[0] = uint32_t(hi >> 32);
         }
     }
-    long long acc[CC][4];
-    float fq[CC];
+    int lead = 32 * LB - 1;  // position of the leading bit
 #pragma unroll
-    for (int cc = 0; cc < CC; ++cc) {
-        fq[cc] = -T.fbias;
+    for (int i = 1; i < LB; ++i) {
+        const bool up = z[0] == 0u;
+#pragma unroll
+        for (int j = 0; j < LB - i; ++j) z[j] = up ? z[j + 1] : z[j];
+        z[LB - i] = up ? 0u : z[LB - i];
+        lead -= up ? 32 : 0;
+    }
+    const int lz = __clz(int(z[0]));
+    const uint32_t t1 = __funnelshift_l(z[1], z[0], lz);
+    uint32_t t0 = __funnelshift_l(z[2], z[1], lz);
+    if constexpr (LB > 2) t0 |= min(__funnelshift_l(z[3], z[2], lz) | (LB > 3 ? z[3] : 0u), 1u);  // sticky
+    unsigned long long mant = (((unsigned long long)t1 << 32) | t0) >> 11;
+    mant += (t0 & 0x7ffu) + (uint32_t(mant) & 1u) > 0x400u ? 1ull : 0ull;
+    const int x = ei + fj - scale;
+    const int be = lead - lz + x + 1023;
+    if (be >= 1 && be <= 2045) {
+        unsigned long long bits = mant + ((unsigned long long)uint32_t(be - 1) << 52);
+        bits |= (unsigned long long)(sgn & 0x80000000u) << 32;
+        return z[0] == 0u ? 0.0 : __longlong_as_double((long long)bits);
+    }
+    if (ei == kNonFinite || fj == kNonFinite) return __longlong_as_double(0x7ff8000000000000ll);
+    if (z[0] == 0u) return 0.0;
+    const double v = ldexp(double(mant), lead - lz - 52 + x);
+    return sgn ? -v : v;
+}
+
+// Residue (CRT) reconstruction of four consecutive outputs of one row for N moduli, all constants
+// compile-time (crt_tables.h).  Per super modulus x = b_p A_s + b_q B_s + K_s < 2^26 is congruent to
+// the super residue u_s (one two-way byte dot product, K_s taking the 128s out), and
+// W = sum_s x_s (P / P_s) in 64-bit sums of 32-bit limb products.  The multiple of P to remove is
+// round(W / P), from an FP32 estimate of sum_s x_s / P_s (below 2^13, off by less than 0.01): the
+// product of the scaled integers has |value| < P / 2.125, so W / P lies at least 0.029 from a half
+// integer.  It is removed by adding the multiple of 2^(32 LB) - P, all modulo 2^(32 LB).
+template <int N>
+__device__ __forceinline__ void crt_cols(const CrtWords<N>& r, const uint8_t* __restrict__ res, int64_t S, int64_t off,
+                                         int nseg, int max_levels, int scale, int ei, const int (&fj)[4], double (&v)[4]) {
+    constexpr CrtTable T = kCrtTables[N - 2];
+    constexpr int NS = T.nsup, LB = T.limbs;
+    unsigned long long acc[4][4];
+    float fq[4];
+#pragma unroll
+    for (int cc = 0; cc < 4; ++cc) {
+        fq[cc] = 0.f;
 #pragma unroll
         for (int l = 0; l < 4; ++l) acc[cc][l] = 0;
     }
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
         constexpr uint32_t one = 1u;
-        const CrtSuper& S = T.sup[s];
+        const CrtSuper& Q = T.sup[s];
+        const bool pair = Q.q > one;
+        uint32_t x[4];
+        if (nseg > 1) {
 #pragma unroll
-        for (int cc = 0; cc < CC; ++cc) {
-            const uint32_t ha = rq[2 * s][cc >> 1];
-            uint32_t cp = (cc & 1) ? (ha >> 16) : (ha & 0xffffu);
-            if (nseg > 1) cp = mod_small(cp, S.p, S.pinv32);
-            uint32_t x = cp * S.A;
-            if (S.q > one) {
-                const uint32_t hb = rq[2 * s + 1][cc >> 1];
-                uint32_t cq = (cc & 1) ? (hb >> 16) : (hb & 0xffffu);
-                if (nseg > 1) cq = mod_small(cq, S.q, S.qinv32);
-                x += cq * S.B;
+            for (int cc = 0; cc < 4; ++cc) {
+                x[cc] = crt_seg_sum<N>(res, S, max_levels, off, nseg, Q.ia, cc, Q.p, Q.pinv32) * Q.A + Q.K;
+                if (pair) x[cc] += crt_seg_sum<N>(res, S, max_levels, off, nseg, Q.ib, cc, Q.q, Q.qinv32) * Q.B;
             }
-            uint32_t u = x - __umulhi(x, S.Psinv32) * S.Ps;
-            u = min(u, u - S.Ps);
-            fq[cc] = fmaf(__uint_as_float(0x4B000000u | u), S.finv, fq[cc]);
+        } else if (Q.ia == 0) {
+#pragma unroll
+            for (int cc = 0; cc < 4; ++cc) {
+                x[cc] = ((cc & 1) ? r.w0[cc >> 1] >> 16 : r.w0[cc >> 1] & 0xffffu) * Q.A + Q.K;
+                if (pair) x[cc] += __byte_perm(r.w[Q.ib], 0, 0x4440 + cc) * Q.B;
+            }
+        } else if (pair) {
+            // bytes (p, q) of columns 0, 1 and of columns 2, 3 side by side
+            const uint32_t t01 = __byte_perm(r.w[Q.ia], r.w[Q.ib], 0x5140), t23 = __byte_perm(r.w[Q.ia], r.w[Q.ib], 0x7362);
+            const uint32_t AB = Q.A | (Q.B << 16);
+            x[0] = __dp2a_lo(AB, t01, Q.K);
+            x[1] = __dp2a_hi(AB, t01, Q.K);
+            x[2] = __dp2a_lo(AB, t23, Q.K);
+            x[3] = __dp2a_hi(AB, t23, Q.K);
+        } else {
+            x[0] = __dp2a_lo(Q.A, r.w[Q.ia], Q.K);
+            x[1] = __dp2a_lo(Q.A << 16, r.w[Q.ia], Q.K);
+            x[2] = __dp2a_hi(Q.A, r.w[Q.ia], Q.K);
+            x[3] = __dp2a_hi(Q.A << 16, r.w[Q.ia], Q.K);
+        }
+#pragma unroll
+        for (int cc = 0; cc < 4; ++cc) {
+            fq[cc] = fmaf(__uint2float_rn(x[cc]), Q.finv, fq[cc]);
 #pragma unroll
             for (int l = 0; l < LB; ++l)
-                if (S.M[l]) acc[cc][l] += (unsigned long long)u * S.M[l];
+                if (Q.M[l]) acc[cc][l] += (unsigned long long)x[cc] * Q.M[l];
         }
     }
 #pragma unroll
-    for (int cc = 0; cc < CC; ++cc) {
+    for (int cc = 0; cc < 4; ++cc) {
         const uint32_t qm = __float_as_uint(fq[cc] + MAGIC) - MAGIC_BITS;
-        long long a[4];
+        uint32_t w[4] = {0u, 0u, 0u, 0u};
+        unsigned long long carry = 0;
 #pragma unroll
         for (int l = 0; l < LB; ++l) {
-            a[l] = acc[cc][l] - (long long)((unsigned long long)qm * T.P[l]);
-            if (l > 0) a[l] += a[l - 1] >> 32;
+            const unsigned long long a = acc[cc][l] + (unsigned long long)qm * T.negP[l] + carry;
+            w[l] = uint32_t(a);
+            carry = a >> 32;
         }
-        unsigned long long hi, lo;
-        if (LB == 1) {
-            lo = (unsigned long long)a[0];
-            hi = (unsigned long long)(a[0] >> 63);
-        } else {
-            lo = ((unsigned long long)a[1] << 32) | uint32_t(a[0]);
-            if (LB == 2) hi = (unsigned long long)(a[1] >> 32);
-            else if (LB == 3) hi = (unsigned long long)a[2];
-            else hi = ((unsigned long long)a[LB - 1] << 32) | uint32_t(a[LB - 2]);
-        }
-        if (ei == kNonFinite || fj[cc] == kNonFinite) v[cc] = __longlong_as_double(0x7ff8000000000000ll);
-        else v[cc] = i128_to_double_scaled(hi, lo, ei + fj[cc] - scale);
+        v[cc] = words_to_double<LB>(w, ei, fj[cc], scale);
     }
 }
 
-// Residue (CRT) reconstruction and epilogue, CC columns a thread (row i on blockIdx.y, striding by
-// gridDim.y; the column exponents are read once): C = alpha * W 2^(e_i + f_j - scale) + beta * C.
-// Measured at 2048^3 and 8192^3: 4 columns beat 2 (latency-bound, less work in flight) and 8
-// (fewer resident warps); reading the column exponents once took 4 % off the 8192^3 time.
-template <int CC>
-__global__ void __launch_bounds__(128, 8) crt_combine_kernel(const uint16_t* __restrict__ res16, int nseg,
-                                                             int max_levels, int64_t mpad, int64_t npad,
-                                                             const SplitInfo* __restrict__ info,
-                                                             const int* __restrict__ eA, const int* __restrict__ eB,
-                                                             int64_t m, int64_t n, double alpha, double beta,
-                                                             double* __restrict__ C, int64_t ldc) {
-    const int64_t j0 = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) * CC;
-    if (j0 >= n) return;
-    const int64_t plane = mpad * npad;
-    const int scale = info->beta + info->beta_b;
-    const int N = info->slices;
-    int fj[CC];
-#pragma unroll
-    for (int cc = 0; cc < CC; ++cc) fj[cc] = (j0 + cc < n) ? eB[j0 + cc] : 0;
-    const bool plain = (alpha == 1.0 && beta == 0.0);
-    for (int64_t i = blockIdx.y; i < m; i += gridDim.y) {
-        const int64_t off = i * npad + j0;
-        const int ei = eA[i];
-        double v[CC];
-        switch (N) {
-#define GB_CRT_CASE(NN) \
-    case NN: crt_cols<NN, CC>(res16, plane, off, nseg, max_levels, scale, ei, fj, v); break;
-            GB_CRT_CASE(2) GB_CRT_CASE(3) GB_CRT_CASE(4) GB_CRT_CASE(5) GB_CRT_CASE(6) GB_CRT_CASE(7)
-            GB_CRT_CASE(8) GB_CRT_CASE(9) GB_CRT_CASE(10) GB_CRT_CASE(11) GB_CRT_CASE(12) GB_CRT_CASE(13)
-            GB_CRT_CASE(14) GB_CRT_CASE(15)
-#undef GB_CRT_CASE
-            default:
-#pragma unroll
-                for (int cc = 0; cc < CC; ++cc) v[cc] = __longlong_as_double(0x7ff8000000000000ll);
+struct CrtCombine {
+    const uint8_t* res;      // residue planes
+    int64_t mpad, npad;
+    int nseg, max_levels;
+    int64_t col0;            // first column of this launch in the planes, eB and C
+    int64_t m, n;            // rows, columns of this launch
+    const int *eA, *eB;
+    double alpha, beta;
+    double* C;
+    int64_t ldc;
+};
+
+// The rows i, i + gridDim.y, ... of four columns a thread, the next row's residues on their way while
+// one row is reconstructed.
+template <int N>
+__device__ __forceinline__ void crt_rows(const CrtCombine& p, int scale, int64_t j0, const int (&fj)[4]) {
+    const int64_t S = p.mpad * p.npad, step = int64_t(gridDim.y) * p.npad;
+    const bool plain = p.alpha == 1.0 && p.beta == 0.0;
+    const bool pairs = j0 + 4 <= p.n && (p.ldc & 1) == 0 && (reinterpret_cast<uintptr_t>(p.C + p.col0) & 15) == 0;
+    int64_t i = blockIdx.y, off = i * p.npad + p.col0 + j0;
+    if (i >= p.m) return;
+    CrtWords<N> w = crt_load<N>(p.res, S, p.max_levels, off);
+    int ei = p.eA[i];
+    while (true) {
+        const int64_t inext = i + gridDim.y;
+        const bool more = inext < p.m;
+        CrtWords<N> wn = w;
+        int en = ei;
+        if (more) {
+            wn = crt_load<N>(p.res, S, p.max_levels, off + step);
+            en = p.eA[inext];
         }
-        double* crow = C + i * ldc;
+        double v[4];
+        crt_cols<N>(w, p.res, S, off, p.nseg, p.max_levels, scale, ei, fj, v);
+        double* crow = p.C + i * p.ldc + p.col0 + j0;
+        if (plain && pairs) {
+            *reinterpret_cast<double2*>(crow) = make_double2(v[0], v[1]);
+            *reinterpret_cast<double2*>(crow + 2) = make_double2(v[2], v[3]);
+        } else {
 #pragma unroll
-        for (int cc = 0; cc < CC; ++cc) {
-            const int64_t j = j0 + cc;
-            if (j >= n) break;
-            if (plain) crow[j] = v[cc];
-            else {
-                const double x = alpha * v[cc];
-                crow[j] = (beta == 0.0) ? x : fma(beta, crow[j], x);
+            for (int cc = 0; cc < 4; ++cc) {
+                if (j0 + cc >= p.n) break;
+                if (plain) crow[cc] = v[cc];
+                else {
+                    const double x = p.alpha * v[cc];
+                    crow[cc] = (p.beta == 0.0) ? x : fma(p.beta, crow[cc], x);
+                }
             }
         }
+        if (!more) return;
+        w = wn;
+        ei = en;
+        i = inext;
+        off += step;
     }
 }
 
-constexpr int CRT_COMBINE_COLS = 4;
+// Residue (CRT) reconstruction and epilogue: C = alpha * W 2^(e_i + f_j - scale) + beta * C.  Bound by
+// instruction issue and latency (about 160 instructions an output at 13 moduli, half the issue slots
+// busy; 118 MB read and 134 MB written take 38 us of the 72 at 32768 x 256).  Byte planes and the
+// straight-line conversion to double against 16-bit planes, a reduction of every super residue and a
+// branching conversion: 33.5 M outputs at 12 moduli 285 -> 243 us, 8.4 M at 13 moduli 90 -> 72.  Eight
+// blocks an SM (64 registers) beat six or five by up to 3 %, and let a block run beside a
+// tensor-core CTA; two columns at a time instead of four took 186 instructions an output.
+constexpr int kCombineBlocks = 8;
+__global__ void __launch_bounds__(128, kCombineBlocks) crt_combine_kernel(const CrtCombine p, const SplitInfo* __restrict__ info) {
+    const int64_t j0 = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) * 4;
+    if (j0 >= p.n) return;
+    const int scale = info->beta + info->beta_b;
+    int fj[4];
+#pragma unroll
+    for (int cc = 0; cc < 4; ++cc) fj[cc] = (j0 + cc < p.n) ? p.eB[p.col0 + j0 + cc] : 0;
+    switch (info->slices) {
+#define GB_CRT_CASE(NN) \
+    case NN: crt_rows<NN>(p, scale, j0, fj); break;
+        GB_CRT_CASE(2) GB_CRT_CASE(3) GB_CRT_CASE(4) GB_CRT_CASE(5) GB_CRT_CASE(6) GB_CRT_CASE(7)
+        GB_CRT_CASE(8) GB_CRT_CASE(9) GB_CRT_CASE(10) GB_CRT_CASE(11) GB_CRT_CASE(12) GB_CRT_CASE(13)
+        GB_CRT_CASE(14) GB_CRT_CASE(15)
+#undef GB_CRT_CASE
+        default: break;  // the plan gives 2 to 15 moduli
+    }
+}
+
+// Grid of the reconstruction: rows on y, as many blocks as are resident on every SM together.
+dim3 crt_combine_grid(int64_t m, int64_t n, int num_sms) {
+    const int64_t x = ((n + 3) / 4 + 127) / 128;
+    const int64_t y = std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(m, 65535), int64_t(num_sms) * kCombineBlocks / x));
+    return dim3(unsigned(x), unsigned(y));
+}
 
 __global__ void __launch_bounds__(128, 8) combine_kernel(const int32_t* __restrict__ levels, int nseg, int max_levels, int64_t mpad,
                                int64_t npad, int mode, const SplitInfo* __restrict__ info,
@@ -1662,6 +1766,17 @@ cudaError_t launch_convert(int64_t rows, int64_t cols, const S* src, int64_t ld_
 
 // ---- host orchestration ------------------------------------------------------------------------
 namespace {
+
+// The residue planes (crt_plane) as the 2-D arrays the epilogue's TMA stores address: 16-bit rows
+// (first modulus) and byte rows (the others).
+bool crt_plane_maps(CUtensorMap* t16, CUtensorMap* t8, const void* planes, int nseg, int max_levels, int64_t mpad,
+                    int64_t npad, std::string* err) {
+    const uint64_t rows = uint64_t(nseg) * uint64_t(max_levels + 1) * uint64_t(mpad);  // of npad bytes
+    return encode_tmap_2d(t16, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, planes, rows / 2, npad, npad, 32, 64,
+                          CU_TENSOR_MAP_SWIZZLE_128B, err) &&
+           encode_tmap_2d(t8, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, planes, rows, npad, npad, 32, 128,
+                          CU_TENSOR_MAP_SWIZZLE_128B, err);
+}
 
 int native_product(const Gemm& g, const LaunchCtl& ctl, cudaStream_t st, Workspace& ws, SplitResult* out,
                    std::string* err) {
@@ -2019,12 +2134,8 @@ int device_product(const Gemm& g_in, const SplitRequest& req, const LaunchCtl& c
                         CU_TENSOR_MAP_SWIZZLE_128B, err))
         return GB300_ERR_CUDA;
 
-    // residue planes as a 2-D array of 16-bit values for the epilogue's TMA stores
-    CUtensorMap tC = tA;
-    if (mode == kCrt &&
-        !encode_tmap_2d(&tC, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, lv, uint64_t(nseg) * max_levels * mpad, npad, npad, 32,
-                        64, CU_TENSOR_MAP_SWIZZLE_128B, err))
-        return GB300_ERR_CUDA;
+    CUtensorMap tC0 = tA, tC = tA;
+    if (mode == kCrt && !crt_plane_maps(&tC0, &tC, lv, nseg, max_levels, mpad, npad, err)) return GB300_ERR_CUDA;
 
     TcParams p;
     p.mode = mode;
@@ -2059,15 +2170,13 @@ int device_product(const Gemm& g_in, const SplitRequest& req, const LaunchCtl& c
         const int units = m_tiles * nt * nseg * max_levels;
         const int grid = 2 * std::max(1, std::min(units, sms / 2));
         KernelTimer timer("tc_gemm", st);
-        kern<<<grid, THREADS, kTcSmem, st>>>(tA, tB, tC, q);
+        kern<<<grid, THREADS, kTcSmem, st>>>(tA, tB, tC0, tC, q);
     };
     // reconstruction of C's columns [c0, c0 + nc) on stream s
     auto launch_crt_combine = [&](int64_t c0, int64_t nc, cudaStream_t s) {
-        const int64_t colgroups = (nc + CRT_COMBINE_COLS - 1) / CRT_COMBINE_COLS;
-        dim3 cgrid(unsigned((colgroups + 127) / 128), unsigned(std::min<int64_t>(m, 65535)));
-        crt_combine_kernel<CRT_COMBINE_COLS><<<cgrid, 128, 0, s>>>(
-            reinterpret_cast<const uint16_t*>(lv) + c0, nseg, max_levels, mpad, npad, info, eA, eB + c0, m, nc,
-            g.alpha, g.beta, static_cast<double*>(g.C) + c0, g.ldc);
+        const CrtCombine q{reinterpret_cast<const uint8_t*>(lv), mpad, npad, nseg, max_levels, c0, m, nc, eA, eB,
+                           g.alpha, g.beta, static_cast<double*>(g.C), g.ldc};
+        crt_combine_kernel<<<crt_combine_grid(m, nc, r.num_sms), 128, 0, s>>>(q, info);
     };
     const bool in_parts = mode == kCrt && n_tiles >= 2 && m_tiles * n_tiles >= sms && req.max_sms <= 0;
     if (in_parts) {
@@ -2335,16 +2444,14 @@ int device_product_host_panels(const Gemm& g, const SplitRequest& req, const Lau
     };
 
     // ---- tensor maps: A panel planes, the B planes, the level planes of a launch ----
-    CUtensorMap tA, tB, tC[2];
+    CUtensorMap tA, tB, tC0[2], tC[2];
     if (!encode_tmap_2d(&tA, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, pa, uint64_t(max_planes) * mpad, kpad, kpad, TM, TK,
                         CU_TENSOR_MAP_SWIZZLE_128B, err) ||
         !encode_tmap_2d(&tB, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, pb, uint64_t(max_planes) * npb, kpad, kpad, TNH, TK,
                         CU_TENSOR_MAP_SWIZZLE_128B, err))
         return GB300_ERR_CUDA;
     for (int b = 0; b < 2; ++b)
-        if (!encode_tmap_2d(&tC[b], CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, lv + b * lv_elems,
-                            uint64_t(nseg) * max_levels * mpad, npb, npb, 32, 64, CU_TENSOR_MAP_SWIZZLE_128B, err))
-            return GB300_ERR_CUDA;
+        if (!crt_plane_maps(&tC0[b], &tC[b], lv + b * lv_elems, nseg, max_levels, mpad, npb, err)) return GB300_ERR_CUDA;
     e = cudaFuncSetAttribute(tc_gemm_kernel<kCrt>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTcSmem));
     if (e != cudaSuccess) return cuda_fail("tc_gemm_kernel smem attribute", e);
 
@@ -2426,17 +2533,15 @@ int device_product_host_panels(const Gemm& g, const SplitRequest& req, const Lau
         const int grid = 2 * std::max(1, std::min(units, r.num_sms / 2));
         {
             KernelTimer timer("tc_gemm", st);
-            tc_gemm_kernel<kCrt><<<grid, THREADS, kTcSmem, st>>>(tA, tB, tC[buf], tp);
+            tc_gemm_kernel<kCrt><<<grid, THREADS, kTcSmem, st>>>(tA, tB, tC0[buf], tC[buf], tp);
         }
         cudaEventRecord(tc_done_ev(l), st);
         cudaStreamWaitEvent(aux, tc_done_ev(l), 0);
         for (int j = j0; j < j1; ++j) {
             const int64_t cj = int64_t(j) * Nq, nj = std::min(Nq, n - cj);
-            const int64_t colgroups = (nj + CRT_COMBINE_COLS - 1) / CRT_COMBINE_COLS;
-            crt_combine_kernel<CRT_COMBINE_COLS>
-                <<<dim3(unsigned((colgroups + 127) / 128), unsigned(std::min<int64_t>(mi, 65535))), 128, 0, aux>>>(
-                    reinterpret_cast<const uint16_t*>(lvb) + cj, nseg, max_levels, mpad, npb,
-                    info_at(P + Q + i * Q + j), eA + r0, eB + cj, mi, nj, g.alpha, g.beta, dC + r0 * n + cj, n);
+            const CrtCombine q{reinterpret_cast<const uint8_t*>(lvb), mpad, npb, nseg, max_levels, cj, mi, nj, eA + r0, eB,
+                               g.alpha, g.beta, dC + r0 * n, n};
+            crt_combine_kernel<<<crt_combine_grid(mi, nj, r.num_sms), 128, 0, aux>>>(q, info_at(P + Q + i * Q + j));
             if ((e = cudaGetLastError()) != cudaSuccess) return;
             cudaEventRecord(block_ev(i, j), aux);
             if (c_locked) copy_block_out(i, j);

@@ -1,8 +1,9 @@
 """The tensor-core epilogue's residues (residue2 in split_gemm.cu), evaluated exactly: for an FP32
 integer x, q = rint(x inv) with inv = 1 / p rounded to FP32 and r = x - p q.  Next to every half
 multiple of p, where the estimate comes closest to the wrong multiple, |r| <= (p + 1) / 2 for
-|x| <= 2^24 (a drain group's sum) and |r| <= p / 2 for |x| < 2^23 (a sum of residues), and what the
-epilogue stores, r + p, stays inside the range the reconstruction's reduction takes."""
+|x| <= 2^24 (a drain group's sum) and |r| <= p / 2 for |x| < 2^23 (a sum of residues).  The
+reconstruction gives back every integer of the plan's range from the bytes r + 128 that the epilogue
+stores."""
 import importlib.util
 import os
 import struct
@@ -46,13 +47,42 @@ def test_residue_magnitude(p, limit, slack):
     assert np.all(np.abs(p * ((x - r) // p)) < 1 << 25)  # p q is exact inside the multiply-add
 
 
+def _replay(t, residues, gen):
+    """The reconstruction of one output from its stored bytes r + 128 (crt_cols): x = b_p A + b_q B + K,
+    W - round(estimate) P modulo 2^(32 limbs)."""
+    from fractions import Fraction
+    f32 = np.float32
+    fq = f32(0)
+    W = 0
+    for s in t["sups"]:
+        x = residues[s["ia"]] * s["A"] + s["K"] + (residues[s["ib"]] * s["B"] if s["ib"] >= 0 else 0)
+        assert 0 <= x < 1 << 26
+        # x rounded to FP32, then one rounding of x finv + fq: a double holds the product's 48 bits, and
+        # the sum's error stays far below half an FP32 unit except at ties, which do not matter here
+        fq = f32(float(f32(x)) * float(f32(1.0 / s["Ps"])) + float(fq))
+        W += x * (t["P"] // s["Ps"])
+        assert all(x * ((t["P"] // s["Ps"] >> 32 * l) & 0xFFFFFFFF) < 1 << 58 for l in range(4))
+    assert 0 <= fq < 1 << 14
+    assert abs(Fraction(float(fq)) - Fraction(W, t["P"])) < Fraction(1, 100)  # the half integers are 0.029 away
+    q = int(round(Fraction(float(fq))))
+    mod = 1 << (32 * t["limbs"])
+    w = (W + q * t["negP"]) % mod
+    return w - mod if w >= mod // 2 else w
+
+
 @pytest.mark.parametrize("n", list(range(2, 16)))
-def test_stored_residues_reduce(n):
-    """x = c_p A + c_q B for the largest stored residues, and its 32-bit Barrett reduction."""
-    for s in _gen().table(n)["sups"]:
-        cp, cq = s["p"] + (s["p"] + 1) // 2, (s["q"] + (s["q"] + 1) // 2) if s["ib"] >= 0 else 0
-        x = cp * s["A"] + cq * s["B"]
-        assert x < 1 << 26
-        for v in (x, x - x % s["Ps"], x - x % s["Ps"] - 1):
-            u = v - ((v * s["Psinv32"]) >> 32) * s["Ps"]
-            assert 0 <= u < 2 * s["Ps"]
+def test_reconstruction_from_stored_bytes(n):
+    import random
+    gen = _gen()
+    t = gen.table(n)
+    lim = t["P"] * 1000 // 2125  # |T| < P / 2.125
+    rng = random.Random(n)
+    cases = [0, 1, -1, lim - 1, 1 - lim] + [rng.randrange(1 - lim, lim) for _ in range(400)]
+    for T in cases:
+        res = []
+        for p in gen.MODULI[:n]:
+            r = T % p
+            r = r - p if r > p // 2 else r  # symmetric
+            assert 0 <= r + 128 <= (256 if p == 257 else 255) or p == 256
+            res.append((r + 128) % 256 if p != 257 else r + 128)
+        assert _replay(t, res, gen) == T, (n, T)
