@@ -158,6 +158,10 @@ __device__ __forceinline__ void cp_async4(uint32_t dst, const void* src, bool va
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(valid ? 4 : 0)
                  : "memory");
 }
+// Sixteen bytes (dst and src 16-byte aligned), of which the first `bytes` are read and the others zero.
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 // Wait until at most N committed groups of this thread are still in flight.
 template <int N>

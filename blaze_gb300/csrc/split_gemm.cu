@@ -163,25 +163,31 @@ struct RowAcc {
     int pad;
 };
 
-// Operands stream through shared memory in tiles of 32 rows x 64 k, TILE_KT tiles per block, with
-// two buffers filled by cp.async: the copies of the next tile are in flight while the current one
-// is processed.
-constexpr int TILE_KT = 8;
+// Operands stream through shared memory in tiles of 32 rows x 64 k, a few tiles per block
+// (tiles_per_block), with two buffers filled by cp.async: the copies of the next tile are in flight
+// while the current one is processed.
+constexpr int TILE_KT = 8;  // at most
 
-// The eight copies of one thread per tile: element (rr0 + i drr, pp0 + i dpp) of the tile,
-// i = 0..7, coalesced along whichever index of X(r, p) = X[r*sr + p*sp] is contiguous (a warp
-// reads 256 consecutive bytes); src points at the first one in tile 0, di and dk step to copy i
-// and to the next tile of 64 k.
+// The copies of one thread per tile, coalesced along whichever index of X(r, p) = X[r*sr + p*sp] is
+// contiguous: eight elements (rr0 + i drr, pp0 + i dpp), a warp reading 256 consecutive bytes, or,
+// where every row is contiguous and 16-byte aligned (vec), four pairs of elements, a warp reading
+// 512.  src points at the first one in tile 0, di and dk step to copy i and to the next tile of 64 k.
 struct TileSrc {
     const unsigned long long* src;
     int64_t di, dk;
     int rr0, pp0, drr, dpp;
+    bool vec;
 };
 
 __device__ __forceinline__ TileSrc tile_src(const double* X, int64_t sr, int64_t sp, int64_t r0) {
     const int t = threadIdx.x;  // 256 threads
     TileSrc s;
-    if (sp == 1) {
+    s.vec = sp == 1 && (sr & 1) == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0;
+    if (s.vec) {
+        s.rr0 = t >> 5; s.drr = 8; s.pp0 = 2 * (t & 31); s.dpp = 0;
+        s.di = 8 * sr;
+        s.dk = 64;
+    } else if (sp == 1) {
         s.rr0 = t >> 6; s.drr = 4; s.pp0 = t & 63; s.dpp = 0;
         s.di = 4 * sr;
         s.dk = 64;
@@ -195,16 +201,29 @@ __device__ __forceinline__ TileSrc tile_src(const double* X, int64_t sr, int64_t
 }
 
 // Issue the copies of tile `it` (k from 64 it) into the buffer at shared address sbuf, where
-// off(rr, pp) places element (rr, pp); zeros outside R x K; one commit group per tile.
+// off(rr, pp) places element (rr, pp), an even pp and the next one side by side; zeros outside R x K;
+// one commit group per tile.
 template <typename Off>
 __device__ __forceinline__ void tile_issue(uint32_t sbuf, const TileSrc& s, const double* X, int64_t R, int64_t K,
                                            int64_t r0, int64_t it, Off off) {
     const unsigned long long* src = s.src + it * s.dk;
+    const bool full = r0 + 32 <= R && it * 64 + 64 <= K;  // the whole tile lies inside the matrix
+    if (s.vec) {
+        const int64_t left = K - it * 64 - s.pp0;
+        const int bytes = full || left >= 2 ? 16 : left == 1 ? 8 : 0;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int rr = s.rr0 + i * s.drr, pp = s.pp0 + i * s.dpp;
-        const bool ok = r0 + rr < R && it * 64 + pp < K;
-        cp_async8(sbuf + off(rr, pp), ok ? src + i * s.di : reinterpret_cast<const unsigned long long*>(X), ok);
+        for (int i = 0; i < 4; ++i) {
+            const int rr = s.rr0 + i * s.drr;
+            const int n = full || r0 + rr < R ? bytes : 0;
+            cp_async16(sbuf + off(rr, s.pp0), n ? src + i * s.di : reinterpret_cast<const unsigned long long*>(X), n);
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int rr = s.rr0 + i * s.drr, pp = s.pp0 + i * s.dpp;
+            const bool ok = full || (r0 + rr < R && it * 64 + pp < K);
+            cp_async8(sbuf + off(rr, pp), ok ? src + i * s.di : reinterpret_cast<const unsigned long long*>(X), ok);
+        }
     }
     cp_async_commit();
 }
@@ -212,29 +231,31 @@ __device__ __forceinline__ void tile_issue(uint32_t sbuf, const TileSrc& s, cons
 // 2^x in FP32 for x <= 127, 0 below the normal range.
 __device__ __forceinline__ float pow2f_or0(int x) { return x < -126 ? 0.f : __uint_as_float(uint32_t(x + 127) << 23); }
 
-// Row statistics over TILE_KT tiles: thread (rr = t % 32, g = t / 32) keeps, for row rr and the
+// Row statistics over kt tiles: thread (rr = t % 32, g = t / 32) keeps, for row rr and the
 // eight k of group g in every tile, the largest high word of |x|, the OR of the low words and the
 // sum of squares in FP32 relative to its running largest exponent `base`: f = |x| 2^(1023 - base)
 // is the high word times 8 (exponent and 20 mantissa bits moved into FP32 position) minus
-// (base - 127) 2^23, one integer multiply-add, valid for exponents above base - 127 (smaller
-// values add less than 2^-252 relative and are dropped; zeros and subnormals always are).  The
-// running sum is rescaled exactly by a power of two when a larger exponent arrives.  The block
-// folds the eight groups of a row and issues one set of atomics per row; an Inf/NaN shows as a
-// largest exponent of 0x7ff.
+// (base - 127) 2^23, one integer multiply-add, valid for exponents above base - 127.  High words below
+// that are raised to its lowest value, whose square is zero in FP32.  `base` moves once per tile, to
+// the exponent of the largest high word so far, and the running sum is rescaled exactly by a power of
+// two.  Bound by the integer ALU: these four ALU operations an element, the maximum and the OR taken
+// two elements at a time; with `base` checked at every element it was seven (1 GiB of operands: 215 us, now 169, 6.4 TB/s).
+// The block folds the eight groups of a row and issues one set of atomics per row; an Inf/NaN shows as
+// a largest exponent of 0x7ff.
 __device__ __forceinline__ void stats_rows(const double* __restrict__ X, int64_t R, int64_t K, int64_t sr, int64_t sp,
-                                           RowAcc* __restrict__ acc, int by) {
-    __shared__ __align__(16) unsigned long long tile[2][32][65];
+                                           RowAcc* __restrict__ acc, int by, int kt) {
+    constexpr uint32_t ROWB = 528, BUF = 32 * ROWB;  // rows 33 chunks of 16 bytes apart: no bank conflicts
+    __shared__ __align__(16) unsigned char tbuf[2 * BUF];
     __shared__ uint32_t red_mx[8][32], red_lo[8][32];
     __shared__ int red_base[8][32];
     __shared__ float red_sq[8][32];
     const int t = threadIdx.x, rr = t & 31, g = t >> 5;
     const int64_t r0 = int64_t(by) * 32;
     const int64_t ntiles = (K + 63) / 64;
-    const int64_t tb = int64_t(blockIdx.x) * TILE_KT, te = min(ntiles, tb + TILE_KT);
-    const uint32_t s0 = smem_u32(&tile[0][0][0]);
-    constexpr uint32_t BUF = 32 * 65 * 8;
-    auto off = [](int r_, int p_) { return uint32_t(r_ * 65 + p_) * 8u; };
-    uint32_t mx = 0, lo = 0, cbias = 0;
+    const int64_t tb = int64_t(blockIdx.x) * kt, te = min(ntiles, tb + kt);
+    const uint32_t s0 = smem_u32(tbuf);
+    auto off = [](int r_, int p_) { return uint32_t(r_) * ROWB + uint32_t(p_) * 8u; };
+    uint32_t mx = 0, lo = 0;
     int base = 127;  // f = |x| 2^(1023 - base); values with exponent field 0 never count
     float sq = 0.f;
     const TileSrc ts = tile_src(X, sr, sp, r0);
@@ -245,19 +266,25 @@ __device__ __forceinline__ void stats_rows(const double* __restrict__ X, int64_t
         else cp_async_commit();  // an empty group keeps the wait count uniform
         cp_async_wait1();
         __syncthreads();
+        uint32_t hi[8];
+        const unsigned char* row = tbuf + b * BUF + rr * ROWB + g * 64;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint4 v = *reinterpret_cast<const uint4*>(row + 16 * q);
+            hi[2 * q] = v.y & 0x7fffffffu;
+            hi[2 * q + 1] = v.w & 0x7fffffffu;
+            lo |= v.x | v.z;
+            mx = max(mx, max(hi[2 * q], hi[2 * q + 1]));
+        }
+        const int top = int(mx >> 20);
+        if (top > base) {
+            sq *= pow2f_or0(2 * (base - top));
+            base = top;
+        }
+        const uint32_t cbias = uint32_t(base - 127) << 23, least = uint32_t(base - 126) << 20;
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-            const unsigned long long a = tile[b][rr][8 * g + q];
-            const uint32_t hi = uint32_t(a >> 32) & 0x7fffffffu;
-            lo |= uint32_t(a);
-            mx = max(mx, hi);
-            const int ea = int(hi >> 20);
-            if (ea > base) {
-                sq *= pow2f_or0(2 * (base - ea));
-                base = ea;
-                cbias = uint32_t(base - 127) << 23;
-            }
-            const float f = ea > base - 127 ? __uint_as_float(hi * 8u - cbias) : 0.f;
+            const float f = __uint_as_float(max(hi[q], least) * 8u - cbias);
             sq = fmaf(f, f, sq);
         }
         __syncthreads();
@@ -339,10 +366,10 @@ struct OperandPair {
     unsigned yb0;  // row blocks of A
 };
 
-__global__ void __launch_bounds__(256, 4) stats_tile_kernel(const OperandPair op, int64_t K) {
+__global__ void __launch_bounds__(256, 4) stats_tile_kernel(const OperandPair op, int64_t K, int kt) {
     const int w = blockIdx.y < op.yb0 ? 0 : 1;
     const int by = w ? int(blockIdx.y - op.yb0) : int(blockIdx.y);
-    stats_rows(op.X[w], op.R[w], K, op.sr[w], op.sp[w], op.acc[w], by);
+    stats_rows(op.X[w], op.R[w], K, op.sr[w], op.sp[w], op.acc[w], by, kt);
 }
 
 // Per-block summary of the row statistics of one operand side, for split_info_kernel: Inf/NaN
@@ -832,41 +859,58 @@ __device__ __forceinline__ uint32_t mod_small(uint32_t x, uint32_t p, uint32_t i
 
 // Planes of eight consecutive elements xv of one row (row exponent e, bad: the row holds Inf/NaN)
 // at dst, plane stride pstride; sl = slices (digits) or moduli (CRT), bt = beta (CRT).
+// A modulus' constants as packed pairs (k_3, k_2, k_1 = symmetric residues of 2^42, 2^28, 2^14;
+// fl(1/p); -p), in shared memory: three 16-byte reads a modulus serve eight elements, and the packed
+// arithmetic takes half the instructions that bound this pass (8192^3 at 12 moduli 750 -> 725 us, 5.9 TB/s; 403 x 517 x 389
+// 20 -> 7.6 us with the smaller blocks of tiles_per_block).
+struct __align__(16) SliceConst {
+    ulonglong2 k32, k1_inv, pneg;
+};
+
 template <int mode>
 __device__ __forceinline__ void slice_emit(const unsigned long long (&xv)[8], int sl, int bt, int e, bool bad,
-                                           uint16_t* __restrict__ dst, int64_t pstride) {
+                                           const SliceConst* tab, uint16_t* __restrict__ dst, int64_t pstride) {
     if (mode == kCrt) {
         const int N = sl, beta = bt;
-        // U = |round(a 2^(beta-e))| < 2^56 in signed FP32 chunks (the sign of a applied to each)
-        float w0[8], w1[8], w2[8], w3[8];
+        // U = |round(a 2^(beta-e))| < 2^56 in signed FP32 chunks (the sign of a applied to each), two
+        // elements to a packed pair
+        uint64_t w0[4], w1[4], w2[4], w3[4];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const unsigned long long bits = bad ? 0ull : xv[q];
-            const unsigned long long U = int_magnitude(bits, beta - e);
-            const float sg = (bits >> 63) ? -1.f : 1.f, off = (bits >> 63) ? 8388608.f : -8388608.f;
-            w0[q] = fmaf(__uint_as_float(0x4B000000u | (uint32_t(U) & 0x3fffu)), sg, off);
-            w1[q] = fmaf(__uint_as_float(0x4B000000u | (uint32_t(U >> 14) & 0x3fffu)), sg, off);
-            w2[q] = fmaf(__uint_as_float(0x4B000000u | (uint32_t(U >> 28) & 0x3fffu)), sg, off);
-            w3[q] = fmaf(__uint_as_float(0x4B000000u | uint32_t(U >> 42)), sg, off);
+        for (int q = 0; q < 4; ++q) {
+            uint32_t c[4][2];
+            float sg[2], off[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const unsigned long long bits = bad ? 0ull : xv[2 * q + h];
+                const unsigned long long U = int_magnitude(bits, beta - e);
+                sg[h] = (bits >> 63) ? -1.f : 1.f;
+                off[h] = (bits >> 63) ? 8388608.f : -8388608.f;
+                c[0][h] = 0x4B000000u | (uint32_t(U) & 0x3fffu);
+                c[1][h] = 0x4B000000u | (uint32_t(U >> 14) & 0x3fffu);
+                c[2][h] = 0x4B000000u | (uint32_t(U >> 28) & 0x3fffu);
+                c[3][h] = 0x4B000000u | uint32_t(U >> 42);
+            }
+            const uint64_t sg2 = f32x2(sg[0], sg[1]), off2 = f32x2(off[0], off[1]);
+            w0[q] = fma2(f32x2_bits(c[0][0], c[0][1]), sg2, off2);
+            w1[q] = fma2(f32x2_bits(c[1][0], c[1][1]), sg2, off2);
+            w2[q] = fma2(f32x2_bits(c[2][0], c[2][1]), sg2, off2);
+            w3[q] = fma2(f32x2_bits(c[3][0], c[3][1]), sg2, off2);
         }
+        const uint64_t magic = f32x2(MAGIC, MAGIC), nmagic = f32x2(-MAGIC, -MAGIC);
         for (int t = 0; t < N; ++t) {
-            const float pf = c_modf[t], inv = c_modf_inv[t];
-            const float k1 = c_mod_k14[0][t], k2 = c_mod_k14[1][t], k3 = c_mod_k14[2][t];
-            uint32_t fb[8];
+            const ulonglong2 k32 = tab[t].k32, k1i = tab[t].k1_inv;
+            const uint64_t pneg = tab[t].pneg.x;
+            uint32_t d[4];
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                const float x = fmaf(w3[q], k3, fmaf(w2[q], k2, fmaf(w1[q], k1, w0[q])));
-                const float qf = fmaf(x, inv, MAGIC) - MAGIC;
+            for (int q = 0; q < 4; ++q) {
+                const uint64_t x = fma2(w3[q], k32.x, fma2(w2[q], k32.y, fma2(w1[q], k1i.x, w0[q])));
+                const uint64_t qf = add2(fma2(x, k1i.y, magic), nmagic);
                 // exact symmetric residue, an integer of at most 8 significant bits: its FP32
                 // pattern's upper half is the BF16 pattern
-                fb[q] = __float_as_uint(fmaf(-pf, qf, x));
+                const uint64_t f = fma2(pneg, qf, x);
+                d[q] = __byte_perm(uint32_t(f), uint32_t(f >> 32), 0x7632);
             }
-            uint4 w;
-            w.x = __byte_perm(fb[0], fb[1], 0x7632);
-            w.y = __byte_perm(fb[2], fb[3], 0x7632);
-            w.z = __byte_perm(fb[4], fb[5], 0x7632);
-            w.w = __byte_perm(fb[6], fb[7], 0x7632);
-            *reinterpret_cast<uint4*>(dst + t * pstride) = w;
+            *reinterpret_cast<uint4*>(dst + t * pstride) = make_uint4(d[0], d[1], d[2], d[3]);
         }
     } else if (mode == kExact) {
         const int S = sl;
@@ -897,20 +941,28 @@ __device__ __forceinline__ void slice_emit(const unsigned long long (&xv)[8], in
     }
 }
 
-// Planes of 32 rows over TILE_KT k-tiles.  Thread (rr = t / 8, L = t % 8) handles elements
+// Planes of 32 rows over kt k-tiles.  Thread (rr = t / 8, L = t % 8) handles elements
 // 8L..8L+7 of row rr and writes 16 bytes per plane (a warp: four 128-byte row segments).  The tile
 // buffer keeps rows of 528 bytes with 16-byte chunk c of a row stored at c ^ (c >> 3), so that the
 // eight threads of a row read their chunks 4L + j from eight different bank groups.
 template <int mode>
 __device__ __forceinline__ void slice_rows(int which, const double* __restrict__ X, int64_t R, int64_t K, int64_t sr,
                                            int64_t sp, const int* __restrict__ rexp, const SplitInfo* __restrict__ info,
-                                           __nv_bfloat16* __restrict__ planes, int64_t rpad, int64_t kpad, int by) {
+                                           __nv_bfloat16* __restrict__ planes, int64_t rpad, int64_t kpad, int by,
+                                           int kt) {
     constexpr uint32_t ROWB = 528, BUF = 32 * ROWB;
     __shared__ __align__(16) unsigned char tbuf[2 * BUF];
+    __shared__ SliceConst tab[mode == kCrt ? MAX_MODULI : 1];
     const int t = threadIdx.x, rr = t >> 3, L = t & 7;
+    if (mode == kCrt && t < MAX_MODULI) {  // visible after the first tile's barrier
+        auto two = [](float v) { return f32x2(v, v); };
+        tab[t].k32 = make_ulonglong2(two(c_mod_k14[2][t]), two(c_mod_k14[1][t]));
+        tab[t].k1_inv = make_ulonglong2(two(c_mod_k14[0][t]), two(c_modf_inv[t]));
+        tab[t].pneg = make_ulonglong2(two(-c_modf[t]), 0ull);
+    }
     const int64_t r0 = int64_t(by) * 32, r = r0 + rr;
     const int64_t ntiles = kpad / 64;
-    const int64_t tb = int64_t(blockIdx.x) * TILE_KT, te = min(ntiles, tb + TILE_KT);
+    const int64_t tb = int64_t(blockIdx.x) * kt, te = min(ntiles, tb + kt);
     const uint32_t s0 = smem_u32(tbuf);
     auto off = [](int r_, int p_) {
         const uint32_t c = uint32_t(p_) >> 1;
@@ -938,7 +990,7 @@ __device__ __forceinline__ void slice_rows(int which, const double* __restrict__
             xv[2 * j + 1] = (unsigned long long)v.z | ((unsigned long long)v.w << 32);
         }
         if (r < rpad)
-            slice_emit<mode>(xv, sl, bt, e, bad, reinterpret_cast<uint16_t*>(planes) + r * kpad + it * 64 + 8 * L,
+            slice_emit<mode>(xv, sl, bt, e, bad, tab, reinterpret_cast<uint16_t*>(planes) + r * kpad + it * 64 + 8 * L,
                              pstride);
         __syncthreads();
     }
@@ -946,10 +998,10 @@ __device__ __forceinline__ void slice_rows(int which, const double* __restrict__
 
 template <int MODE>
 __global__ void __launch_bounds__(256, 3) slice_kernel(const OperandPair op, int64_t K, const SplitInfo* __restrict__ info,
-                                                       int64_t kpad) {
+                                                       int64_t kpad, int kt) {
     const int w = blockIdx.y < op.yb0 ? 0 : 1;
     const int by = w ? int(blockIdx.y - op.yb0) : int(blockIdx.y);
-    slice_rows<MODE>(w, op.X[w], op.R[w], K, op.sr[w], op.sp[w], op.rexp[w], info, op.planes[w], op.rpad[w], kpad, by);
+    slice_rows<MODE>(w, op.X[w], op.R[w], K, op.sr[w], op.sp[w], op.rexp[w], info, op.planes[w], op.rpad[w], kpad, by, kt);
 }
 
 // ---- level / pair schedule ---------------------------------------------------------------------
@@ -1767,6 +1819,12 @@ cudaError_t launch_convert(int64_t rows, int64_t cols, const S* src, int64_t ld_
 // ---- host orchestration ------------------------------------------------------------------------
 namespace {
 
+// k-tiles per block of the pre-pass kernels: TILE_KT, or fewer where that would leave an SM without
+// several blocks (1024^3: 128 blocks of eight tiles took 9 us for the statistics and 23 for slicing, smaller ones 7 and 16).
+int tiles_per_block(int64_t tiles, int64_t row_blocks, int num_sms) {
+    return int(std::max<int64_t>(1, std::min<int64_t>(TILE_KT, tiles * row_blocks / (int64_t(num_sms) * 6))));
+}
+
 // The residue planes (crt_plane) as the 2-D arrays the epilogue's TMA stores address: 16-bit rows
 // (first modulus) and byte rows (the others).
 bool crt_plane_maps(CUtensorMap* t16, CUtensorMap* t8, const void* planes, int nseg, int max_levels, int64_t mpad,
@@ -2102,8 +2160,9 @@ int device_product(const Gemm& g_in, const SplitRequest& req, const LaunchCtl& c
     op.rpad[0] = mpad; op.rpad[1] = npad;
     op.yb0 = unsigned((m + 31) / 32);
     {
-        dim3 grid(unsigned(((k + 63) / 64 + TILE_KT - 1) / TILE_KT), unsigned((m + 31) / 32 + (n + 31) / 32));
-        stats_tile_kernel<<<grid, 256, 0, st>>>(op, k);
+        const int64_t yb = (m + 31) / 32 + (n + 31) / 32, tiles = (k + 63) / 64;
+        const int kt = tiles_per_block(tiles, yb, r.num_sms);
+        stats_tile_kernel<<<dim3(unsigned((tiles + kt - 1) / kt), unsigned(yb)), 256, 0, st>>>(op, k, kt);
         stats_finalize_pair_kernel<<<xb0 + xb1, 256, 0, st>>>(op, k, xb0, part);
     }
     const double target = req.target_error > 0 ? req.target_error : double(k) * 0x1p-53;
@@ -2116,10 +2175,12 @@ int device_product(const Gemm& g_in, const SplitRequest& req, const LaunchCtl& c
     {
         OperandPair sp2 = op;
         sp2.yb0 = unsigned(mpad / 32);
-        dim3 grid(unsigned((kpad / 64 + TILE_KT - 1) / TILE_KT), unsigned(mpad / 32 + npad / 32));
+        const int64_t yb = mpad / 32 + npad / 32, tiles = kpad / 64;
+        const int kt = tiles_per_block(tiles, yb, r.num_sms);
+        const dim3 grid(unsigned((tiles + kt - 1) / kt), unsigned(yb));
         auto sk = mode == kCrt ? slice_kernel<kCrt>
                                : (mode == kExact ? slice_kernel<kExact> : (mode == kBf16 ? slice_kernel<kBf16> : slice_kernel<kBf16x3>));
-        sk<<<grid, 256, 0, st>>>(sp2, k, info, kpad);
+        sk<<<grid, 256, 0, st>>>(sp2, k, info, kpad, kt);
     }
     count_launches(4);
     if (cudaError_t le = cudaGetLastError(); le != cudaSuccess) {
@@ -2391,8 +2452,17 @@ int device_product_host_panels(const Gemm& g, const SplitRequest& req, const Lau
         cudaEventRecord(ev[P + j], r.copy_in);
     };
     cudaMemsetAsync(racc, 0, size_t(m + n) * sizeof(RowAcc), st);
-    const unsigned ktiles = unsigned(((k + 63) / 64 + TILE_KT - 1) / TILE_KT);
-    const unsigned stiles = unsigned((kpad / 64 + TILE_KT - 1) / TILE_KT);
+    // the pre-pass launches over a panel or a column block
+    auto run_stats = [&](const OperandPair& o, int64_t yb) {
+        const int64_t tiles = (k + 63) / 64;
+        const int kt = tiles_per_block(tiles, yb, r.num_sms);
+        stats_tile_kernel<<<dim3(unsigned((tiles + kt - 1) / kt), unsigned(yb)), 256, 0, st>>>(o, k, kt);
+    };
+    auto run_slice = [&](const OperandPair& o, int64_t yb, const SplitInfo* info) {
+        const int64_t tiles = kpad / 64;
+        const int kt = tiles_per_block(tiles, yb, r.num_sms);
+        slice_kernel<kCrt><<<dim3(unsigned((tiles + kt - 1) / kt), unsigned(yb)), 256, 0, st>>>(o, k, info, kpad, kt);
+    };
     const int64_t a_sr = g.ta ? 1 : a_cols, a_sp = g.ta ? a_cols : 1;
     const int64_t b_sr = g.tb ? b_cols : 1, b_sp = g.tb ? 1 : b_cols;
     OperandPair base;
@@ -2416,12 +2486,12 @@ int device_product_host_panels(const Gemm& g, const SplitRequest& req, const Lau
         o.rexp[0] = eA + r0;
         o.rsq[0] = sqA + r0;
         o.yb0 = unsigned((mi + 31) / 32);
-        stats_tile_kernel<<<dim3(ktiles, o.yb0), 256, 0, st>>>(o, k);
+        run_stats(o, o.yb0);
         const unsigned xb0 = unsigned((mi + 255) / 256);
         stats_finalize_pair_kernel<<<xb0, 256, 0, st>>>(o, k, xb0, nullptr);
         split_side_kernel<<<1, 1024, 0, st>>>(eA + r0, sqA + r0, mi, k, max_planes, target, info_at(i));
         o.yb0 = unsigned(mpad / 32);
-        slice_kernel<kCrt><<<dim3(stiles, o.yb0), 256, 0, st>>>(o, k, info_at(i), kpad);
+        run_slice(o, o.yb0, info_at(i));
         count_launches(4);
     };
     // statistics, side scaling and planes of B's column block j (rows j*Nq.. of the B planes)
@@ -2436,10 +2506,10 @@ int device_product_host_panels(const Gemm& g, const SplitRequest& req, const Lau
         o.planes[1] = pb + size_t(j) * size_t(Nq) * size_t(kpad);
         o.rpad[1] = npb;
         o.yb0 = 0;
-        stats_tile_kernel<<<dim3(ktiles, unsigned((nj + 31) / 32)), 256, 0, st>>>(o, k);
+        run_stats(o, (nj + 31) / 32);
         stats_finalize_pair_kernel<<<unsigned((nj + 255) / 256), 256, 0, st>>>(o, k, 0u, nullptr);
         split_side_kernel<<<1, 1024, 0, st>>>(eB + c0, sqB + c0, nj, k, max_planes, target, info_at(P + j));
-        slice_kernel<kCrt><<<dim3(stiles, unsigned(Nq / 32)), 256, 0, st>>>(o, k, info_at(P + j), kpad);
+        run_slice(o, Nq / 32, info_at(P + j));
         count_launches(4);
     };
 
