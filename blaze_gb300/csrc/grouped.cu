@@ -9,15 +9,12 @@
 //
 // Design:
 //   * Every product is brought to the row-major form (as for the single products) and tiled with
-//     the warp-tile shape chosen for its (m, n, k) class.  Warp tile = (8*R) x (4*C) outputs, lane
-//     (ly, lx) of an 8 x 4 lane grid owning rows ly + 8r and columns lx + 4c, so a warp's B loads
-//     are coalesced runs and its A loads are 8 broadcast rows.
+//     the warp-tile shape chosen for its (m, n, k) class: FP32 warp tiles of (8*R) x (4*C) outputs, FP64
+//     tiles of at most that many, taken as flat lists of outputs (warp_tile_flat).
 //   * One flat tile list, sorted by descending work (longest first), is consumed by persistent
 //     warps through a global atomic counter (warp-granular work stealing): uneven products
 //     balance across SMs without a per-product launch.
-//   * Operands are read through L1 (__ldg): a small product's panels stay cache-resident across the
-//     k loop, and on this chip the FP64 pipe (about 2 DFMA/clock/SM) — not the load path — bounds
-//     the FP64 form, so the tile shapes exist to avoid multiply-adds on padding.
+//   * Operands are staged in the warp's own shared memory, so a warp waits for no other.
 //   * The launch (counter reset + kernel) is captured once into a CUDA graph owned by the plan;
 //     running the plan is one graph launch.
 #include <cuda_runtime.h>
@@ -33,6 +30,7 @@
 #include <vector>
 
 #include "../../include/gb300_blas.h"
+#include "ptx.cuh"
 #include "runtime.h"
 
 namespace gb {
@@ -55,6 +53,7 @@ struct DevProblem {
     int m, n, k;
     int ta, tb;
     int shape;
+    int tr, tc;  // rows and columns of its tiles (the last ones of a row or column may be smaller)
     double alpha, beta;
 };
 
@@ -64,64 +63,121 @@ struct DevTile {
     int pad;
 };
 
-template <typename T, int R, int C>
-__device__ __forceinline__ void warp_tile(const DevProblem& p, int tm, int tn, int lane) {
-    const int ly = lane >> 2, lx = lane & 3;
-    const int row0 = tm * (8 * R) + ly;
-    const int col0 = tn * (4 * C) + lx;
-    // A(i, kk) = A[i*a_rs + kk*a_ks], B(kk, j) = B[kk*b_ks + j*b_cs]; one running pointer per operand
-    const int64_t a_rs = p.ta ? 1 : p.lda, a_ks = p.ta ? p.lda : 1;
-    const int64_t b_cs = p.tb ? p.ldb : 1, b_ks = p.tb ? 1 : p.ldb;
-    const int64_t a8 = 8 * a_rs, b4 = 4 * b_cs;
-    const T* pa = static_cast<const T*>(p.A) + int64_t(row0) * a_rs;
-    const T* pb = static_cast<const T*>(p.B) + int64_t(col0) * b_cs;
-    uint32_t rmask = 0, cmask = 0;
-#pragma unroll
-    for (int r = 0; r < R; ++r) rmask |= (row0 + 8 * r < p.m) ? (1u << r) : 0u;
-#pragma unroll
-    for (int c = 0; c < C; ++c) cmask |= (col0 + 4 * c < p.n) ? (1u << c) : 0u;
-    T acc[R][C];
-#pragma unroll
-    for (int r = 0; r < R; ++r)
-#pragma unroll
-        for (int c = 0; c < C; ++c) acc[r][c] = T(0);
-    auto step = [&]() {
-        T a0[R], b0[C];
-#pragma unroll
-        for (int r = 0; r < R; ++r) a0[r] = (rmask >> r) & 1u ? __ldg(pa + r * a8) : T(0);
-#pragma unroll
-        for (int c = 0; c < C; ++c) b0[c] = (cmask >> c) & 1u ? __ldg(pb + c * b4) : T(0);
-#pragma unroll
-        for (int r = 0; r < R; ++r)
-#pragma unroll
-            for (int c = 0; c < C; ++c) acc[r][c] = fma(a0[r], b0[c], acc[r][c]);
-        pa += a_ks;
-        pb += b_ks;
-    };
-    // FP64: unrolled so that the loads of the next k step issue before this step's multiply-adds
-    // retire; FP32: not unrolled, which keeps every shape within the 128 registers that let an SM
-    // hold two blocks (latency is hidden by warps instead).  The accumulation order of every output
-    // stays k = 0, 1, 2, ... either way.
-    if constexpr (sizeof(T) == 8) {
+// FP64 warp tiles.  On this chip a multiply-add of a warp holds its SM quarter's FP64 pipe for 64
+// clocks, so what a tile costs is the number of its multiply-add instructions, and loads are free.  A
+// warp therefore takes its tile's outputs as one flat list, 32 at a time, whatever the tile's rows and
+// columns are: output o of lane l in round u is o = l + 32 u, row o / cols, column o % cols, each lane
+// reading its own A and B value from the warp's staged chunk for every multiply-add.  A product is
+// split into tiles of equal parts (tr x tc, within the shape's rows and columns), which leaves at most
+// 31 idle outputs a tile: 1.03 times the useful work on 10,000 products of 4 to 256 rows, columns and
+// steps, against 1.22 with tiles of fixed 8 R x 4 C outputs (4.58 ms, now 3.77, 0.94 of the FP64
+// peak).  The operands come in by
+// cp.async, DKC k-steps ahead of the ones being used.  Every output sums k in order.
+constexpr int DKC = 16;
+constexpr int DPA = DKC + 1;                        // A row pitch (doubles): rows 2 banks apart
+constexpr int kDStage = 32 * DPA + DKC * 17;       // doubles per buffer: 32 x 16 tiles need most, then 16 x 32
+static_assert(kDStage >= 16 * DPA + DKC * 33, "16 x 32 tiles");
+constexpr int kDStageBytes = 8 * 2 * kDStage * int(sizeof(double));  // per 256-thread block
+
+// kc k-steps of the first U rounds.  U is a template argument so that no multiply-add is issued for the
+// rounds a tile does not have: one that is predicated off for the whole warp holds the FP64 pipe as
+// long as any other (4.75 ms against 3.93 before the epilogue was split as well).
+template <int U, int UMAX>
+__device__ __forceinline__ void flat_steps(const double* __restrict__ buf, int kc, int pb, const int (&ao)[UMAX],
+                                           const int (&bo)[UMAX], double (&acc)[UMAX]) {
 #pragma unroll 2
-        for (int kk = 0; kk < p.k; ++kk) step();
-    } else {
-#pragma unroll 1
-        for (int kk = 0; kk < p.k; ++kk) step();
+    for (int kk = 0; kk < kc; ++kk) {
+        const double* a = buf + kk;
+        const double* c = buf + kk * pb;
+#pragma unroll
+        for (int u = 0; u < U; ++u) acc[u] = fma(a[ao[u]], c[bo[u]], acc[u]);
     }
-    T* Cp = static_cast<T*>(p.C);
-    const T alpha = T(p.alpha), beta = T(p.beta);
+}
+
+// The flat tile of `rows` x `cols` outputs at (i0, j0), UMAX rounds at most.
+constexpr int UMAX = 16;
+__device__ __forceinline__ void warp_tile_flat(const DevProblem& p, int i0, int j0, int rows, int cols, int lane,
+                                               double* __restrict__ sw) {
+    const int outs = rows * cols, U = (outs + 31) >> 5;
+    const int pb = cols | 1, bbase = rows * DPA;  // B row pitch, and where B's chunk begins
+    const double* A = static_cast<const double*>(p.A) + (p.ta ? int64_t(i0) : int64_t(i0) * p.lda);
+    const double* B = static_cast<const double*>(p.B) + (p.tb ? int64_t(j0) * p.ldb : int64_t(j0));
+    double acc[UMAX];
+    int ao[UMAX], bo[UMAX];
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-        if (!((rmask >> r) & 1u)) continue;
-        T* crow = Cp + int64_t(row0 + 8 * r) * p.ldc;
-#pragma unroll
-        for (int c = 0; c < C; ++c) {
-            if (!((cmask >> c) & 1u)) continue;
-            const int j = col0 + 4 * c;
-            const T v = alpha * acc[r][c];
-            crow[j] = (beta == T(0)) ? v : fma(beta, crow[j], v);
+    for (int u = 0; u < UMAX; ++u) {
+        const int o = min(lane + 32 * u, outs - 1);
+        const int i = o / cols;
+        ao[u] = i * DPA;
+        bo[u] = bbase + o - i * cols;
+        acc[u] = 0.0;
+    }
+    // k-steps k0 .. k0 + kc - 1 of the tile's rows of A and columns of B into a buffer
+    auto stage = [&](double* buf, int k0) {
+        const int kc = min(DKC, p.k - k0);
+        const uint32_t sa = smem_u32(buf), sb = smem_u32(buf + bbase);
+        if (!p.ta) {
+            const int kk = lane & (DKC - 1);
+            if (kk < kc)
+                for (int i = lane / DKC; i < rows; i += 32 / DKC)
+                    cp_async8(sa + uint32_t(i * DPA + kk) * 8u, A + int64_t(i) * p.lda + k0 + kk, true);
+        } else {
+            for (int e = lane; e < rows * kc; e += 32) {
+                const int kk = e / rows, i = e - kk * rows;
+                cp_async8(sa + uint32_t(i * DPA + kk) * 8u, A + int64_t(k0 + kk) * p.lda + i, true);
+            }
         }
+        if (!p.tb) {
+            for (int e = lane; e < cols * kc; e += 32) {
+                const int kk = e / cols, j = e - kk * cols;
+                cp_async8(sb + uint32_t(kk * pb + j) * 8u, B + int64_t(k0 + kk) * p.ldb + j, true);
+            }
+        } else {
+            const int kk = lane & (DKC - 1);
+            if (kk < kc)
+                for (int j = lane / DKC; j < cols; j += 32 / DKC)
+                    cp_async8(sb + uint32_t(kk * pb + j) * 8u, B + int64_t(j) * p.ldb + k0 + kk, true);
+        }
+    };
+    if (p.k > 0) stage(sw, 0);
+    cp_async_commit();
+    int b = 0;
+    for (int k0 = 0; k0 < p.k; k0 += DKC, b ^= 1) {
+        if (k0 + DKC < p.k) stage(sw + (b ^ 1) * kDStage, k0 + DKC);
+        cp_async_commit();  // an empty group keeps the wait count uniform
+        cp_async_wait1();
+        __syncwarp();
+        const double* buf = sw + b * kDStage;
+        const int kc = min(DKC, p.k - k0);
+        switch (U) {
+#define GB_FLAT(n) \
+    case n: flat_steps<n>(buf, kc, pb, ao, bo, acc); break;
+            GB_FLAT(1) GB_FLAT(2) GB_FLAT(3) GB_FLAT(4) GB_FLAT(5) GB_FLAT(6) GB_FLAT(7) GB_FLAT(8)
+            GB_FLAT(9) GB_FLAT(10) GB_FLAT(11) GB_FLAT(12) GB_FLAT(13) GB_FLAT(14) GB_FLAT(15)
+#undef GB_FLAT
+            default: flat_steps<16>(buf, kc, pb, ao, bo, acc); break;
+        }
+        __syncwarp();  // the buffer is free for the chunk after next
+    }
+    double* C = static_cast<double*>(p.C) + int64_t(i0) * p.ldc + j0;
+    const double alpha = p.alpha, beta = p.beta;
+    // a loop of its own where C = A B: multiplies by one would cost as much as a k-step
+    if (alpha == 1.0 && beta == 0.0) {
+#pragma unroll
+        for (int u = 0; u < UMAX; ++u) {
+            if (lane + 32 * u >= outs) break;
+            const int i = ao[u] / DPA, j = bo[u] - bbase;
+            C[int64_t(i) * p.ldc + j] = acc[u];
+        }
+        return;
+    }
+#pragma unroll
+    for (int u = 0; u < UMAX; ++u) {
+        if (lane + 32 * u >= outs) break;
+        const int i = ao[u] / DPA, j = bo[u] - bbase;
+        double* c = C + int64_t(i) * p.ldc + j;
+        const double v = alpha * acc[u];
+        *c = (beta == 0.0) ? v : fma(beta, *c, v);
     }
 }
 
@@ -250,9 +306,8 @@ __device__ __forceinline__ void warp_tile_staged(const DevProblem& p, int tm, in
     }
 }
 
-// Shapes available per element type: FP64 stops at 16x32 / 32x16 warp tiles (16 accumulators per
-// lane): on the FP64 pipe a larger tile only adds padding, and the smaller register footprint lets an
-// SM hold twice the warps.  FP32 stops at 32x32 (32 accumulators per lane), so that an SM holds three
+// Shapes available per element type: FP64 stops at 16x32 / 32x16 warp tiles (16 outputs per lane), whose
+// staging lets an SM hold 16 warps.  FP32 stops at 32x32 (32 accumulators per lane), so that an SM holds three
 // 256-thread blocks (24 warps) to cover the latency of the staging loads.
 template <typename T>
 __host__ __device__ constexpr int max_shape() { return sizeof(T) == 8 ? 3 : 4; }
@@ -262,8 +317,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 2 : 3)
 grouped_kernel(const DevProblem* __restrict__ probs, const DevTile* __restrict__ tiles, int ntiles,
                int* __restrict__ counter) {
     const int lane = threadIdx.x & 31;
-    // FP32: the warp's staging region (dynamic shared memory of kStageBytes per block)
-    extern __shared__ float stage_smem[];
+    // the warps' staging regions (dynamic shared memory of kStageBytes or kDStageBytes per block)
+    extern __shared__ __align__(16) float stage_smem[];
     float* sw = stage_smem + (threadIdx.x >> 5) * kStageWarp;
     (void)sw;
     int t = 0;
@@ -286,18 +341,10 @@ grouped_kernel(const DevProblem* __restrict__ probs, const DevTile* __restrict__
                 default: warp_tile_staged<4, 8>(p, tl.tm, tl.tn, lane, sw); break;
             }
         } else {
-            switch (p.shape) {
-                case 0: warp_tile<T, 1, 2>(p, tl.tm, tl.tn, lane); break;
-                case 1: warp_tile<T, 2, 4>(p, tl.tm, tl.tn, lane); break;
-                case 2: warp_tile<T, 4, 4>(p, tl.tm, tl.tn, lane); break;
-                case 3: warp_tile<T, 2, 8>(p, tl.tm, tl.tn, lane); break;
-                case 4:
-                    if constexpr (max_shape<T>() >= 4) warp_tile<T, 4, 8>(p, tl.tm, tl.tn, lane);
-                    break;
-                default:
-                    if constexpr (max_shape<T>() >= 5) warp_tile<T, 8, 8>(p, tl.tm, tl.tn, lane);
-                    break;
-            }
+            const int i0 = tl.tm * p.tr, j0 = tl.tn * p.tc;
+            const int rows = min(p.tr, p.m - i0), cols = min(p.tc, p.n - j0);
+            double* sd = reinterpret_cast<double*>(stage_smem) + (threadIdx.x >> 5) * (2 * kDStage);
+            warp_tile_flat(p, i0, j0, rows, cols, lane, sd);
         }
         t = __shfl_sync(0xffffffffu, next, 0);
     }
@@ -333,12 +380,32 @@ bool g_tune_init = false;
 // Default choice (no measurements): the shape with the least padded work, larger tiles on ties.
 // tile_w < 0: the cost is the padded area plus 64 a tile (k left out); tile_w >= 0: the padded
 // multiply-adds (area x k) plus tile_w multiply-adds' worth of overhead a tile.
-int model_shape(int m, int n, int nshapes, int k = 1, double tile_w = -1.0) {
+// FP64 (flat): a product's tiles are equal parts of at most the shape's size, each a whole number of 32
+// outputs (warp_tile_flat).
+struct Parts {
+    int count, size;  // parts of `size`, the last one the rest
+};
+Parts equal_parts(int x, int limit) {
+    const int c = (x + limit - 1) / limit;
+    const int size = (x + c - 1) / c;
+    return {(x + size - 1) / size, size};
+}
+double padded_outputs(int m, int n, int s, bool flat) {
+    const int tr = shape_rows(s), tc = shape_cols(s);
+    if (!flat) return std::ceil(m / double(tr)) * tr * std::ceil(n / double(tc)) * tc;
+    const Parts r = equal_parts(m, tr), c = equal_parts(n, tc);
+    const int lr = m - (r.count - 1) * r.size, lc = n - (c.count - 1) * c.size;
+    auto warp = [](int a, int b) { return double((int64_t(a) * b + 31) / 32 * 32); };
+    return double(r.count - 1) * (c.count - 1) * warp(r.size, c.size) + double(r.count - 1) * warp(r.size, lc) +
+           double(c.count - 1) * warp(lr, c.size) + warp(lr, lc);
+}
+
+int model_shape(int m, int n, int nshapes, bool flat, int k = 1, double tile_w = -1.0) {
     int best = 0;
     double best_cost = 1e300;
     for (int s = 0; s < nshapes; ++s) {
         const double tr = shape_rows(s), tc = shape_cols(s);
-        const double padded = std::ceil(m / tr) * tr * std::ceil(n / tc) * tc;
+        const double padded = padded_outputs(m, n, s, flat);
         const double tiles = std::ceil(m / tr) * std::ceil(n / tc);
         // a small per-tile overhead favours fewer, larger tiles when the padding is equal
         const double cost = tile_w < 0 ? padded + 64.0 * tiles : padded * double(std::max(k, 1)) + tile_w * tiles;
@@ -358,7 +425,7 @@ void tune_defaults() {
             for (int b = 0; b < kMB; ++b)
                 for (int c = 0; c < kKB; ++c)
                     g_tune.shape[d][a][b][c] =
-                        model_shape(rep[a], rep[b], d == 0 ? max_shape<double>() + 1 : max_shape<float>() + 1);
+                        model_shape(rep[a], rep[b], d == 0 ? max_shape<double>() + 1 : max_shape<float>() + 1, d == 0);
     g_tune_init = true;
 }
 
@@ -375,8 +442,7 @@ int pick_shape(int dtype_idx, int m, int n, int k, int mode_override = -1) {
             for (int s = 0; s < nshapes; ++s) {
                 const float per = g_tune.cost[dtype_idx][a][b][c][s];
                 if (per <= 0.f) continue;
-                const double tr = shape_rows(s), tc = shape_cols(s);
-                const double cost = std::ceil(m / tr) * tr * std::ceil(n / tc) * tc * double(per);
+                const double cost = padded_outputs(m, n, s, dtype_idx == 0) * double(per);
                 if (cost < best_cost) {
                     best_cost = cost;
                     best = s;
@@ -384,7 +450,7 @@ int pick_shape(int dtype_idx, int m, int n, int k, int mode_override = -1) {
             }
             return best;
         }
-        default: return model_shape(m, n, nshapes, k, g_tune.tile_w[dtype_idx]);
+        default: return model_shape(m, n, nshapes, dtype_idx == 0, k, g_tune.tile_w[dtype_idx]);
     }
 }
 
@@ -462,38 +528,40 @@ int build_tables(const gb300_gemm_problem* probs, int64_t count, int force_shape
         if (d.m == 0 || d.n == 0) continue;
         if (d.k == 0 || x.alpha == 0.0) d.k = 0;  // C = beta*C through the same kernel
         d.shape = force_shape >= 0 ? force_shape : pick_shape(didx, d.m, d.n, d.k, policy);
-        const int tr = shape_rows(d.shape), tc = shape_cols(d.shape);
-        const int mt = (d.m + tr - 1) / tr, nt = (d.n + tc - 1) / tc;
+        d.tr = shape_rows(d.shape);
+        d.tc = shape_cols(d.shape);
+        if (sizeof(T) == 8) {
+            d.tr = equal_parts(d.m, d.tr).size;
+            d.tc = equal_parts(d.n, d.tc).size;
+        }
+        const int mt = (d.m + d.tr - 1) / d.tr, nt = (d.n + d.tc - 1) / d.tc;
         const int pid = int(hp.size());
         hp.push_back(d);
         for (int a = 0; a < mt; ++a)
             for (int b = 0; b < nt; ++b) ht.push_back(DevTile{pid, a, b, 0});
         useful += 2.0 * d.m * d.n * d.k;
-        padded += 2.0 * double(mt) * tr * double(nt) * tc * d.k;
+        padded += 2.0 * padded_outputs(d.m, d.n, d.shape, sizeof(T) == 8) * d.k;
     }
     // longest first: tiles ordered by their k times tile area (descending)
     std::stable_sort(ht.begin(), ht.end(), [&](const DevTile& a, const DevTile& b) {
         const DevProblem& pa = hp[a.prob];
         const DevProblem& pb = hp[b.prob];
-        const double wa = double(pa.k) * shape_rows(pa.shape) * shape_cols(pa.shape);
-        const double wb = double(pb.k) * shape_rows(pb.shape) * shape_cols(pb.shape);
+        const double wa = double(pa.k) * pa.tr * pa.tc;
+        const double wb = double(pb.k) * pb.tr * pb.tc;
         return wa > wb;
     });
     return GB300_OK;
 }
 
-// Dynamic shared memory of a block: the FP32 staging regions (none for FP64).
+// Dynamic shared memory of a block: its warps' staging regions.
 template <typename T>
 int grouped_smem() {
-    if constexpr (sizeof(T) == 4) {
-        static const bool set = [] {
-            return cudaFuncSetAttribute(grouped_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        kStageBytes) == cudaSuccess;
-        }();
-        (void)set;
-        return kStageBytes;
-    }
-    return 0;
+    constexpr int bytes = sizeof(T) == 4 ? kStageBytes : kDStageBytes;
+    static const bool set = [] {
+        return cudaFuncSetAttribute(grouped_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
+    }();
+    (void)set;
+    return bytes;
 }
 
 // Persistent grid for `ntiles` warp tiles: every SM's resident blocks, or fewer for a short list.
@@ -800,7 +868,7 @@ int grouped_lane_launch(GroupedLane* l, const gb300_gemm_problem* probs, int64_t
     if (e == cudaSuccess) e = cudaMemsetAsync(l->d_counter, 0, sizeof(int), l->stream);
     if (e == cudaSuccess) {
         const int grid = grouped_grid<double>(int64_t(l->ht.size()), runtime().num_sms);
-        grouped_kernel<double><<<grid, 256, 0, l->stream>>>(reinterpret_cast<const DevProblem*>(d),
+        grouped_kernel<double><<<grid, 256, grouped_smem<double>(), l->stream>>>(reinterpret_cast<const DevProblem*>(d),
                                                             reinterpret_cast<const DevTile*>(d + off_t),
                                                             int(l->ht.size()), l->d_counter);
         count_launches(1);
