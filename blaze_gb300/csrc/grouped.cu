@@ -181,128 +181,191 @@ __device__ __forceinline__ void warp_tile_flat(const DevProblem& p, int i0, int 
     }
 }
 
-// FP32 warp tiles stage their operands through shared memory, KC k-steps at a time: a warp reads
-// its A rows and B columns with coalesced loads (the contiguous dimension across lanes) into its own
-// region, then every k step reads them back from there.  Read straight from global memory, each k
-// step of an A row costs one cache line per row of the tile for one multiply-add per row and
-// column, which bounds small FP32 tiles by L1 line traffic rather than by the FFMA pipe.  Lane
-// (ly, lx) owns rows ly + 8r and the C contiguous columns lx*C .. lx*C + C-1 of the tile, so a k
-// step reads its B values with 16-byte shared loads (8-byte for C = 2), and one 16-byte load of an
-// A row serves KV = 4 k steps (2 for the 8 x 8 shape, whose accumulators leave fewer registers).
-// Rows of both staging arrays are padded to multiples of 16 bytes; the 16-byte reads of a warp then
-// touch distinct banks (A: rows 36 floats apart land 4 banks apart).  Every output still sums k in
-// order, so the results are those of the unstaged tile.
-constexpr int KC = 32;                                   // k-steps per staged block
-constexpr int PA = KC + 4;                               // A row pitch (floats)
-constexpr int kStageA = 32 * PA;                         // up to 32 rows (FP32 tiles stop at 32 x 32)
-constexpr int kStageB = KC * (32 + 4);                   // up to 32 columns, pitch TC + 4
-constexpr int kStageWarp = kStageA + kStageB;            // floats per warp
-constexpr int kStageBytes = 8 * kStageWarp * int(sizeof(float));  // per 256-thread block
+// FP32 warp tiles of (8 R) x (4 C) outputs: lane (ly, lx) of an 8 x 4 grid owns rows ly + 8 r and the C
+// contiguous columns lx C .. lx C + C - 1.  A and B are staged KC k-steps at a time in the warp's own
+// shared memory by cp.async, the next chunk on its way while one is used (16 bytes a copy where base
+// and leading dimension allow it, else 4), so that a chunk costs its instructions and not its latency:
+// with plain loads and stores through registers a warp waited for every row, 24 us a tile of some
+// 24 x 24 x 60.  One 16-byte read of an A row serves four k-steps; its chunks are rotated by the row
+// so that a warp's eight rows fall on different banks.  A k-step reads a lane's B columns 16 bytes at
+// a time (8 for C = 2), and its multiply-adds are packed in pairs of columns.  Rows and columns
+// outside the product are never copied in and never stored, and k-steps past the end are not added:
+// every output sums its k range in order.
+constexpr int KC = 16;                                    // k-steps per staged chunk
+constexpr int kStageA = 32 * KC;                          // up to 32 rows (FP32 tiles stop at 32 x 32)
+constexpr int kStageB = KC * (32 + 4);                    // up to 32 columns, pitch PB
+constexpr int kStageBuf = kStageA + kStageB;              // floats per buffer
+constexpr int kStageBytes = 8 * 2 * kStageBuf * int(sizeof(float));  // per 256-thread block
 
-// C consecutive floats from 16-byte (or, for C = 2, 8-byte) aligned shared memory.
+// Offset of A(row, kk): 16-byte chunk kk / 4 of a row at chunk ^ (row / 2 % 4).
+__device__ __forceinline__ int a_slot(int row, int kk) { return row * KC + ((((kk >> 2) ^ (row >> 1)) & 3) << 2) + (kk & 3); }
+
+// C consecutive floats from 16-byte (or, for C = 2, 8-byte) aligned shared memory, as packed pairs.
 template <int C>
-__device__ __forceinline__ void lds_vec(const float* __restrict__ src, float (&v)[C]) {
+__device__ __forceinline__ void lds_pairs(const float* __restrict__ src, uint64_t (&v)[C / 2]) {
     if constexpr (C == 2) {
-        const float2 t = *reinterpret_cast<const float2*>(src);
-        v[0] = t.x; v[1] = t.y;
+        v[0] = *reinterpret_cast<const uint64_t*>(src);
     } else {
 #pragma unroll
         for (int q = 0; q < C / 4; ++q) {
-            const float4 t = *reinterpret_cast<const float4*>(src + 4 * q);
-            v[4 * q] = t.x; v[4 * q + 1] = t.y; v[4 * q + 2] = t.z; v[4 * q + 3] = t.w;
+            const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(src + 4 * q);
+            v[2 * q] = t.x;
+            v[2 * q + 1] = t.y;
         }
     }
 }
 
+constexpr int PB = 36;  // B row pitch (floats)
+constexpr int kAcc = 16;  // packed accumulators a lane: 4 x 8 outputs
+
+// kc k-steps of a staged chunk.
 template <int R, int C>
-__device__ __forceinline__ void warp_tile_staged(const DevProblem& p, int tm, int tn, int lane, float* __restrict__ sw) {
-    constexpr int TR = 8 * R, TC = 4 * C, PB = TC + 4;
-    constexpr int KV = R >= 8 ? 2 : 4;  // k steps per A load
-    float* As = sw;            // As[r * PA + kk]
-    float* Bs = sw + kStageA;  // Bs[kk * PB + c]
-    const int ly = lane >> 2, lx = lane & 3;
-    const int i0 = tm * TR, j0 = tn * TC;
-    const float* A = static_cast<const float*>(p.A);
-    const float* B = static_cast<const float*>(p.B);
-    float acc[R][C];
-#pragma unroll
-    for (int r = 0; r < R; ++r)
-#pragma unroll
-        for (int c = 0; c < C; ++c) acc[r][c] = 0.f;
-    for (int k0 = 0; k0 < p.k; k0 += KC) {
-        const int kc = min(KC, p.k - k0);
-        // A(i, kk) = A[i lda + kk] (k contiguous) or A[kk lda + i] (m contiguous); zeros outside
-        if (!p.ta) {
-            for (int r = 0; r < TR; ++r) {
-                const int i = i0 + r;
-                As[r * PA + lane] = (i < p.m && lane < kc) ? __ldg(A + int64_t(i) * p.lda + k0 + lane) : 0.f;
-            }
-        } else {
-            for (int idx = lane; idx < TR * KC; idx += 32) {
-                const int r = idx % TR, kk = idx / TR, i = i0 + r;
-                As[r * PA + kk] = (i < p.m && kk < kc) ? __ldg(A + int64_t(k0 + kk) * p.lda + i) : 0.f;
-            }
-        }
-        // B(kk, j) = B[kk ldb + j] (n contiguous) or B[j ldb + kk] (k contiguous)
-        if (!p.tb) {
-            for (int idx = lane; idx < KC * TC; idx += 32) {
-                const int c = idx % TC, kk = idx / TC, j = j0 + c;
-                Bs[kk * PB + c] = (j < p.n && kk < kc) ? __ldg(B + int64_t(k0 + kk) * p.ldb + j) : 0.f;
-            }
-        } else {
-            for (int c = 0; c < TC; ++c) {
-                const int j = j0 + c;
-                Bs[lane * PB + c] = (j < p.n && lane < kc) ? __ldg(B + int64_t(j) * p.ldb + k0 + lane) : 0.f;
-            }
-        }
-        __syncwarp();
-        const float* arow = As + ly * PA;
-        const float* bcol = Bs + lx * C;
-        const int kv = kc & ~(KV - 1);
+__device__ __forceinline__ void f32_steps(const float* __restrict__ As, int kc, int ly, int lx, uint64_t (&acc)[kAcc]) {
+    const float* bcol = As + kStageA + lx * C;
+    const int kv = kc & ~3;
 #pragma unroll 1
-        for (int kk = 0; kk < kv; kk += KV) {
-            float a[R][KV];
+    for (int kk = 0; kk < kv; kk += 4) {
+        float4 a[R];
 #pragma unroll
-            for (int r = 0; r < R; ++r) lds_vec<KV>(arow + 8 * r * PA + kk, a[r]);
+        for (int r = 0; r < R; ++r) a[r] = *reinterpret_cast<const float4*>(As + a_slot(ly + 8 * r, kk));
 #pragma unroll
-            for (int q = 0; q < KV; ++q) {
-                float b[C];
-                lds_vec<C>(bcol + (kk + q) * PB, b);
-#pragma unroll
-                for (int r = 0; r < R; ++r)
-#pragma unroll
-                    for (int c = 0; c < C; ++c) acc[r][c] = fmaf(a[r][q], b[c], acc[r][c]);
-            }
-        }
-        // the last kc % KV steps one at a time (the staged zeros beyond kc are never added, so an
-        // output's sum is exactly that of its k range)
-#pragma unroll 1
-        for (int kk = kv; kk < kc; ++kk) {
-            float b[C];
-            lds_vec<C>(bcol + kk * PB, b);
+        for (int q = 0; q < 4; ++q) {
+            uint64_t bv[C / 2];
+            lds_pairs<C>(bcol + (kk + q) * PB, bv);
 #pragma unroll
             for (int r = 0; r < R; ++r) {
-                const float a = arow[8 * r * PA + kk];
+                const float x = q == 0 ? a[r].x : q == 1 ? a[r].y : q == 2 ? a[r].z : a[r].w;
+                const uint64_t x2 = f32x2(x, x);
 #pragma unroll
-                for (int c = 0; c < C; ++c) acc[r][c] = fmaf(a, b[c], acc[r][c]);
+                for (int c = 0; c < C / 2; ++c) acc[r * (C / 2) + c] = fma2(x2, bv[c], acc[r * (C / 2) + c]);
             }
         }
-        __syncwarp();
     }
-    float* Cp = static_cast<float*>(p.C);
+    // the last k-steps one at a time: what lies behind the end in the buffer is never added
+#pragma unroll 1
+    for (int kk = kv; kk < kc; ++kk) {
+        uint64_t bv[C / 2];
+        lds_pairs<C>(bcol + kk * PB, bv);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const float x = As[a_slot(ly + 8 * r, kk)];
+            const uint64_t x2 = f32x2(x, x);
+#pragma unroll
+            for (int c = 0; c < C / 2; ++c) acc[r * (C / 2) + c] = fma2(x2, bv[c], acc[r * (C / 2) + c]);
+        }
+    }
+}
+
+// C = alpha acc + beta C for the lane's rows and columns inside the product.
+template <int R, int C>
+__device__ __forceinline__ void f32_store(const DevProblem& p, int i0, int j0, int rows, int cols, int ly, int lx,
+                                          const uint64_t (&acc)[kAcc]) {
     const float alpha = float(p.alpha), beta = float(p.beta);
+    float* Cp = static_cast<float*>(p.C) + int64_t(i0) * p.ldc + j0 + lx * C;
+    const int left = cols - lx * C;  // of this lane's columns
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-        const int i = i0 + ly + 8 * r;
-        if (i >= p.m) continue;
-        float* crow = Cp + int64_t(i) * p.ldc;
+        if (ly + 8 * r >= rows) break;
+        float* crow = Cp + int64_t(ly + 8 * r) * p.ldc;
 #pragma unroll
         for (int c = 0; c < C; ++c) {
-            const int j = j0 + lx * C + c;
-            if (j >= p.n) continue;
-            const float v = alpha * acc[r][c];
-            crow[j] = (beta == 0.f) ? v : fmaf(beta, crow[j], v);
+            if (c >= left) break;
+            const float v = alpha * __uint_as_float(uint32_t(acc[r * (C / 2) + c / 2] >> ((c & 1) * 32)));
+            crow[c] = (beta == 0.f) ? v : fmaf(beta, crow[c], v);
         }
+    }
+}
+
+// k-steps k0 .. of the tile's rows of A and columns of B into a buffer.  One short loop per layout for
+// every tile shape: copies are asynchronous, so nothing is gained by unrolling them, and code that
+// is unrolled for each shape no longer fits the instruction cache (628 us for 10,000 products instead
+// of 369, two thirds of the stalls waiting for instructions).
+__device__ __forceinline__ void f32_stage(const DevProblem& p, const float* __restrict__ A, const float* __restrict__ B,
+                                          bool va, bool vb, int rows, int cols, int k0, int lane, uint32_t sa) {
+    const int kc = min(KC, p.k - k0);
+    const uint32_t sb = sa + kStageA * 4u;
+    if (va) {
+        const int c4 = (lane & 3) * 4, bytes = min(16, (kc - c4) * 4);
+        const float* src = A + int64_t(lane >> 2) * p.lda + k0 + c4;
+        if (bytes > 0)
+#pragma unroll 1
+            for (int i = lane >> 2; i < rows; i += 8, src += 8 * p.lda) cp_async16(sa + 4u * uint32_t(a_slot(i, c4)), src, bytes);
+    } else if (!p.ta) {
+        const int kk = lane & 15;
+        const float* src = A + int64_t(lane >> 4) * p.lda + k0 + kk;
+        if (kk < kc)
+#pragma unroll 2
+            for (int i = lane >> 4; i < rows; i += 2, src += 2 * p.lda) cp_async4(sa + 4u * uint32_t(a_slot(i, kk)), src, true);
+    } else if (lane < rows) {
+        const float* src = A + int64_t(k0) * p.lda + lane;
+#pragma unroll 2
+        for (int kk = 0; kk < kc; ++kk, src += p.lda) cp_async4(sa + 4u * uint32_t(a_slot(lane, kk)), src, true);
+    }
+    if (vb) {
+        const int c4 = (lane & 7) * 4, bytes = min(16, (cols - c4) * 4);
+        const float* src = B + int64_t(k0 + (lane >> 3)) * p.ldb + c4;
+        if (bytes > 0)
+#pragma unroll 1
+            for (int kk = lane >> 3; kk < kc; kk += 4, src += 4 * p.ldb) cp_async16(sb + 4u * uint32_t(kk * PB + c4), src, bytes);
+    } else if (p.tb) {
+        const int kk = lane & 15;
+        const float* src = B + int64_t(lane >> 4) * p.ldb + k0 + kk;
+        if (kk < kc)
+#pragma unroll 2
+            for (int j = lane >> 4; j < cols; j += 2, src += 2 * p.ldb) cp_async4(sb + 4u * uint32_t(kk * PB + j), src, true);
+    } else if (cols > 16) {
+        const float* src = B + int64_t(k0) * p.ldb + lane;
+        if (lane < cols)
+#pragma unroll 2
+            for (int kk = 0; kk < kc; ++kk, src += p.ldb) cp_async4(sb + 4u * uint32_t(kk * PB + lane), src, true);
+    } else {  // two k-steps a copy instruction
+        const int j = lane & 15;
+        const float* src = B + int64_t(k0 + (lane >> 4)) * p.ldb + j;
+        if (j < cols)
+#pragma unroll 2
+            for (int kk = lane >> 4; kk < kc; kk += 2, src += 2 * p.ldb) cp_async4(sb + 4u * uint32_t(kk * PB + j), src, true);
+    }
+}
+
+__device__ __forceinline__ void warp_tile_staged(const DevProblem& p, int tm, int tn, int lane, float* __restrict__ sw) {
+    const int ly = lane >> 2, lx = lane & 3;
+    const int i0 = tm * p.tr, j0 = tn * p.tc;
+    const int rows = min(p.tr, p.m - i0), cols = min(p.tc, p.n - j0);
+    const float* A = static_cast<const float*>(p.A) + (p.ta ? int64_t(i0) : int64_t(i0) * p.lda);
+    const float* B = static_cast<const float*>(p.B) + (p.tb ? int64_t(j0) * p.ldb : int64_t(j0));
+    // rows (or k-steps) that can be copied 16 bytes at a time
+    const bool va = !p.ta && ((reinterpret_cast<uintptr_t>(A) | uintptr_t(p.lda * 4)) & 15) == 0;
+    const bool vb = !p.tb && ((reinterpret_cast<uintptr_t>(B) | uintptr_t(p.ldb * 4)) & 15) == 0;
+    const uint32_t s0 = smem_u32(sw);
+    uint64_t acc[kAcc];
+#pragma unroll
+    for (int q = 0; q < kAcc; ++q) acc[q] = 0ull;
+    const int chunks = (p.k + KC - 1) / KC;
+#pragma unroll 1
+    for (int c = -1; c < chunks; ++c) {
+        if (c + 1 < chunks)
+            f32_stage(p, A, B, va, vb, rows, cols, (c + 1) * KC, lane, s0 + uint32_t((c + 1) & 1) * (kStageBuf * 4u));
+        cp_async_commit();  // an empty group keeps the wait count uniform
+        if (c < 0) continue;
+        cp_async_wait1();
+        __syncwarp();
+        const float* buf = sw + (c & 1) * kStageBuf;
+        const int kc = min(KC, p.k - c * KC);
+        switch (p.shape) {
+            case 0: f32_steps<1, 2>(buf, kc, ly, lx, acc); break;
+            case 1: f32_steps<2, 4>(buf, kc, ly, lx, acc); break;
+            case 2: f32_steps<4, 4>(buf, kc, ly, lx, acc); break;
+            case 3: f32_steps<2, 8>(buf, kc, ly, lx, acc); break;
+            default: f32_steps<4, 8>(buf, kc, ly, lx, acc); break;
+        }
+        __syncwarp();  // the buffer is free for the chunk after next
+    }
+    switch (p.shape) {
+        case 0: f32_store<1, 2>(p, i0, j0, rows, cols, ly, lx, acc); break;
+        case 1: f32_store<2, 4>(p, i0, j0, rows, cols, ly, lx, acc); break;
+        case 2: f32_store<4, 4>(p, i0, j0, rows, cols, ly, lx, acc); break;
+        case 3: f32_store<2, 8>(p, i0, j0, rows, cols, ly, lx, acc); break;
+        default: f32_store<4, 8>(p, i0, j0, rows, cols, ly, lx, acc); break;
     }
 }
 
@@ -319,34 +382,34 @@ grouped_kernel(const DevProblem* __restrict__ probs, const DevTile* __restrict__
     const int lane = threadIdx.x & 31;
     // the warps' staging regions (dynamic shared memory of kStageBytes or kDStageBytes per block)
     extern __shared__ __align__(16) float stage_smem[];
-    float* sw = stage_smem + (threadIdx.x >> 5) * kStageWarp;
+    float* sw = stage_smem + (threadIdx.x >> 5) * (2 * kStageBuf);
     (void)sw;
-    int t = 0;
-    if (lane == 0) t = atomicAdd(counter, 1);
+    // The tickets run two tiles ahead and the tile descriptions one: the ticket after next is taken and
+    // the next tile's description read while this tile is worked on, so neither round trip precedes a
+    // tile (small tiles are a few hundred clocks of multiply-adds).
+    int t = 0, next = 0;
+    if (lane == 0) {
+        t = atomicAdd(counter, 1);
+        next = atomicAdd(counter, 1);
+    }
     t = __shfl_sync(0xffffffffu, t, 0);
-    while (t < ntiles) {
-        // the next tile's ticket is taken now and read after this tile: the atomic's round trip
-        // overlaps the tile's work instead of preceding every tile (small tiles are a few hundred
-        // clocks of multiply-adds)
-        int next = 0;
+    if (t >= ntiles) return;
+    DevTile tl = tiles[t];
+    while (true) {
+        t = __shfl_sync(0xffffffffu, next, 0);
         if (lane == 0) next = atomicAdd(counter, 1);
-        const DevTile tl = tiles[t];
+        const DevTile tn = tiles[min(t, ntiles - 1)];
         const DevProblem p = probs[tl.prob];
         if constexpr (sizeof(T) == 4) {
-            switch (p.shape) {
-                case 0: warp_tile_staged<1, 2>(p, tl.tm, tl.tn, lane, sw); break;
-                case 1: warp_tile_staged<2, 4>(p, tl.tm, tl.tn, lane, sw); break;
-                case 2: warp_tile_staged<4, 4>(p, tl.tm, tl.tn, lane, sw); break;
-                case 3: warp_tile_staged<2, 8>(p, tl.tm, tl.tn, lane, sw); break;
-                default: warp_tile_staged<4, 8>(p, tl.tm, tl.tn, lane, sw); break;
-            }
+            warp_tile_staged(p, tl.tm, tl.tn, lane, sw);
         } else {
             const int i0 = tl.tm * p.tr, j0 = tl.tn * p.tc;
             const int rows = min(p.tr, p.m - i0), cols = min(p.tc, p.n - j0);
             double* sd = reinterpret_cast<double*>(stage_smem) + (threadIdx.x >> 5) * (2 * kDStage);
             warp_tile_flat(p, i0, j0, rows, cols, lane, sd);
         }
-        t = __shfl_sync(0xffffffffu, next, 0);
+        if (t >= ntiles) return;
+        tl = tn;
     }
 }
 
@@ -377,7 +440,20 @@ std::mutex g_tune_mu;
 TuneTable g_tune;
 bool g_tune_init = false;
 
-// Default choice (no measurements): the shape with the least padded work, larger tiles on ties.
+// Instructions of one FP32 warp tile of `rows` x `cols` used outputs (shape s, k steps): per staged
+// chunk its copies and its multiply-adds, per tile its description, set-up and stores.  The small
+// shapes waste little on padding but pay five times as many instructions a multiply-add as 32 x 32.
+double f32_tile_cost(int s, int rows, int cols, int k) {
+    const int R = shape_rows(s) / 8, C = shape_cols(s) / 4;
+    const double steps = 4.0 * (R + 4.0 * (std::max(1, C / 4) + R + R * C / 2));
+    const double copies = 3.5 * rows + (cols > 16 ? 112.0 : 56.0);
+    return 400.0 + (k + KC - 1) / KC * (60.0 + copies) + k / double(KC) * steps;
+}
+
+// Default choice (no measurements).  FP64: the shape with the least padded work, larger tiles on ties;
+// FP32: the one with the fewest instructions (f32_tile_cost), since they bound its tiles (10,000
+// products: 369 us with the least padded work, 323 with this, which also holds the ticket and
+// description look-ahead of grouped_kernel).
 // tile_w < 0: the cost is the padded area plus 64 a tile (k left out); tile_w >= 0: the padded
 // multiply-adds (area x k) plus tile_w multiply-adds' worth of overhead a tile.
 // FP64 (flat): a product's tiles are equal parts of at most the shape's size, each a whole number of 32
@@ -408,7 +484,9 @@ int model_shape(int m, int n, int nshapes, bool flat, int k = 1, double tile_w =
         const double padded = padded_outputs(m, n, s, flat);
         const double tiles = std::ceil(m / tr) * std::ceil(n / tc);
         // a small per-tile overhead favours fewer, larger tiles when the padding is equal
-        const double cost = tile_w < 0 ? padded + 64.0 * tiles : padded * double(std::max(k, 1)) + tile_w * tiles;
+        const double cost = tile_w < 0 && !flat ? tiles * f32_tile_cost(s, std::min(m, int(tr)), std::min(n, int(tc)), k)
+                            : tile_w < 0        ? padded + 64.0 * tiles
+                                                : padded * double(std::max(k, 1)) + tile_w * tiles;
         if (cost < best_cost - 1e-9) {
             best_cost = cost;
             best = s;
@@ -419,13 +497,13 @@ int model_shape(int m, int n, int nshapes, bool flat, int k = 1, double tile_w =
 
 void tune_defaults() {
     if (g_tune_init) return;
-    const int rep[kMB] = {6, 12, 24, 48, 96, 192};
+    const int rep[kMB] = {6, 12, 24, 48, 96, 192}, rep_k[kKB] = {10, 40, 160};
     for (int d = 0; d < 2; ++d)
         for (int a = 0; a < kMB; ++a)
             for (int b = 0; b < kMB; ++b)
                 for (int c = 0; c < kKB; ++c)
                     g_tune.shape[d][a][b][c] =
-                        model_shape(rep[a], rep[b], d == 0 ? max_shape<double>() + 1 : max_shape<float>() + 1, d == 0);
+                        model_shape(rep[a], rep[b], d == 0 ? max_shape<double>() + 1 : max_shape<float>() + 1, d == 0, rep_k[c]);
     g_tune_init = true;
 }
 
