@@ -85,6 +85,7 @@ constexpr int THREADS = 64 + EPI_WARPS * 32;
 constexpr int MAX_SLICES = 10;
 constexpr int KSEG_UNIT = 256;          // k-segments are multiples of this
 constexpr int kPipeMaxQ = 2;            // column blocks of B in the host-operand pipeline
+constexpr int kPipeMaxEvents = 64;      // of a pipeline of P panels and Q column blocks, P + Q + 2 P Q + 1
 constexpr uint32_t MAGIC_BITS = 0x4B400000u;  // bits of 1.5 * 2^23
 constexpr float MAGIC = 12582912.0f;
 
@@ -98,11 +99,14 @@ enum Mode : int { kExact = 0, kBf16 = 1, kBf16x3 = 2, kCrt = 3 };
 // 239; 233; 229; 227; 223; 7,31; 211; 199.  Product of all 15: about 2^118.2.
 constexpr int MAX_MODULI = 15;
 __constant__ uint32_t c_mod[MAX_MODULI] = {257, 256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 217, 211, 199};
-// log2 of each modulus (device copy: the plan kernels sum these instead of calling log2).
-__constant__ double c_mod_log2[MAX_MODULI] = {
-    8.005624549193879, 8.0, 7.994353436858858, 7.98299357469431, 7.971543553950772, 7.948367231584678,
-    7.912889336229962, 7.900866807980749, 7.864186144654281, 7.839203788096944, 7.826548487290915,
-    7.800899899920305, 7.7615512324444795, 7.721099188707185, 7.636624620543649};
+// Running products of the moduli rounded to FP64: entry N for the first N (device copy).
+__constant__ double c_mod_prod[MAX_MODULI + 1] = {
+    0x1.0p+0, 0x1.0100000000000p+8, 0x1.0100000000000p+16, 0x1.fffe000000000p+23,
+    0x1.f9fe060000000p+31, 0x1.f01c0fe200000p+39, 0x1.deab13530e000p+47, 0x1.c29f0d31302e0p+55,
+    0x1.a4b27d50ebfafp+63, 0x1.7ee6740ea6c76p+71, 0x1.568425d11b306p+79, 0x1.2fb72d886b1bep+87,
+    0x1.089090a9d54d5p+95, 0x1.c085153feb9d1p+102, 0x1.71adb083af327p+110, 0x1.1f5e04365d303p+118};
+// What the product of the moduli must exceed the largest |T| by: 2^1.0875, just above 2.125.
+constexpr double kModMargin = 0x1.1001cb22b792cp+1;
 // log2 of the running products of the moduli (host-side copy for the worst-case plan).
 constexpr double kModLog2[MAX_MODULI] = {8.00562, 8.0, 7.99435, 7.98299, 7.97154, 7.94837, 7.91289, 7.90087,
                                          7.86419, 7.83920, 7.82655, 7.80090, 7.76155, 7.72110, 7.63662};
@@ -143,86 +147,55 @@ struct SplitInfo {
 // ---- pre-pass ------------------------------------------------------------------------------
 // Row statistics of a logical R x K operand X(r,p) = X[r*sr + p*sp]: e_r = frexp exponent of
 // max |X(r,:)| (kNonFinite if the row holds Inf/NaN) and q_r = sum_p (X(r,p) * 2^-e_r)^2, the
-// row's sum of squares relative to 2^(2 e_r) (so that norms of huge or tiny inputs stay finite).
-//
-// stats_tile_kernel reads 32-row x 64-k tiles (coalesced along whichever dimension is
-// contiguous, like slice_kernel) and folds each row's tile maximum and sum of squares into
-// per-row accumulators with atomics; stats_finalize_kernel turns them into (e_r, q_r).  A row
-// whose values leave [2^-500, 2^500] would over- or underflow the unscaled sum of squares; the
-// finalize kernel recomputes such (rare) rows on scaled values.
+// row's sum of squares relative to 2^(2 e_r) (so that norms of huge or tiny inputs stay finite), and
+// from them the plan (SplitInfo).  All of it is one launch, stats_kernel: its blocks read 32-row x 64-k
+// tiles (coalesced along whichever dimension is contiguous, like slice_kernel), the last block to
+// finish a row block folds the partial sums of the row block's k-chunks into (e_r, q_r) and one
+// RowPartial, and the last block of all plans from those.  The counters that find the last block are
+// zero before the launch; no block waits for another.
 constexpr int kNonFinite = 0x7fff;
-
-struct RowAcc {
-    // max |x| to its high 32 bits (sign, exponent, 20 mantissa bits; non-negative doubles order
-    // like integers), bit 0 set when some value has non-zero low bits: the frexp exponent of the
-    // maximum follows whenever the high word is a normal number, and a row whose high words are
-    // all zero or subnormal is rescanned exactly
-    unsigned long long maxbits;
-    double sumsq;
-    int flags;                   // 1: non-finite value seen
-    int pad;
-};
 
 // Operands stream through shared memory in tiles of 32 rows x 64 k, a few tiles per block
 // (tiles_per_block), with two buffers filled by cp.async: the copies of the next tile are in flight
 // while the current one is processed.
 constexpr int TILE_KT = 8;  // at most
 
-// The copies of one thread per tile, coalesced along whichever index of X(r, p) = X[r*sr + p*sp] is
-// contiguous: eight elements (rr0 + i drr, pp0 + i dpp), a warp reading 256 consecutive bytes, or,
-// where every row is contiguous and 16-byte aligned (vec), four pairs of elements, a warp reading
-// 512.  src points at the first one in tile 0, di and dk step to copy i and to the next tile of 64 k.
-struct TileSrc {
-    const unsigned long long* src;
-    int64_t di, dk;
-    int rr0, pp0, drr, dpp;
-    bool vec;
-};
-
-__device__ __forceinline__ TileSrc tile_src(const double* X, int64_t sr, int64_t sp, int64_t r0) {
-    const int t = threadIdx.x;  // 256 threads
-    TileSrc s;
-    s.vec = sp == 1 && (sr & 1) == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0;
-    if (s.vec) {
-        s.rr0 = t >> 5; s.drr = 8; s.pp0 = 2 * (t & 31); s.dpp = 0;
-        s.di = 8 * sr;
-        s.dk = 64;
-    } else if (sp == 1) {
-        s.rr0 = t >> 6; s.drr = 4; s.pp0 = t & 63; s.dpp = 0;
-        s.di = 4 * sr;
-        s.dk = 64;
-    } else {
-        s.rr0 = t & 31; s.drr = 0; s.pp0 = t >> 5; s.dpp = 8;
-        s.di = 8 * sp;
-        s.dk = 64 * sp;
-    }
-    s.src = reinterpret_cast<const unsigned long long*>(X) + (r0 + s.rr0) * sr + int64_t(s.pp0) * sp;
-    return s;
+// Whether an operand's rows are contiguous and 16-byte aligned.
+__device__ __forceinline__ bool rows_vec(const double* X, int64_t sr, int64_t sp) {
+    return sp == 1 && (sr & 1) == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0;
 }
 
 // Issue the copies of tile `it` (k from 64 it) into the buffer at shared address sbuf, where
 // off(rr, pp) places element (rr, pp), an even pp and the next one side by side; zeros outside R x K;
-// one commit group per tile.
+// one commit group per tile.  The copies are coalesced along whichever index of
+// X(r, p) = X[r*sr + p*sp] is contiguous: eight elements a thread, a warp reading 256 consecutive
+// bytes, or, where rows_vec, four pairs of elements, a warp reading 512.  Addresses are formed anew for
+// each tile: kept across tiles they spilled from the slicing's 80 registers (725 -> 879 us at 8192^3).
 template <typename Off>
-__device__ __forceinline__ void tile_issue(uint32_t sbuf, const TileSrc& s, const double* X, int64_t R, int64_t K,
-                                           int64_t r0, int64_t it, Off off) {
-    const unsigned long long* src = s.src + it * s.dk;
+__device__ __forceinline__ void tile_issue(uint32_t sbuf, const double* X, int64_t R, int64_t K, int64_t sr, int64_t sp,
+                                           bool vec, int64_t r0, int64_t it, Off off) {
+    const int t = threadIdx.x;  // 256 threads
     const bool full = r0 + 32 <= R && it * 64 + 64 <= K;  // the whole tile lies inside the matrix
-    if (s.vec) {
-        const int64_t left = K - it * 64 - s.pp0;
+    if (vec) {
+        const int rr0 = t >> 5, pp = 2 * (t & 31);
+        const int64_t left = K - it * 64 - pp;
         const int bytes = full || left >= 2 ? 16 : left == 1 ? 8 : 0;
+        const double* src = X + (r0 + rr0) * sr + it * 64 + pp;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const int rr = s.rr0 + i * s.drr;
-            const int n = full || r0 + rr < R ? bytes : 0;
-            cp_async16(sbuf + off(rr, s.pp0), n ? src + i * s.di : reinterpret_cast<const unsigned long long*>(X), n);
+            const int n = full || r0 + rr0 + 8 * i < R ? bytes : 0;
+            cp_async16(sbuf + off(rr0 + 8 * i, pp), n ? src + 8 * i * sr : X, n);
         }
     } else {
+        const int rr0 = sp == 1 ? t >> 6 : t & 31, pp0 = sp == 1 ? t & 63 : t >> 5;
+        const int drr = sp == 1 ? 4 : 0, dpp = sp == 1 ? 0 : 8;
+        const double* src = X + (r0 + rr0) * sr + (it * 64 + pp0) * sp;
+        const int64_t di = sp == 1 ? 4 * sr : 8 * sp;
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-            const int rr = s.rr0 + i * s.drr, pp = s.pp0 + i * s.dpp;
+            const int rr = rr0 + i * drr, pp = pp0 + i * dpp;
             const bool ok = full || (r0 + rr < R && it * 64 + pp < K);
-            cp_async8(sbuf + off(rr, pp), ok ? src + i * s.di : reinterpret_cast<const unsigned long long*>(X), ok);
+            cp_async8(sbuf + off(rr, pp), ok ? src + i * di : X, ok);
         }
     }
     cp_async_commit();
@@ -231,7 +204,86 @@ __device__ __forceinline__ void tile_issue(uint32_t sbuf, const TileSrc& s, cons
 // 2^x in FP32 for x <= 127, 0 below the normal range.
 __device__ __forceinline__ float pow2f_or0(int x) { return x < -126 ? 0.f : __uint_as_float(uint32_t(x + 127) << 23); }
 
-// Row statistics over kt tiles: thread (rr = t % 32, g = t / 32) keeps, for row rr and the
+// Both operands of a product go through one launch: blocks with blockIdx.y < yb0 work on A (its
+// rows), the others on B (its columns), so the two passes overlap on the device.
+struct OperandPair {
+    const double* X[2];
+    int64_t R[2], sr[2], sp[2];
+    int* rexp[2];
+    __nv_bfloat16* planes[2];
+    int64_t rpad[2];
+    unsigned yb0;  // row blocks of A
+};
+
+// Summary of 32 rows (or of many): Inf/NaN flag, largest exponent E of the rows with q > 0 (kNoRows
+// when none), largest q, s = sum 2^(2(e - E)) and nrm = sum 2^(2(e - E)) q.  FP32: the sums feed norms
+// and bounds, and the plan allows q 2^-10 for rounding.
+constexpr int kNoRows = -100000;
+struct RowPartial {
+    int bad, E;
+    float Q, s, nrm;
+};
+
+__device__ __forceinline__ RowPartial merge(const RowPartial& a, const RowPartial& b) {
+    RowPartial r;
+    r.bad = a.bad | b.bad;
+    r.E = max(a.E, b.E);
+    r.Q = fmaxf(a.Q, b.Q);
+    const float wa = pow2f_or0(2 * (a.E - r.E)), wb = pow2f_or0(2 * (b.E - r.E));
+    r.s = fmaf(wa, a.s, wb * b.s);
+    r.nrm = fmaf(wa, a.nrm, wb * b.nrm);
+    return r;
+}
+
+// The merge over the calling warp's lanes (all lanes get it).
+__device__ __forceinline__ RowPartial warp_merge(RowPartial v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        RowPartial w;
+        w.bad = __shfl_xor_sync(0xffffffffu, v.bad, o);
+        w.E = __shfl_xor_sync(0xffffffffu, v.E, o);
+        w.Q = __shfl_xor_sync(0xffffffffu, v.Q, o);
+        w.s = __shfl_xor_sync(0xffffffffu, v.s, o);
+        w.nrm = __shfl_xor_sync(0xffffffffu, v.nrm, o);
+        v = merge(v, w);
+    }
+    return v;
+}
+
+// What the last block of a statistics launch plans.
+enum PlanKind : int { kPlanProduct = 0, kPlanSide = 1 };
+struct PlanArgs {
+    int kind, mode, fixed_slices, cap_planes;
+    double target;
+    SplitInfo* info;
+};
+
+__device__ void plan_product(const RowPartial& A, const RowPartial& B, int64_t k, const PlanArgs& plan);
+__device__ void plan_side(const RowPartial& S, int64_t k, const PlanArgs& plan);
+
+struct StatsArgs {
+    OperandPair op;
+    int64_t K;
+    int kt, chunks;        // k-tiles per block, blocks per row block
+    uint2* part;           // chunks > 1: [rows of A, then of B][chunks] of (high word and low flag, sum)
+    unsigned* count;       // one counter per row block, one for the launch; zero before the launch
+    RowPartial* group;     // one per row block
+    PlanArgs plan;
+};
+
+// Whether this block is the last of `n` to arrive at the counter (uniform over the block).  What the
+// arriving blocks wrote before is visible to the last one.
+__device__ __forceinline__ bool last_to_arrive(unsigned* counter, unsigned n) {
+    __shared__ unsigned last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(counter, 1u) + 1u == n ? 1u : 0u;
+    __syncthreads();
+    if (last != 0u) __threadfence();
+    return last != 0u;
+}
+
+// Thread (rr = t % 32, g = t / 32) keeps, for row rr and the
 // eight k of group g in every tile, the largest high word of |x|, the OR of the low words and the
 // sum of squares in FP32 relative to its running largest exponent `base`: f = |x| 2^(1023 - base)
 // is the high word times 8 (exponent and 20 mantissa bits moved into FP32 position) minus
@@ -239,30 +291,36 @@ __device__ __forceinline__ float pow2f_or0(int x) { return x < -126 ? 0.f : __ui
 // that are raised to its lowest value, whose square is zero in FP32.  `base` moves once per tile, to
 // the exponent of the largest high word so far, and the running sum is rescaled exactly by a power of
 // two.  Bound by the integer ALU: these four ALU operations an element, the maximum and the OR taken
-// two elements at a time; with `base` checked at every element it was seven (1 GiB of operands: 215 us, now 169, 6.4 TB/s).
-// The block folds the eight groups of a row and issues one set of atomics per row; an Inf/NaN shows as
-// a largest exponent of 0x7ff.
-__device__ __forceinline__ void stats_rows(const double* __restrict__ X, int64_t R, int64_t K, int64_t sr, int64_t sp,
-                                           RowAcc* __restrict__ acc, int by, int kt) {
+// two elements at a time; with `base` checked at every element it was seven (1 GiB of operands: 215
+// us, now 169, 6.4 TB/s).  An Inf/NaN shows as a largest exponent of 0x7ff.
+//
+// Small operands are bound by the launches and by the plan's chain of FP64 functions instead: with the
+// row totals in a kernel of their own (atomics and a memset before it) and the plan in another, these
+// steps took 23 us of a 403 x 517 x 389 product and 26 of 1024^3 with the gaps between four launches
+// beside them, now 13 and 17.
+__global__ void __launch_bounds__(256, 4) stats_kernel(const StatsArgs a) {
     constexpr uint32_t ROWB = 528, BUF = 32 * ROWB;  // rows 33 chunks of 16 bytes apart: no bank conflicts
     __shared__ __align__(16) unsigned char tbuf[2 * BUF];
-    __shared__ uint32_t red_mx[8][32], red_lo[8][32];
-    __shared__ int red_base[8][32];
+    __shared__ uint32_t red_mx[8][32];
     __shared__ float red_sq[8][32];
+    const int w = blockIdx.y < a.op.yb0 ? 0 : 1;
+    const int by = w ? int(blockIdx.y - a.op.yb0) : int(blockIdx.y);
+    const double* __restrict__ X = a.op.X[w];
+    const int64_t R = a.op.R[w], sr = a.op.sr[w], sp = a.op.sp[w], K = a.K;
     const int t = threadIdx.x, rr = t & 31, g = t >> 5;
     const int64_t r0 = int64_t(by) * 32;
     const int64_t ntiles = (K + 63) / 64;
-    const int64_t tb = int64_t(blockIdx.x) * kt, te = min(ntiles, tb + kt);
+    const int64_t tb = int64_t(blockIdx.x) * a.kt, te = min(ntiles, tb + a.kt);
     const uint32_t s0 = smem_u32(tbuf);
     auto off = [](int r_, int p_) { return uint32_t(r_) * ROWB + uint32_t(p_) * 8u; };
     uint32_t mx = 0, lo = 0;
     int base = 127;  // f = |x| 2^(1023 - base); values with exponent field 0 never count
     float sq = 0.f;
-    const TileSrc ts = tile_src(X, sr, sp, r0);
-    if (tb < te) tile_issue(s0, ts, X, R, K, r0, tb, off);
+    const bool vec = rows_vec(X, sr, sp);
+    if (tb < te) tile_issue(s0, X, R, K, sr, sp, vec, r0, tb, off);
     for (int64_t it = tb; it < te; ++it) {
         const int b = int(it - tb) & 1;
-        if (it + 1 < te) tile_issue(s0 + uint32_t(b ^ 1) * BUF, ts, X, R, K, r0, it + 1, off);
+        if (it + 1 < te) tile_issue(s0 + uint32_t(b ^ 1) * BUF, X, R, K, sr, sp, vec, r0, it + 1, off);
         else cp_async_commit();  // an empty group keeps the wait count uniform
         cp_async_wait1();
         __syncthreads();
@@ -289,156 +347,120 @@ __device__ __forceinline__ void stats_rows(const double* __restrict__ X, int64_t
         }
         __syncthreads();
     }
-    red_mx[g][rr] = mx;
-    red_lo[g][rr] = lo;
-    red_base[g][rr] = base;
+    // a row's largest high word with the low words' flag in bit 0, and its sum of squares relative to
+    // the exponent of that high word (at least 127)
+    auto exponent = [](uint32_t m) { return max(127, int(m >> 21)); };
+    red_mx[g][rr] = (mx << 1) | (lo != 0u ? 1u : 0u);
     red_sq[g][rr] = sq;
     __syncthreads();
-    if (g == 0) {
-        int E = 0;
-        uint32_t m = 0, l = 0;
+    auto fold = [&](uint32_t& m, float& s) {  // the eight groups' values of row rr
+        m = 0;
+        uint32_t flag = 0;
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-            E = max(E, red_base[i][rr]);
-            m = max(m, red_mx[i][rr]);
-            l |= red_lo[i][rr];
+            m = max(m, red_mx[i][rr] & ~1u);
+            flag |= red_mx[i][rr] & 1u;
         }
-        float s = 0.f;
+        m |= flag;
+        const int E = exponent(m);
+        s = 0.f;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) s = fmaf(red_sq[i][rr], pow2f_or0(2 * (red_base[i][rr] - E)), s);
-        const int64_t r = r0 + rr;
-        if (r < R) {
-            if (m >= 0x7ff00000u) atomicOr(&acc[r].flags, 1);
-            if (m != 0 || l != 0) {
-                atomicMax(&acc[r].maxbits, ((unsigned long long)m << 32) | (l != 0 ? 1ull : 0ull));
-                // sum of squares of the unscaled values: s * 2^(2 (E - 1023))
-                if (s > 0.f) atomicAdd(&acc[r].sumsq, ldexp(double(s), 2 * (E - 1023)));
+        for (int i = 0; i < 8; ++i) s = fmaf(red_sq[i][rr], pow2f_or0(2 * (exponent(red_mx[i][rr]) - E)), s);
+    };
+    const int64_t r = r0 + rr;
+    uint32_t m = 0;
+    float s = 0.f;
+    if (g == 0) fold(m, s);
+    if (a.chunks > 1) {
+        uint2* rowpart = a.part + ((w ? a.op.R[0] : 0) + r) * a.chunks;
+        if (g == 0 && r < R) rowpart[blockIdx.x] = make_uint2(m, __float_as_uint(s));
+        if (!last_to_arrive(a.count + blockIdx.y, unsigned(a.chunks))) return;
+        m = 0;
+        s = 0.f;
+        uint32_t flag = 0;
+        if (r < R)
+            for (int c = g; c < a.chunks; c += 8) {  // fixed order: the sums do not depend on which block is last
+                const uint2 v = __ldcg(rowpart + c);
+                const int E = exponent(m), Ec = exponent(v.x);
+                s = Ec > E ? fmaf(s, pow2f_or0(2 * (E - Ec)), __uint_as_float(v.y))
+                           : fmaf(__uint_as_float(v.y), pow2f_or0(2 * (Ec - E)), s);
+                m = max(m, v.x & ~1u);
+                flag |= v.x & 1u;
+            }
+        red_mx[g][rr] = m | flag;
+        red_sq[g][rr] = s;
+        __syncthreads();
+        if (g == 0) fold(m, s);
+    }
+    if (g == 0) {
+        int e = 0;
+        float q = 0.f;
+        const uint32_t hi = m >> 1;
+        if (r < R && m != 0u) {
+            if (hi >= 0x7ff00000u) {
+                e = kNonFinite;
+            } else if (hi >= (191u << 20)) {
+                e = int(hi >> 20) - 1022;
+                q = 0.25f * s;  // |x| 2^-e = f / 2
+            } else {
+                // tiny or subnormal values, whose squares left the FP32 range: the row again, exactly
+                unsigned long long mb = 0;
+                for (int64_t p = 0; p < K; ++p) {
+                    const unsigned long long v =
+                        static_cast<unsigned long long>(__double_as_longlong(X[r * sr + p * sp])) & 0x7fffffffffffffffull;
+                    mb = v > mb ? v : mb;
+                }
+                frexp(__longlong_as_double(static_cast<long long>(mb)), &e);
+                double d = 0.0;
+                for (int64_t p = 0; p < K; ++p) {
+                    const double v = ldexp(X[r * sr + p * sp], -e);
+                    d = fma(v, v, d);
+                }
+                q = float(d);
             }
         }
+        if (r < R) a.op.rexp[w][r] = e;
+        RowPartial pr{e == kNonFinite, q > 0.f ? e : kNoRows, q, q > 0.f ? 1.f : 0.f, q};
+        pr = warp_merge(pr);
+        if (t == 0) a.group[blockIdx.y] = pr;
     }
+    if (!last_to_arrive(a.count + gridDim.y, gridDim.y)) return;
+    // the plan, from every row block
+    __shared__ RowPartial side[2][8];
+    RowPartial acc[2];
+    acc[0] = acc[1] = RowPartial{0, kNoRows, 0.f, 0.f, 0.f};
+#pragma unroll 4
+    for (unsigned i = t; i < gridDim.y; i += 256) {
+        const int* v = reinterpret_cast<const int*>(a.group + i);
+        const RowPartial pr{__ldcg(v), __ldcg(v + 1), __int_as_float(__ldcg(v + 2)), __int_as_float(__ldcg(v + 3)),
+                            __int_as_float(__ldcg(v + 4))};
+        const RowPartial none{0, kNoRows, 0.f, 0.f, 0.f};
+        acc[0] = merge(acc[0], i < a.op.yb0 ? pr : none);
+        acc[1] = merge(acc[1], i < a.op.yb0 ? none : pr);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        acc[i] = warp_merge(acc[i]);
+        if (rr == 0) side[i][g] = acc[i];
+    }
+    __syncthreads();
+    if (g != 0) return;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        RowPartial v{0, kNoRows, 0.f, 0.f, 0.f};
+        if (rr < 8) v = side[i][rr];
+        acc[i] = warp_merge(v);
+    }
+    if (a.plan.kind == kPlanProduct) plan_product(acc[0], acc[1], K, a.plan);
+    else plan_side(a.op.yb0 ? acc[0] : acc[1], K, a.plan);
 }
 
-__device__ __forceinline__ void stats_finalize_row(const double* __restrict__ X, int64_t R, int64_t K, int64_t sr,
-                                                   int64_t sp, const RowAcc* __restrict__ acc, int* __restrict__ rexp,
-                                                   double* __restrict__ rsq, int64_t r) {
-    if (r >= R) return;
-    const RowAcc a = acc[r];
-    if (a.flags & 1) {
-        rexp[r] = kNonFinite;
-        rsq[r] = 0.0;
-        return;
-    }
-    unsigned long long mb = a.maxbits;
-    if (mb != 0 && (mb >> 52) == 0) {
-        // every high word zero or subnormal: the exact maximum decides the exponent
-        mb = 0;
-        for (int64_t p = 0; p < K; ++p) {
-            const unsigned long long v =
-                static_cast<unsigned long long>(__double_as_longlong(X[r * sr + p * sp])) & 0x7fffffffffffffffull;
-            mb = v > mb ? v : mb;
-        }
-    }
-    const double mx = __longlong_as_double(static_cast<long long>(mb));
-    int e = 0;
-    if (mx > 0.0) frexp(mx, &e);
-    double q = ldexp(a.sumsq, -2 * e);
-    if (mx > 0.0 && (e > 500 || e < -500)) {
-        q = 0.0;
-        for (int64_t p = 0; p < K; ++p) {
-            const double v = ldexp(X[r * sr + p * sp], -e);
-            q = fma(v, v, q);
-        }
-    }
-    rexp[r] = e;
-    rsq[r] = q;
-}
-
-// Both operands of a product go through one launch: blocks with blockIdx.y < yb0 work on A (its
-// rows), the others on B (its columns), so the two passes overlap on the device.
-struct OperandPair {
-    const double* X[2];
-    int64_t R[2], sr[2], sp[2];
-    RowAcc* acc[2];
-    int* rexp[2];
-    double* rsq[2];
-    __nv_bfloat16* planes[2];
-    int64_t rpad[2];
-    unsigned yb0;  // row blocks of A
-};
-
-__global__ void __launch_bounds__(256, 4) stats_tile_kernel(const OperandPair op, int64_t K, int kt) {
-    const int w = blockIdx.y < op.yb0 ? 0 : 1;
-    const int by = w ? int(blockIdx.y - op.yb0) : int(blockIdx.y);
-    stats_rows(op.X[w], op.R[w], K, op.sr[w], op.sp[w], op.acc[w], by, kt);
-}
-
-// Per-block summary of the row statistics of one operand side, for split_info_kernel: Inf/NaN
-// flag, largest exponent E of the rows with q > 0 (kNoRows when none), largest q (its bit pattern:
-// non-negative doubles order like integers), s = sum 2^(2(e - E)) and nrm = sum 2^(2(e - E)) q.
-constexpr int kNoRows = -100000;
-struct RowPartial {
-    int bad, E;
-    long long Qbits;
-    double s, nrm;
-};
-
-__device__ double block_sum(double v, double* red);
-__device__ long long block_max_ll(long long v, long long* red);
-__device__ int block_max_int(int v, int* red);
-__device__ __forceinline__ double pow2i(int x);
-
-// blockIdx.x < xb0: rows of A, else columns of B (256 a block); with `part`, each block also
-// writes its RowPartial (part[blockIdx.x]).
-__global__ void __launch_bounds__(256) stats_finalize_pair_kernel(const OperandPair op, int64_t K, unsigned xb0,
-                                                                  RowPartial* __restrict__ part) {
-    const int w = blockIdx.x < xb0 ? 0 : 1;
-    const int64_t r = int64_t(w ? blockIdx.x - xb0 : blockIdx.x) * blockDim.x + threadIdx.x;
-    stats_finalize_row(op.X[w], op.R[w], K, op.sr[w], op.sp[w], op.acc[w], op.rexp[w], op.rsq[w], r);
-    if (part == nullptr) return;  // uniform over the launch
-    __shared__ double redd[32];
-    __shared__ int redi[32];
-    int e = kNoRows, bad = 0;
-    double q = 0.0;
-    if (r < op.R[w]) {
-        e = op.rexp[w][r];
-        q = op.rsq[w][r];
-        if (e == kNonFinite) {
-            bad = 1;
-            e = kNoRows;
-            q = 0.0;
-        }
-    }
-    const long long qb = __double_as_longlong(q);
-    RowPartial pr;
-    pr.bad = block_max_int(bad, redi);
-    pr.E = block_max_int(qb > 0 ? e : kNoRows, redi);
-    pr.Qbits = block_max_ll(qb, reinterpret_cast<long long*>(redd));
-    const double wgt = (qb > 0 && pr.E != kNoRows) ? pow2i(2 * (e - pr.E)) : 0.0;
-    pr.s = block_sum(wgt, redd);
-    pr.nrm = block_sum(wgt * q, redd);
-    if (threadIdx.x == 0) part[blockIdx.x] = pr;
-}
-
-// One block: norms, scale norms, slice count and bound.  Sums are formed relative to the largest
+// The plans: norms, slice count and bound, by one warp.  Sums come relative to the largest
 // row exponent, so the ratio rho = ||2^e|| ||2^f|| / (||A|| ||B||) is finite for any finite input.
 //
-// On GB300 every FP64 warp instruction occupies the narrow FP64 pipe for many cycles whatever the
-// number of active lanes, so these planning kernels keep FP64 work off long serial chains: block
-// sums finish in one warp's shuffles, and the searches below test 32 candidates per instruction.
-__device__ double block_sum(double v, double* red) {
-    __shared__ double total;
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        double t = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.0;
-        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-        if (threadIdx.x == 0) total = t;
-    }
-    __syncthreads();
-    return total;
-}
+// On GB300 every FP64 instruction of a warp holds its SM quarter's FP64 pipe for 64 clocks whatever the
+// number of active lanes, so the plan keeps FP64 work off serial chains: each function runs once with
+// a different argument in each lane, and the searches test 32 candidates per instruction.
 
 // Smallest b in [lo, hi] with ok(b), hi + 1 when there is none (ok false, then true as b grows):
 // the 32 lanes of the calling warp test 32 candidates at a time.
@@ -465,234 +487,122 @@ __device__ int warp_last_true(int lo, int hi, F ok) {
     return lo - 1;
 }
 
-__device__ long long block_max_ll(long long v, long long* red) {
-    for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    long long t = red[0];
-    for (int i = 1; i < int(blockDim.x >> 5); ++i) t = max(t, red[i]);
-    return t;
-}
-
-__device__ int block_max_int(int v, int* red) {
-    for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    int t = red[0];
-    for (int i = 1; i < int(blockDim.x >> 5); ++i) t = max(t, red[i]);
-    return t;
-}
-
-// 2^x for an integer x <= 0 from the bit pattern (0 below the normal range, where the weight of a
-// row in a norm sum no longer matters)
+// 2^x for an integer x <= 0 from the bit pattern (0 below the normal range)
 __device__ __forceinline__ double pow2i(int x) {
     return x < -1022 ? 0.0 : __longlong_as_double((long long)(x + 1023) << 52);
 }
 
-// One warp: the partials are few (one per 256 rows or columns), and the shuffle reductions need no
-// barriers.  A block of 1024 threads spent most of the kernel's 25 us in the barriers and the
-// serial combining steps of nine block-wide reductions.
-__device__ __forceinline__ int warp_max(int v) {
-    for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-__device__ __forceinline__ long long warp_max(long long v) {
-    for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-__device__ __forceinline__ double warp_sum(double v) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
+// The fewest moduli, two at least and `cap` at most, whose product is at least `need`.
+__device__ __forceinline__ int moduli_for(double need, int cap) {
+    const int first = warp_first_true(2, MAX_MODULI, [&](int n) { return c_mod_prod[n] >= need; });
+    return max(2, min(cap, first));
 }
 
-__global__ void __launch_bounds__(32) split_info_kernel(const RowPartial* __restrict__ part, int nA, int nB, int64_t k,
-                                                         int mode, int fixed_slices, int cap_planes, double target,
-                                                         SplitInfo* info) {
-    // the per-block partials of A (the first nA) and B: Inf/NaN flag, largest exponents, largest
-    // row / column sums of squares relative to 2^(2e)
-    int bad = 0, EA = kNoRows, EB = kNoRows;
-    long long QAb = 0, QBb = 0;
-    for (int i = threadIdx.x; i < nA + nB; i += 32) {
-        const RowPartial p = part[i];
-        bad |= p.bad;
-        if (i < nA) {
-            EA = max(EA, p.E);
-            QAb = max(QAb, p.Qbits);
-        } else {
-            EB = max(EB, p.E);
-            QBb = max(QBb, p.Qbits);
-        }
-    }
-    bad = warp_max(bad);
-    EA = warp_max(EA);
-    EB = warp_max(EB);
-    const double QA = __longlong_as_double(warp_max(QAb));
-    const double QB = __longlong_as_double(warp_max(QBb));
-    // the sums relative to the largest exponent: each block's relative to its own, rescaled by an
-    // exact power of two
-    double sa = 0, na = 0, sb = 0, nb = 0;
-    for (int i = threadIdx.x; i < nA + nB; i += 32) {
-        const RowPartial p = part[i];
-        if (p.E == kNoRows) continue;
-        if (i < nA) {
-            const double w = pow2i(2 * (p.E - EA));
-            sa += w * p.s;
-            na += w * p.nrm;
-        } else {
-            const double w = pow2i(2 * (p.E - EB));
-            sb += w * p.s;
-            nb += w * p.nrm;
-        }
-    }
-    sa = warp_sum(sa);
-    na = warp_sum(na);
-    sb = warp_sum(sb);
-    nb = warp_sum(nb);
-    if (threadIdx.x < 32) {  // warp 0 plans; lane 0 writes
-        const int lane = threadIdx.x;
-        // Each FP64 function below runs once for the warp with a different argument in each lane
-        // (the cost of one evaluation, same operations as one at a time): lanes 0-3 the norms, 4-5
-        // sqrt(k s / n), 6-7 sqrt(Q (1 + 2^-10)), 8 sqrt(k), 9-10 sqrt(s / n).
-        double num = 0.0, den = 1.0;
-        switch (lane) {
-            case 0: num = na; break;
-            case 1: num = nb; break;
-            case 2: num = sa; break;
-            case 3: num = sb; break;
-            case 4: num = double(k) * sa; den = na > 0 ? na : 1.0; break;
-            case 5: num = double(k) * sb; den = nb > 0 ? nb : 1.0; break;
-            case 6: num = QA * (1.0 + 0x1p-10); break;
-            case 7: num = QB * (1.0 + 0x1p-10); break;
-            case 8: num = double(k); break;
-            case 9: num = sa; den = na > 0 ? na : 1.0; break;
-            case 10: num = sb; den = nb > 0 ? nb : 1.0; break;
-            default: break;
-        }
-        const double root = sqrt(num / den);
-        const double scaled = ldexp(root, (lane == 0 || lane == 2) ? EA : EB);  // lanes 0-3
-        auto from = [&](double v, int l) { return __shfl_sync(0xffffffffu, v, l); };
-        const double nA_ = from(scaled, 0), nB_ = from(scaled, 1), sA_ = from(scaled, 2), sB_ = from(scaled, 3);
-        const double rAk = from(root, 4), rBk = from(root, 5), sqa = from(root, 6), sqb = from(root, 7);
-        const double sqk = from(root, 8), ra = from(root, 9), rb = from(root, 10);
-        SplitInfo r;
-        r.nonfinite = bad;
-        r.normA = (na > 0) ? nA_ : 0.0;
-        r.normB = (nb > 0) ? nB_ : 0.0;
-        r.scaleA = (sa > 0) ? sA_ : 0.0;
-        r.scaleB = (sb > 0) ? sB_ : 0.0;
-        const double rho = (na > 0 && nb > 0) ? ra * rb : 0.0;
-        if (mode == kCrt) {
-            // operands rounded to beta-bit integers: |dA_ip| <= 2^(e_i-beta-1), so
-            // ||dC||_F/(||A|| ||B||) <= 2^(-beta-1)(rA + rB) + 2^(-2beta-2) rA rB + 2^-52 with
-            // rA = sqrt(k) ||2^e|| / ||A|| (and 2^-52 for the final conversion and the alpha scaling)
-            const double rA = (na > 0) ? rAk : 0.0;
-            const double rB = (nb > 0) ? rBk : 0.0;
-            auto bnd = [&](int b) {
-                return pow2i(-b - 1) * (rA + rB) + pow2i(-2 * b - 2) * rA * rB + pow2i(-52);
-            };
-            // the smallest beta in [1, 55] that meets the target (beta <= 55 keeps |A'| < 2^56, the
-            // range of the residue extraction)
-            int beta = min(55, warp_first_true(1, 54, [&](int b) { return bnd(b) <= target; }));
-            // The scaled rows satisfy ||A'_i|| <= 2^beta sqrt(Q_A) + sqrt(k)/2 (the rounding adds
-            // at most 1/2 per entry), so by Cauchy-Schwarz every exact product entry T has
-            // |T| <= (2^beta sqrt(Q_A) + sqrt(k)/2)(2^beta sqrt(Q_B) + sqrt(k)/2).  The moduli's
-            // product P must exceed 2.125 |T| (symmetric residues, with room for the FP32 quotient
-            // estimate of the reconstruction); Q carries a 2^-10 allowance for its own rounding.
-            const double hk = 0.5 * sqk;
-            auto need = [&](int b) {
-                const double x = ldexp(sqa, b) + hk, y = ldexp(sqb, b) + hk;
-                return 1.0875 + log2(x) + log2(y);
-            };
-            // lanes 0-1: the two factors of need(beta); lanes 2-3: log2 sqa and log2 sqb
-            const double lg = log2(ldexp((lane & 1) ? sqb : sqa, lane < 2 ? beta : 0) + (lane < 2 ? hk : 0.0));
-            const double lg0 = from(lg, 0), lg1 = from(lg, 1), lsqa = from(lg, 2), lsqb = from(lg, 3);
-            double have = 0.0;
-            // a fixed count is used as given (at least two); otherwise the fewest that carry the
-            // target, within the planes the host sized for
-            int N = 0;
-            const int nfix = fixed_slices > 0 ? (fixed_slices < 2 ? 2 : fixed_slices) : 0;
-            const double need0 = 1.0875 + lg0 + lg1;  // need(beta)
-            while (nfix ? N < nfix : (N < 2 || (N < cap_planes && have < need0))) {
-                have += c_mod_log2[N];
-                ++N;
-            }
-            // the moduli chosen may carry more bits than needed: round to as many bits as they allow.
-            // need(b) exceeds 1.0875 + 2b + log2(sqa sqb), so no b above b0 qualifies: the largest b
-            // in (-60, b0] with need(b) <= have, -60 when none
-            int bhi = 55;
-            if (sqa > 0 && sqb > 0) {
-                const int b0 = int(floor((have - 1.0875 - lsqa - lsqb) / 2.0));
-                bhi = b0 < 55 ? (b0 > -60 ? b0 : -60) : 55;
-            }
-            beta = warp_last_true(-59, bhi, [&](int b) { return need(b) <= have; });
-            r.slices = N;
-            r.beta = beta;
-            r.beta_b = beta;
-            r.qmaxB = QB;
-            // a beta the search found has need(beta) <= have; -60 (none found) was not tested.  Too
-            // few moduli for even the coarsest rounding: no bound
-            const bool fits = beta >= -59 || need(beta) <= have;
-            r.bound = fits ? bnd(beta) : __longlong_as_double(0x7ff0000000000000ll);
-        } else if (mode == kExact) {
-            int S = fixed_slices;
-            if (S <= 0) {
-                S = MAX_SLICES;
-                for (int s = 2; s <= MAX_SLICES; ++s) {
-                    const double b = (s + 1) * double(k) * ldexp(1.0, -8 * s) * rho + (s + 3) * ldexp(1.0, -53);
-                    if (b <= target) { S = s; break; }
-                }
-            }
-            r.slices = S;
-            r.bound = (S + 1) * double(k) * ldexp(1.0, -8 * S) * rho + (S + 3) * ldexp(1.0, -53);
-        } else if (mode == kBf16) {
-            // each operand rounded to 8 significant bits, FP32 accumulation
-            r.slices = 1;
-            r.bound = 2.0 * ldexp(1.0, -8) + double(k) * ldexp(1.0, -24);
-        } else {
-            // hi/lo split keeps 16 bits; the dropped lo*lo term and the FP32 accumulation remain
-            r.slices = 2;
-            r.bound = 3.0 * ldexp(1.0, -16) + double(k) * ldexp(1.0, -24);
-        }
-        if (threadIdx.x == 0) *info = r;
-    }
-}
+// floor(log2 |x|) of a normal x.
+__device__ __forceinline__ int exponent_of(double x) { return int((__double2hiint(x) >> 20) & 0x7ff) - 1023; }
 
-// ---- panel pipeline (host operands): B is sliced ahead of A -----------------------------------
-// Block-wide statistics of one operand side from its row exponents e and relative sums of squares
-// q: Inf/NaN flag, largest exponent E, largest q, s = sum 2^(2(e-E)) and nrm = sum 2^(2(e-E)) q.
-struct SideStats {
-    int bad, E;
-    double Q, s, nrm;
-};
-
-__device__ SideStats side_stats(const int* __restrict__ e, const double* __restrict__ q, int64_t count, double* redd,
-                                int* redi) {
-    SideStats r;
-    int bad = 0, E = -100000;
-    long long Qb = 0;  // non-negative doubles: their bit patterns order like integers
-    for (int64_t i = threadIdx.x; i < count; i += blockDim.x) {
-        if (e[i] == kNonFinite) bad = 1;
-        else {
-            const long long qb = __double_as_longlong(q[i]);
-            if (qb > 0) E = max(E, e[i]);
-            Qb = max(Qb, qb);
+__device__ void plan_product(const RowPartial& A, const RowPartial& B, int64_t k, const PlanArgs& plan) {
+    const int lane = threadIdx.x & 31, EA = A.E, EB = B.E, bad = A.bad | B.bad;
+    const double QA = A.Q, QB = B.Q, sa = A.s, na = A.nrm, sb = B.s, nb = B.nrm;
+    const int mode = plan.mode, fixed_slices = plan.fixed_slices, cap_planes = plan.cap_planes;
+    const double target = plan.target;
+    // Each FP64 function below runs once for the warp with a different argument in each lane
+    // (the cost of one evaluation, same operations as one at a time): lanes 0-3 the norms, 4-5
+    // sqrt(k s / n), 6-7 sqrt(Q (1 + 2^-10)), 8 sqrt(k), 9-10 sqrt(s / n).
+    double num = 1.0, den = 1.0;  // one, not zero, in the idle lanes: zeros take the functions' slow paths
+    switch (lane) {
+        case 0: num = na; break;
+        case 1: num = nb; break;
+        case 2: num = sa; break;
+        case 3: num = sb; break;
+        case 4: num = double(k) * sa; den = na > 0 ? na : 1.0; break;
+        case 5: num = double(k) * sb; den = nb > 0 ? nb : 1.0; break;
+        case 6: num = QA * (1.0 + 0x1p-10); break;
+        case 7: num = QB * (1.0 + 0x1p-10); break;
+        case 8: num = double(k); break;
+        case 9: num = sa; den = na > 0 ? na : 1.0; break;
+        case 10: num = sb; den = nb > 0 ? nb : 1.0; break;
+        default: break;
+    }
+    const double root = sqrt(num / den);
+    const double scaled = ldexp(root, (lane == 0 || lane == 2) ? EA : EB);  // lanes 0-3
+    auto from = [&](double v, int l) { return __shfl_sync(0xffffffffu, v, l); };
+    const double nA_ = from(scaled, 0), nB_ = from(scaled, 1), sA_ = from(scaled, 2), sB_ = from(scaled, 3);
+    const double rAk = from(root, 4), rBk = from(root, 5), sqa = from(root, 6), sqb = from(root, 7);
+    const double sqk = from(root, 8), ra = from(root, 9), rb = from(root, 10);
+    SplitInfo r;
+    r.nonfinite = bad;
+    r.normA = (na > 0) ? nA_ : 0.0;
+    r.normB = (nb > 0) ? nB_ : 0.0;
+    r.scaleA = (sa > 0) ? sA_ : 0.0;
+    r.scaleB = (sb > 0) ? sB_ : 0.0;
+    const double rho = (na > 0 && nb > 0) ? ra * rb : 0.0;
+    if (mode == kCrt) {
+        // operands rounded to beta-bit integers: |dA_ip| <= 2^(e_i-beta-1), so
+        // ||dC||_F/(||A|| ||B||) <= 2^(-beta-1)(rA + rB) + 2^(-2beta-2) rA rB + 2^-52 with
+        // rA = sqrt(k) ||2^e|| / ||A|| (and 2^-52 for the final conversion and the alpha scaling)
+        const double rA = (na > 0) ? rAk : 0.0;
+        const double rB = (nb > 0) ? rBk : 0.0;
+        auto bnd = [&](int b) {
+            return pow2i(-b - 1) * (rA + rB) + pow2i(-2 * b - 2) * rA * rB + pow2i(-52);
+        };
+        // the smallest beta in [1, 55] that meets the target (beta <= 55 keeps |A'| < 2^56, the
+        // range of the residue extraction); below `lo` the first term alone exceeds it
+        int lo = 1;
+        if (rA + rB > 0.0 && target > 0x1p-1000) lo = exponent_of(rA + rB) - exponent_of(target) - 2;
+        int beta = min(55, warp_first_true(max(1, min(lo, 54)), 54, [&](int b) { return bnd(b) <= target; }));
+        // The scaled rows satisfy ||A'_i|| <= 2^beta sqrt(Q_A) + sqrt(k)/2 (the rounding adds
+        // at most 1/2 per entry), so by Cauchy-Schwarz every exact product entry T has
+        // |T| <= (2^beta sqrt(Q_A) + sqrt(k)/2)(2^beta sqrt(Q_B) + sqrt(k)/2).  The moduli's
+        // product P must exceed 2.125 |T| (symmetric residues, with room for the FP32 quotient
+        // estimate of the reconstruction); Q carries a 2^-10 allowance for its own rounding.
+        const double hk = 0.5 * sqk;
+        auto need = [&](int b) {
+            const double p2 = __hiloint2double((b + 1023) << 20, 0);
+            return kModMargin * fma(sqa, p2, hk) * fma(sqb, p2, hk);
+        };
+        // a fixed count is used as given (at least two); otherwise the fewest that carry the
+        // target, within the planes the host sized for
+        const int N = fixed_slices > 0 ? max(2, fixed_slices) : moduli_for(need(beta), cap_planes);
+        const double have = c_mod_prod[N];
+        // the moduli chosen may carry more bits than needed: round to as many bits as they allow.
+        // need(b) exceeds 2 4^b sqa sqb, so no b above b0 qualifies: the largest b in (-60, b0] with
+        // need(b) <= have, -60 when none
+        int bhi = 55;
+        if (sqa > 0 && sqb > 0) {
+            const int b0 = (exponent_of(have) - exponent_of(sqa) - exponent_of(sqb)) >> 1;
+            bhi = b0 < 55 ? (b0 > -60 ? b0 : -60) : 55;
         }
+        beta = warp_last_true(-59, bhi, [&](int b) { return need(b) <= have; });
+        r.slices = N;
+        r.beta = beta;
+        r.beta_b = beta;
+        r.qmaxB = QB;
+        // a beta the search found has need(beta) <= have; -60 (none found) was not tested.  Too
+        // few moduli for even the coarsest rounding: no bound
+        const bool fits = beta >= -59 || need(beta) <= have;
+        r.bound = fits ? bnd(beta) : __longlong_as_double(0x7ff0000000000000ll);
+    } else if (mode == kExact) {
+        int S = fixed_slices;
+        if (S <= 0) {
+            S = MAX_SLICES;
+            for (int s = 2; s <= MAX_SLICES; ++s) {
+                const double b = (s + 1) * double(k) * ldexp(1.0, -8 * s) * rho + (s + 3) * ldexp(1.0, -53);
+                if (b <= target) { S = s; break; }
+            }
+        }
+        r.slices = S;
+        r.bound = (S + 1) * double(k) * ldexp(1.0, -8 * S) * rho + (S + 3) * ldexp(1.0, -53);
+    } else if (mode == kBf16) {
+        // each operand rounded to 8 significant bits, FP32 accumulation
+        r.slices = 1;
+        r.bound = 2.0 * ldexp(1.0, -8) + double(k) * ldexp(1.0, -24);
+    } else {
+        // hi/lo split keeps 16 bits; the dropped lo*lo term and the FP32 accumulation remain
+        r.slices = 2;
+        r.bound = 3.0 * ldexp(1.0, -16) + double(k) * ldexp(1.0, -24);
     }
-    r.bad = block_max_int(bad, redi);
-    r.E = block_max_int(E, redi);
-    r.Q = __longlong_as_double(block_max_ll(Qb, reinterpret_cast<long long*>(redd)));
-    double sv = 0, nv = 0;
-    for (int64_t i = threadIdx.x; i < count; i += blockDim.x) {
-        if (e[i] == kNonFinite || q[i] <= 0.0) continue;
-        const double w = pow2i(2 * (e[i] - r.E));
-        sv += w;
-        nv += w * q[i];
-    }
-    r.s = block_sum(sv, redd);
-    r.nrm = block_sum(nv, redd);
-    return r;
+    if (lane == 0) *plan.info = r;
 }
 
 // One operand side of a block of the host pipeline (a row panel of A or a column block of B): its
@@ -700,25 +610,25 @@ __device__ SideStats side_stats(const int* __restrict__ e, const double* __restr
 // smallest beta with 2^(-beta-1) r <= target / 2: each side takes half of the bound for its own
 // rounding, so the two sides are sliced independently.  `slices` = the planes the side is sliced
 // into (the host's largest modulus count).
-__global__ void __launch_bounds__(1024) split_side_kernel(const int* __restrict__ e, const double* __restrict__ q,
-                                                          int64_t count, int64_t k, int planes, double target,
-                                                          SplitInfo* out) {
-    __shared__ double redd[32];
-    __shared__ int redi[32];
-    const SideStats t = side_stats(e, q, count, redd, redi);
-    if (threadIdx.x < 32) {  // warp 0 plans; lane 0 writes
-        SplitInfo r;
-        r.nonfinite = t.bad;
-        r.normA = r.normB = (t.nrm > 0) ? ldexp(sqrt(t.nrm), t.E) : 0.0;
-        r.scaleA = r.scaleB = (t.s > 0) ? ldexp(sqrt(t.s), t.E) : 0.0;
-        r.qmaxA = r.qmaxB = t.Q;
-        const double rr = (t.nrm > 0) ? sqrt(double(k) * t.s / t.nrm) : 0.0;
-        const int beta = min(55, warp_first_true(1, 54, [&](int b) { return pow2i(-b - 1) * rr <= 0.5 * target; }));
-        r.beta = r.beta_b = beta;
-        r.slices = planes;
-        r.bound = 0.0;
-        if (threadIdx.x == 0) *out = r;
-    }
+__device__ void plan_side(const RowPartial& S, int64_t k, const PlanArgs& plan) {
+    const int lane = threadIdx.x & 31;
+    const double s = S.s, nrm = S.nrm;
+    // lane 0 the norm, 1 the scale, 2 sqrt(k s / nrm)
+    const double root = sqrt((lane == 0 ? nrm : lane == 1 ? s : double(k) * s) / (lane == 2 && nrm > 0 ? nrm : 1.0));
+    const double scaled = ldexp(root, S.E);
+    SplitInfo r;
+    r.nonfinite = S.bad;
+    r.normA = r.normB = nrm > 0 ? __shfl_sync(0xffffffffu, scaled, 0) : 0.0;
+    r.scaleA = r.scaleB = s > 0 ? __shfl_sync(0xffffffffu, scaled, 1) : 0.0;
+    r.qmaxA = r.qmaxB = S.Q;
+    const double rr = nrm > 0 ? __shfl_sync(0xffffffffu, root, 2) : 0.0;
+    int lo = 1;
+    if (rr > 0.0 && plan.target > 0x1p-1000) lo = exponent_of(rr) - exponent_of(plan.target) - 1;
+    r.beta = r.beta_b = min(55, warp_first_true(max(1, min(lo, 54)), 54,
+                                                [&](int b) { return pow2i(-b - 1) * rr <= 0.5 * plan.target; }));
+    r.slices = plan.cap_planes;
+    r.bound = 0.0;
+    if (lane == 0) *plan.info = r;
 }
 
 // A block (row panel i of A, column block j of B) from the two sides: the moduli that carry
@@ -728,7 +638,6 @@ __global__ void __launch_bounds__(1024) split_side_kernel(const int* __restrict_
 // moduli are too few).
 __global__ void split_block_kernel(const SplitInfo* __restrict__ ia, const SplitInfo* __restrict__ ib, int64_t k,
                                    int cap_planes, SplitInfo* out) {
-    if (threadIdx.x != 0) return;
     const SplitInfo A = *ia, B = *ib;
     SplitInfo r;
     r.nonfinite = A.nonfinite | B.nonfinite;
@@ -738,24 +647,23 @@ __global__ void split_block_kernel(const SplitInfo* __restrict__ ia, const Split
     r.normB = B.normB;
     r.scaleB = B.scaleB;
     r.qmaxB = B.qmaxB;
-    const double rA = (A.normA > 0) ? sqrt(double(k)) * A.scaleA / A.normA : 0.0;
-    const double rB = (B.normB > 0) ? sqrt(double(k)) * B.scaleB / B.normB : 0.0;
+    // lanes 0, 1: r_A and r_B; 2, 3: the square roots of the Qs; 4: sqrt(k), one evaluation each
+    const int lane = threadIdx.x;
+    const double root = sqrt(lane == 2 ? A.qmaxA * (1.0 + 0x1p-10) : lane == 3 ? B.qmaxB * (1.0 + 0x1p-10) : double(k));
+    const double ratio = lane == 0 ? (A.normA > 0 ? A.scaleA / A.normA : 0.0) : (B.normB > 0 ? B.scaleB / B.normB : 0.0);
+    auto from = [&](double v, int l) { return __shfl_sync(0xffffffffu, v, l); };
+    const double rA = from(root * ratio, 0), rB = from(root * ratio, 1);
     const int ba = A.beta, bb = B.beta_b;
-    const double hk = 0.5 * sqrt(double(k));
-    const double need = 1.0875 + log2(ldexp(sqrt(A.qmaxA * (1.0 + 0x1p-10)), ba) + hk) +
-                        log2(ldexp(sqrt(B.qmaxB * (1.0 + 0x1p-10)), bb) + hk);
-    double have = 0.0;
-    int N = 0;
-    while (N < 2 || (N < cap_planes && have < need)) {
-        have += c_mod_log2[N];
-        ++N;
-    }
+    const double hk = 0.5 * from(root, 4);
+    const double need = kModMargin * (ldexp(from(root, 2), ba) + hk) * (ldexp(from(root, 3), bb) + hk);
+    const int N = moduli_for(need, cap_planes);
+    const double have = c_mod_prod[N];
     r.slices = N;
     r.beta = ba;
     r.beta_b = bb;
     r.bound = need > have ? __longlong_as_double(0x7ff0000000000000ll)
                           : pow2i(-ba - 1) * rA + pow2i(-bb - 1) * rB + pow2i(-ba - bb - 2) * rA * rB + pow2i(-52);
-    *out = r;
+    if (lane == 0) *out = r;
 }
 
 // Summary of the blocks for the caller: the largest modulus count and bound (infos `stride` bytes
@@ -836,17 +744,28 @@ __device__ __forceinline__ void write_planes(const U_t (&V)[8], const bool (&neg
     }
 }
 
+// 64-bit shifts whose counts above 63 give zero.
+__device__ __forceinline__ unsigned long long shl64(unsigned long long v, int n) {
+    unsigned long long r;
+    asm("shl.b64 %0, %1, %2;" : "=l"(r) : "l"(v), "r"(n));
+    return r;
+}
+__device__ __forceinline__ unsigned long long shr64(unsigned long long v, int n) {
+    unsigned long long r;
+    asm("shr.u64 %0, %1, %2;" : "=l"(r) : "l"(v), "r"(n));
+    return r;
+}
+
 // |round(a * 2^sh)| for a finite double given by its bits (round half up); the result must fit in
-// 56 bits, which the CRT plan guarantees (beta <= 55 and |a| < 2^e).
+// 56 bits, which the CRT plan guarantees (beta <= 55 and |a| < 2^e).  The mantissa, 10 bits up (below
+// 2^63), goes down by n = 10 minus its exponent, from n = 64 on to zero; n is at least 8 for normal
+// numbers, and only a subnormal one in a row of subnormals goes up instead.
 __device__ __forceinline__ unsigned long long int_magnitude(unsigned long long bits, int sh_total) {
     const int eb = int((bits >> 52) & 0x7ff);
-    const unsigned long long mant = bits & 0xfffffffffffffull;
-    const unsigned long long M = eb ? (mant | (1ull << 52)) : mant;
-    const int sh = (eb ? eb : 1) - 1075 + sh_total;
-    if (M == 0) return 0;
-    if (sh >= 0) return M << sh;
-    if (sh > -64) return (M + (1ull << (-sh - 1))) >> (-sh);
-    return 0;
+    const unsigned long long M = (bits & 0xfffffffffffffull) | (eb ? 1ull << 52 : 0ull);
+    const int n = 1085 - max(eb, 1) - sh_total;
+    if (n <= 0) return shl64(M << 10, -n);
+    return shr64((M << 10) + shl64(1ull, n - 1), n);
 }
 
 // x mod p for x < 2^32 and p <= 257 with inv = floor(2^32 / p): the quotient estimate is at most
@@ -862,7 +781,8 @@ __device__ __forceinline__ uint32_t mod_small(uint32_t x, uint32_t p, uint32_t i
 // A modulus' constants as packed pairs (k_3, k_2, k_1 = symmetric residues of 2^42, 2^28, 2^14;
 // fl(1/p); -p), in shared memory: three 16-byte reads a modulus serve eight elements, and the packed
 // arithmetic takes half the instructions that bound this pass (8192^3 at 12 moduli 750 -> 725 us, 5.9 TB/s; 403 x 517 x 389
-// 20 -> 7.6 us with the smaller blocks of tiles_per_block).
+// 20 -> 8 us with the smaller blocks of tiles_per_block; 61 % of the issue slots busy, so the planes'
+// writes bound it now).
 struct __align__(16) SliceConst {
     ulonglong2 k32, k1_inv, pneg;
 };
@@ -873,30 +793,50 @@ __device__ __forceinline__ void slice_emit(const unsigned long long (&xv)[8], in
     if (mode == kCrt) {
         const int N = sl, beta = bt;
         // U = |round(a 2^(beta-e))| < 2^56 in signed FP32 chunks (the sign of a applied to each), two
-        // elements to a packed pair
+        // elements to a packed pair.  H = 2 U + (0 or 1): the mantissa with its implicit bit, 3 bits up,
+        // goes down to one bit below the rounding point, and adding one there rounds half up; counts
+        // above 63 leave nothing.  A zero or subnormal element of such a row ends there too; a row of
+        // numbers below 2^-960 takes the general int_magnitude.  About twenty integer
+        // instructions an element.
+        // (Rows with Inf / NaN have e = kNonFinite and come out as zeros.)
         uint64_t w0[4], w1[4], w2[4], w3[4];
+        unsigned long long Hs[8];
+        if (e < -960) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) Hs[q] = int_magnitude(xv[q], beta - e) << 1;
+        } else {
+            const int down = 1077 - beta + e;  // shift count for a biased exponent of zero
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const uint32_t hi = uint32_t(xv[q] >> 32), lo = uint32_t(xv[q]);
+                const uint32_t vh = (__funnelshift_l(lo, hi, 3) & 0x007fffffu) | 0x00800000u;
+                Hs[q] = shr64(((unsigned long long)vh << 32) | (lo << 3), down - int((hi >> 20) & 0x7ffu)) + 1ull;
+            }
+        }
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            uint32_t c[4][2];
-            float sg[2], off[2];
+            uint32_t c[4][2], sign[2];
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const unsigned long long bits = bad ? 0ull : xv[2 * q + h];
-                const unsigned long long U = int_magnitude(bits, beta - e);
-                sg[h] = (bits >> 63) ? -1.f : 1.f;
-                off[h] = (bits >> 63) ? 8388608.f : -8388608.f;
-                c[0][h] = 0x4B000000u | (uint32_t(U) & 0x3fffu);
-                c[1][h] = 0x4B000000u | (uint32_t(U >> 14) & 0x3fffu);
-                c[2][h] = 0x4B000000u | (uint32_t(U >> 28) & 0x3fffu);
-                c[3][h] = 0x4B000000u | uint32_t(U >> 42);
+                const unsigned long long H = Hs[2 * q + h];
+                const uint32_t hi = uint32_t(xv[2 * q + h] >> 32);
+                const uint32_t hh = uint32_t(H >> 32), hl = uint32_t(H);
+                sign[h] = hi & 0x80000000u;
+                c[0][h] = 0x4B000000u | ((hl >> 1) & 0x3fffu);
+                c[1][h] = 0x4B000000u | ((hl >> 15) & 0x3fffu);
+                c[2][h] = 0x4B000000u | (__funnelshift_r(hl, hh, 29) & 0x3fffu);
+                c[3][h] = 0x4B000000u | (hh >> 11);
             }
-            const uint64_t sg2 = f32x2(sg[0], sg[1]), off2 = f32x2(off[0], off[1]);
+            // chunk c = 2^23 + w: +-(c - 2^23)
+            const uint64_t sg2 = f32x2_bits(0x3f800000u | sign[0], 0x3f800000u | sign[1]);
+            const uint64_t off2 = f32x2_bits(0xcb000000u ^ sign[0], 0xcb000000u ^ sign[1]);
             w0[q] = fma2(f32x2_bits(c[0][0], c[0][1]), sg2, off2);
             w1[q] = fma2(f32x2_bits(c[1][0], c[1][1]), sg2, off2);
             w2[q] = fma2(f32x2_bits(c[2][0], c[2][1]), sg2, off2);
             w3[q] = fma2(f32x2_bits(c[3][0], c[3][1]), sg2, off2);
         }
         const uint64_t magic = f32x2(MAGIC, MAGIC), nmagic = f32x2(-MAGIC, -MAGIC);
+#pragma unroll 1
         for (int t = 0; t < N; ++t) {
             const ulonglong2 k32 = tab[t].k32, k1i = tab[t].k1_inv;
             const uint64_t pneg = tab[t].pneg.x;
@@ -973,11 +913,11 @@ __device__ __forceinline__ void slice_rows(int which, const double* __restrict__
     const int e = (r < R) ? rexp[r] : 0;
     const bool bad = (mode == kExact || mode == kCrt) && e == kNonFinite;
     const int64_t pstride = rpad * kpad;
-    const TileSrc ts = tile_src(X, sr, sp, r0);
-    if (tb < te) tile_issue(s0, ts, X, R, K, r0, tb, off);
+    const bool vec = rows_vec(X, sr, sp);
+    if (tb < te) tile_issue(s0, X, R, K, sr, sp, vec, r0, tb, off);
     for (int64_t it = tb; it < te; ++it) {
         const int b = int(it - tb) & 1;
-        if (it + 1 < te) tile_issue(s0 + uint32_t(b ^ 1) * BUF, ts, X, R, K, r0, it + 1, off);
+        if (it + 1 < te) tile_issue(s0 + uint32_t(b ^ 1) * BUF, X, R, K, sr, sp, vec, r0, it + 1, off);
         else cp_async_commit();  // an empty group keeps the wait count uniform
         cp_async_wait1();
         __syncthreads();
@@ -1626,7 +1566,7 @@ struct CrtCombine {
     const uint8_t* res;      // residue planes
     int64_t mpad, npad;
     int nseg, max_levels;
-    int64_t col0;            // first column of this launch in the planes, eB and C
+    int64_t row0, col0;      // first row and column of this launch in the planes, the exponents and C
     int64_t m, n;            // rows, columns of this launch
     const int *eA, *eB;
     double alpha, beta;
@@ -1641,13 +1581,14 @@ __device__ __forceinline__ void crt_rows(const CrtCombine& p, int scale, int64_t
     const int64_t S = p.mpad * p.npad, step = int64_t(gridDim.y) * p.npad;
     const bool plain = p.alpha == 1.0 && p.beta == 0.0;
     const bool pairs = j0 + 4 <= p.n && (p.ldc & 1) == 0 && (reinterpret_cast<uintptr_t>(p.C + p.col0) & 15) == 0;
-    int64_t i = blockIdx.y, off = i * p.npad + p.col0 + j0;
-    if (i >= p.m) return;
+    int64_t i = p.row0 + blockIdx.y, off = i * p.npad + p.col0 + j0;
+    const int64_t end = p.row0 + p.m;
+    if (i >= end) return;
     CrtWords<N> w = crt_load<N>(p.res, S, p.max_levels, off);
     int ei = p.eA[i];
     while (true) {
         const int64_t inext = i + gridDim.y;
-        const bool more = inext < p.m;
+        const bool more = inext < end;
         CrtWords<N> wn = w;
         int en = ei;
         if (more) {
@@ -1942,6 +1883,34 @@ SplitGeometry split_geometry(const Gemm& g, const SplitRequest& req, int num_sms
     return G;
 }
 
+// Level planes of a product: int32 sums, FP32 tiles or, in the residue form, 16 bits for the first
+// modulus and a byte for each other one (crt_plane).
+size_t level_bytes(const SplitGeometry& G) {
+    const size_t S = size_t(G.nseg) * size_t(G.mpad) * size_t(G.npad);
+    return G.mode == kCrt ? S * size_t(G.max_levels + 1) : S * size_t(G.max_levels) * 4;
+}
+
+// Statistics buffers of `rows_a` rows of A and `rows_b` columns of B over k.  kSlotScaleA: exponents
+// (int), SplitInfo, one RowPartial per row block; kSlotScaleB: the counters, then the chunk partials.
+struct StatsLayout {
+    int kt, chunks;
+    int64_t blocks;  // row blocks of both
+    size_t off_info, off_group, bytes_a, off_part, bytes_b;
+};
+StatsLayout stats_layout(int64_t rows_a, int64_t rows_b, int64_t k, int num_sms) {
+    StatsLayout L;
+    L.blocks = (rows_a + 31) / 32 + (rows_b + 31) / 32;
+    const int64_t tiles = (k + 63) / 64;
+    L.kt = tiles_per_block(tiles, L.blocks, num_sms);
+    L.chunks = int((tiles + L.kt - 1) / L.kt);
+    L.off_info = size_t(round_up((rows_a + rows_b) * int64_t(sizeof(int)), 256));
+    L.off_group = L.off_info + (sizeof(SplitInfo) + 255) / 256 * 256;
+    L.bytes_a = L.off_group + size_t(L.blocks) * sizeof(RowPartial);
+    L.off_part = size_t(round_up((L.blocks + 1) * int64_t(sizeof(unsigned)), 256));
+    L.bytes_b = L.off_part + (L.chunks > 1 ? size_t(rows_a + rows_b) * size_t(L.chunks) * sizeof(uint2) : 0);
+    return L;
+}
+
 // Stored (row-major) shape of the operands of a logical product.
 void stored_a(const Gemm& g, int64_t* rows, int64_t* cols) { *rows = g.ta ? g.k : g.m; *cols = g.ta ? g.m : g.k; }
 void stored_b(const Gemm& g, int64_t* rows, int64_t* cols) { *rows = g.tb ? g.n : g.k; *cols = g.tb ? g.k : g.n; }
@@ -2007,12 +1976,10 @@ void device_product_slot_needs(const Gemm& g, const SplitRequest& req, size_t ne
     const SplitGeometry G = split_geometry(g, req, r.num_sms);
     need[kSlotSliceA] = rounded(size_t(G.max_planes) * size_t(G.mpad) * size_t(G.kpad) * 2);
     need[kSlotSliceB] = rounded(size_t(G.max_planes) * size_t(G.npad) * size_t(G.kpad) * 2);
-    need[kSlotLevels] = rounded(size_t(G.nseg) * G.max_levels * size_t(G.mpad) * size_t(G.npad) * 4);
-    const int64_t off_sq = round_up((g.m + g.n) * int64_t(sizeof(int)), 256);
-    const int64_t off_info = round_up(off_sq + (g.m + g.n) * int64_t(sizeof(double)), 256);
-    const size_t off_part = size_t(off_info) + ((sizeof(SplitInfo) + 255) / 256) * 256;
-    need[kSlotScaleA] = rounded(off_part + size_t((g.m + 255) / 256 + (g.n + 255) / 256) * sizeof(RowPartial));
-    need[kSlotScaleB] = rounded(size_t(g.m + g.n) * sizeof(RowAcc));
+    need[kSlotLevels] = rounded(level_bytes(G));
+    const StatsLayout SL = stats_layout(g.m, g.n, g.k, r.num_sms);
+    need[kSlotScaleA] = rounded(SL.bytes_a);
+    need[kSlotScaleB] = rounded(SL.bytes_b);
 }
 
 size_t device_product_footprint(const Gemm& g, const SplitRequest& req) {
@@ -2122,22 +2089,14 @@ int device_product(const Gemm& g_in, const SplitRequest& req, const LaunchCtl& c
     const size_t planesB = size_t(max_planes) * size_t(npad) * size_t(kpad);
     auto* pa = static_cast<__nv_bfloat16*>(ws.get(kSlotSliceA, planesA * 2, err));
     auto* pb = static_cast<__nv_bfloat16*>(ws.get(kSlotSliceB, planesB * 2, err));
-    auto* lv = static_cast<int32_t*>(
-        ws.get(kSlotLevels, size_t(nseg) * max_levels * size_t(mpad) * size_t(npad) * 4, err));
-    // statistics block: exponents (int), relative sums of squares (double), SplitInfo
-    const int64_t off_sq = round_up((m + n) * int64_t(sizeof(int)), 256);
-    const int64_t off_info = round_up(off_sq + (m + n) * int64_t(sizeof(double)), 256);
-    const int64_t off_part = off_info + int64_t((sizeof(SplitInfo) + 255) / 256) * 256;
-    const unsigned xb0 = unsigned((m + 255) / 256), xb1 = unsigned((n + 255) / 256);
-    const size_t stat_bytes = size_t(off_part) + size_t(xb0 + xb1) * sizeof(RowPartial);
-    auto* stats = static_cast<uint8_t*>(ws.get(kSlotScaleA, stat_bytes, err));
-    if (!pa || !pb || !lv || !stats) return GB300_ERR_NO_MEMORY;
+    auto* lv = static_cast<int32_t*>(ws.get(kSlotLevels, level_bytes(G), err));
+    const StatsLayout SL = stats_layout(m, n, k, r.num_sms);
+    auto* stats = static_cast<uint8_t*>(ws.get(kSlotScaleA, SL.bytes_a, err));
+    auto* scratch = static_cast<uint8_t*>(ws.get(kSlotScaleB, SL.bytes_b, err));
+    if (!pa || !pb || !lv || !stats || !scratch) return GB300_ERR_NO_MEMORY;
     int* eA = reinterpret_cast<int*>(stats);
     int* eB = eA + m;
-    double* sqA = reinterpret_cast<double*>(stats + off_sq);
-    double* sqB = sqA + m;
-    auto* info = reinterpret_cast<SplitInfo*>(stats + off_info);
-    auto* part = reinterpret_cast<RowPartial*>(stats + off_part);
+    auto* info = reinterpret_cast<SplitInfo*>(stats + SL.off_info);
 
     // operand strides of the logical R x K views
     const int64_t a_sr = g.ta ? 1 : g.lda, a_sp = g.ta ? g.lda : 1;
@@ -2145,29 +2104,29 @@ int device_product(const Gemm& g_in, const SplitRequest& req, const LaunchCtl& c
     const double* A = static_cast<const double*>(g.A);
     const double* B = static_cast<const double*>(g.B);
 
-    RowAcc* racc = static_cast<RowAcc*>(ws.get(kSlotScaleB, size_t(m + n) * sizeof(RowAcc), err));
-    if (!racc) return GB300_ERR_NO_MEMORY;
-    cudaMemsetAsync(racc, 0, size_t(m + n) * sizeof(RowAcc), st);
     OperandPair op;
     op.X[0] = A; op.X[1] = B;
     op.R[0] = m; op.R[1] = n;
     op.sr[0] = a_sr; op.sr[1] = b_sr;
     op.sp[0] = a_sp; op.sp[1] = b_sp;
-    op.acc[0] = racc; op.acc[1] = racc + m;
     op.rexp[0] = eA; op.rexp[1] = eB;
-    op.rsq[0] = sqA; op.rsq[1] = sqB;
     op.planes[0] = pa; op.planes[1] = pb;
     op.rpad[0] = mpad; op.rpad[1] = npad;
     op.yb0 = unsigned((m + 31) / 32);
     {
-        const int64_t yb = (m + 31) / 32 + (n + 31) / 32, tiles = (k + 63) / 64;
-        const int kt = tiles_per_block(tiles, yb, r.num_sms);
-        stats_tile_kernel<<<dim3(unsigned((tiles + kt - 1) / kt), unsigned(yb)), 256, 0, st>>>(op, k, kt);
-        stats_finalize_pair_kernel<<<xb0 + xb1, 256, 0, st>>>(op, k, xb0, part);
+        StatsArgs sa;
+        sa.op = op;
+        sa.K = k;
+        sa.kt = SL.kt;
+        sa.chunks = SL.chunks;
+        sa.count = reinterpret_cast<unsigned*>(scratch);
+        sa.part = reinterpret_cast<uint2*>(scratch + SL.off_part);
+        sa.group = reinterpret_cast<RowPartial*>(stats + SL.off_group);
+        const double target = req.target_error > 0 ? req.target_error : double(k) * 0x1p-53;
+        sa.plan = PlanArgs{kPlanProduct, mode, req.slices > 0 ? max_planes : 0, max_planes, target, info};
+        cudaMemsetAsync(sa.count, 0, size_t(SL.blocks + 1) * sizeof(unsigned), st);
+        stats_kernel<<<dim3(unsigned(SL.chunks), unsigned(SL.blocks)), 256, 0, st>>>(sa);
     }
-    const double target = req.target_error > 0 ? req.target_error : double(k) * 0x1p-53;
-    split_info_kernel<<<1, 32, 0, st>>>(part, int(xb0), int(xb1), k, mode, req.slices > 0 ? max_planes : 0,
-                                         max_planes, target, info);
     if (cudaError_t le = cudaGetLastError(); le != cudaSuccess) {
         if (err) *err = std::string("split pre-pass launch: ") + cudaGetErrorString(le);
         return GB300_ERR_CUDA;
@@ -2182,7 +2141,7 @@ int device_product(const Gemm& g_in, const SplitRequest& req, const LaunchCtl& c
                                : (mode == kExact ? slice_kernel<kExact> : (mode == kBf16 ? slice_kernel<kBf16> : slice_kernel<kBf16x3>));
         sk<<<grid, 256, 0, st>>>(sp2, k, info, kpad, kt);
     }
-    count_launches(4);
+    count_launches(2);
     if (cudaError_t le = cudaGetLastError(); le != cudaSuccess) {
         if (err) *err = std::string("split slicing launch: ") + cudaGetErrorString(le);
         return GB300_ERR_CUDA;
@@ -2235,7 +2194,7 @@ int device_product(const Gemm& g_in, const SplitRequest& req, const LaunchCtl& c
     };
     // reconstruction of C's columns [c0, c0 + nc) on stream s
     auto launch_crt_combine = [&](int64_t c0, int64_t nc, cudaStream_t s) {
-        const CrtCombine q{reinterpret_cast<const uint8_t*>(lv), mpad, npad, nseg, max_levels, c0, m, nc, eA, eB,
+        const CrtCombine q{reinterpret_cast<const uint8_t*>(lv), mpad, npad, nseg, max_levels, 0, c0, m, nc, eA, eB,
                            g.alpha, g.beta, static_cast<double*>(g.C), g.ldc};
         crt_combine_kernel<<<crt_combine_grid(m, nc, r.num_sms), 128, 0, s>>>(q, info);
     };
@@ -2394,28 +2353,36 @@ int device_product_host_panels(const Gemm& g, const SplitRequest& req, const Lau
     auto* pb = static_cast<__nv_bfloat16*>(ws.get(kSlotSliceB, size_t(max_planes) * size_t(npb) * size_t(kpad) * 2, err));
     // level planes of a launch over the whole width, two buffers: launch L's reconstructions (on the
     // second stream) read buffer L % 2 while launch L + 1's tensor-core work writes the other
-    const size_t lv_elems = size_t(nseg) * max_levels * size_t(mpad) * size_t(npb);
+    const size_t lv_elems = level_bytes(Gp) / size_t(mpad) / size_t(Gp.npad) * size_t(mpad) * size_t(npb) / 4;
     auto* lv = static_cast<int32_t*>(ws.get(kSlotLevels, 2 * lv_elems * 4, err));
-    const int64_t off_sq = round_up((m + n) * int64_t(sizeof(int)), 256);
-    const int64_t off_info = round_up(off_sq + (m + n) * int64_t(sizeof(double)), 256);
+    // exponents, then the infos; counters of every panel and column block, then the row blocks' partials
+    // and the chunk partials of the one being worked on (they follow one another on st)
+    const int64_t off_info = round_up((m + n) * int64_t(sizeof(int)), 256);
     const int ninfo = P + Q + P * Q + P + 1;
     const size_t info_stride = ((sizeof(SplitInfo) + 255) / 256) * 256;
+    const StatsLayout LA = stats_layout(Mp, 0, k, r.num_sms), LB = stats_layout(0, Nq, k, r.num_sms);
+    const size_t count_bytes = size_t(round_up((int64_t(P) * (LA.blocks + 1) + int64_t(Q) * (LB.blocks + 1)) * 4, 256));
+    const size_t group_bytes = size_t(round_up(std::max(LA.blocks, LB.blocks) * int64_t(sizeof(RowPartial)), 256));
+    auto part_bytes = [&](int64_t rows) {  // whatever chunks a last, shorter panel takes
+        return size_t(rows) * size_t((k + 63) / 64) * sizeof(uint2);
+    };
     auto* stats = static_cast<uint8_t*>(ws.get(kSlotScaleA, size_t(off_info) + size_t(ninfo) * info_stride, err));
-    auto* racc = static_cast<RowAcc*>(ws.get(kSlotScaleB, size_t(m + n) * sizeof(RowAcc), err));
-    if (!dA || !dB || !dC || !pa || !pb || !lv || !stats || !racc) return GB300_ERR_NO_MEMORY;
+    auto* scratch = static_cast<uint8_t*>(
+        ws.get(kSlotScaleB, count_bytes + group_bytes + part_bytes(std::max(Mp, Nq)), err));
+    if (!dA || !dB || !dC || !pa || !pb || !lv || !stats || !scratch) return GB300_ERR_NO_MEMORY;
     int* eA = reinterpret_cast<int*>(stats);
     int* eB = eA + m;
-    double* sqA = reinterpret_cast<double*>(stats + off_sq);
-    double* sqB = sqA + m;
     auto info_at = [&](int i) { return reinterpret_cast<SplitInfo*>(stats + off_info + size_t(i) * info_stride); };
     // infos: [0, P) panels of A, [P, P+Q) blocks of B, [P+Q, P+Q+PQ) blocks of C, [P+Q+PQ,
     // P+Q+PQ+P) the launches over a whole panel (the largest level count of its blocks), last: summary
     SplitInfo* info_sum = info_at(ninfo - 1);
     const double target = req.target_error > 0 ? req.target_error : double(k) * 0x1p-53;
     // events: [0, P) A panels in, [P, P+Q) B blocks in, [P+Q, P+Q+PQ) C blocks computed, next:
-    // all out, then [P+Q+PQ+1, P+Q+2PQ+1) the launches' tensor-core work done
+    // all out, then [P+Q+PQ+1, P+Q+2PQ+1) the launches' tensor-core work done, then PQ for the first
+    // row halves of the C blocks
     cudaEvent_t* ev = r.pipe_ev;
-    if (P + Q + 2 * P * Q + 1 > Runtime::kPipeEvents) return GB300_ERR_NOT_SUPPORTED;
+    if (P + Q + 2 * P * Q + 1 > kPipeMaxEvents) return GB300_ERR_NOT_SUPPORTED;
+    static_assert(Runtime::kPipeEvents >= kPipeMaxEvents + kPipeMaxEvents / 2, "events of the row halves");
     cudaStream_t aux = aux_stream_for(st, err);
     if (!aux) return GB300_ERR_CUDA;
     auto cuda_fail = [&](const char* what, cudaError_t e) {
@@ -2451,12 +2418,19 @@ int device_product_host_panels(const Gemm& g, const SplitRequest& req, const Lau
                                   cudaMemcpyHostToDevice, r.copy_in);
         cudaEventRecord(ev[P + j], r.copy_in);
     };
-    cudaMemsetAsync(racc, 0, size_t(m + n) * sizeof(RowAcc), st);
+    cudaMemsetAsync(scratch, 0, count_bytes, st);
     // the pre-pass launches over a panel or a column block
-    auto run_stats = [&](const OperandPair& o, int64_t yb) {
-        const int64_t tiles = (k + 63) / 64;
-        const int kt = tiles_per_block(tiles, yb, r.num_sms);
-        stats_tile_kernel<<<dim3(unsigned((tiles + kt - 1) / kt), unsigned(yb)), 256, 0, st>>>(o, k, kt);
+    auto run_stats = [&](const OperandPair& o, const StatsLayout& L, int64_t first_counter, SplitInfo* info) {
+        StatsArgs sa;
+        sa.op = o;
+        sa.K = k;
+        sa.kt = L.kt;
+        sa.chunks = L.chunks;
+        sa.count = reinterpret_cast<unsigned*>(scratch) + first_counter;
+        sa.group = reinterpret_cast<RowPartial*>(scratch + count_bytes);
+        sa.part = reinterpret_cast<uint2*>(scratch + count_bytes + group_bytes);
+        sa.plan = PlanArgs{kPlanSide, kCrt, 0, max_planes, target, info};
+        stats_kernel<<<dim3(unsigned(L.chunks), unsigned(L.blocks)), 256, 0, st>>>(sa);
     };
     auto run_slice = [&](const OperandPair& o, int64_t yb, const SplitInfo* info) {
         const int64_t tiles = kpad / 64;
@@ -2470,9 +2444,7 @@ int device_product_host_panels(const Gemm& g, const SplitRequest& req, const Lau
     base.R[0] = 0; base.R[1] = 0;
     base.sr[0] = a_sr; base.sr[1] = b_sr;
     base.sp[0] = a_sp; base.sp[1] = b_sp;
-    base.acc[0] = racc; base.acc[1] = racc + m;
     base.rexp[0] = eA; base.rexp[1] = eB;
-    base.rsq[0] = sqA; base.rsq[1] = sqB;
     base.planes[0] = pa; base.planes[1] = pb;
     base.rpad[0] = mpad; base.rpad[1] = npb;
     base.yb0 = 0;
@@ -2482,17 +2454,12 @@ int device_product_host_panels(const Gemm& g, const SplitRequest& req, const Lau
         OperandPair o = base;
         o.X[0] = g.ta ? dA + r0 : dA + r0 * a_cols;
         o.R[0] = mi;
-        o.acc[0] = racc + r0;
         o.rexp[0] = eA + r0;
-        o.rsq[0] = sqA + r0;
         o.yb0 = unsigned((mi + 31) / 32);
-        run_stats(o, o.yb0);
-        const unsigned xb0 = unsigned((mi + 255) / 256);
-        stats_finalize_pair_kernel<<<xb0, 256, 0, st>>>(o, k, xb0, nullptr);
-        split_side_kernel<<<1, 1024, 0, st>>>(eA + r0, sqA + r0, mi, k, max_planes, target, info_at(i));
+        run_stats(o, stats_layout(mi, 0, k, r.num_sms), int64_t(i) * (LA.blocks + 1), info_at(i));
         o.yb0 = unsigned(mpad / 32);
         run_slice(o, o.yb0, info_at(i));
-        count_launches(4);
+        count_launches(2);
     };
     // statistics, side scaling and planes of B's column block j (rows j*Nq.. of the B planes)
     auto prep_b = [&](int j) {
@@ -2500,17 +2467,14 @@ int device_product_host_panels(const Gemm& g, const SplitRequest& req, const Lau
         OperandPair o = base;
         o.X[1] = g.tb ? dB + c0 * b_cols : dB + c0;
         o.R[1] = nj;
-        o.acc[1] = racc + m + c0;
         o.rexp[1] = eB + c0;
-        o.rsq[1] = sqB + c0;
         o.planes[1] = pb + size_t(j) * size_t(Nq) * size_t(kpad);
         o.rpad[1] = npb;
         o.yb0 = 0;
-        run_stats(o, (nj + 31) / 32);
-        stats_finalize_pair_kernel<<<unsigned((nj + 255) / 256), 256, 0, st>>>(o, k, 0u, nullptr);
-        split_side_kernel<<<1, 1024, 0, st>>>(eB + c0, sqB + c0, nj, k, max_planes, target, info_at(P + j));
+        run_stats(o, stats_layout(0, nj, k, r.num_sms), int64_t(P) * (LA.blocks + 1) + int64_t(j) * (LB.blocks + 1),
+                  info_at(P + j));
         run_slice(o, Nq / 32, info_at(P + j));
-        count_launches(4);
+        count_launches(2);
     };
 
     // ---- tensor maps: A panel planes, the B planes, the level planes of a launch ----
@@ -2536,12 +2500,18 @@ int device_product_host_panels(const Gemm& g, const SplitRequest& req, const Lau
     // copy_to_host), else per block.
     const bool c_per_panel = !c_locked && Q > 1 && g.ldc == n;
     auto block_ev = [&](int i, int j) { return ev[P + Q + i * Q + j]; };
+    auto half_ev = [&](int i, int j) { return ev[P + Q + 2 * P * Q + 1 + i * Q + j]; };
+    auto half_rows = [](int64_t rows) { return (rows + 1) / 2; };
     auto copy_block_out = [&](int i, int j) {
         const int64_t r0 = int64_t(i) * Mp, mi = std::min(Mp, m - r0);
         const int64_t c0 = int64_t(j) * Nq, nj = std::min(Nq, n - c0);
-        cudaStreamWaitEvent(r.copy_out, block_ev(i, j), 0);
-        e = copy_to_host(hC + r0 * g.ldc + c0, size_t(g.ldc) * 8, dC + r0 * n + c0, size_t(n) * 8, size_t(nj) * 8,
-                         size_t(mi), r.copy_out);
+        for (int h = 0; h < 2 && e == cudaSuccess; ++h) {
+            const int64_t h0 = h ? half_rows(mi) : 0, h1 = h ? mi : half_rows(mi);
+            if (h1 == h0) continue;
+            cudaStreamWaitEvent(r.copy_out, h ? block_ev(i, j) : half_ev(i, j), 0);
+            e = copy_to_host(hC + (r0 + h0) * g.ldc + c0, size_t(g.ldc) * 8, dC + (r0 + h0) * n + c0, size_t(n) * 8,
+                             size_t(nj) * 8, size_t(h1 - h0), r.copy_out);
+        }
     };
     auto copy_panel_out = [&](int i) {
         if (!c_per_panel) {
@@ -2609,14 +2579,18 @@ int device_product_host_panels(const Gemm& g, const SplitRequest& req, const Lau
         cudaStreamWaitEvent(aux, tc_done_ev(l), 0);
         for (int j = j0; j < j1; ++j) {
             const int64_t cj = int64_t(j) * Nq, nj = std::min(Nq, n - cj);
-            const CrtCombine q{reinterpret_cast<const uint8_t*>(lvb), mpad, npb, nseg, max_levels, cj, mi, nj, eA + r0, eB,
-                               g.alpha, g.beta, dC + r0 * n, n};
-            crt_combine_kernel<<<crt_combine_grid(mi, nj, r.num_sms), 128, 0, aux>>>(q, info_at(P + Q + i * Q + j));
-            if ((e = cudaGetLastError()) != cudaSuccess) return;
-            cudaEventRecord(block_ev(i, j), aux);
+            // in two row halves, so that the first one's copy back starts while the second is reconstructed
+            for (int h = 0; h < 2; ++h) {
+                const int64_t h0 = h ? half_rows(mi) : 0, h1 = h ? mi : half_rows(mi);
+                const CrtCombine q{reinterpret_cast<const uint8_t*>(lvb), mpad, npb, nseg, max_levels, h0, cj, h1 - h0, nj,
+                                   eA + r0, eB, g.alpha, g.beta, dC + r0 * n, n};
+                crt_combine_kernel<<<crt_combine_grid(h1 - h0, nj, r.num_sms), 128, 0, aux>>>(q, info_at(P + Q + i * Q + j));
+                if ((e = cudaGetLastError()) != cudaSuccess) return;
+                cudaEventRecord(h ? block_ev(i, j) : half_ev(i, j), aux);
+            }
             if (c_locked) copy_block_out(i, j);
         }
-        count_launches(1 + 2 * (j1 - j0));
+        count_launches(1 + 3 * (j1 - j0));
     };
     bool have_a[16] = {}, have_b[kPipeMaxQ] = {};
     int nb = 0;  // B blocks in
