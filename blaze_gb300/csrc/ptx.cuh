@@ -178,6 +178,17 @@ __device__ __forceinline__ uint32_t swz128(uint32_t off) {
     return off ^ (((off >> 7) & 7u) << 4);
 }
 
+// ---- programmatic dependent launch -----------------------------------------------------------------
+// A kernel launched with launch_dependent (runtime.h) may start before the kernel ahead of it on the
+// stream has finished, once every block of that one has called griddep_launch (or ended).  Before it
+// touches anything that kernel or an earlier one writes or still reads, it calls griddep_wait, which
+// returns when the kernel ahead has completed and its writes are visible.  A kernel launched the
+// plain way passes through both.
+__device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Orders generic-proxy writes that are visible to this thread before its later TMA accesses.
+__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async;" ::: "memory"); }
+
 // ---- packed FP32 pairs -----------------------------------------------------------------------------
 __device__ __forceinline__ uint64_t f32x2_bits(uint32_t lo, uint32_t hi) {
     uint64_t d;

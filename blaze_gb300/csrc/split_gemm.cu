@@ -303,6 +303,7 @@ __global__ void __launch_bounds__(256, 4) stats_kernel(const StatsArgs a) {
     __shared__ __align__(16) unsigned char tbuf[2 * BUF];
     __shared__ uint32_t red_mx[8][32];
     __shared__ float red_sq[8][32];
+    griddep_launch();  // the slicing's first tiles may come in meanwhile
     const int w = blockIdx.y < a.op.yb0 ? 0 : 1;
     const int by = w ? int(blockIdx.y - a.op.yb0) : int(blockIdx.y);
     const double* __restrict__ X = a.op.X[w];
@@ -908,13 +909,17 @@ __device__ __forceinline__ void slice_rows(int which, const double* __restrict__
         const uint32_t c = uint32_t(p_) >> 1;
         return uint32_t(r_) * ROWB + ((c ^ (c >> 3)) << 4) + ((uint32_t(p_) & 1u) << 3);
     };
+    const int64_t pstride = rpad * kpad;
+    const bool vec = rows_vec(X, sr, sp);
+    if (tb < te) tile_issue(s0, X, R, K, sr, sp, vec, r0, tb, off);
+    // the operand is the caller's and was there before; the plan, the exponents and the planes (which
+    // an earlier product may still be reading) have to wait
+    griddep_launch();
+    griddep_wait();
     const int sl = (mode == kExact || mode == kCrt) ? info->slices : 0;
     const int bt = (mode == kCrt) ? (which ? info->beta_b : info->beta) : 0;
     const int e = (r < R) ? rexp[r] : 0;
     const bool bad = (mode == kExact || mode == kCrt) && e == kNonFinite;
-    const int64_t pstride = rpad * kpad;
-    const bool vec = rows_vec(X, sr, sp);
-    if (tb < te) tile_issue(s0, X, R, K, sr, sp, vec, r0, tb, off);
     for (int64_t it = tb; it < te; ++it) {
         const int b = int(it - tb) & 1;
         if (it + 1 < te) tile_issue(s0 + uint32_t(b ^ 1) * BUF, X, R, K, sr, sp, vec, r0, it + 1, off);
@@ -1051,10 +1056,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
     // the epilogue's arithmetic is fixed at compile time: residues, exact integer sums or FP32 tiles
     constexpr int mode = MODE;
-    const int S = (mode == kExact || mode == kCrt) ? p.info->slices : 1;
-    const int nlev = num_levels(mode, S);
-    const int units = p.m_tiles * p.n_tiles * p.nseg * nlev;
-
+    griddep_launch();
     if (threadIdx.x == 0) {
         tma_prefetch_desc(&tmA);
         tma_prefetch_desc(&tmB);
@@ -1085,10 +1087,16 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     cluster_sync();
     tc_fence_after();
     const uint32_t tmem = bars->tmem_base;
+    // everything above overlaps the slicing; the plan and the planes are ready from here on
+    griddep_wait();
+    const int S = (mode == kExact || mode == kCrt) ? p.info->slices : 1;
+    const int nlev = num_levels(mode, S);
+    const int units = p.m_tiles * p.n_tiles * p.nseg * nlev;
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------
         if (lane == 0 && !p.inject_stall) {
+            fence_proxy_async();
             uint32_t it = 0;
             bool ok = true;
             for (int u = pair; u < units && ok; u += npairs) {
@@ -1629,6 +1637,7 @@ __device__ __forceinline__ void crt_rows(const CrtCombine& p, int scale, int64_t
 // tensor-core CTA; two columns at a time instead of four took 186 instructions an output.
 constexpr int kCombineBlocks = 8;
 __global__ void __launch_bounds__(128, kCombineBlocks) crt_combine_kernel(const CrtCombine p, const SplitInfo* __restrict__ info) {
+    griddep_wait();
     const int64_t j0 = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) * 4;
     if (j0 >= p.n) return;
     const int scale = info->beta + info->beta_b;
@@ -1657,6 +1666,7 @@ __global__ void __launch_bounds__(128, 8) combine_kernel(const int32_t* __restri
                                int64_t npad, int mode, const SplitInfo* __restrict__ info,
                                const int* __restrict__ eA, const int* __restrict__ eB, int64_t m, int64_t n,
                                double alpha, double beta, double* __restrict__ C, int64_t ldc) {
+    griddep_wait();
     const int64_t j0 = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) * COMBINE_COLS;
     if (j0 >= n) return;
     const int64_t plane = mpad * npad;
@@ -2139,7 +2149,7 @@ int device_product(const Gemm& g_in, const SplitRequest& req, const LaunchCtl& c
         const dim3 grid(unsigned((tiles + kt - 1) / kt), unsigned(yb));
         auto sk = mode == kCrt ? slice_kernel<kCrt>
                                : (mode == kExact ? slice_kernel<kExact> : (mode == kBf16 ? slice_kernel<kBf16> : slice_kernel<kBf16x3>));
-        sk<<<grid, 256, 0, st>>>(sp2, k, info, kpad, kt);
+        launch_dependent(sk, grid, dim3(256), 0, st, sp2, k, info, kpad, kt);
     }
     count_launches(2);
     if (cudaError_t le = cudaGetLastError(); le != cudaSuccess) {
@@ -2190,13 +2200,14 @@ int device_product(const Gemm& g_in, const SplitRequest& req, const LaunchCtl& c
         const int units = m_tiles * nt * nseg * max_levels;
         const int grid = 2 * std::max(1, std::min(units, sms / 2));
         KernelTimer timer("tc_gemm", st);
-        kern<<<grid, THREADS, kTcSmem, st>>>(tA, tB, tC0, tC, q);
+        launch_dependent(kern, dim3(unsigned(grid)), dim3(THREADS), kTcSmem, st, tA, tB, tC0, tC, q);
     };
     // reconstruction of C's columns [c0, c0 + nc) on stream s
     auto launch_crt_combine = [&](int64_t c0, int64_t nc, cudaStream_t s) {
         const CrtCombine q{reinterpret_cast<const uint8_t*>(lv), mpad, npad, nseg, max_levels, 0, c0, m, nc, eA, eB,
                            g.alpha, g.beta, static_cast<double*>(g.C), g.ldc};
-        crt_combine_kernel<<<crt_combine_grid(m, nc, r.num_sms), 128, 0, s>>>(q, info);
+        if (s == st) launch_dependent(crt_combine_kernel, crt_combine_grid(m, nc, r.num_sms), dim3(128), 0, s, q, info);
+        else crt_combine_kernel<<<crt_combine_grid(m, nc, r.num_sms), 128, 0, s>>>(q, info);  // behind an event
     };
     const bool in_parts = mode == kCrt && n_tiles >= 2 && m_tiles * n_tiles >= sms && req.max_sms <= 0;
     if (in_parts) {
@@ -2221,8 +2232,8 @@ int device_product(const Gemm& g_in, const SplitRequest& req, const LaunchCtl& c
         } else {
             const int64_t colgroups = (n + COMBINE_COLS - 1) / COMBINE_COLS;
             dim3 cgrid(unsigned((colgroups + 127) / 128), unsigned(std::min<int64_t>(m, 65535)));
-            combine_kernel<<<cgrid, 128, 0, st>>>(lv, nseg, max_levels, mpad, npad, mode, info, eA, eB, m, n,
-                                                  g.alpha, g.beta, static_cast<double*>(g.C), g.ldc);
+            launch_dependent(combine_kernel, cgrid, dim3(128), 0, st, lv, nseg, max_levels, mpad, npad, mode, info, eA, eB,
+                             m, n, g.alpha, g.beta, static_cast<double*>(g.C), g.ldc);
         }
     }
     count_launches(2);
@@ -2435,7 +2446,8 @@ int device_product_host_panels(const Gemm& g, const SplitRequest& req, const Lau
     auto run_slice = [&](const OperandPair& o, int64_t yb, const SplitInfo* info) {
         const int64_t tiles = kpad / 64;
         const int kt = tiles_per_block(tiles, yb, r.num_sms);
-        slice_kernel<kCrt><<<dim3(unsigned((tiles + kt - 1) / kt), unsigned(yb)), 256, 0, st>>>(o, k, info, kpad, kt);
+        launch_dependent(slice_kernel<kCrt>, dim3(unsigned((tiles + kt - 1) / kt), unsigned(yb)), dim3(256), 0, st, o, k,
+                         info, kpad, kt);
     };
     const int64_t a_sr = g.ta ? 1 : a_cols, a_sp = g.ta ? a_cols : 1;
     const int64_t b_sr = g.tb ? b_cols : 1, b_sp = g.tb ? 1 : b_cols;
@@ -2573,7 +2585,8 @@ int device_product_host_panels(const Gemm& g, const SplitRequest& req, const Lau
         const int grid = 2 * std::max(1, std::min(units, r.num_sms / 2));
         {
             KernelTimer timer("tc_gemm", st);
-            tc_gemm_kernel<kCrt><<<grid, THREADS, kTcSmem, st>>>(tA, tB, tC0[buf], tC[buf], tp);
+            launch_dependent(tc_gemm_kernel<kCrt>, dim3(unsigned(grid)), dim3(THREADS), kTcSmem, st, tA, tB, tC0[buf],
+                             tC[buf], tp);
         }
         cudaEventRecord(tc_done_ev(l), st);
         cudaStreamWaitEvent(aux, tc_done_ev(l), 0);
