@@ -217,7 +217,7 @@ int gemm_entry(int order, int transA, int transB, int64_t m, int64_t n, int64_t 
     Stored da = sa, db = sb, dc = sc;
     bool c_staged = false;
     if (!done) {
-    // float: the split forms run on double copies at the float target (device_product_float); small
+    // float: the split forms run at the float target (device_product_float); small
     // products under `auto` stay on the native kernel, as for double
     const bool split_path = product && method != GB300_METHOD_NATIVE &&
                             (is_double || !(method == GB300_METHOD_AUTO && split_auto_uses_native(g)));
@@ -258,7 +258,7 @@ int gemm_entry(int order, int transA, int transB, int64_t m, int64_t n, int64_t 
         req.target_error = opts ? opts->target_error : 0.0;
         SplitResult res_out;
         st = is_double ? device_product(g, req, ctl, s, r.ws, &res_out, &err)
-                       : device_product_float(g, req, ctl, s, r.ws, r.aux, &res_out, &err);
+                       : device_product_float(g, req, ctl, s, r.ws, &res_out, &err);
         if (st != GB300_OK) return fail(st, err);
         used = res_out.method_used;
         info_dev = res_out.info_dev;

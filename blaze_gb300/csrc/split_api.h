@@ -42,11 +42,11 @@ int device_product(const Gemm& g, const SplitRequest& req, const LaunchCtl& ctl,
 // True when the `auto` method runs a product on the native kernel (small products, short k).
 bool split_auto_uses_native(const Gemm& g);
 
-// The same for float operands (device, float, caller's pitches): widened to double in `conv`
-// (slots 0-2), computed at the float target k 2^-24 unless the request sets one, rounded once to
-// float.  The bound includes the final rounding (2^-24).
+// The same for float operands and result (device, caller's pitches): computed at the float target
+// k 2^-24 unless the request sets one, rounded once to float.  The bound includes the final rounding
+// (2^-24).  The tensor-core forms only: the caller runs native float products itself.
 int device_product_float(const Gemm& g, const SplitRequest& req, const LaunchCtl& ctl, cudaStream_t s, Workspace& ws,
-                         Workspace& conv, SplitResult* out, std::string* err);
+                         SplitResult* out, std::string* err);
 
 // FP64-accurate product of host operands (page-locked or pageable) in row panels of A: B is copied
 // and sliced once, then each panel's copy in, product and copy of C back run on three streams so

@@ -160,45 +160,61 @@ constexpr int kNonFinite = 0x7fff;
 // while the current one is processed.
 constexpr int TILE_KT = 8;  // at most
 
+// A row of a tile buffer: 64 elements and 16 bytes, so that rows start on different banks.
+template <typename TX>
+constexpr uint32_t kTileRow = 64 * sizeof(TX) + 16;
+
 // Whether an operand's rows are contiguous and 16-byte aligned.
-__device__ __forceinline__ bool rows_vec(const double* X, int64_t sr, int64_t sp) {
-    return sp == 1 && (sr & 1) == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0;
+template <typename TX>
+__device__ __forceinline__ bool rows_vec(const TX* X, int64_t sr, int64_t sp) {
+    return sp == 1 && (sr * int64_t(sizeof(TX))) % 16 == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0;
 }
 
 // Issue the copies of tile `it` (k from 64 it) into the buffer at shared address sbuf, where
-// off(rr, pp) places element (rr, pp), an even pp and the next one side by side; zeros outside R x K;
-// one commit group per tile.  The copies are coalesced along whichever index of
-// X(r, p) = X[r*sr + p*sp] is contiguous: eight elements a thread, a warp reading 256 consecutive
-// bytes, or, where rows_vec, four pairs of elements, a warp reading 512.  Addresses are formed anew for
+// off(rr, pp) places element (rr, pp), the elements of an aligned 16 bytes side by side; zeros outside
+// R x K; one commit group per tile.  The copies are coalesced along whichever index of
+// X(r, p) = X[r*sr + p*sp] is contiguous: eight elements a thread, a warp reading 32 consecutive ones,
+// or, where rows_vec, 16 bytes at a time.  Addresses are formed anew for
 // each tile: kept across tiles they spilled from the slicing's 80 registers (725 -> 879 us at 8192^3).
-template <typename Off>
-__device__ __forceinline__ void tile_issue(uint32_t sbuf, const double* X, int64_t R, int64_t K, int64_t sr, int64_t sp,
+template <typename TX, typename Off>
+__device__ __forceinline__ void tile_issue(uint32_t sbuf, const TX* X, int64_t R, int64_t K, int64_t sr, int64_t sp,
                                            bool vec, int64_t r0, int64_t it, Off off) {
     const int t = threadIdx.x;  // 256 threads
     const bool full = r0 + 32 <= R && it * 64 + 64 <= K;  // the whole tile lies inside the matrix
     if (vec) {
-        const int rr0 = t >> 5, pp = 2 * (t & 31);
+        constexpr int V = 16 / sizeof(TX), CH = 64 / V, STEP = 256 / CH;  // elements, chunks a row, rows a pass
+        const int rr0 = t / CH, pp = V * (t % CH);
         const int64_t left = K - it * 64 - pp;
-        const int bytes = full || left >= 2 ? 16 : left == 1 ? 8 : 0;
-        const double* src = X + (r0 + rr0) * sr + it * 64 + pp;
+        const int bytes = full || left >= V ? 16 : left > 0 ? int(left) * int(sizeof(TX)) : 0;
+        const TX* src = X + (r0 + rr0) * sr + it * 64 + pp;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int n = full || r0 + rr0 + 8 * i < R ? bytes : 0;
-            cp_async16(sbuf + off(rr0 + 8 * i, pp), n ? src + 8 * i * sr : X, n);
+        for (int i = 0; i < 32 / STEP; ++i) {
+            const int n = full || r0 + rr0 + STEP * i < R ? bytes : 0;
+            cp_async16(sbuf + off(rr0 + STEP * i, pp), n ? src + STEP * i * sr : X, n);
         }
     } else {
         const int rr0 = sp == 1 ? t >> 6 : t & 31, pp0 = sp == 1 ? t & 63 : t >> 5;
         const int drr = sp == 1 ? 4 : 0, dpp = sp == 1 ? 0 : 8;
-        const double* src = X + (r0 + rr0) * sr + (it * 64 + pp0) * sp;
+        const TX* src = X + (r0 + rr0) * sr + (it * 64 + pp0) * sp;
         const int64_t di = sp == 1 ? 4 * sr : 8 * sp;
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const int rr = rr0 + i * drr, pp = pp0 + i * dpp;
             const bool ok = full || (r0 + rr < R && it * 64 + pp < K);
-            cp_async8(sbuf + off(rr, pp), ok ? src + i * di : X, ok);
+            if constexpr (sizeof(TX) == 8) cp_async8(sbuf + off(rr, pp), ok ? src + i * di : X, ok);
+            else cp_async4(sbuf + off(rr, pp), ok ? src + i * di : X, ok);
         }
     }
     cp_async_commit();
+}
+
+// The bits of a float operand's element as a double (exact).
+__device__ __forceinline__ unsigned long long widened_bits(uint32_t b) {
+    const uint32_t mag = b & 0x7fffffffu;
+    if (mag - 1u < 0x007fffffu || mag >= 0x7f800000u)  // subnormal, Inf, NaN
+        return static_cast<unsigned long long>(__double_as_longlong(double(__uint_as_float(b))));
+    const uint32_t hi = (b & 0x80000000u) | (mag ? (mag >> 3) + 0x38000000u : 0u);
+    return ((unsigned long long)hi << 32) | (mag << 29);
 }
 
 // 2^x in FP32 for x <= 127, 0 below the normal range.
@@ -207,7 +223,7 @@ __device__ __forceinline__ float pow2f_or0(int x) { return x < -126 ? 0.f : __ui
 // Both operands of a product go through one launch: blocks with blockIdx.y < yb0 work on A (its
 // rows), the others on B (its columns), so the two passes overlap on the device.
 struct OperandPair {
-    const double* X[2];
+    const void* X[2];  // double or float elements
     int64_t R[2], sr[2], sp[2];
     int* rexp[2];
     __nv_bfloat16* planes[2];
@@ -298,22 +314,30 @@ __device__ __forceinline__ bool last_to_arrive(unsigned* counter, unsigned n) {
 // row totals in a kernel of their own (atomics and a memset before it) and the plan in another, these
 // steps took 23 us of a 403 x 517 x 389 product and 26 of 1024^3 with the gaps between four launches
 // beside them, now 13 and 17.
+//
+// A float's high word as a double is its magnitude shifted by 3 with the exponent rebased.  A zero or
+// subnormal float gets exponent field 896 that way, no matter next to a row's larger values: rows
+// without values above 2^-86 are read again like tiny doubles, and all-zero rows known by their OR.
+template <typename TX>
 __global__ void __launch_bounds__(256, 4) stats_kernel(const StatsArgs a) {
-    constexpr uint32_t ROWB = 528, BUF = 32 * ROWB;  // rows 33 chunks of 16 bytes apart: no bank conflicts
+    constexpr bool F32 = sizeof(TX) == 4;
+    constexpr uint32_t ROWB = kTileRow<TX>, BUF = 32 * ROWB;  // an odd count of 16-byte chunks: no bank conflicts
+    constexpr uint32_t kInfHi = F32 ? 0x47f00000u : 0x7ff00000u;
+    constexpr uint32_t kTinyExp = F32 ? 937u : 191u;
     __shared__ __align__(16) unsigned char tbuf[2 * BUF];
     __shared__ uint32_t red_mx[8][32];
     __shared__ float red_sq[8][32];
     griddep_launch();  // the slicing's first tiles may come in meanwhile
     const int w = blockIdx.y < a.op.yb0 ? 0 : 1;
     const int by = w ? int(blockIdx.y - a.op.yb0) : int(blockIdx.y);
-    const double* __restrict__ X = a.op.X[w];
+    const TX* __restrict__ X = static_cast<const TX*>(a.op.X[w]);
     const int64_t R = a.op.R[w], sr = a.op.sr[w], sp = a.op.sp[w], K = a.K;
     const int t = threadIdx.x, rr = t & 31, g = t >> 5;
     const int64_t r0 = int64_t(by) * 32;
     const int64_t ntiles = (K + 63) / 64;
     const int64_t tb = int64_t(blockIdx.x) * a.kt, te = min(ntiles, tb + a.kt);
     const uint32_t s0 = smem_u32(tbuf);
-    auto off = [](int r_, int p_) { return uint32_t(r_) * ROWB + uint32_t(p_) * 8u; };
+    auto off = [](int r_, int p_) { return uint32_t(r_) * ROWB + uint32_t(p_) * uint32_t(sizeof(TX)); };
     uint32_t mx = 0, lo = 0;
     int base = 127;  // f = |x| 2^(1023 - base); values with exponent field 0 never count
     float sq = 0.f;
@@ -326,14 +350,27 @@ __global__ void __launch_bounds__(256, 4) stats_kernel(const StatsArgs a) {
         cp_async_wait1();
         __syncthreads();
         uint32_t hi[8];
-        const unsigned char* row = tbuf + b * BUF + rr * ROWB + g * 64;
+        const unsigned char* row = tbuf + b * BUF + rr * ROWB + g * 8 * uint32_t(sizeof(TX));
+        if constexpr (F32) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const uint4 v = *reinterpret_cast<const uint4*>(row + 16 * q);
-            hi[2 * q] = v.y & 0x7fffffffu;
-            hi[2 * q + 1] = v.w & 0x7fffffffu;
-            lo |= v.x | v.z;
-            mx = max(mx, max(hi[2 * q], hi[2 * q + 1]));
+            for (int q = 0; q < 2; ++q) {
+                const uint4 v = *reinterpret_cast<const uint4*>(row + 16 * q);
+                const uint32_t m4[4] = {v.x & 0x7fffffffu, v.y & 0x7fffffffu, v.z & 0x7fffffffu, v.w & 0x7fffffffu};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) hi[4 * q + i] = (m4[i] >> 3) + 0x38000000u;
+                lo |= m4[0] | m4[1];
+                lo |= m4[2] | m4[3];
+                mx = max(mx, max(max(hi[4 * q], hi[4 * q + 1]), max(hi[4 * q + 2], hi[4 * q + 3])));
+            }
+        } else {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const uint4 v = *reinterpret_cast<const uint4*>(row + 16 * q);
+                hi[2 * q] = v.y & 0x7fffffffu;
+                hi[2 * q + 1] = v.w & 0x7fffffffu;
+                lo |= v.x | v.z;
+                mx = max(mx, max(hi[2 * q], hi[2 * q + 1]));
+            }
         }
         const int top = int(mx >> 20);
         if (top > base) {
@@ -351,6 +388,10 @@ __global__ void __launch_bounds__(256, 4) stats_kernel(const StatsArgs a) {
     // a row's largest high word with the low words' flag in bit 0, and its sum of squares relative to
     // the exponent of that high word (at least 127)
     auto exponent = [](uint32_t m) { return max(127, int(m >> 21)); };
+    if (F32 && lo == 0u) {
+        mx = 0u;
+        sq = 0.f;
+    }
     red_mx[g][rr] = (mx << 1) | (lo != 0u ? 1u : 0u);
     red_sq[g][rr] = sq;
     __syncthreads();
@@ -398,9 +439,9 @@ __global__ void __launch_bounds__(256, 4) stats_kernel(const StatsArgs a) {
         float q = 0.f;
         const uint32_t hi = m >> 1;
         if (r < R && m != 0u) {
-            if (hi >= 0x7ff00000u) {
+            if (hi >= kInfHi) {
                 e = kNonFinite;
-            } else if (hi >= (191u << 20)) {
+            } else if (hi >= (kTinyExp << 20)) {
                 e = int(hi >> 20) - 1022;
                 q = 0.25f * s;  // |x| 2^-e = f / 2
             } else {
@@ -408,13 +449,13 @@ __global__ void __launch_bounds__(256, 4) stats_kernel(const StatsArgs a) {
                 unsigned long long mb = 0;
                 for (int64_t p = 0; p < K; ++p) {
                     const unsigned long long v =
-                        static_cast<unsigned long long>(__double_as_longlong(X[r * sr + p * sp])) & 0x7fffffffffffffffull;
+                        static_cast<unsigned long long>(__double_as_longlong(double(X[r * sr + p * sp]))) & 0x7fffffffffffffffull;
                     mb = v > mb ? v : mb;
                 }
                 frexp(__longlong_as_double(static_cast<long long>(mb)), &e);
                 double d = 0.0;
                 for (int64_t p = 0; p < K; ++p) {
-                    const double v = ldexp(X[r * sr + p * sp], -e);
+                    const double v = ldexp(double(X[r * sr + p * sp]), -e);
                     d = fma(v, v, d);
                 }
                 q = float(d);
@@ -886,12 +927,12 @@ __device__ __forceinline__ void slice_emit(const unsigned long long (&xv)[8], in
 // 8L..8L+7 of row rr and writes 16 bytes per plane (a warp: four 128-byte row segments).  The tile
 // buffer keeps rows of 528 bytes with 16-byte chunk c of a row stored at c ^ (c >> 3), so that the
 // eight threads of a row read their chunks 4L + j from eight different bank groups.
-template <int mode>
-__device__ __forceinline__ void slice_rows(int which, const double* __restrict__ X, int64_t R, int64_t K, int64_t sr,
+template <int mode, typename TX>
+__device__ __forceinline__ void slice_rows(int which, const TX* __restrict__ X, int64_t R, int64_t K, int64_t sr,
                                            int64_t sp, const int* __restrict__ rexp, const SplitInfo* __restrict__ info,
                                            __nv_bfloat16* __restrict__ planes, int64_t rpad, int64_t kpad, int by,
                                            int kt) {
-    constexpr uint32_t ROWB = 528, BUF = 32 * ROWB;
+    constexpr uint32_t ROWB = kTileRow<TX>, BUF = 32 * ROWB, V = 16 / sizeof(TX);
     __shared__ __align__(16) unsigned char tbuf[2 * BUF];
     __shared__ SliceConst tab[mode == kCrt ? MAX_MODULI : 1];
     const int t = threadIdx.x, rr = t >> 3, L = t & 7;
@@ -906,8 +947,8 @@ __device__ __forceinline__ void slice_rows(int which, const double* __restrict__
     const int64_t tb = int64_t(blockIdx.x) * kt, te = min(ntiles, tb + kt);
     const uint32_t s0 = smem_u32(tbuf);
     auto off = [](int r_, int p_) {
-        const uint32_t c = uint32_t(p_) >> 1;
-        return uint32_t(r_) * ROWB + ((c ^ (c >> 3)) << 4) + ((uint32_t(p_) & 1u) << 3);
+        const uint32_t c = uint32_t(p_) / V;
+        return uint32_t(r_) * ROWB + ((c ^ (c >> 3)) << 4) + (uint32_t(p_) % V) * uint32_t(sizeof(TX));
     };
     const int64_t pstride = rpad * kpad;
     const bool vec = rows_vec(X, sr, sp);
@@ -928,11 +969,18 @@ __device__ __forceinline__ void slice_rows(int which, const double* __restrict__
         __syncthreads();
         unsigned long long xv[8];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const uint32_t c = uint32_t(4 * L + j);
+        for (int j = 0; j < int(8 / V); ++j) {
+            const uint32_t c = uint32_t(8 / V * L + j);
             const uint4 v = *reinterpret_cast<const uint4*>(tbuf + b * BUF + rr * ROWB + ((c ^ (c >> 3)) << 4));
-            xv[2 * j] = (unsigned long long)v.x | ((unsigned long long)v.y << 32);
-            xv[2 * j + 1] = (unsigned long long)v.z | ((unsigned long long)v.w << 32);
+            if constexpr (sizeof(TX) == 8) {
+                xv[2 * j] = (unsigned long long)v.x | ((unsigned long long)v.y << 32);
+                xv[2 * j + 1] = (unsigned long long)v.z | ((unsigned long long)v.w << 32);
+            } else {
+                xv[4 * j] = widened_bits(v.x);
+                xv[4 * j + 1] = widened_bits(v.y);
+                xv[4 * j + 2] = widened_bits(v.z);
+                xv[4 * j + 3] = widened_bits(v.w);
+            }
         }
         if (r < rpad)
             slice_emit<mode>(xv, sl, bt, e, bad, tab, reinterpret_cast<uint16_t*>(planes) + r * kpad + it * 64 + 8 * L,
@@ -941,12 +989,12 @@ __device__ __forceinline__ void slice_rows(int which, const double* __restrict__
     }
 }
 
-template <int MODE>
+template <int MODE, typename TX>
 __global__ void __launch_bounds__(256, 3) slice_kernel(const OperandPair op, int64_t K, const SplitInfo* __restrict__ info,
                                                        int64_t kpad, int kt) {
     const int w = blockIdx.y < op.yb0 ? 0 : 1;
     const int by = w ? int(blockIdx.y - op.yb0) : int(blockIdx.y);
-    slice_rows<MODE>(w, op.X[w], op.R[w], K, op.sr[w], op.sp[w], op.rexp[w], info, op.planes[w], op.rpad[w], kpad, by, kt);
+    slice_rows<MODE, TX>(w, static_cast<const TX*>(op.X[w]), op.R[w], K, op.sr[w], op.sp[w], op.rexp[w], info, op.planes[w], op.rpad[w], kpad, by, kt);
 }
 
 // ---- level / pair schedule ---------------------------------------------------------------------
@@ -1570,6 +1618,7 @@ __device__ __forceinline__ void crt_cols(const CrtWords<N>& r, const uint8_t* __
     }
 }
 
+template <typename TC>
 struct CrtCombine {
     const uint8_t* res;      // residue planes
     int64_t mpad, npad;
@@ -1578,17 +1627,26 @@ struct CrtCombine {
     int64_t m, n;            // rows, columns of this launch
     const int *eA, *eB;
     double alpha, beta;
-    double* C;
+    TC* C;
     int64_t ldc;
 };
 
+// alpha v + beta c in double precision, rounded once to the result's type.
+template <typename TC>
+__device__ __forceinline__ TC scaled(double v, double alpha, double beta, const TC* c) {
+    const double x = alpha * v;
+    return TC((beta == 0.0) ? x : fma(beta, double(*c), x));
+}
+
 // The rows i, i + gridDim.y, ... of four columns a thread, the next row's residues on their way while
 // one row is reconstructed.
-template <int N>
-__device__ __forceinline__ void crt_rows(const CrtCombine& p, int scale, int64_t j0, const int (&fj)[4]) {
+template <int N, typename TC>
+__device__ __forceinline__ void crt_rows(const CrtCombine<TC>& p, int scale, int64_t j0, const int (&fj)[4]) {
     const int64_t S = p.mpad * p.npad, step = int64_t(gridDim.y) * p.npad;
     const bool plain = p.alpha == 1.0 && p.beta == 0.0;
-    const bool pairs = j0 + 4 <= p.n && (p.ldc & 1) == 0 && (reinterpret_cast<uintptr_t>(p.C + p.col0) & 15) == 0;
+    // whole groups of four columns, 16-byte aligned in every row
+    const bool vec = j0 + 4 <= p.n && (p.ldc * int64_t(sizeof(TC))) % 16 == 0 &&
+                     (reinterpret_cast<uintptr_t>(p.C + p.col0) & 15) == 0;
     int64_t i = p.row0 + blockIdx.y, off = i * p.npad + p.col0 + j0;
     const int64_t end = p.row0 + p.m;
     if (i >= end) return;
@@ -1605,19 +1663,19 @@ __device__ __forceinline__ void crt_rows(const CrtCombine& p, int scale, int64_t
         }
         double v[4];
         crt_cols<N>(w, p.res, S, off, p.nseg, p.max_levels, scale, ei, fj, v);
-        double* crow = p.C + i * p.ldc + p.col0 + j0;
-        if (plain && pairs) {
-            *reinterpret_cast<double2*>(crow) = make_double2(v[0], v[1]);
-            *reinterpret_cast<double2*>(crow + 2) = make_double2(v[2], v[3]);
+        TC* crow = p.C + i * p.ldc + p.col0 + j0;
+        if (plain && vec) {
+            if constexpr (sizeof(TC) == 8) {
+                *reinterpret_cast<double2*>(crow) = make_double2(v[0], v[1]);
+                *reinterpret_cast<double2*>(crow + 2) = make_double2(v[2], v[3]);
+            } else {
+                *reinterpret_cast<float4*>(crow) = make_float4(float(v[0]), float(v[1]), float(v[2]), float(v[3]));
+            }
         } else {
 #pragma unroll
             for (int cc = 0; cc < 4; ++cc) {
                 if (j0 + cc >= p.n) break;
-                if (plain) crow[cc] = v[cc];
-                else {
-                    const double x = p.alpha * v[cc];
-                    crow[cc] = (p.beta == 0.0) ? x : fma(p.beta, crow[cc], x);
-                }
+                crow[cc] = plain ? TC(v[cc]) : scaled(v[cc], p.alpha, p.beta, crow + cc);
             }
         }
         if (!more) return;
@@ -1636,7 +1694,9 @@ __device__ __forceinline__ void crt_rows(const CrtCombine& p, int scale, int64_t
 // blocks an SM (64 registers) beat six or five by up to 3 %, and let a block run beside a
 // tensor-core CTA; two columns at a time instead of four took 186 instructions an output.
 constexpr int kCombineBlocks = 8;
-__global__ void __launch_bounds__(128, kCombineBlocks) crt_combine_kernel(const CrtCombine p, const SplitInfo* __restrict__ info) {
+template <typename TC>
+__global__ void __launch_bounds__(128, kCombineBlocks) crt_combine_kernel(const CrtCombine<TC> p,
+                                                                          const SplitInfo* __restrict__ info) {
     griddep_wait();
     const int64_t j0 = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) * 4;
     if (j0 >= p.n) return;
@@ -1646,7 +1706,7 @@ __global__ void __launch_bounds__(128, kCombineBlocks) crt_combine_kernel(const 
     for (int cc = 0; cc < 4; ++cc) fj[cc] = (j0 + cc < p.n) ? p.eB[p.col0 + j0 + cc] : 0;
     switch (info->slices) {
 #define GB_CRT_CASE(NN) \
-    case NN: crt_rows<NN>(p, scale, j0, fj); break;
+    case NN: crt_rows<NN, TC>(p, scale, j0, fj); break;
         GB_CRT_CASE(2) GB_CRT_CASE(3) GB_CRT_CASE(4) GB_CRT_CASE(5) GB_CRT_CASE(6) GB_CRT_CASE(7)
         GB_CRT_CASE(8) GB_CRT_CASE(9) GB_CRT_CASE(10) GB_CRT_CASE(11) GB_CRT_CASE(12) GB_CRT_CASE(13)
         GB_CRT_CASE(14) GB_CRT_CASE(15)
@@ -1662,10 +1722,11 @@ dim3 crt_combine_grid(int64_t m, int64_t n, int num_sms) {
     return dim3(unsigned(x), unsigned(y));
 }
 
+template <typename TC>
 __global__ void __launch_bounds__(128, 8) combine_kernel(const int32_t* __restrict__ levels, int nseg, int max_levels, int64_t mpad,
                                int64_t npad, int mode, const SplitInfo* __restrict__ info,
                                const int* __restrict__ eA, const int* __restrict__ eB, int64_t m, int64_t n,
-                               double alpha, double beta, double* __restrict__ C, int64_t ldc) {
+                               double alpha, double beta, TC* __restrict__ C, int64_t ldc) {
     griddep_wait();
     const int64_t j0 = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) * COMBINE_COLS;
     if (j0 >= n) return;
@@ -1709,16 +1770,12 @@ __global__ void __launch_bounds__(128, 8) combine_kernel(const int32_t* __restri
         for (int c = 0; c < COMBINE_COLS; ++c) v[c] = dacc[c];
     }
     const bool plain = (alpha == 1.0 && beta == 0.0);
-    double* crow = C + i * ldc;
+    TC* crow = C + i * ldc;
 #pragma unroll
     for (int c = 0; c < COMBINE_COLS; ++c) {
         const int64_t j = j0 + c;
         if (j >= n) break;
-        if (plain) crow[j] = v[c];
-        else {
-            const double x = alpha * v[c];
-            crow[j] = (beta == 0.0) ? x : fma(beta, crow[j], x);
-        }
+        crow[j] = plain ? TC(v[c]) : scaled(v[c], alpha, beta, crow + j);
     }
     }
 }
@@ -1743,29 +1800,6 @@ void split_decode_info(const void* info_host, int* slices, double* bound) {
     *slices = h.slices;
     *bound = h.bound;
 }
-
-namespace {
-// dst (rows x cols, pitch ld_d) = src (pitch ld_s), element-wise conversion: rows on blockIdx.y
-// (striding by gridDim.y), columns on threads.
-template <typename S, typename D>
-__global__ void convert_kernel(int64_t rows, int64_t cols, const S* __restrict__ src, int64_t ld_s, D* __restrict__ dst,
-                               int64_t ld_d) {
-    for (int64_t r = blockIdx.y; r < rows; r += gridDim.y)
-        for (int64_t c = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; c < cols; c += int64_t(gridDim.x) * blockDim.x)
-            dst[r * ld_d + c] = D(src[r * ld_s + c]);
-}
-
-template <typename S, typename D>
-cudaError_t launch_convert(int64_t rows, int64_t cols, const S* src, int64_t ld_s, D* dst, int64_t ld_d,
-                           cudaStream_t st) {
-    if (rows <= 0 || cols <= 0) return cudaSuccess;
-    const int64_t x = std::max<int64_t>(1, std::min<int64_t>((cols + 255) / 256, 64));
-    const int64_t y = std::max<int64_t>(1, std::min<int64_t>(rows, int64_t(runtime().num_sms) * 16 / x));
-    convert_kernel<S, D><<<dim3(unsigned(x), unsigned(y)), 256, 0, st>>>(rows, cols, src, ld_s, dst, ld_d);
-    count_launches(1);
-    return cudaGetLastError();
-}
-}  // namespace
 
 // ---- host orchestration ------------------------------------------------------------------------
 namespace {
@@ -1937,25 +1971,25 @@ bool runs_tma_tiles(const Gemm& g, const SplitRequest& req, bool stall) {
 
 // An operand read in place: by TMA when it is 16-byte aligned in base and pitch, by every other
 // kernel (single-element loads) when its base is aligned for a double.
-bool read_in_place(const void* p, int64_t ld, bool tma) {
-    return tma ? tma_ready(p, ld) : reinterpret_cast<uintptr_t>(p) % 8 == 0;
+bool read_in_place(const void* p, int64_t ld, bool tma, size_t elem = 8) {
+    return tma ? tma_ready(p, ld) : reinterpret_cast<uintptr_t>(p) % elem == 0;
 }
 
 // Copy operands that cannot be read in place into the workspace.
-int realign_operands(Gemm& g, bool tma, Workspace& ws, cudaStream_t st, std::string* err) {
+int realign_operands(Gemm& g, bool tma, size_t elem, Workspace& ws, cudaStream_t st, std::string* err) {
     if (g.k == 0) return GB300_OK;
     for (int which = 0; which < 2; ++which) {
         const void*& p = which == 0 ? g.A : g.B;
         int64_t& ld = which == 0 ? g.lda : g.ldb;
-        if (read_in_place(p, ld, tma)) continue;
+        if (read_in_place(p, ld, tma, elem)) continue;
         int64_t rows, cols;
         if (which == 0) stored_a(g, &rows, &cols);
         else stored_b(g, &rows, &cols);
         const int64_t ldp = (cols + 1) / 2 * 2;
-        void* d = ws.get(which == 0 ? kSlotA : kSlotB, size_t(rows) * size_t(ldp) * 8, err);
+        void* d = ws.get(which == 0 ? kSlotA : kSlotB, size_t(rows) * size_t(ldp) * elem, err);
         if (!d) return GB300_ERR_NO_MEMORY;
-        const cudaError_t e = cudaMemcpy2DAsync(d, size_t(ldp) * 8, p, size_t(ld) * 8, size_t(cols) * 8, size_t(rows),
-                                                cudaMemcpyDeviceToDevice, st);
+        const cudaError_t e = cudaMemcpy2DAsync(d, size_t(ldp) * elem, p, size_t(ld) * elem, size_t(cols) * elem,
+                                                size_t(rows), cudaMemcpyDeviceToDevice, st);
         if (e != cudaSuccess) {
             if (err) *err = std::string("operand realignment: ") + cudaGetErrorString(e);
             return GB300_ERR_CUDA;
@@ -2075,15 +2109,12 @@ static void part_events_put(const PartEvents& pe) {
     r.part_events.push_back(pe.done0);
 }
 
-int device_product(const Gemm& g_in, const SplitRequest& req, const LaunchCtl& ctl, cudaStream_t st, Workspace& ws,
+namespace {
+// The tensor-core forms on operands and result of type T (double or float).
+template <typename T>
+int tensor_product(const Gemm& g, const SplitRequest& req, const LaunchCtl& ctl, cudaStream_t st, Workspace& ws,
                    SplitResult* out, std::string* err) {
     Runtime& r = runtime();
-    Gemm g = g_in;
-    {
-        const int rst = realign_operands(g, runs_tma_tiles(g, req, ctl.inject_stall != 0), ws, st, err);
-        if (rst != GB300_OK) return rst;
-    }
-    if (runs_native(g, req)) return native_product(g, ctl, st, ws, out, err);
 
     const SplitGeometry G = split_geometry(g, req, r.num_sms);
     const int mode = G.mode;
@@ -2111,11 +2142,8 @@ int device_product(const Gemm& g_in, const SplitRequest& req, const LaunchCtl& c
     // operand strides of the logical R x K views
     const int64_t a_sr = g.ta ? 1 : g.lda, a_sp = g.ta ? g.lda : 1;
     const int64_t b_sr = g.tb ? g.ldb : 1, b_sp = g.tb ? 1 : g.ldb;
-    const double* A = static_cast<const double*>(g.A);
-    const double* B = static_cast<const double*>(g.B);
-
     OperandPair op;
-    op.X[0] = A; op.X[1] = B;
+    op.X[0] = g.A; op.X[1] = g.B;
     op.R[0] = m; op.R[1] = n;
     op.sr[0] = a_sr; op.sr[1] = b_sr;
     op.sp[0] = a_sp; op.sp[1] = b_sp;
@@ -2135,7 +2163,7 @@ int device_product(const Gemm& g_in, const SplitRequest& req, const LaunchCtl& c
         const double target = req.target_error > 0 ? req.target_error : double(k) * 0x1p-53;
         sa.plan = PlanArgs{kPlanProduct, mode, req.slices > 0 ? max_planes : 0, max_planes, target, info};
         cudaMemsetAsync(sa.count, 0, size_t(SL.blocks + 1) * sizeof(unsigned), st);
-        stats_kernel<<<dim3(unsigned(SL.chunks), unsigned(SL.blocks)), 256, 0, st>>>(sa);
+        stats_kernel<T><<<dim3(unsigned(SL.chunks), unsigned(SL.blocks)), 256, 0, st>>>(sa);
     }
     if (cudaError_t le = cudaGetLastError(); le != cudaSuccess) {
         if (err) *err = std::string("split pre-pass launch: ") + cudaGetErrorString(le);
@@ -2147,8 +2175,10 @@ int device_product(const Gemm& g_in, const SplitRequest& req, const LaunchCtl& c
         const int64_t yb = mpad / 32 + npad / 32, tiles = kpad / 64;
         const int kt = tiles_per_block(tiles, yb, r.num_sms);
         const dim3 grid(unsigned((tiles + kt - 1) / kt), unsigned(yb));
-        auto sk = mode == kCrt ? slice_kernel<kCrt>
-                               : (mode == kExact ? slice_kernel<kExact> : (mode == kBf16 ? slice_kernel<kBf16> : slice_kernel<kBf16x3>));
+        auto sk = mode == kCrt     ? slice_kernel<kCrt, T>
+                  : mode == kExact ? slice_kernel<kExact, T>
+                  : mode == kBf16  ? slice_kernel<kBf16, T>
+                                   : slice_kernel<kBf16x3, T>;
         launch_dependent(sk, grid, dim3(256), 0, st, sp2, k, info, kpad, kt);
     }
     count_launches(2);
@@ -2204,10 +2234,10 @@ int device_product(const Gemm& g_in, const SplitRequest& req, const LaunchCtl& c
     };
     // reconstruction of C's columns [c0, c0 + nc) on stream s
     auto launch_crt_combine = [&](int64_t c0, int64_t nc, cudaStream_t s) {
-        const CrtCombine q{reinterpret_cast<const uint8_t*>(lv), mpad, npad, nseg, max_levels, 0, c0, m, nc, eA, eB,
-                           g.alpha, g.beta, static_cast<double*>(g.C), g.ldc};
-        if (s == st) launch_dependent(crt_combine_kernel, crt_combine_grid(m, nc, r.num_sms), dim3(128), 0, s, q, info);
-        else crt_combine_kernel<<<crt_combine_grid(m, nc, r.num_sms), 128, 0, s>>>(q, info);  // behind an event
+        const CrtCombine<T> q{reinterpret_cast<const uint8_t*>(lv), mpad, npad, nseg, max_levels, 0, c0, m, nc, eA, eB,
+                              g.alpha, g.beta, static_cast<T*>(g.C), g.ldc};
+        if (s == st) launch_dependent(crt_combine_kernel<T>, crt_combine_grid(m, nc, r.num_sms), dim3(128), 0, s, q, info);
+        else crt_combine_kernel<T><<<crt_combine_grid(m, nc, r.num_sms), 128, 0, s>>>(q, info);  // behind an event
     };
     const bool in_parts = mode == kCrt && n_tiles >= 2 && m_tiles * n_tiles >= sms && req.max_sms <= 0;
     if (in_parts) {
@@ -2232,8 +2262,8 @@ int device_product(const Gemm& g_in, const SplitRequest& req, const LaunchCtl& c
         } else {
             const int64_t colgroups = (n + COMBINE_COLS - 1) / COMBINE_COLS;
             dim3 cgrid(unsigned((colgroups + 127) / 128), unsigned(std::min<int64_t>(m, 65535)));
-            launch_dependent(combine_kernel, cgrid, dim3(128), 0, st, lv, nseg, max_levels, mpad, npad, mode, info, eA, eB,
-                             m, n, g.alpha, g.beta, static_cast<double*>(g.C), g.ldc);
+            launch_dependent(combine_kernel<T>, cgrid, dim3(128), 0, st, lv, nseg, max_levels, mpad, npad, mode, info, eA,
+                             eB, m, n, g.alpha, g.beta, static_cast<T*>(g.C), g.ldc);
         }
     }
     count_launches(2);
@@ -2253,43 +2283,32 @@ int device_product(const Gemm& g_in, const SplitRequest& req, const LaunchCtl& c
 }
 
 
-// A float product through the FP64-accurate machinery: A and B (device, float, the caller's
-// pitches) are widened to double in `conv`'s slots 0 and 1 (exact), C in slot 2 (read only when
-// beta != 0), device_product runs at the float target (k 2^-24 unless the request sets one), and
-// the double result is rounded once to float into C.  The reported bound adds 2^-24 for that final
-// rounding.
-int device_product_float(const Gemm& g, const SplitRequest& req_in, const LaunchCtl& ctl, cudaStream_t st,
-                         Workspace& ws, Workspace& conv, SplitResult* out, std::string* err) {
-    const int64_t a_rows = g.ta ? g.k : g.m, a_cols = g.ta ? g.m : g.k;
-    const int64_t b_rows = g.tb ? g.n : g.k, b_cols = g.tb ? g.k : g.n;
-    const int64_t pa = (a_cols + 1) / 2 * 2, pb = (b_cols + 1) / 2 * 2, pc = (g.n + 1) / 2 * 2;  // 16-byte pitches
-    auto* dA = static_cast<double*>(conv.get(0, size_t(a_rows) * size_t(pa) * 8, err));
-    auto* dB = static_cast<double*>(conv.get(1, size_t(b_rows) * size_t(pb) * 8, err));
-    auto* dC = static_cast<double*>(conv.get(2, size_t(g.m) * size_t(pc) * 8, err));
-    if (!dA || !dB || !dC) return GB300_ERR_NO_MEMORY;
-    cudaError_t e = launch_convert(a_rows, a_cols, static_cast<const float*>(g.A), g.lda, dA, pa, st);
-    if (e == cudaSuccess) e = launch_convert(b_rows, b_cols, static_cast<const float*>(g.B), g.ldb, dB, pb, st);
-    if (e == cudaSuccess && g.beta != 0.0)
-        e = launch_convert(g.m, g.n, static_cast<const float*>(g.C), g.ldc, dC, pc, st);
-    if (e != cudaSuccess) {
-        if (err) *err = std::string("float widening: ") + cudaGetErrorString(e);
-        return GB300_ERR_CUDA;
-    }
-    Gemm g64 = g;
-    g64.A = dA; g64.lda = pa;
-    g64.B = dB; g64.ldb = pb;
-    g64.C = dC; g64.ldc = pc;
+}  // namespace
+
+int device_product(const Gemm& g_in, const SplitRequest& req, const LaunchCtl& ctl, cudaStream_t st, Workspace& ws,
+                   SplitResult* out, std::string* err) {
+    Gemm g = g_in;
+    const int rst = realign_operands(g, runs_tma_tiles(g, req, ctl.inject_stall != 0), 8, ws, st, err);
+    if (rst != GB300_OK) return rst;
+    if (runs_native(g, req)) return native_product(g, ctl, st, ws, out, err);
+    return tensor_product<double>(g, req, ctl, st, ws, out, err);
+}
+
+// A float product through the FP64-accurate machinery at the float target (k 2^-24 unless the request
+// sets one).  The statistics and the slicing read the float operands, whose values a double holds
+// exactly, and the reconstruction's double result (with alpha and beta applied in double) is rounded
+// once to float; widened copies of A, B and C beside them took 39 us of a 2048^3 product.  The
+// reported bound adds 2^-24 for that rounding.
+int device_product_float(const Gemm& g_in, const SplitRequest& req_in, const LaunchCtl& ctl, cudaStream_t st,
+                         Workspace& ws, SplitResult* out, std::string* err) {
+    Gemm g = g_in;
+    const int rst = realign_operands(g, false, 4, ws, st, err);
+    if (rst != GB300_OK) return rst;
     SplitRequest req = req_in;
     if (req.target_error <= 0) req.target_error = double(std::max<int64_t>(g.k, 1)) * 0x1p-24;
-    const int st_ = device_product(g64, req, ctl, st, ws, out, err);
-    if (st_ != GB300_OK) return st_;
-    e = launch_convert(g.m, g.n, static_cast<const double*>(dC), pc, static_cast<float*>(g.C), g.ldc, st);
-    if (e != cudaSuccess) {
-        if (err) *err = std::string("float rounding: ") + cudaGetErrorString(e);
-        return GB300_ERR_CUDA;
-    }
-    if (out->error_bound >= 0) out->error_bound += 0x1p-24;
-    return GB300_OK;
+    const int st_ = tensor_product<float>(g, req, ctl, st, ws, out, err);
+    if (st_ == GB300_OK && out->error_bound >= 0) out->error_bound += 0x1p-24;
+    return st_;
 }
 
 namespace {
@@ -2441,12 +2460,12 @@ int device_product_host_panels(const Gemm& g, const SplitRequest& req, const Lau
         sa.group = reinterpret_cast<RowPartial*>(scratch + count_bytes);
         sa.part = reinterpret_cast<uint2*>(scratch + count_bytes + group_bytes);
         sa.plan = PlanArgs{kPlanSide, kCrt, 0, max_planes, target, info};
-        stats_kernel<<<dim3(unsigned(L.chunks), unsigned(L.blocks)), 256, 0, st>>>(sa);
+        stats_kernel<double><<<dim3(unsigned(L.chunks), unsigned(L.blocks)), 256, 0, st>>>(sa);
     };
     auto run_slice = [&](const OperandPair& o, int64_t yb, const SplitInfo* info) {
         const int64_t tiles = kpad / 64;
         const int kt = tiles_per_block(tiles, yb, r.num_sms);
-        launch_dependent(slice_kernel<kCrt>, dim3(unsigned((tiles + kt - 1) / kt), unsigned(yb)), dim3(256), 0, st, o, k,
+        launch_dependent(slice_kernel<kCrt, double>, dim3(unsigned((tiles + kt - 1) / kt), unsigned(yb)), dim3(256), 0, st, o, k,
                          info, kpad, kt);
     };
     const int64_t a_sr = g.ta ? 1 : a_cols, a_sp = g.ta ? a_cols : 1;
@@ -2595,9 +2614,9 @@ int device_product_host_panels(const Gemm& g, const SplitRequest& req, const Lau
             // in two row halves, so that the first one's copy back starts while the second is reconstructed
             for (int h = 0; h < 2; ++h) {
                 const int64_t h0 = h ? half_rows(mi) : 0, h1 = h ? mi : half_rows(mi);
-                const CrtCombine q{reinterpret_cast<const uint8_t*>(lvb), mpad, npb, nseg, max_levels, h0, cj, h1 - h0, nj,
-                                   eA + r0, eB, g.alpha, g.beta, dC + r0 * n, n};
-                crt_combine_kernel<<<crt_combine_grid(h1 - h0, nj, r.num_sms), 128, 0, aux>>>(q, info_at(P + Q + i * Q + j));
+                const CrtCombine<double> q{reinterpret_cast<const uint8_t*>(lvb), mpad, npb, nseg, max_levels, h0, cj, h1 - h0, nj,
+                                           eA + r0, eB, g.alpha, g.beta, dC + r0 * n, n};
+                crt_combine_kernel<double><<<crt_combine_grid(h1 - h0, nj, r.num_sms), 128, 0, aux>>>(q, info_at(P + Q + i * Q + j));
                 if ((e = cudaGetLastError()) != cudaSuccess) return;
                 cudaEventRecord(h ? block_ev(i, j) : half_ev(i, j), aux);
             }
