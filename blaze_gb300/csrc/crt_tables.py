@@ -70,8 +70,10 @@ def table(n):
             assert (cp * s["A"] + cq * s["B"]) % Ps == x * ys % Ps
         assert (p - 1) * s["A"] + (q - 1) * s["B"] < 1 << 26
     fbias = sum((1 << 23) / s["Ps"] for s in sups)
-    limbs = (P.bit_length() + 1 + 31) // 32  # signed result |W| < P / 2
-    return dict(n=n, P=P, sups=sups, fbias=fbias, limbs=limbs, negP=(1 << (32 * limbs)) - P)
+    bits = (P * 1000 // 2125).bit_length() + 1  # the signed result, |T| < P / 2.125
+    limbs = (bits + 31) // 32
+    assert P < 1 << (32 * limbs)
+    return dict(n=n, P=P, sups=sups, fbias=fbias, limbs=limbs, negP=(1 << (32 * limbs)) - P, bits=bits)
 
 
 def emit(path):
@@ -95,6 +97,7 @@ def emit(path):
         "",
         "struct CrtTable {",
         "    int nsup, limbs;            // super moduli; 32-bit limbs of the signed result",
+        "    int bits;                   // bits of the signed result",
         "    uint32_t negP[4];           // 2^(32 limbs) - product of the moduli, 32-bit limbs",
         f"    CrtSuper sup[{MAX_SUP}];",
         "};",
@@ -105,7 +108,7 @@ def emit(path):
     for n in range(2, 16):
         t = table(n)
         P32 = ", ".join(f"{(t['negP'] >> (32 * l)) & 0xFFFFFFFF}u" for l in range(4))
-        lines.append(f"    {{{len(t['sups'])}, {t['limbs']}, {{{P32}}}, {{  // N = {n}")
+        lines.append(f"    {{{len(t['sups'])}, {t['limbs']}, {t['bits']}, {{{P32}}}, {{  // N = {n}")
         for s in t["sups"]:
             M = ", ".join(f"{m}u" for m in s["M"])
             finv = f32hex(1.0 / s["Ps"])

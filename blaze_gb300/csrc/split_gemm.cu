@@ -1466,14 +1466,16 @@ struct CrtWords {
     uint32_t w[N];  // w[0] unused
 };
 
+// row: the plane offset of the block's row and the launch's first column, j: the thread's column from
+// there; row is the same for the whole block, so the addresses are formed once per warp.
 template <int N>
-__device__ __forceinline__ CrtWords<N> crt_load(const uint8_t* __restrict__ res, int64_t S, int max_levels, int64_t off) {
+__device__ __forceinline__ CrtWords<N> crt_load(const uint8_t* __restrict__ res, int64_t S, int64_t row, uint32_t j) {
     CrtWords<N> r;
-    const uint2 z = *reinterpret_cast<const uint2*>(res + 2 * off);
+    const uint2 z = *reinterpret_cast<const uint2*>(res + 2 * row + 2u * j);
     r.w0[0] = z.x;
     r.w0[1] = z.y;
 #pragma unroll
-    for (int t = 1; t < N; ++t) r.w[t] = *reinterpret_cast<const uint32_t*>(res + crt_plane(S, max_levels, 0, t) + off);
+    for (int t = 1; t < N; ++t) r.w[t] = *reinterpret_cast<const uint32_t*>(res + crt_plane(S, 0, 0, t) + row + j);
     return r;
 }
 
@@ -1490,57 +1492,73 @@ __device__ __forceinline__ uint32_t crt_seg_sum(const uint8_t* __restrict__ res,
     return mod_small(sum + 128u * (p - 1u) * uint32_t(nseg - 1), p, pinv32);
 }
 
-// sign |W| 2^x for the two's-complement integer W of LB 32-bit words (low word first), rounded to nearest
-// even.  Straight-line code: the magnitude's words move up until the top one is not zero, a funnel
-// shift brings the leading bit to the top, and the 53-bit mantissa is rounded on integers; adding
-// (be - 1) << 52 to it writes the exponent, a rounding carry into 2^53 moving it up by itself.  Results
-// that are not normal numbers take the FP64 path (ldexp), rows or columns with Inf / NaN (whose
-// exponent kNonFinite lands there too) give NaN.
+// The double W 2^(x) of the two's-complement integer W of LB 32-bit words (low word first), rounded to
+// nearest even, where W fits `bits` bits with its sign: rows or columns with Inf / NaN (exponent
+// kNonFinite) give NaN, and results that are not normal numbers take the FP64 path (ldexp).  General
+// form, for outputs whose leading words are all sign: the magnitude's words move up until the top
+// one is not zero.
 template <int LB>
-__device__ __forceinline__ double words_to_double(const uint32_t (&w)[4], int ei, int fj, int scale) {
+__device__ __noinline__ double words_to_double_any(uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3, int ei, int fj,
+                                                   int scale) {
+    if (ei == kNonFinite || fj == kNonFinite) return __longlong_as_double(0x7ff8000000000000ll);
+    const uint32_t w[4] = {w0, w1, w2, w3};
     const uint32_t sgn = uint32_t(int32_t(w[LB - 1]) >> 31);
     uint32_t z[4] = {0u, 0u, 0u, 0u};  // the magnitude, top word first
-    if constexpr (LB == 1) {
-        z[0] = (w[0] ^ sgn) - sgn;
-    } else {
-        unsigned long long lo = (unsigned long long)w[0] | ((unsigned long long)w[1] << 32);
-        lo = (lo ^ (unsigned long long)(long long)int32_t(sgn)) - (unsigned long long)(long long)int32_t(sgn);
-        z[LB - 1] = uint32_t(lo);
-        z[LB - 2] = uint32_t(lo >> 32);
-        if constexpr (LB > 2) {
-            const unsigned long long carry = (sgn != 0u && lo == 0ull) ? 1ull : 0ull;
-            unsigned long long hi = (unsigned long long)w[2] | (LB > 3 ? (unsigned long long)w[LB - 1] << 32 : 0ull);
-            hi = (hi ^ (unsigned long long)(long long)int32_t(sgn)) + carry;
-            z[LB - 3] = uint32_t(hi);
-            if constexpr (LB > 3) z[0] = uint32_t(hi >> 32);
-        }
+    uint32_t carry = sgn & 1u;
+#pragma unroll
+    for (int i = 0; i < LB; ++i) {
+        const unsigned long long t = (unsigned long long)(w[i] ^ sgn) + carry;
+        z[LB - 1 - i] = uint32_t(t);
+        carry = uint32_t(t >> 32);
     }
     int lead = 32 * LB - 1;  // position of the leading bit
 #pragma unroll
-    for (int i = 1; i < LB; ++i) {
-        const bool up = z[0] == 0u;
+    for (int i = 1; i < LB; ++i)
+        if (z[0] == 0u) {
 #pragma unroll
-        for (int j = 0; j < LB - i; ++j) z[j] = up ? z[j + 1] : z[j];
-        z[LB - i] = up ? 0u : z[LB - i];
-        lead -= up ? 32 : 0;
-    }
+            for (int j = 0; j < 3; ++j) z[j] = z[j + 1];
+            z[3] = 0u;
+            lead -= 32;
+        }
+    if (z[0] == 0u) return 0.0;
     const int lz = __clz(int(z[0]));
     const uint32_t t1 = __funnelshift_l(z[1], z[0], lz);
-    uint32_t t0 = __funnelshift_l(z[2], z[1], lz);
-    if constexpr (LB > 2) t0 |= min(__funnelshift_l(z[3], z[2], lz) | (LB > 3 ? z[3] : 0u), 1u);  // sticky
+    const uint32_t t0 = __funnelshift_l(z[2], z[1], lz) | min(__funnelshift_l(z[3], z[2], lz) | z[3], 1u);  // sticky
     unsigned long long mant = (((unsigned long long)t1 << 32) | t0) >> 11;
     mant += (t0 & 0x7ffu) + (uint32_t(mant) & 1u) > 0x400u ? 1ull : 0ull;
-    const int x = ei + fj - scale;
-    const int be = lead - lz + x + 1023;
-    if (be >= 1 && be <= 2045) {
-        unsigned long long bits = mant + ((unsigned long long)uint32_t(be - 1) << 52);
-        bits |= (unsigned long long)(sgn & 0x80000000u) << 32;
-        return z[0] == 0u ? 0.0 : __longlong_as_double((long long)bits);
-    }
-    if (ei == kNonFinite || fj == kNonFinite) return __longlong_as_double(0x7ff8000000000000ll);
-    if (z[0] == 0u) return 0.0;
-    const double v = ldexp(double(mant), lead - lz - 52 + x);
+    const double v = ldexp(double(mant), lead - lz - 52 + ei + fj - scale);
     return sgn ? -v : v;
+}
+
+// The usual case in straight-line code: W, moved up by the constant that brings its sign bit to the top,
+// has a bit that is not sign in its top word; the funnel shift that puts that bit below the sign
+// leaves 64 bits whose rounding to nearest even (symmetric, so no magnitude is formed before it) is
+// an integer addition, and adding the exponent's bits to the 53-bit magnitude writes it, a rounding
+// carry into 2^53 moving the exponent up by itself.  About 30 instructions; with the magnitude formed
+// first and the words moved up one at a time it was about 55.
+template <int LB, int BITS>
+__device__ __forceinline__ double words_to_double(const uint32_t (&w)[4], int ei, int fj, int scale) {
+    constexpr int UP = 32 * LB - BITS;  // 0 <= UP < 32
+    uint32_t z[4] = {0u, 0u, 0u, 0u};  // top word first
+#pragma unroll
+    for (int i = 0; i < LB; ++i) z[i] = UP == 0 ? w[LB - 1 - i] : __funnelshift_l(i + 1 < LB ? w[LB - 2 - i] : 0u, w[LB - 1 - i], UP);
+    const uint32_t sgn = uint32_t(int32_t(z[0]) >> 31);
+    const int lz = __clz(int(z[0] ^ sgn));  // at least 1, 32 when the top word is all sign
+    const int sh = lz - 1;
+    uint32_t t1 = __funnelshift_l(z[1], z[0], sh), t0 = __funnelshift_l(z[2], z[1], sh);
+    if constexpr (LB > 2) t0 |= min(__funnelshift_l(z[3], z[2], sh) | (LB > 3 ? z[3] : 0u), 1u);  // sticky
+    // mantissa in bits 62..10
+    unsigned long long v = ((unsigned long long)t1 << 32) | t0;
+    v += 0x1ffu + ((t0 >> 10) & 1u);
+    const uint32_t rl = uint32_t(v >> 10), rh = uint32_t(int32_t(uint32_t(v >> 32)) >> 10);
+    unsigned long long m = ((unsigned long long)(rh ^ sgn) << 32) | (rl ^ sgn);
+    m += sgn & 1u;
+    const int be = BITS - 1 - lz + ei + fj - scale + 1023;  // the leading bit is bit BITS - 1 - lz of W
+    if (lz < 32 && be >= 1 && be <= 2045) {
+        const uint32_t hi = uint32_t(m >> 32) + (uint32_t(be - 1) << 20) + (sgn & 0x80000000u);
+        return __hiloint2double(int(hi), int(uint32_t(m)));
+    }
+    return words_to_double_any<LB>(w[0], w[1], w[2], w[3], ei, fj, scale);
 }
 
 // Residue (CRT) reconstruction of four consecutive outputs of one row for N moduli, all constants
@@ -1614,7 +1632,7 @@ __device__ __forceinline__ void crt_cols(const CrtWords<N>& r, const uint8_t* __
             w[l] = uint32_t(a);
             carry = a >> 32;
         }
-        v[cc] = words_to_double<LB>(w, ei, fj[cc], scale);
+        v[cc] = words_to_double<LB, T.bits>(w, ei, fj[cc], scale);
     }
 }
 
@@ -1638,8 +1656,7 @@ __device__ __forceinline__ TC scaled(double v, double alpha, double beta, const 
     return TC((beta == 0.0) ? x : fma(beta, double(*c), x));
 }
 
-// The rows i, i + gridDim.y, ... of four columns a thread, the next row's residues on their way while
-// one row is reconstructed.
+// The rows i, i + gridDim.y, ... of four columns a thread.
 template <int N, typename TC>
 __device__ __forceinline__ void crt_rows(const CrtCombine<TC>& p, int scale, int64_t j0, const int (&fj)[4]) {
     const int64_t S = p.mpad * p.npad, step = int64_t(gridDim.y) * p.npad;
@@ -1647,22 +1664,17 @@ __device__ __forceinline__ void crt_rows(const CrtCombine<TC>& p, int scale, int
     // whole groups of four columns, 16-byte aligned in every row
     const bool vec = j0 + 4 <= p.n && (p.ldc * int64_t(sizeof(TC))) % 16 == 0 &&
                      (reinterpret_cast<uintptr_t>(p.C + p.col0) & 15) == 0;
-    int64_t i = p.row0 + blockIdx.y, off = i * p.npad + p.col0 + j0;
+    int64_t i = p.row0 + blockIdx.y, row = i * p.npad + p.col0;
     const int64_t end = p.row0 + p.m;
     if (i >= end) return;
-    CrtWords<N> w = crt_load<N>(p.res, S, p.max_levels, off);
-    int ei = p.eA[i];
+    const uint32_t j = uint32_t(j0);
     while (true) {
         const int64_t inext = i + gridDim.y;
         const bool more = inext < end;
-        CrtWords<N> wn = w;
-        int en = ei;
-        if (more) {
-            wn = crt_load<N>(p.res, S, p.max_levels, off + step);
-            en = p.eA[inext];
-        }
+        const CrtWords<N> w = crt_load<N>(p.res, S, row, j);
+        const int ei = p.eA[i];
         double v[4];
-        crt_cols<N>(w, p.res, S, off, p.nseg, p.max_levels, scale, ei, fj, v);
+        crt_cols<N>(w, p.res, S, row + j0, p.nseg, p.max_levels, scale, ei, fj, v);
         TC* crow = p.C + i * p.ldc + p.col0 + j0;
         if (plain && vec) {
             if constexpr (sizeof(TC) == 8) {
@@ -1679,20 +1691,19 @@ __device__ __forceinline__ void crt_rows(const CrtCombine<TC>& p, int scale, int
             }
         }
         if (!more) return;
-        w = wn;
-        ei = en;
         i = inext;
-        off += step;
+        row += step;
     }
 }
 
 // Residue (CRT) reconstruction and epilogue: C = alpha * W 2^(e_i + f_j - scale) + beta * C.  Bound by
-// instruction issue and latency (about 160 instructions an output at 13 moduli, half the issue slots
-// busy; 118 MB read and 134 MB written take 38 us of the 72 at 32768 x 256).  Byte planes and the
-// straight-line conversion to double against 16-bit planes, a reduction of every super residue and a
-// branching conversion: 33.5 M outputs at 12 moduli 285 -> 243 us, 8.4 M at 13 moduli 90 -> 72.  Eight
-// blocks an SM (64 registers) beat six or five by up to 3 %, and let a block run beside a
-// tensor-core CTA; two columns at a time instead of four took 186 instructions an output.
+// instruction issue and latency (about 137 instructions an output at 13 moduli, half the issue slots
+// busy; 118 MB read and 134 MB written would take 38 us of the 63 at 32768 x 256).  Byte planes, super
+// residues left unreduced and a straight-line conversion to double against 16-bit planes, a reduction of
+// every super residue and a branching conversion: 8.4 M outputs at 13 moduli 90 -> 63 us, 33.5 M at 12
+// moduli 285 -> 184.  Eight blocks an SM (64 registers) measured like six and 4 % faster than five, and
+// let a block run beside a tensor-core CTA; fetching the next row's residues ahead cost the registers of
+// it (66 us), two columns at a time instead of four took 40 % more instructions.
 constexpr int kCombineBlocks = 8;
 template <typename TC>
 __global__ void __launch_bounds__(128, kCombineBlocks) crt_combine_kernel(const CrtCombine<TC> p,
