@@ -142,6 +142,19 @@ int real_product(const Gemm& g, const LaunchCtl& ctl, cudaStream_t st, std::stri
     return e == cudaSuccess ? GB300_OK : GB300_ERR_CUDA;
 }
 
+// Whether a product M x N x K reads its operands before it writes its result, so that the result may
+// take an operand's place: the tensor-core forms slice both operands first, and a complex product
+// goes through planes.  The native kernel reads as it writes.
+template <typename T, bool CPLX>
+bool reads_before_writing(int64_t M, int64_t N, int64_t K) {
+    if (CPLX) return true;
+    if (sizeof(T) != 8) return false;
+    const int method = library_default_method();
+    Gemm g;
+    g.m = M; g.n = N; g.k = K;
+    return method != GB300_METHOD_NATIVE && !(method == GB300_METHOD_AUTO && split_auto_uses_native(g));
+}
+
 LaunchCtl fresh_ctl(cudaStream_t st) {
     Runtime& r = runtime();
     LaunchCtl ctl;
@@ -676,7 +689,7 @@ struct SolveForm {
 // leaf size solve_block().  The half whose unknowns do not depend on the other is solved first, then one
 // product subtracts its contribution from the other half's right-hand sides (alpha = -1,
 // beta = 1), then the other half is solved.  A range of at most one leaf is multiplied by its
-// block's inverse, into `tmp` and copied back.
+// block's inverse, in place or into `tmp` and copied back.
 template <typename T, bool CPLX>
 int solve_range(const SolveForm& f, int64_t lo, int64_t hi, int64_t sbr, int64_t sbc, const T* SA, int64_t lda,
                 T* SB, int64_t ldb, const T* inv, T* tmp, const LaunchCtl& ctl, cudaStream_t s, std::string* err) {
@@ -706,6 +719,11 @@ int solve_range(const SolveForm& f, int64_t lo, int64_t hi, int64_t sbr, int64_t
     if (hi - lo <= nb) {
         const int64_t nk = hi - lo;
         const T* Ib = inv + (lo / nb) * int64_t(nb) * nb * w;
+        // straight into the right-hand sides where the product has read them by then, else through tmp
+        if (f.left && reads_before_writing<T, CPLX>(nk, sbc, nk))
+            return product(nk, sbc, nk, false, false, false, false, Ib, nb, rows_of(lo), ldb, false, rows_of(lo), ldb);
+        if (!f.left && reads_before_writing<T, CPLX>(sbr, nk, nk))
+            return product(sbr, nk, nk, false, false, false, false, cols_of(lo), ldb, Ib, nb, false, cols_of(lo), ldb);
         int st;
         cudaError_t e;
         if (f.left) {

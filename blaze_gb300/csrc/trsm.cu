@@ -20,6 +20,7 @@
 #include "cplx.cuh"
 #include "gb300_internal.h"
 #include "level23.h"
+#include "ptx.cuh"
 #include "runtime.h"
 
 namespace gb {
@@ -91,6 +92,7 @@ template <typename V>
 __global__ void __launch_bounds__(32) tri_base_kernel(const TriArgs<V> a) {
     using A = Ar<V>;
     __shared__ V Ls[2][kTriBase][kTriBase + 1];
+    griddep_launch();
     const int per = a.nb / kTriBase, c = threadIdx.x % kTriBase, h = threadIdx.x / kTriBase;
     V (&L)[kTriBase][kTriBase + 1] = Ls[h];
     const int g = int(blockIdx.x) * 2 + h;
@@ -131,6 +133,8 @@ template <typename V, bool SECOND>
 __global__ void __launch_bounds__(256) tri_join_kernel(const TriArgs<V> a, int s) {
     using A = Ar<V>;
     __shared__ V As[16][17], Bs[16][17];
+    griddep_launch();
+    griddep_wait();
     const int pairs = a.nb / (2 * s);
     const TriBlock<V> t(a, blockIdx.y / pairs);
     const int q0 = int(blockIdx.y % pairs) * 2 * s;   // first row of the upper half
@@ -177,6 +181,7 @@ __global__ void __launch_bounds__(256) tri_join_kernel(const TriArgs<V> a, int s
 // Zeros above the diagonal of every inverted block.
 template <typename V>
 __global__ void __launch_bounds__(256) tri_zero_kernel(const TriArgs<V> a) {
+    griddep_wait();
     const TriBlock<V> t(a, blockIdx.y);
     for (int r = blockIdx.x; r < t.rows; r += gridDim.x)
         for (int c = r + 1 + threadIdx.x; c < t.rows; c += blockDim.x) t.out[r * t.orow + c * t.ocol] = Ar<V>::zero();
@@ -217,10 +222,10 @@ cudaError_t launch_tri_inverse(int64_t ka, int nb, const T* SA, int64_t lda, boo
     for (int s = kTriBase; s < rows; s *= 2, launches += 2) {
         // gridDim.y holds at most 65535 pairs: ka / 32 of them on the first level
         const dim3 grid(unsigned((s / 16) * (s / 16)), unsigned(blocks * (nb / (2 * s))));
-        tri_join_kernel<V, false><<<grid, 256, 0, st>>>(a, s);
-        tri_join_kernel<V, true><<<grid, 256, 0, st>>>(a, s);
+        launch_dependent(tri_join_kernel<V, false>, grid, dim3(256), 0, st, a, s);
+        launch_dependent(tri_join_kernel<V, true>, grid, dim3(256), 0, st, a, s);
     }
-    tri_zero_kernel<V><<<dim3(unsigned(std::min<int64_t>(rows, 64)), unsigned(blocks)), 256, 0, st>>>(a);
+    launch_dependent(tri_zero_kernel<V>, dim3(unsigned(std::min<int64_t>(rows, 64)), unsigned(blocks)), dim3(256), 0, st, a);
     count_launches(launches);
     return cudaGetLastError();
 }
