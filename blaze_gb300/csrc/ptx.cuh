@@ -183,7 +183,9 @@ __device__ __forceinline__ uint32_t swz128(uint32_t off) {
 // stream has finished, once every block of that one has called griddep_launch (or ended).  Before it
 // touches anything that kernel or an earlier one writes or still reads, it calls griddep_wait, which
 // returns when the kernel ahead has completed and its writes are visible.  A kernel launched the
-// plain way passes through both.
+// plain way passes through both.  No pointer to what an earlier kernel writes is __restrict__ in such a
+// kernel: that promises the compiler that nothing else writes there, and its loads may then move up
+// across the wait.
 __device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Orders generic-proxy writes that are visible to this thread before its later TMA accesses.

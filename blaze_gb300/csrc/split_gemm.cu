@@ -928,10 +928,9 @@ __device__ __forceinline__ void slice_emit(const unsigned long long (&xv)[8], in
 // buffer keeps rows of 528 bytes with 16-byte chunk c of a row stored at c ^ (c >> 3), so that the
 // eight threads of a row read their chunks 4L + j from eight different bank groups.
 template <int mode, typename TX>
-__device__ __forceinline__ void slice_rows(int which, const TX* __restrict__ X, int64_t R, int64_t K, int64_t sr,
-                                           int64_t sp, const int* __restrict__ rexp, const SplitInfo* __restrict__ info,
-                                           __nv_bfloat16* __restrict__ planes, int64_t rpad, int64_t kpad, int by,
-                                           int kt) {
+__device__ __forceinline__ void slice_rows(int which, const TX* X, int64_t R, int64_t K, int64_t sr, int64_t sp,
+                                           const int* rexp, const SplitInfo* info, __nv_bfloat16* planes, int64_t rpad,
+                                           int64_t kpad, int by, int kt) {
     constexpr uint32_t ROWB = kTileRow<TX>, BUF = 32 * ROWB, V = 16 / sizeof(TX);
     __shared__ __align__(16) unsigned char tbuf[2 * BUF];
     __shared__ SliceConst tab[mode == kCrt ? MAX_MODULI : 1];
@@ -990,8 +989,8 @@ __device__ __forceinline__ void slice_rows(int which, const TX* __restrict__ X, 
 }
 
 template <int MODE, typename TX>
-__global__ void __launch_bounds__(256, 3) slice_kernel(const OperandPair op, int64_t K, const SplitInfo* __restrict__ info,
-                                                       int64_t kpad, int kt) {
+__global__ void __launch_bounds__(256, 3) slice_kernel(const OperandPair op, int64_t K,
+                                                       const SplitInfo* info, int64_t kpad, int kt) {
     const int w = blockIdx.y < op.yb0 ? 0 : 1;
     const int by = w ? int(blockIdx.y - op.yb0) : int(blockIdx.y);
     slice_rows<MODE, TX>(w, static_cast<const TX*>(op.X[w]), op.R[w], K, op.sr[w], op.sp[w], op.rexp[w], info, op.planes[w], op.rpad[w], kpad, by, kt);
@@ -1469,7 +1468,7 @@ struct CrtWords {
 // row: the plane offset of the block's row and the launch's first column, j: the thread's column from
 // there; row is the same for the whole block, so the addresses are formed once per warp.
 template <int N>
-__device__ __forceinline__ CrtWords<N> crt_load(const uint8_t* __restrict__ res, int64_t S, int64_t row, uint32_t j) {
+__device__ __forceinline__ CrtWords<N> crt_load(const uint8_t* res, int64_t S, int64_t row, uint32_t j) {
     CrtWords<N> r;
     const uint2 z = *reinterpret_cast<const uint2*>(res + 2 * row + 2u * j);
     r.w0[0] = z.x;
@@ -1482,7 +1481,7 @@ __device__ __forceinline__ CrtWords<N> crt_load(const uint8_t* __restrict__ res,
 // With k in segments: the sum of the residues b = r + 128 of column cc over the segments, reduced to
 // [0, p) and congruent to (sum of r) + 128, as the single segment's b is.
 template <int N>
-__device__ __forceinline__ uint32_t crt_seg_sum(const uint8_t* __restrict__ res, int64_t S, int max_levels, int64_t off,
+__device__ __forceinline__ uint32_t crt_seg_sum(const uint8_t* res, int64_t S, int max_levels, int64_t off,
                                                 int nseg, int t, int cc, uint32_t p, uint32_t pinv32) {
     uint32_t sum = 0;
     for (int g = 0; g < nseg; ++g) {
@@ -1569,7 +1568,7 @@ __device__ __forceinline__ double words_to_double(const uint32_t (&w)[4], int ei
 // product of the scaled integers has |value| < P / 2.125, so W / P lies at least 0.029 from a half
 // integer.  It is removed by adding the multiple of 2^(32 LB) - P, all modulo 2^(32 LB).
 template <int N>
-__device__ __forceinline__ void crt_cols(const CrtWords<N>& r, const uint8_t* __restrict__ res, int64_t S, int64_t off,
+__device__ __forceinline__ void crt_cols(const CrtWords<N>& r, const uint8_t* res, int64_t S, int64_t off,
                                          int nseg, int max_levels, int scale, int ei, const int (&fj)[4], double (&v)[4]) {
     constexpr CrtTable T = kCrtTables[N - 2];
     constexpr int NS = T.nsup, LB = T.limbs;
@@ -1714,7 +1713,7 @@ __device__ __forceinline__ void crt_rows(const CrtCombine<TC>& p, int scale, int
 constexpr int kCombineBlocks = 8;
 template <typename TC>
 __global__ void __launch_bounds__(128, kCombineBlocks) crt_combine_kernel(const CrtCombine<TC> p,
-                                                                          const SplitInfo* __restrict__ info) {
+                                                                          const SplitInfo* info) {
     griddep_wait();
     const int64_t j0 = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) * 4;
     if (j0 >= p.n) return;
@@ -1741,10 +1740,9 @@ dim3 crt_combine_grid(int64_t m, int64_t n, int num_sms) {
 }
 
 template <typename TC>
-__global__ void __launch_bounds__(128, 8) combine_kernel(const int32_t* __restrict__ levels, int nseg, int max_levels, int64_t mpad,
-                               int64_t npad, int mode, const SplitInfo* __restrict__ info,
-                               const int* __restrict__ eA, const int* __restrict__ eB, int64_t m, int64_t n,
-                               double alpha, double beta, TC* __restrict__ C, int64_t ldc) {
+__global__ void __launch_bounds__(128, 8) combine_kernel(const int32_t* levels, int nseg, int max_levels, int64_t mpad,
+                               int64_t npad, int mode, const SplitInfo* info, const int* eA, const int* eB, int64_t m,
+                               int64_t n, double alpha, double beta, TC* C, int64_t ldc) {
     griddep_wait();
     const int64_t j0 = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) * COMBINE_COLS;
     if (j0 >= n) return;
