@@ -83,7 +83,7 @@ constexpr int kDStageBytes = 8 * 2 * kDStage * int(sizeof(double));  // per 256-
 // rounds a tile does not have: one that is predicated off for the whole warp holds the FP64 pipe as
 // long as any other (4.75 ms against 3.93 before the epilogue was split as well).
 template <int U, int UMAX>
-__device__ __forceinline__ void flat_steps(const double* __restrict__ buf, int kc, int pb, const int (&ao)[UMAX],
+__device__ __forceinline__ void flat_steps(const double* buf, int kc, int pb, const int (&ao)[UMAX],
                                            const int (&bo)[UMAX], double (&acc)[UMAX]) {
 #pragma unroll 2
     for (int kk = 0; kk < kc; ++kk) {
@@ -97,7 +97,7 @@ __device__ __forceinline__ void flat_steps(const double* __restrict__ buf, int k
 // The flat tile of `rows` x `cols` outputs at (i0, j0), UMAX rounds at most.
 constexpr int UMAX = 16;
 __device__ __forceinline__ void warp_tile_flat(const DevProblem& p, int i0, int j0, int rows, int cols, int lane,
-                                               double* __restrict__ sw) {
+                                               double* sw) {
     const int outs = rows * cols, U = (outs + 31) >> 5;
     const int pb = cols | 1, bbase = rows * DPA;  // B row pitch, and where B's chunk begins
     const double* A = static_cast<const double*>(p.A) + (p.ta ? int64_t(i0) : int64_t(i0) * p.lda);
@@ -202,7 +202,7 @@ __device__ __forceinline__ int a_slot(int row, int kk) { return row * KC + ((((k
 
 // C consecutive floats from 16-byte (or, for C = 2, 8-byte) aligned shared memory, as packed pairs.
 template <int C>
-__device__ __forceinline__ void lds_pairs(const float* __restrict__ src, uint64_t (&v)[C / 2]) {
+__device__ __forceinline__ void lds_pairs(const float* src, uint64_t (&v)[C / 2]) {
     if constexpr (C == 2) {
         v[0] = *reinterpret_cast<const uint64_t*>(src);
     } else {
@@ -220,7 +220,7 @@ constexpr int kAcc = 16;  // packed accumulators a lane: 4 x 8 outputs
 
 // kc k-steps of a staged chunk.
 template <int R, int C>
-__device__ __forceinline__ void f32_steps(const float* __restrict__ As, int kc, int ly, int lx, uint64_t (&acc)[kAcc]) {
+__device__ __forceinline__ void f32_steps(const float* As, int kc, int ly, int lx, uint64_t (&acc)[kAcc]) {
     const float* bcol = As + kStageA + lx * C;
     const int kv = kc & ~3;
 #pragma unroll 1
@@ -327,7 +327,7 @@ __device__ __forceinline__ void f32_stage(const DevProblem& p, const float* __re
     }
 }
 
-__device__ __forceinline__ void warp_tile_staged(const DevProblem& p, int tm, int tn, int lane, float* __restrict__ sw) {
+__device__ __forceinline__ void warp_tile_staged(const DevProblem& p, int tm, int tn, int lane, float* sw) {
     const int ly = lane >> 2, lx = lane & 3;
     const int i0 = tm * p.tr, j0 = tn * p.tc;
     const int rows = min(p.tr, p.m - i0), cols = min(p.tc, p.n - j0);
