@@ -2,11 +2,12 @@
 //
 //   GB300_METHOD_SPLIT   Ozaki-style split-precision product that reaches FP64-level normwise
 //                        accuracy: A and B are scaled per row / per column by powers of two and
-//                        cut into BF16 "digit" slices; the slice products run on tcgen05 tensor
-//                        cores (FP32 accumulators in TMEM) in groups whose sums stay exactly
-//                        representable, so every partial product is an exact integer; the
-//                        integers are accumulated exactly (int32) and only the final
-//                        recombination, the exponent rescale and alpha/beta run in FP64.
+//                        cut into BF16 planes, residues of the scaled integers modulo 2 to 15
+//                        moduli (by default) or base-256 digits (explicit slice counts); the plane
+//                        products run on tcgen05 tensor cores (FP32 accumulators in TMEM) in groups
+//                        whose sums stay exactly representable; the group sums are reduced modulo
+//                        their modulus (digits: added in int32) exactly, and only the final
+//                        rounding, the exponent rescale and alpha/beta run in FP64.
 //   GB300_METHOD_BF16X3  hi*hi + hi*lo + lo*hi with BF16 hi/lo parts, FP32 accumulation.
 //   GB300_METHOD_BF16    one BF16 product, FP32 accumulation.
 //   GB300_METHOD_AUTO    the split form when it is predicted faster than the native kernel.
@@ -14,7 +15,7 @@
 // They replace the same CBLAS dgemm call as the native kernel (blaze/math/blas/cblas/gemm.h:
 // 156-162, reached from DMatDMatMultExpr.h:2021-2037 and siblings).
 //
-// ---- split arithmetic --------------------------------------------------------------------------
+// ---- digit arithmetic (the residue form's stands at c_mod below) --------------------------------------------------------------------------
 // Row i of op(A) is scaled by 2^-e_i with e_i = frexp exponent of max_p |A(i,p)|, so the scaled
 // entries x satisfy |x| < 1.  Digits: d_1 = rint(x*2^7), r_1 = x*2^7 - d_1, then
 // d_s = rint(r_{s-1}*2^8), r_s = r_{s-1}*2^8 - d_s (all exact in FP64; |d_s| <= 128, |r_s| <= 1/2),
@@ -34,18 +35,21 @@
 //   chosen on the device, so the whole product is stream-ordered without a host round trip.
 //
 // ---- kernel structure (tc_gemm_kernel) ---------------------------------------------------------
-// Persistent CTAs, one per SM, each owning whole 128 x 256 output tiles (and a k-segment).
-//   warp 0      TMA producer: 128x64 A-plane box + 256x64 B-plane box per item, 128B swizzle,
-//               4-stage ring of 48 KB stages.
-//   warp 1      TMEM allocator and MMA issuer: 4 x tcgen05.mma (M=128, N=256, K=16, BF16->FP32)
-//               per item; tcgen05.commit releases the smem stage and, at the end of a drain
-//               group, hands the accumulator buffer to the epilogue.  Two 256-column TMEM
-//               accumulators let the MMAs of one group overlap the drain of the previous one.
-//   warps 2-9   epilogue: tcgen05.ld of its 32 lanes x 128 columns, exact integer accumulation
-//               in registers, and at each level end a store of the int32 level sums (float
-//               modes: the FP32 tile) to the level planes in global memory.
-// A separate combine kernel forms C = alpha * 2^(e_i+f_j) * sum_L 2^(-14-8L) T_L + beta*C in FP64
-// (float modes: alpha * sum of segment partials + beta*C).  Every wait is bounded.
+// Persistent pairs of CTAs (a cluster of two, one CTA per SM), each pair owning 256 x 256 output
+// tiles (and a k-segment) of one level at a time.
+//   warp 0      TMA producer: 128x64 A-plane box + the CTA's 128x64 half of the B-plane box per item,
+//               128B swizzle, 6-stage ring of 32 KB stages.
+//   warp 1      TMEM allocator; the even CTA's issues the pair's 4 x tcgen05.mma (M=256, N=256, K=16,
+//               BF16->FP32) per item; tcgen05.commit releases the smem stage in both CTAs and, at the
+//               end of a drain group, hands the accumulator buffer to both epilogues.  Two 256-column
+//               TMEM accumulators let the MMAs of one group overlap the drain of the previous one.
+//   warps 2-9   epilogue: tcgen05.ld of its 32 lanes x 128 columns; residue form: the groups' residues
+//               summed in packed FP32, and at each level end a TMA store of them as bytes (16 bits for
+//               the modulus 257); digit form: exact int32 sums (float modes: the FP32 tile), stored to
+//               the level planes in global memory.
+// A separate kernel reconstructs C from the residue planes (crt_combine_kernel) or recombines the
+// level sums, C = alpha * 2^(e_i+f_j) * sum_L 2^(-14-8L) T_L + beta*C in FP64 (float modes: alpha *
+// sum of segment partials + beta*C).  Every wait is bounded.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -675,7 +679,7 @@ __device__ void plan_side(const RowPartial& S, int64_t k, const PlanArgs& plan) 
 
 // A block (row panel i of A, column block j of B) from the two sides: the moduli that carry
 // (2^beta_a sqrt(Q_A) + sqrt(k)/2)(2^beta_b sqrt(Q_B) + sqrt(k)/2) with the margin of
-// split_info_kernel, and the block's bound 2^(-beta_a-1) r_A + 2^(-beta_b-1) r_B +
+// plan_product, and the block's bound 2^(-beta_a-1) r_A + 2^(-beta_b-1) r_B +
 // 2^(-beta_a-beta_b-2) r_A r_B + 2^-52 relative to ||A_i|| ||B_j|| (infinite when even cap_planes
 // moduli are too few).
 __global__ void split_block_kernel(const SplitInfo* __restrict__ ia, const SplitInfo* __restrict__ ib, int64_t k,
@@ -822,9 +826,9 @@ __device__ __forceinline__ uint32_t mod_small(uint32_t x, uint32_t p, uint32_t i
 // at dst, plane stride pstride; sl = slices (digits) or moduli (CRT), bt = beta (CRT).
 // A modulus' constants as packed pairs (k_3, k_2, k_1 = symmetric residues of 2^42, 2^28, 2^14;
 // fl(1/p); -p), in shared memory: three 16-byte reads a modulus serve eight elements, and the packed
-// arithmetic takes half the instructions that bound this pass (8192^3 at 12 moduli 750 -> 725 us, 5.9 TB/s; 403 x 517 x 389
-// 20 -> 8 us with the smaller blocks of tiles_per_block; 61 % of the issue slots busy, so the planes'
-// writes bound it now).
+// arithmetic takes half the instructions that bound this pass (8192^3 at 12 moduli 750 -> 725 us, now
+// 685, 6.3 TB/s; 403 x 517 x 389 20 -> 7 us with the smaller blocks of tiles_per_block); the planes'
+// writes bound it now.
 struct __align__(16) SliceConst {
     ulonglong2 k32, k1_inv, pneg;
 };
@@ -1914,12 +1918,12 @@ SplitGeometry split_geometry(const Gemm& g, const SplitRequest& req, int num_sms
         G.max_planes = (G.mode == kExact) ? (req.slices > 0 ? std::min(req.slices, MAX_SLICES) : MAX_SLICES)
                                           : (G.mode == kBf16 ? 1 : 2);
     G.max_levels = (G.mode == kExact || G.mode == kCrt) ? G.max_planes : 1;
-    // k-segments: exactness (int32 level sums) and parallelism for few output tiles; decided from the
+    // k-segments: exactness (int32 level sums, sums of group residues) and parallelism for few output tiles; decided from the
     // device's SM count only, so a capped grid computes the same segments (and the same result)
     int64_t kseg = G.kpad;
     if (G.mode == kExact || G.mode == kCrt) {
-        // n_L * Kseg products of at most 2^14 each must stay below 2^31 (one pair per level in
-        // CRT mode)
+        // n_L * Kseg products of at most 2^14 each must stay below 2^31 (residue form, one pair per
+        // level: 128 groups' residues of at most 130, exact in FP32 by far)
         const int64_t cap = (int64_t(511) / (G.mode == kCrt ? 1 : G.max_planes)) * KSEG_UNIT;
         kseg = std::min(kseg, std::max<int64_t>(cap, KSEG_UNIT));
     }
@@ -1928,7 +1932,7 @@ SplitGeometry split_geometry(const Gemm& g, const SplitRequest& req, int num_sms
     // spill into a second, partial wave) and it multiplies the residue planes the reconstruction
     // reads; at 64 tiles on 76 pairs two segments made a 512 x 8192 x 512 product 1.6 times slower.
     // A segment keeps at least one TMEM drain group of k (1024): a unit of 256 k has about 1.3 us of
-    // products against about 3 us of epilogue (drain, modular reduction, residue store), and every
+    // products against about 3 us of epilogue (measured with its integer reductions), and every
     // extra segment adds residue planes for the reconstruction; 1024^3 split into four 256-k
     // segments took 59 us in the tensor-core kernel and 55 us in the reconstruction.
     const int tiles = G.m_tiles * G.n_tiles, pairs = std::max(1, num_sms / 2);
