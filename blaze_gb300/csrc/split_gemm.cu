@@ -1555,8 +1555,9 @@ __device__ __forceinline__ double words_to_double(const uint32_t (&w)[4], int ei
     // mantissa in bits 62..10
     unsigned long long v = ((unsigned long long)t1 << 32) | t0;
     v += 0x1ffu + ((t0 >> 10) & 1u);
-    const uint32_t rl = uint32_t(v >> 10), rh = uint32_t(int32_t(uint32_t(v >> 32)) >> 10);
-    unsigned long long m = ((unsigned long long)(rh ^ sgn) << 32) | (rl ^ sgn);
+    // the sign bits go before the shift down: a positive carry into bit 63 is a magnitude, not a sign
+    const uint32_t rl = uint32_t(v >> 10) ^ sgn, rh = (uint32_t(v >> 32) ^ sgn) >> 10;
+    unsigned long long m = ((unsigned long long)rh << 32) | rl;
     m += sgn & 1u;
     const int be = BITS - 1 - lz + ei + fj - scale + 1023;  // the leading bit is bit BITS - 1 - lz of W
     if (lz < 32 && be >= 1 && be <= 2045) {
