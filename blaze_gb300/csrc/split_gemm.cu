@@ -235,39 +235,83 @@ struct OperandPair {
     unsigned yb0;  // row blocks of A
 };
 
+// 64-bit shifts whose counts above 63 give zero.
+__device__ __forceinline__ unsigned long long shl64(unsigned long long v, int n) {
+    unsigned long long r;
+    asm("shl.b64 %0, %1, %2;" : "=l"(r) : "l"(v), "r"(n));
+    return r;
+}
+__device__ __forceinline__ unsigned long long shr64(unsigned long long v, int n) {
+    unsigned long long r;
+    asm("shr.u64 %0, %1, %2;" : "=l"(r) : "l"(v), "r"(n));
+    return r;
+}
+
+// v 2^x of a zero or normal v >= 0 for x <= 0, zero below the normal range: integer operations only (an
+// FP64 instruction of a warp holds its SM quarter's FP64 pipe for 64 clocks).
+__device__ __forceinline__ double down2(double v, int x) {
+    const int hi = __double2hiint(v);
+    return (hi >> 20) + x > 0 ? __hiloint2double(hi + x * (1 << 20), __double2loint(v)) : 0.0;
+}
+
+// A float sum (zero or normal, not negative) as a double.
+__device__ __forceinline__ double widened_sum(float v) {
+    return __longlong_as_double(static_cast<long long>(widened_bits(__float_as_uint(v))));
+}
+
 // Summary of 32 rows (or of many): Inf/NaN flag, largest exponent E of the rows with q > 0 (kNoRows
-// when none), largest q, s = sum 2^(2(e - E)) and nrm = sum 2^(2(e - E)) q.  FP32: the sums feed norms
-// and bounds, and the plan allows q 2^-10 for rounding.
+// when none), bits of the largest q (non-negative doubles order like integers), s = sum 2^(2(e - E)) and
+// nrm = sum 2^(2(e - E)) q.  A block's sums of squares are FP32; everything summed from them is FP64, with
+// the scalings by powers of two done on the exponents.
 constexpr int kNoRows = -100000;
-struct RowPartial {
+struct __align__(16) RowPartial {
     int bad, E;
-    float Q, s, nrm;
+    long long Qbits;
+    double s, nrm;
+    __device__ __forceinline__ double Q() const { return __longlong_as_double(Qbits); }
 };
+
+// The sum over the calling warp's lanes (all of them get it) of zero or normal doubles v 2^x >= 0,
+// x <= 0, in integers: the 53-bit significands, five bits up, aligned to the largest exponent, lose less
+// than 2^-58 of the largest term each, so the sum is within 2^-53 of itself before its one rounding,
+// closer than a chain of FP64 additions.  One copy of the code: a launch runs it a few times a block, from
+// a cold instruction cache.
+__device__ __noinline__ double warp_sum(double v, int x) {
+    const int f = max((__double2hiint(v) >> 20) + x, 0), F = __reduce_max_sync(0xffffffffu, f);
+    const uint32_t hi = (uint32_t(__double2hiint(v)) & 0xfffffu) | 0x100000u;
+    const unsigned long long t = f ? shr64((((unsigned long long)hi << 32) | uint32_t(__double2loint(v))) << 5, F - f) : 0ull;
+    const unsigned a = __reduce_add_sync(0xffffffffu, unsigned(t) & 0xfffffu);
+    const unsigned b = __reduce_add_sync(0xffffffffu, unsigned(t >> 20) & 0xfffffu);
+    const unsigned c = __reduce_add_sync(0xffffffffu, unsigned(t >> 40));
+    unsigned long long T = a + ((unsigned long long)b << 20) + ((unsigned long long)c << 40);  // 0 or 2^57 <= T < 2^63
+    if (T == 0ull) return 0.0;
+    const int sh = 11 - __clzll((long long)T);  // down to 53 bits, to nearest even
+    T += (1ull << (sh - 1)) - 1ull + ((T >> sh) & 1ull);
+    return __longlong_as_double((long long)((T >> sh) + ((unsigned long long)(sh + F - 6) << 52)));
+}
 
 __device__ __forceinline__ RowPartial merge(const RowPartial& a, const RowPartial& b) {
     RowPartial r;
     r.bad = a.bad | b.bad;
     r.E = max(a.E, b.E);
-    r.Q = fmaxf(a.Q, b.Q);
-    const float wa = pow2f_or0(2 * (a.E - r.E)), wb = pow2f_or0(2 * (b.E - r.E));
-    r.s = fmaf(wa, a.s, wb * b.s);
-    r.nrm = fmaf(wa, a.nrm, wb * b.nrm);
+    r.Qbits = max(a.Qbits, b.Qbits);
+    r.s = down2(a.s, 2 * (a.E - r.E)) + down2(b.s, 2 * (b.E - r.E));
+    r.nrm = down2(a.nrm, 2 * (a.E - r.E)) + down2(b.nrm, 2 * (b.E - r.E));
     return r;
 }
 
-// The merge over the calling warp's lanes (all lanes get it).
-__device__ __forceinline__ RowPartial warp_merge(RowPartial v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        RowPartial w;
-        w.bad = __shfl_xor_sync(0xffffffffu, v.bad, o);
-        w.E = __shfl_xor_sync(0xffffffffu, v.E, o);
-        w.Q = __shfl_xor_sync(0xffffffffu, v.Q, o);
-        w.s = __shfl_xor_sync(0xffffffffu, v.s, o);
-        w.nrm = __shfl_xor_sync(0xffffffffu, v.nrm, o);
-        v = merge(v, w);
-    }
-    return v;
+// The merge over the calling warp's lanes (all of them get it).
+__device__ __forceinline__ RowPartial warp_merge(const RowPartial& v) {
+    constexpr unsigned all = 0xffffffffu;
+    RowPartial r;
+    r.bad = __any_sync(all, v.bad);
+    r.E = __reduce_max_sync(all, v.E);
+    const unsigned hi = unsigned(v.Qbits >> 32), top = __reduce_max_sync(all, hi);
+    const unsigned lo = __reduce_max_sync(all, hi == top ? unsigned(v.Qbits) : 0u);
+    r.Qbits = (long long)(((unsigned long long)top << 32) | lo);
+    r.s = warp_sum(v.s, 2 * (v.E - r.E));
+    r.nrm = warp_sum(v.nrm, 2 * (v.E - r.E));
+    return r;
 }
 
 // What the last block of a statistics launch plans.
@@ -415,39 +459,57 @@ __global__ void __launch_bounds__(256, 4) stats_kernel(const StatsArgs a) {
     };
     const int64_t r = r0 + rr;
     uint32_t m = 0;
-    float s = 0.f;
-    if (g == 0) fold(m, s);
+    double s = 0.0;
+    if (g == 0) {
+        float sb;
+        fold(m, sb);
+        s = widened_sum(sb);
+    }
     if (a.chunks > 1) {
         uint2* rowpart = a.part + ((w ? a.op.R[0] : 0) + r) * a.chunks;
-        if (g == 0 && r < R) rowpart[blockIdx.x] = make_uint2(m, __float_as_uint(s));
+        if (g == 0 && r < R) rowpart[blockIdx.x] = make_uint2(m, __float_as_uint(float(s)));
         if (!last_to_arrive(a.count + blockIdx.y, unsigned(a.chunks))) return;
+        double(*const red_s)[32] = reinterpret_cast<double(*)[32]>(tbuf);  // free by now
         m = 0;
-        s = 0.f;
+        s = 0.0;
         uint32_t flag = 0;
         if (r < R)
             for (int c = g; c < a.chunks; c += 8) {  // fixed order: the sums do not depend on which block is last
                 const uint2 v = __ldcg(rowpart + c);
-                const int E = exponent(m), Ec = exponent(v.x);
-                s = Ec > E ? fmaf(s, pow2f_or0(2 * (E - Ec)), __uint_as_float(v.y))
-                           : fmaf(__uint_as_float(v.y), pow2f_or0(2 * (Ec - E)), s);
+                const double sc = widened_sum(__uint_as_float(v.y));
+                const int E = exponent(m), Ec = exponent(v.x), top = max(E, Ec);
+                s = c == g ? sc : down2(s, 2 * (E - top)) + down2(sc, 2 * (Ec - top));
                 m = max(m, v.x & ~1u);
                 flag |= v.x & 1u;
             }
         red_mx[g][rr] = m | flag;
-        red_sq[g][rr] = s;
+        red_s[g][rr] = s;
         __syncthreads();
-        if (g == 0) fold(m, s);
+        if (g == 0) {
+            m = 0;
+            flag = 0;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                m = max(m, red_mx[i][rr] & ~1u);
+                flag |= red_mx[i][rr] & 1u;
+            }
+            m |= flag;
+            const int E = exponent(m);
+            s = down2(red_s[0][rr], 2 * (exponent(red_mx[0][rr]) - E));
+#pragma unroll
+            for (int i = 1; i < 8; ++i) s += down2(red_s[i][rr], 2 * (exponent(red_mx[i][rr]) - E));
+        }
     }
     if (g == 0) {
         int e = 0;
-        float q = 0.f;
+        double q = 0.0;
         const uint32_t hi = m >> 1;
         if (r < R && m != 0u) {
             if (hi >= kInfHi) {
                 e = kNonFinite;
             } else if (hi >= (kTinyExp << 20)) {
                 e = int(hi >> 20) - 1022;
-                q = 0.25f * s;  // |x| 2^-e = f / 2
+                q = down2(s, -2);  // |x| 2^-e = f / 2
             } else {
                 // tiny or subnormal values, whose squares left the FP32 range: the row again, exactly
                 unsigned long long mb = 0;
@@ -462,43 +524,35 @@ __global__ void __launch_bounds__(256, 4) stats_kernel(const StatsArgs a) {
                     const double v = ldexp(double(X[r * sr + p * sp]), -e);
                     d = fma(v, v, d);
                 }
-                q = float(d);
+                q = d;
             }
         }
         if (r < R) a.op.rexp[w][r] = e;
-        RowPartial pr{e == kNonFinite, q > 0.f ? e : kNoRows, q, q > 0.f ? 1.f : 0.f, q};
-        pr = warp_merge(pr);
+        const long long qb = __double_as_longlong(q);
+        const RowPartial pr = warp_merge(RowPartial{e == kNonFinite, qb > 0 ? e : kNoRows, qb, qb > 0 ? 1.0 : 0.0, q});
         if (t == 0) a.group[blockIdx.y] = pr;
     }
     if (!last_to_arrive(a.count + gridDim.y, gridDim.y)) return;
-    // the plan, from every row block
-    __shared__ RowPartial side[2][8];
-    RowPartial acc[2];
-    acc[0] = acc[1] = RowPartial{0, kNoRows, 0.f, 0.f, 0.f};
+    // the plan, from every row block: warps 0-3 sum up A's, 4-7 B's
+    __shared__ RowPartial side[8];
+    const RowPartial none{0, kNoRows, 0, 0.0, 0.0};
+    RowPartial acc = none;
+    const unsigned first = (g < 4 ? 0u : a.op.yb0) + (t & 127), end = g < 4 ? a.op.yb0 : gridDim.y;
 #pragma unroll 4
-    for (unsigned i = t; i < gridDim.y; i += 256) {
-        const int* v = reinterpret_cast<const int*>(a.group + i);
-        const RowPartial pr{__ldcg(v), __ldcg(v + 1), __int_as_float(__ldcg(v + 2)), __int_as_float(__ldcg(v + 3)),
-                            __int_as_float(__ldcg(v + 4))};
-        const RowPartial none{0, kNoRows, 0.f, 0.f, 0.f};
-        acc[0] = merge(acc[0], i < a.op.yb0 ? pr : none);
-        acc[1] = merge(acc[1], i < a.op.yb0 ? none : pr);
+    for (unsigned i = first; i < end; i += 128) {
+        const uint4* v = reinterpret_cast<const uint4*>(a.group + i);
+        const uint4 lo4 = __ldcg(v), hi4 = __ldcg(v + 1);
+        const RowPartial pr{int(lo4.x), int(lo4.y), (long long)(((unsigned long long)lo4.w << 32) | lo4.z),
+                            __hiloint2double(int(hi4.y), int(hi4.x)), __hiloint2double(int(hi4.w), int(hi4.z))};
+        acc = i == first ? pr : merge(acc, pr);
     }
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        acc[i] = warp_merge(acc[i]);
-        if (rr == 0) side[i][g] = acc[i];
-    }
+    acc = warp_merge(acc);
+    if (rr == 0) side[g] = acc;
     __syncthreads();
     if (g != 0) return;
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        RowPartial v{0, kNoRows, 0.f, 0.f, 0.f};
-        if (rr < 8) v = side[i][rr];
-        acc[i] = warp_merge(v);
-    }
-    if (a.plan.kind == kPlanProduct) plan_product(acc[0], acc[1], K, a.plan);
-    else plan_side(a.op.yb0 ? acc[0] : acc[1], K, a.plan);
+    const RowPartial A = warp_merge(rr < 4 ? side[rr & 7] : none), B = warp_merge(rr >= 4 && rr < 8 ? side[rr & 7] : none);
+    if (a.plan.kind == kPlanProduct) plan_product(A, B, K, a.plan);
+    else plan_side(a.op.yb0 ? A : B, K, a.plan);
 }
 
 // The plans: norms, slice count and bound, by one warp.  Sums come relative to the largest
@@ -549,7 +603,7 @@ __device__ __forceinline__ int exponent_of(double x) { return int((__double2hiin
 
 __device__ void plan_product(const RowPartial& A, const RowPartial& B, int64_t k, const PlanArgs& plan) {
     const int lane = threadIdx.x & 31, EA = A.E, EB = B.E, bad = A.bad | B.bad;
-    const double QA = A.Q, QB = B.Q, sa = A.s, na = A.nrm, sb = B.s, nb = B.nrm;
+    const double QA = A.Q(), QB = B.Q(), sa = A.s, na = A.nrm, sb = B.s, nb = B.nrm;
     const int mode = plan.mode, fixed_slices = plan.fixed_slices, cap_planes = plan.cap_planes;
     const double target = plan.target;
     // Each FP64 function below runs once for the warp with a different argument in each lane
@@ -666,7 +720,7 @@ __device__ void plan_side(const RowPartial& S, int64_t k, const PlanArgs& plan) 
     r.nonfinite = S.bad;
     r.normA = r.normB = nrm > 0 ? __shfl_sync(0xffffffffu, scaled, 0) : 0.0;
     r.scaleA = r.scaleB = s > 0 ? __shfl_sync(0xffffffffu, scaled, 1) : 0.0;
-    r.qmaxA = r.qmaxB = S.Q;
+    r.qmaxA = r.qmaxB = S.Q();
     const double rr = nrm > 0 ? __shfl_sync(0xffffffffu, root, 2) : 0.0;
     int lo = 1;
     if (rr > 0.0 && plan.target > 0x1p-1000) lo = exponent_of(rr) - exponent_of(plan.target) - 1;
@@ -788,18 +842,6 @@ __device__ __forceinline__ void write_planes(const U_t (&V)[8], const bool (&neg
         }
         *reinterpret_cast<uint4*>(dst + a * pstride) = *reinterpret_cast<const uint4*>(d);
     }
-}
-
-// 64-bit shifts whose counts above 63 give zero.
-__device__ __forceinline__ unsigned long long shl64(unsigned long long v, int n) {
-    unsigned long long r;
-    asm("shl.b64 %0, %1, %2;" : "=l"(r) : "l"(v), "r"(n));
-    return r;
-}
-__device__ __forceinline__ unsigned long long shr64(unsigned long long v, int n) {
-    unsigned long long r;
-    asm("shr.u64 %0, %1, %2;" : "=l"(r) : "l"(v), "r"(n));
-    return r;
 }
 
 // |round(a * 2^sh)| for a finite double given by its bits (round half up); the result must fit in
