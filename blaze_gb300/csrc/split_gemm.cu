@@ -364,14 +364,15 @@ __device__ __forceinline__ bool last_to_arrive(unsigned* counter, unsigned n) {
 // beside them, now 13 and 17.
 //
 // A float's high word as a double is its magnitude shifted by 3 with the exponent rebased.  A zero or
-// subnormal float gets exponent field 896 that way, no matter next to a row's larger values: rows
-// without values above 2^-86 are read again like tiny doubles, and all-zero rows known by their OR.
+// subnormal float gets exponent field 896 that way, no matter next to a row's larger values: a block with
+// a row that has nothing above 2^-86 goes over its tiles again with the doubles' own high words, and
+// all-zero rows are known by their OR.
 template <typename TX>
 __global__ void __launch_bounds__(256, 4) stats_kernel(const StatsArgs a) {
     constexpr bool F32 = sizeof(TX) == 4;
     constexpr uint32_t ROWB = kTileRow<TX>, BUF = 32 * ROWB;  // an odd count of 16-byte chunks: no bank conflicts
     constexpr uint32_t kInfHi = F32 ? 0x47f00000u : 0x7ff00000u;
-    constexpr uint32_t kTinyExp = F32 ? 937u : 191u;
+    constexpr uint32_t kTinyExp = 191u, kTinyF32Exp = 937u;
     __shared__ __align__(16) unsigned char tbuf[2 * BUF];
     __shared__ uint32_t red_mx[8][32];
     __shared__ float red_sq[8][32];
@@ -386,63 +387,62 @@ __global__ void __launch_bounds__(256, 4) stats_kernel(const StatsArgs a) {
     const int64_t tb = int64_t(blockIdx.x) * a.kt, te = min(ntiles, tb + a.kt);
     const uint32_t s0 = smem_u32(tbuf);
     auto off = [](int r_, int p_) { return uint32_t(r_) * ROWB + uint32_t(p_) * uint32_t(sizeof(TX)); };
-    uint32_t mx = 0, lo = 0;
-    int base = 127;  // f = |x| 2^(1023 - base); values with exponent field 0 never count
-    float sq = 0.f;
+    uint32_t mx, lo;
+    float sq;
     const bool vec = rows_vec(X, sr, sp);
-    if (tb < te) tile_issue(s0, X, R, K, sr, sp, vec, r0, tb, off);
-    for (int64_t it = tb; it < te; ++it) {
-        const int b = int(it - tb) & 1;
-        if (it + 1 < te) tile_issue(s0 + uint32_t(b ^ 1) * BUF, X, R, K, sr, sp, vec, r0, it + 1, off);
-        else cp_async_commit();  // an empty group keeps the wait count uniform
-        cp_async_wait1();
-        __syncthreads();
-        uint32_t hi[8];
-        const unsigned char* row = tbuf + b * BUF + rr * ROWB + g * 8 * uint32_t(sizeof(TX));
-        if constexpr (F32) {
+    auto scan = [&](auto exact) {
+        constexpr bool EXACT = decltype(exact)::value;
+        mx = lo = 0u;
+        sq = 0.f;
+        int base = 127;  // f = |x| 2^(1023 - base); values with exponent field 0 never count
+        if (tb < te) tile_issue(s0, X, R, K, sr, sp, vec, r0, tb, off);
+        for (int64_t it = tb; it < te; ++it) {
+            const int b = int(it - tb) & 1;
+            if (it + 1 < te) tile_issue(s0 + uint32_t(b ^ 1) * BUF, X, R, K, sr, sp, vec, r0, it + 1, off);
+            else cp_async_commit();  // an empty group keeps the wait count uniform
+            cp_async_wait1();
+            __syncthreads();
+            uint32_t hi[8];
+            const unsigned char* row = tbuf + b * BUF + rr * ROWB + g * 8 * uint32_t(sizeof(TX));
+            if constexpr (F32) {
 #pragma unroll
-            for (int q = 0; q < 2; ++q) {
-                const uint4 v = *reinterpret_cast<const uint4*>(row + 16 * q);
-                const uint32_t m4[4] = {v.x & 0x7fffffffu, v.y & 0x7fffffffu, v.z & 0x7fffffffu, v.w & 0x7fffffffu};
+                for (int q = 0; q < 2; ++q) {
+                    const uint4 v = *reinterpret_cast<const uint4*>(row + 16 * q);
+                    const uint32_t m4[4] = {v.x & 0x7fffffffu, v.y & 0x7fffffffu, v.z & 0x7fffffffu, v.w & 0x7fffffffu};
 #pragma unroll
-                for (int i = 0; i < 4; ++i) hi[4 * q + i] = (m4[i] >> 3) + 0x38000000u;
-                lo |= m4[0] | m4[1];
-                lo |= m4[2] | m4[3];
-                mx = max(mx, max(max(hi[4 * q], hi[4 * q + 1]), max(hi[4 * q + 2], hi[4 * q + 3])));
+                    for (int i = 0; i < 4; ++i)
+                        hi[4 * q + i] = EXACT ? uint32_t(widened_bits(m4[i]) >> 32) : (m4[i] >> 3) + 0x38000000u;
+                    lo |= m4[0] | m4[1];
+                    lo |= m4[2] | m4[3];
+                    mx = max(mx, max(max(hi[4 * q], hi[4 * q + 1]), max(hi[4 * q + 2], hi[4 * q + 3])));
+                }
+            } else {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const uint4 v = *reinterpret_cast<const uint4*>(row + 16 * q);
+                    hi[2 * q] = v.y & 0x7fffffffu;
+                    hi[2 * q + 1] = v.w & 0x7fffffffu;
+                    lo |= v.x | v.z;
+                    mx = max(mx, max(hi[2 * q], hi[2 * q + 1]));
+                }
             }
-        } else {
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const uint4 v = *reinterpret_cast<const uint4*>(row + 16 * q);
-                hi[2 * q] = v.y & 0x7fffffffu;
-                hi[2 * q + 1] = v.w & 0x7fffffffu;
-                lo |= v.x | v.z;
-                mx = max(mx, max(hi[2 * q], hi[2 * q + 1]));
+            const int top = int(mx >> 20);
+            if (top > base) {
+                sq *= pow2f_or0(2 * (base - top));
+                base = top;
             }
-        }
-        const int top = int(mx >> 20);
-        if (top > base) {
-            sq *= pow2f_or0(2 * (base - top));
-            base = top;
-        }
-        const uint32_t cbias = uint32_t(base - 127) << 23, least = uint32_t(base - 126) << 20;
+            const uint32_t cbias = uint32_t(base - 127) << 23, least = uint32_t(base - 126) << 20;
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const float f = __uint_as_float(max(hi[q], least) * 8u - cbias);
-            sq = fmaf(f, f, sq);
+            for (int q = 0; q < 8; ++q) {
+                const float f = __uint_as_float(max(hi[q], least) * 8u - cbias);
+                sq = fmaf(f, f, sq);
+            }
+            __syncthreads();
         }
-        __syncthreads();
-    }
+    };
     // a row's largest high word with the low words' flag in bit 0, and its sum of squares relative to
     // the exponent of that high word (at least 127)
     auto exponent = [](uint32_t m) { return max(127, int(m >> 21)); };
-    if (F32 && lo == 0u) {
-        mx = 0u;
-        sq = 0.f;
-    }
-    red_mx[g][rr] = (mx << 1) | (lo != 0u ? 1u : 0u);
-    red_sq[g][rr] = sq;
-    __syncthreads();
     auto fold = [&](uint32_t& m, float& s) {  // the eight groups' values of row rr
         m = 0;
         uint32_t flag = 0;
@@ -460,11 +460,24 @@ __global__ void __launch_bounds__(256, 4) stats_kernel(const StatsArgs a) {
     const int64_t r = r0 + rr;
     uint32_t m = 0;
     double s = 0.0;
-    if (g == 0) {
-        float sb;
-        fold(m, sb);
-        s = widened_sum(sb);
-    }
+    auto block_rows = [&](auto exact) {  // m and s of the block's tiles
+        scan(exact);
+        if (F32 && lo == 0u) {
+            mx = 0u;
+            sq = 0.f;
+        }
+        red_mx[g][rr] = (mx << 1) | (lo != 0u ? 1u : 0u);
+        red_sq[g][rr] = sq;
+        __syncthreads();
+        if (g == 0) {
+            float sb;
+            fold(m, sb);
+            s = widened_sum(sb);
+        }
+    };
+    block_rows(std::false_type{});
+    if constexpr (F32)
+        if (__syncthreads_or(m != 0u && m < (kTinyF32Exp << 21))) block_rows(std::true_type{});
     if (a.chunks > 1) {
         uint2* rowpart = a.part + ((w ? a.op.R[0] : 0) + r) * a.chunks;
         if (g == 0 && r < R) rowpart[blockIdx.x] = make_uint2(m, __float_as_uint(float(s)));
