@@ -11,6 +11,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdlib>
 #include <cstring>
 #include <string>
@@ -25,7 +26,7 @@
 namespace gb {
 namespace {
 
-int g_default_method = -1;
+std::atomic<int> g_default_method{-1};
 
 int default_method() {
     if (g_default_method < 0) {

@@ -104,11 +104,11 @@ int finish(cudaStream_t st, std::string* err) {
 
 // One real product C = alpha op(A) op(B) + beta C of device operands in the logical row-major form:
 // the default method for double (FP64-accurate split precision, or the native kernel for small
-// products and when native is the default), the native kernel for float.
+// products and when native is the default), the native kernel for float.  `method` is the default
+// method, read once for a call: another thread may change it meanwhile.
 template <typename T>
-int real_product(const Gemm& g, const LaunchCtl& ctl, cudaStream_t st, std::string* err) {
+int real_product(const Gemm& g, int method, const LaunchCtl& ctl, cudaStream_t st, std::string* err) {
     Runtime& r = runtime();
-    const int method = library_default_method();
     if (sizeof(T) == 8 && method != GB300_METHOD_NATIVE) {
         SplitRequest req;
         req.method = method;
@@ -142,14 +142,13 @@ int real_product(const Gemm& g, const LaunchCtl& ctl, cudaStream_t st, std::stri
     return e == cudaSuccess ? GB300_OK : GB300_ERR_CUDA;
 }
 
-// Whether a product M x N x K reads its operands before it writes its result, so that the result may
-// take an operand's place: the tensor-core forms slice both operands first, and a complex product
-// goes through planes.  The native kernel reads as it writes.
+// Whether a product M x N x K by `method` reads its operands before it writes its result, so that the
+// result may take an operand's place: the tensor-core forms slice both operands first, and a complex
+// product goes through planes.  The native kernel reads as it writes.
 template <typename T, bool CPLX>
-bool reads_before_writing(int64_t M, int64_t N, int64_t K) {
+bool reads_before_writing(int64_t M, int64_t N, int64_t K, int method) {
     if (CPLX) return true;
     if (sizeof(T) != 8) return false;
-    const int method = library_default_method();
     Gemm g;
     g.m = M; g.n = N; g.k = K;
     return method != GB300_METHOD_NATIVE && !(method == GB300_METHOD_AUTO && split_auto_uses_native(g));
@@ -362,7 +361,7 @@ int complex_product(int64_t M, int64_t N, int64_t k, bool ta, bool tb, bool ca, 
         g.m = 2 * M; g.n = 2 * N; g.k = k; g.ta = ta; g.tb = tb;
         g.A = A2; g.lda = la2; g.B = B2; g.ldb = lb2; g.C = P; g.ldc = 2 * N;
         g.alpha = 1.0; g.beta = 0.0;
-        const int st = real_product<T>(g, ctl, s, err);
+        const int st = real_product<T>(g, library_default_method(), ctl, s, err);
         if (st != GB300_OK) return st;
     } else {
         cudaMemsetAsync(P, 0, size_t(4) * size_t(M) * size_t(N) * sizeof(T), s);
@@ -506,7 +505,7 @@ int trmm_entry(int order, int side, int uplo, int transA, int diag, int64_t m, i
             g.A = dB; g.lda = ldb; g.B = tri; g.ldb = ka;
         }
     }
-    if ((st = real_product<T>(g, ctl, s, &err)) != GB300_OK) return fail(st, err);
+    if ((st = real_product<T>(g, library_default_method(), ctl, s, &err)) != GB300_OK) return fail(st, err);
     // the product back into B (its pitch)
     cudaError_t e = cudaMemcpy2DAsync(bdev ? static_cast<void*>(B) : static_cast<void*>(dB), size_t(ldb) * sizeof(T), tmp,
                                       size_t(sbc) * sizeof(T), size_t(sbc) * sizeof(T), size_t(sbr),
@@ -679,9 +678,11 @@ int dot_entry(int64_t n, const T* x, int64_t incx, const T* y, int64_t incy, T* 
 // ---- trsm --------------------------------------------------------------------------------------
 namespace {
 // A triangular system in row-major storage: op(SA) X = SB (left) or X op(SA) = SB (right), X
-// overwriting SB (sbr x sbc, pitch ldb); SA ka x ka (pitch lda), `lower` its stored triangle.
+// overwriting SB (sbr x sbc, pitch ldb); SA ka x ka (pitch lda), `lower` its stored triangle; `method`
+// runs its real products.
 struct SolveForm {
     bool left = true, lower = true, trans = false, conj = false, unit = false;
+    int method = GB300_METHOD_AUTO;
 };
 
 // Recursive blocked solve.  [lo, hi) is a range of op(SA)'s rows and columns whose right-hand sides
@@ -709,7 +710,7 @@ int solve_range(const SolveForm& f, int64_t lo, int64_t hi, int64_t sbr, int64_t
         g.A = X; g.lda = lx; g.B = Y; g.ldb = ly; g.C = C; g.ldc = ldc;
         g.alpha = update ? -1.0 : 1.0;
         g.beta = update ? 1.0 : 0.0;
-        return real_product<T>(g, ctl, s, err);
+        return real_product<T>(g, f.method, ctl, s, err);
     };
     // the block of op(SA) at rows i0.., columns j0.. as a product operand (stored transposed when
     // op transposes)
@@ -720,9 +721,9 @@ int solve_range(const SolveForm& f, int64_t lo, int64_t hi, int64_t sbr, int64_t
         const int64_t nk = hi - lo;
         const T* Ib = inv + (lo / nb) * int64_t(nb) * nb * w;
         // straight into the right-hand sides where the product has read them by then, else through tmp
-        if (f.left && reads_before_writing<T, CPLX>(nk, sbc, nk))
+        if (f.left && reads_before_writing<T, CPLX>(nk, sbc, nk, f.method))
             return product(nk, sbc, nk, false, false, false, false, Ib, nb, rows_of(lo), ldb, false, rows_of(lo), ldb);
-        if (!f.left && reads_before_writing<T, CPLX>(sbr, nk, nk))
+        if (!f.left && reads_before_writing<T, CPLX>(sbr, nk, nk, f.method))
             return product(sbr, nk, nk, false, false, false, false, cols_of(lo), ldb, Ib, nb, false, cols_of(lo), ldb);
         int st;
         cudaError_t e;
@@ -817,6 +818,7 @@ int trsm_entry(int order, int side, int uplo, int transA, int diag, int64_t m, i
     f.trans = transA != CblasNoTrans;
     f.conj = CPLX && transA == CblasConjTrans;
     f.unit = diag == CblasUnit;
+    f.method = library_default_method();
     const bool bdev = in_place(B, elem);
     T* dB = static_cast<T*>(stage(B, sbr, sbc, ldb, elem, kAuxB, bdev, s, &err));
     if (!dB) return fail(GB300_ERR_NO_MEMORY, err);
