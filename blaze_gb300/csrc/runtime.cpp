@@ -160,19 +160,24 @@ int ensure_init(std::string* err) {
 void status_begin(cudaStream_t s, bool synchronous) {
     Runtime& r = runtime();
     if (!synchronous) r.async_seen = true;
-    if (r.async_seen || !r.status_clean) {
-        *static_cast<volatile int*>(r.h_status) = 0;
-        cudaMemsetAsync(r.d_status, 0, sizeof(int), s);
-    }
-    r.status_clean = false;
+    // a call that returned before status_end may have left kernels queued: like an asynchronous one
+    r.status_ordered = r.async_seen || r.status_open;
+    if (r.status_ordered || !r.status_clean) cudaMemsetAsync(r.d_status, 0, sizeof(int), s);
+    if (!r.status_ordered) *static_cast<volatile int*>(r.h_status) = 0;
+    r.status_open = true;
 }
 
 int status_end() {
     Runtime& r = runtime();
     int status = 0;
-    if (r.async_seen) cudaMemcpy(&status, r.d_status, sizeof(int), cudaMemcpyDeviceToHost);
-    else status = *static_cast<volatile int*>(r.h_status);
+    if (r.status_ordered) {
+        cudaMemcpy(&status, r.d_status, sizeof(int), cudaMemcpyDeviceToHost);
+        *static_cast<volatile int*>(r.h_status) = 0;
+    } else {
+        status = *static_cast<volatile int*>(r.h_status);
+    }
     r.status_clean = status == 0;
+    r.status_open = false;
     return status;
 }
 

@@ -56,7 +56,9 @@ struct Runtime {
     cudaStream_t stream = nullptr;
     int* d_status = nullptr;       // device status word of the default context
     int* h_status = nullptr;       // page-locked word that a failing wait sets too (record_status)
-    bool status_clean = true;      // both words are known to be zero
+    bool status_clean = true;      // both words were zero when the last call ended
+    bool status_open = false;      // a call began and has not ended: its kernels may still be queued
+    bool status_ordered = false;   // the present call's word is cleared and read in stream order
     bool async_seen = false;       // an asynchronous call was made: work may be running between calls
     Workspace ws;                  // default context (stream = `stream`)
     Workspace aux;                 // operands and intermediates of ?gemv, complex ?gemm, ?trmm
@@ -93,8 +95,8 @@ void* pool_get(int s, size_t bytes, std::string* err);
 // the stream has been waited for.  While every call was synchronous, a call that succeeded leaves
 // both words zero and the host reads its own copy, so neither costs the stream anything (clearing
 // and copying back took about 15 us of every call, more than a small product's kernel).  After the
-// first asynchronous call the word is cleared on the stream and copied back in each call: a kernel
-// of an earlier call may still write it.
+// process's first asynchronous call, and in the call after one that returned early, the word is
+// cleared on the stream and copied back: a kernel of an earlier call may still write it.
 void status_begin(cudaStream_t s, bool synchronous);
 int status_end();
 
