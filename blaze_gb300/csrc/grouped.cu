@@ -461,10 +461,11 @@ double f32_tile_cost(int s, int rows, int cols, int k) {
 struct Parts {
     int count, size;  // parts of `size`, the last one the rest
 };
-Parts equal_parts(int x, int limit) {
-    const int c = (x + limit - 1) / limit;
-    const int size = (x + c - 1) / c;
-    return {(x + size - 1) / size, size};
+Parts equal_parts(int64_t x, int limit) {
+    if (x <= 0) return {0, 0};
+    const int64_t c = (x + limit - 1) / limit;
+    const int64_t size = (x + c - 1) / c;
+    return {int((x + size - 1) / size), int(size)};
 }
 double padded_outputs(int m, int n, int s, bool flat) {
     const int tr = shape_rows(s), tc = shape_cols(s);
@@ -612,7 +613,7 @@ int build_tables(const gb300_gemm_problem* probs, int64_t count, int force_shape
             d.tr = equal_parts(d.m, d.tr).size;
             d.tc = equal_parts(d.n, d.tc).size;
         }
-        const int mt = (d.m + d.tr - 1) / d.tr, nt = (d.n + d.tc - 1) / d.tc;
+        const int mt = int((int64_t(d.m) + d.tr - 1) / d.tr), nt = int((int64_t(d.n) + d.tc - 1) / d.tc);
         const int pid = int(hp.size());
         hp.push_back(d);
         for (int a = 0; a < mt; ++a)
