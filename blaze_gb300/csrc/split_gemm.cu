@@ -1770,8 +1770,8 @@ __device__ __forceinline__ void crt_rows(const CrtCombine<TC>& p, int scale, int
 // busy; 118 MB read and 134 MB written would take 38 us of the 63 at 32768 x 256).  Byte planes, super
 // residues left unreduced and a straight-line conversion to double against 16-bit planes, a reduction of
 // every super residue and a branching conversion: 8.4 M outputs at 13 moduli 90 -> 63 us, 33.5 M at 12
-// moduli 285 -> 184.  Eight blocks an SM (64 registers) measured like six and 4 % faster than five, and
-// let a block run beside a tensor-core CTA; fetching the next row's residues ahead cost the registers of
+// moduli 285 -> 184.  Eight blocks an SM (64 registers) measured like six and 4 % faster than
+// five; fetching the next row's residues ahead cost the registers of
 // it (66 us), two columns at a time instead of four took 40 % more instructions.
 constexpr int kCombineBlocks = 8;
 template <typename TC>
@@ -2117,9 +2117,11 @@ size_t device_product_footprint(const Gemm& g, const SplitRequest& req) {
 bool split_auto_uses_native(const Gemm& g) { return auto_uses_native(g); }
 
 // A residue product with at least as many pair tiles as SMs runs its tensor-core work as two
-// launches over the two halves of C's column tiles, and the first half's reconstruction runs on a
-// second stream while the tensor cores work on the second half: a reconstruction block (128
-// threads, no shared memory) fits on an SM beside the tensor-core kernel's one CTA.  The second
+// launches over the two halves of C's column tiles, and the first half's reconstruction waits on a
+// second stream for the first of them.  No reconstruction block fits beside a tensor-core CTA (a quarter
+// of an SM that holds three of its warps at 168 registers has 256 left), so what this hides is the
+// tail: SMs that have no tensor-core unit left start on the first half at once.  65536 x 256 x 256: 403 us
+// in one part, 394 in two; 8192^3 9.11 and 8.81 ms (two runs of one side differ by 2 %).  The second
 // stream belongs to the pair (calling host thread, caller's stream) and has the caller's stream
 // priority, so concurrent callers (user threads, or the server's slots, launched from its one
 // scheduler thread on their own streams) never queue behind one another's reconstructions; the
@@ -2312,12 +2314,12 @@ int tensor_product(const Gemm& g, const SplitRequest& req, const LaunchCtl& ctl,
         KernelTimer timer("tc_gemm", st);
         launch_dependent(kern, dim3(unsigned(grid)), dim3(THREADS), kTcSmem, st, tA, tB, tC0, tC, q);
     };
-    // reconstruction of C's columns [c0, c0 + nc) on stream s
-    auto launch_crt_combine = [&](int64_t c0, int64_t nc, cudaStream_t s) {
+    // reconstruction of C's columns [c0, c0 + nc) on stream s, `dependent` on the launch ahead of it there
+    auto launch_crt_combine = [&](int64_t c0, int64_t nc, cudaStream_t s, bool dependent) {
         const CrtCombine<T> q{reinterpret_cast<const uint8_t*>(lv), mpad, npad, nseg, max_levels, 0, c0, m, nc, eA, eB,
                               g.alpha, g.beta, static_cast<T*>(g.C), g.ldc, false};
-        if (s == st) launch_dependent(crt_combine_kernel<T>, crt_combine_grid(m, nc, r.num_sms), dim3(128), 0, s, q, info);
-        else crt_combine_kernel<T><<<crt_combine_grid(m, nc, r.num_sms), 128, 0, s>>>(q, info);  // behind an event
+        if (dependent) launch_dependent(crt_combine_kernel<T>, crt_combine_grid(m, nc, r.num_sms), dim3(128), 0, s, q, info);
+        else crt_combine_kernel<T><<<crt_combine_grid(m, nc, r.num_sms), 128, 0, s>>>(q, info);
     };
     const bool in_parts = mode == kCrt && n_tiles >= 2 && m_tiles * n_tiles >= sms && req.max_sms <= 0;
     if (in_parts) {
@@ -2329,16 +2331,19 @@ int tensor_product(const Gemm& g, const SplitRequest& req, const LaunchCtl& ctl,
         cudaEventRecord(pe.tc0, st);
         launch_tc(nt0, n_tiles - nt0);
         cudaStreamWaitEvent(pe.aux, pe.tc0, 0);
-        launch_crt_combine(0, c0, pe.aux);
+        launch_crt_combine(0, c0, pe.aux, false);
         cudaEventRecord(pe.done0, pe.aux);
-        launch_crt_combine(c0, n - c0, st);
+        // not dependent: its blocks would be in line from the second tensor-core launch's start and take the
+        // SMs before the first part's (which then ended 50 us after it at 65536 x 256 x 256: 255 us from the
+        // first launch to the end of both, 246 this way)
+        launch_crt_combine(c0, n - c0, st, false);
         cudaStreamWaitEvent(st, pe.done0, 0);
         part_events_put(pe);
         count_launches(2);
     } else {
         launch_tc(0, n_tiles);
         if (mode == kCrt) {
-            launch_crt_combine(0, n, st);
+            launch_crt_combine(0, n, st, true);
         } else {
             const int64_t colgroups = (n + COMBINE_COLS - 1) / COMBINE_COLS;
             dim3 cgrid(unsigned((colgroups + 127) / 128), unsigned(std::min<int64_t>(m, 65535)));
