@@ -414,6 +414,7 @@ grouped_kernel(const DevProblem* __restrict__ probs, const DevTile* __restrict__
 }
 
 // ---- tuning table ------------------------------------------------------------------------------
+constexpr int kTuneKernels = 2;  // version of the kernels and of padded_outputs that costs refer to
 // Size classes: m and n bucketed by powers of two (<=8, <=16, <=32, <=64, <=128, >128), k by
 // (<=16, <=64, >64).  Entry = warp-tile shape index.
 constexpr int kMB = 6, kKB = 3;
@@ -454,8 +455,8 @@ double f32_tile_cost(int s, int rows, int cols, int k) {
 // FP32: the one with the fewest instructions (f32_tile_cost), since they bound its tiles (10,000
 // products: 369 us with the least padded work, 323 with this, which also holds the ticket and
 // description look-ahead of grouped_kernel).
-// tile_w < 0: the cost is the padded area plus 64 a tile (k left out); tile_w >= 0: the padded
-// multiply-adds (area x k) plus tile_w multiply-adds' worth of overhead a tile.
+// tile_w < 0, the default: FP64 the padded outputs plus 64 a tile (k left out), FP32 f32_tile_cost (with
+// k); tile_w >= 0: the padded multiply-adds (outputs x k) plus tile_w multiply-adds' worth a tile.
 // FP64 (flat): a product's tiles are equal parts of at most the shape's size, each a whole number of 32
 // outputs (warp_tile_flat).
 struct Parts {
@@ -1100,8 +1101,11 @@ int gb300_grouped_autotune(int elem_bytes, int effort) {
 
 // Tuning files: "gb300-grouped-tune v1" then one line per class, `dtype m-class n-class k-class
 // shape`; an autotuned table is saved as "gb300-grouped-tune v2", each line followed by the measured
-// ns per padded multiply-add of every shape (0: not measured).  Loading v1 makes plans use the
-// class shapes, loading v2 the measured costs.
+// ns per padded multiply-add of every shape (0: not measured), after a line "mode <double> <float>
+// <weight> <weight> kernels <n>".  Loading v1 makes plans use the class shapes, loading v2 the measured
+// costs, or what its mode line says.  Costs and weights belong to the kernels that they were measured on
+// (what a padded multiply-add is has changed with them): a mode line of other kernels loads the class
+// shapes and leaves the default choice in place.
 int gb300_grouped_tuning_save(const char* path) {
     std::lock_guard<std::mutex> lock(gb::g_tune_mu);
     gb::tune_defaults();
@@ -1117,7 +1121,7 @@ int gb300_grouped_tuning_save(const char* path) {
     f << (costs ? "gb300-grouped-tune v2\n" : "gb300-grouped-tune v1\n");
     if (costs)
         f << "mode " << gb::g_tune.mode[0] << ' ' << gb::g_tune.mode[1] << ' ' << gb::g_tune.tile_w[0] << ' '
-          << gb::g_tune.tile_w[1] << '\n';
+          << gb::g_tune.tile_w[1] << " kernels " << gb::kTuneKernels << '\n';
     for (int d = 0; d < 2; ++d)
         for (int a = 0; a < gb::kMB; ++a)
             for (int b = 0; b < gb::kMB; ++b)
@@ -1157,9 +1161,17 @@ int gb300_grouped_tuning_load(const char* path) {
                 return GB300_ERR_INVALID_ARG;
             }
             double w0 = -1.0, w1 = -1.0;
-            if (ms >> w0 >> w1) {  // the model's per-tile weights (absent in older v2 files)
-                t.tile_w[0] = w0;
+            std::string tag;
+            int kernels = 0;
+            ms >> w0 >> w1 >> tag >> kernels;
+            if (ms && tag == "kernels" && kernels == gb::kTuneKernels) {
+                t.tile_w[0] = w0;  // the model's per-tile weights
                 t.tile_w[1] = w1;
+            } else {
+                for (int d = 0; d < 2; ++d) {
+                    if (modes[d] == gb::kPickCost) modes[d] = gb::kPickModel;
+                    t.tile_w[d] = -1.0;
+                }
             }
             continue;
         }
