@@ -20,7 +20,9 @@ LIB = os.path.join(HERE, "libgb300blas.so")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden",
+# (--no-compress: past some size nvcc compresses the device code, line table included, and the first call of a
+# process that needs it waits 10 ms for the unpacking)
+COMMON = ["-O3", "-std=c++17", "-lineinfo", "--no-compress", "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden",
           "-Xcompiler", "-Wall", "-I", INCLUDE, "-I", CSRC]
 
 # (source, object, extra flags)
