@@ -347,6 +347,79 @@ __device__ __forceinline__ bool last_to_arrive(unsigned* counter, unsigned n) {
     return last != 0u;
 }
 
+// One thread's part of a statistics block: the largest high word `mx` and the OR of the low words (float:
+// of the magnitudes) `lo` of row rr, eight k of every tile of [tb, te), and their sum of squares in FP32
+// relative to the exponent of mx.  EXACT (float): high words of the widened values instead of the shifted
+// ones.
+struct ThreadStats {
+    uint32_t mx, lo;
+    float sq;
+};
+template <typename TX, bool EXACT>
+__device__ __forceinline__ ThreadStats scan_tiles(unsigned char* tbuf, const TX* __restrict__ X, int64_t R, int64_t K, int64_t sr,
+                                                  int64_t sp, int64_t r0, int64_t tb, int64_t te) {
+    constexpr bool F32 = sizeof(TX) == 4;
+    constexpr uint32_t ROWB = kTileRow<TX>, BUF = 32 * ROWB;
+    const int rr = threadIdx.x & 31, g = threadIdx.x >> 5;
+    const uint32_t s0 = smem_u32(tbuf);
+    const bool vec = rows_vec(X, sr, sp);
+    auto off = [](int r_, int p_) { return uint32_t(r_) * ROWB + uint32_t(p_) * uint32_t(sizeof(TX)); };
+    uint32_t mx = 0, lo = 0;
+    float sq = 0.f;
+    int base = 127;  // f = |x| 2^(1023 - base); values with exponent field 0 never count
+    if (tb < te) tile_issue(s0, X, R, K, sr, sp, vec, r0, tb, off);
+    for (int64_t it = tb; it < te; ++it) {
+        const int b = int(it - tb) & 1;
+        if (it + 1 < te) tile_issue(s0 + uint32_t(b ^ 1) * BUF, X, R, K, sr, sp, vec, r0, it + 1, off);
+        else cp_async_commit();  // an empty group keeps the wait count uniform
+        cp_async_wait1();
+        __syncthreads();
+        uint32_t hi[8];
+        const unsigned char* row = tbuf + b * BUF + rr * ROWB + g * 8 * uint32_t(sizeof(TX));
+        if constexpr (F32) {
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const uint4 v = *reinterpret_cast<const uint4*>(row + 16 * q);
+                const uint32_t m4[4] = {v.x & 0x7fffffffu, v.y & 0x7fffffffu, v.z & 0x7fffffffu, v.w & 0x7fffffffu};
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    hi[4 * q + i] = EXACT ? uint32_t(widened_bits(m4[i]) >> 32) : (m4[i] >> 3) + 0x38000000u;
+                lo |= m4[0] | m4[1];
+                lo |= m4[2] | m4[3];
+                mx = max(mx, max(max(hi[4 * q], hi[4 * q + 1]), max(hi[4 * q + 2], hi[4 * q + 3])));
+            }
+        } else {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const uint4 v = *reinterpret_cast<const uint4*>(row + 16 * q);
+                hi[2 * q] = v.y & 0x7fffffffu;
+                hi[2 * q + 1] = v.w & 0x7fffffffu;
+                lo |= v.x | v.z;
+                mx = max(mx, max(hi[2 * q], hi[2 * q + 1]));
+            }
+        }
+        const int top = int(mx >> 20);
+        if (top > base) {
+            sq *= pow2f_or0(2 * (base - top));
+            base = top;
+        }
+        const uint32_t cbias = uint32_t(base - 127) << 23, least = uint32_t(base - 126) << 20;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const float f = __uint_as_float(max(hi[q], least) * 8u - cbias);
+            sq = fmaf(f, f, sq);
+        }
+        __syncthreads();
+    }
+    return {mx, lo, sq};
+}
+// Out of line: it is rarely run, and its registers and code stay out of the kernel's way.
+template <typename TX>
+__device__ __noinline__ ThreadStats scan_tiles_exact(unsigned char* tbuf, const TX* X, int64_t R, int64_t K, int64_t sr,
+                                                     int64_t sp, int64_t r0, int64_t tb, int64_t te) {
+    return scan_tiles<TX, true>(tbuf, X, R, K, sr, sp, r0, tb, te);
+}
+
 // Thread (rr = t % 32, g = t / 32) keeps, for row rr and the
 // eight k of group g in every tile, the largest high word of |x|, the OR of the low words and the
 // sum of squares in FP32 relative to its running largest exponent `base`: f = |x| 2^(1023 - base)
@@ -385,61 +458,6 @@ __global__ void __launch_bounds__(256, 4) stats_kernel(const StatsArgs a) {
     const int64_t r0 = int64_t(by) * 32;
     const int64_t ntiles = (K + 63) / 64;
     const int64_t tb = int64_t(blockIdx.x) * a.kt, te = min(ntiles, tb + a.kt);
-    const uint32_t s0 = smem_u32(tbuf);
-    auto off = [](int r_, int p_) { return uint32_t(r_) * ROWB + uint32_t(p_) * uint32_t(sizeof(TX)); };
-    uint32_t mx, lo;
-    float sq;
-    const bool vec = rows_vec(X, sr, sp);
-    auto scan = [&](auto exact) {
-        constexpr bool EXACT = decltype(exact)::value;
-        mx = lo = 0u;
-        sq = 0.f;
-        int base = 127;  // f = |x| 2^(1023 - base); values with exponent field 0 never count
-        if (tb < te) tile_issue(s0, X, R, K, sr, sp, vec, r0, tb, off);
-        for (int64_t it = tb; it < te; ++it) {
-            const int b = int(it - tb) & 1;
-            if (it + 1 < te) tile_issue(s0 + uint32_t(b ^ 1) * BUF, X, R, K, sr, sp, vec, r0, it + 1, off);
-            else cp_async_commit();  // an empty group keeps the wait count uniform
-            cp_async_wait1();
-            __syncthreads();
-            uint32_t hi[8];
-            const unsigned char* row = tbuf + b * BUF + rr * ROWB + g * 8 * uint32_t(sizeof(TX));
-            if constexpr (F32) {
-#pragma unroll
-                for (int q = 0; q < 2; ++q) {
-                    const uint4 v = *reinterpret_cast<const uint4*>(row + 16 * q);
-                    const uint32_t m4[4] = {v.x & 0x7fffffffu, v.y & 0x7fffffffu, v.z & 0x7fffffffu, v.w & 0x7fffffffu};
-#pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        hi[4 * q + i] = EXACT ? uint32_t(widened_bits(m4[i]) >> 32) : (m4[i] >> 3) + 0x38000000u;
-                    lo |= m4[0] | m4[1];
-                    lo |= m4[2] | m4[3];
-                    mx = max(mx, max(max(hi[4 * q], hi[4 * q + 1]), max(hi[4 * q + 2], hi[4 * q + 3])));
-                }
-            } else {
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const uint4 v = *reinterpret_cast<const uint4*>(row + 16 * q);
-                    hi[2 * q] = v.y & 0x7fffffffu;
-                    hi[2 * q + 1] = v.w & 0x7fffffffu;
-                    lo |= v.x | v.z;
-                    mx = max(mx, max(hi[2 * q], hi[2 * q + 1]));
-                }
-            }
-            const int top = int(mx >> 20);
-            if (top > base) {
-                sq *= pow2f_or0(2 * (base - top));
-                base = top;
-            }
-            const uint32_t cbias = uint32_t(base - 127) << 23, least = uint32_t(base - 126) << 20;
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                const float f = __uint_as_float(max(hi[q], least) * 8u - cbias);
-                sq = fmaf(f, f, sq);
-            }
-            __syncthreads();
-        }
-    };
     // a row's largest high word with the low words' flag in bit 0, and its sum of squares relative to
     // the exponent of that high word (at least 127)
     auto exponent = [](uint32_t m) { return max(127, int(m >> 21)); };
@@ -460,14 +478,13 @@ __global__ void __launch_bounds__(256, 4) stats_kernel(const StatsArgs a) {
     const int64_t r = r0 + rr;
     uint32_t m = 0;
     double s = 0.0;
-    auto block_rows = [&](auto exact) {  // m and s of the block's tiles
-        scan(exact);
-        if (F32 && lo == 0u) {
-            mx = 0u;
-            sq = 0.f;
+    auto block_rows = [&](ThreadStats v) {  // m and s of the block's tiles
+        if (F32 && v.lo == 0u) {
+            v.mx = 0u;
+            v.sq = 0.f;
         }
-        red_mx[g][rr] = (mx << 1) | (lo != 0u ? 1u : 0u);
-        red_sq[g][rr] = sq;
+        red_mx[g][rr] = (v.mx << 1) | (v.lo != 0u ? 1u : 0u);
+        red_sq[g][rr] = v.sq;
         __syncthreads();
         if (g == 0) {
             float sb;
@@ -475,9 +492,10 @@ __global__ void __launch_bounds__(256, 4) stats_kernel(const StatsArgs a) {
             s = widened_sum(sb);
         }
     };
-    block_rows(std::false_type{});
+    block_rows(scan_tiles<TX, false>(tbuf, X, R, K, sr, sp, r0, tb, te));
     if constexpr (F32)
-        if (__syncthreads_or(m != 0u && m < (kTinyF32Exp << 21))) block_rows(std::true_type{});
+        if (__syncthreads_or(m != 0u && m < (kTinyF32Exp << 21)))
+            block_rows(scan_tiles_exact<TX>(tbuf, X, R, K, sr, sp, r0, tb, te));
     if (a.chunks > 1) {
         uint2* rowpart = a.part + ((w ? a.op.R[0] : 0) + r) * a.chunks;
         if (g == 0 && r < R) rowpart[blockIdx.x] = make_uint2(m, __float_as_uint(float(s)));
