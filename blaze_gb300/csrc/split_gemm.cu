@@ -15,7 +15,8 @@
 // They replace the same CBLAS dgemm call as the native kernel (blaze/math/blas/cblas/gemm.h:
 // 156-162, reached from DMatDMatMultExpr.h:2021-2037 and siblings).
 //
-// ---- digit arithmetic (the residue form's stands at c_mod below) --------------------------------------------------------------------------
+// ---- digit arithmetic --------------------------------------------------------------------------
+// (The residue form's stands at c_mod below.)
 // Row i of op(A) is scaled by 2^-e_i with e_i = frexp exponent of max_p |A(i,p)|, so the scaled
 // entries x satisfy |x| < 1.  Digits: d_1 = rint(x*2^7), r_1 = x*2^7 - d_1, then
 // d_s = rint(r_{s-1}*2^8), r_s = r_{s-1}*2^8 - d_s (all exact in FP64; |d_s| <= 128, |r_s| <= 1/2),
@@ -347,10 +348,21 @@ __device__ __forceinline__ bool last_to_arrive(unsigned* counter, unsigned n) {
     return last != 0u;
 }
 
-// One thread's part of a statistics block: the largest high word `mx` and the OR of the low words (float:
-// of the magnitudes) `lo` of row rr, eight k of every tile of [tb, te), and their sum of squares in FP32
-// relative to the exponent of mx.  EXACT (float): high words of the widened values instead of the shifted
-// ones.
+// One thread's part of a statistics block: over row rr = t % 32 and the eight k of group g = t / 32 in
+// every tile of [tb, te), the largest high word of |x| (mx), the OR of the low words (float: of the
+// magnitudes; lo) and the sum of squares in FP32 relative to the exponent of mx (sq).
+//
+// The sum runs relative to the largest exponent so far, `base`: f = |x| 2^(1023 - base) is the high word
+// times 8 (exponent and 20 mantissa bits moved into FP32 position) minus (base - 127) 2^23, one integer
+// multiply-add, valid for exponents above base - 127.  High words below that are raised to its lowest
+// value, whose square is zero in FP32.  `base` moves once per tile, and the sum is rescaled exactly by a
+// power of two.  An Inf/NaN shows as a largest exponent of 0x7ff.  Bound by the integer ALU (73 % active at
+// 4096^3): four operations an element, the maximum and the OR two elements at a time; with `base` checked at
+// every element it was seven (1 GiB of operands 215 us, now 190).
+//
+// A float's high word as a double is its magnitude shifted by 3 with the exponent rebased.  A zero or
+// subnormal float gets exponent field 896 that way, no matter next to a row's larger values; EXACT takes
+// the high words of the widened values instead.
 struct ThreadStats {
     uint32_t mx, lo;
     float sq;
@@ -420,26 +432,14 @@ __device__ __noinline__ ThreadStats scan_tiles_exact(unsigned char* tbuf, const 
     return scan_tiles<TX, true>(tbuf, X, R, K, sr, sp, r0, tb, te);
 }
 
-// Thread (rr = t % 32, g = t / 32) keeps, for row rr and the
-// eight k of group g in every tile, the largest high word of |x|, the OR of the low words and the
-// sum of squares in FP32 relative to its running largest exponent `base`: f = |x| 2^(1023 - base)
-// is the high word times 8 (exponent and 20 mantissa bits moved into FP32 position) minus
-// (base - 127) 2^23, one integer multiply-add, valid for exponents above base - 127.  High words below
-// that are raised to its lowest value, whose square is zero in FP32.  `base` moves once per tile, to
-// the exponent of the largest high word so far, and the running sum is rescaled exactly by a power of
-// two.  Bound by the integer ALU: these four ALU operations an element, the maximum and the OR taken
-// two elements at a time; with `base` checked at every element it was seven (1 GiB of operands: 215
-// us, now 169, 6.4 TB/s).  An Inf/NaN shows as a largest exponent of 0x7ff.
+// The statistics of both operands and the plan, in one launch: scan_tiles per thread, folded per row block
+// over its k-chunks, then over the row blocks.  Small operands are bound by the launches and by the serial
+// folds and FP64 functions behind them: with the row totals in a kernel of their own (atomics and a memset
+// before it) and the plan in another, these steps took 23 us of a 403 x 517 x 389 product and 26 of
+// 1024^3, with the gaps between four launches beside them; this kernel takes 13 and 18.
 //
-// Small operands are bound by the launches and by the plan's chain of FP64 functions instead: with the
-// row totals in a kernel of their own (atomics and a memset before it) and the plan in another, these
-// steps took 23 us of a 403 x 517 x 389 product and 26 of 1024^3 with the gaps between four launches
-// beside them, now 13 and 17.
-//
-// A float's high word as a double is its magnitude shifted by 3 with the exponent rebased.  A zero or
-// subnormal float gets exponent field 896 that way, no matter next to a row's larger values: a block with
-// a row that has nothing above 2^-86 goes over its tiles again with the doubles' own high words, and
-// all-zero rows are known by their OR.
+// A float block with a row that has nothing above 2^-86 goes over its tiles again with EXACT; all-zero rows
+// are known by their OR.
 template <typename TX>
 __global__ void __launch_bounds__(256, 4) stats_kernel(const StatsArgs a) {
     constexpr bool F32 = sizeof(TX) == 4;
@@ -797,10 +797,9 @@ __global__ void split_block_kernel(const SplitInfo* __restrict__ ia, const Split
     if (lane == 0) *out = r;
 }
 
-// Summary of the blocks for the caller: the largest modulus count and bound (infos `stride` bytes
-// apart).
 // The level count of a launch that covers several blocks of one panel: the largest of its blocks'
 // (each block's reconstruction reads its own count of levels; the launch reads only the count).
+// Infos `stride` bytes apart.
 __global__ void split_max_slices_kernel(const uint8_t* __restrict__ infos, size_t stride, int count,
                                         SplitInfo* __restrict__ out) {
     if (threadIdx.x != 0) return;
@@ -810,6 +809,7 @@ __global__ void split_max_slices_kernel(const uint8_t* __restrict__ infos, size_
     *out = r;
 }
 
+// Summary of the blocks for the caller: the largest modulus count and bound.
 __global__ void split_panels_summary_kernel(const uint8_t* __restrict__ infos, size_t stride, int count,
                                             SplitInfo* out) {
     if (threadIdx.x != 0) return;
@@ -895,17 +895,17 @@ __device__ __forceinline__ uint32_t mod_small(uint32_t x, uint32_t p, uint32_t i
     return r >= p ? r - p : r;
 }
 
-// Planes of eight consecutive elements xv of one row (row exponent e, bad: the row holds Inf/NaN)
-// at dst, plane stride pstride; sl = slices (digits) or moduli (CRT), bt = beta (CRT).
 // A modulus' constants as packed pairs (k_3, k_2, k_1 = symmetric residues of 2^42, 2^28, 2^14;
 // fl(1/p); -p), in shared memory: three 16-byte reads a modulus serve eight elements, and the packed
-// arithmetic takes half the instructions that bound this pass (8192^3 at 12 moduli 750 -> 725 us, now
-// 685, 6.3 TB/s; 403 x 517 x 389 20 -> 7 us with the smaller blocks of tiles_per_block); the planes'
-// writes bound it now.
+// arithmetic takes half the instructions that bound this pass.  The planes' writes bound it now (DRAM 71 %
+// busy at 4096^3): 8192^3 at 12 moduli 750 us before, now 690, 6.1 TB/s; 403 x 517 x 389 20, now 7, with
+// the smaller blocks of tiles_per_block.
 struct __align__(16) SliceConst {
     ulonglong2 k32, k1_inv, pneg;
 };
 
+// Planes of eight consecutive elements xv of one row (row exponent e, bad: the row holds Inf/NaN)
+// at dst, plane stride pstride; sl = slices (digits) or moduli (CRT), bt = beta (CRT).
 template <int mode>
 __device__ __forceinline__ void slice_emit(const unsigned long long (&xv)[8], int sl, int bt, int e, bool bad,
                                            const SliceConst* tab, uint16_t* __restrict__ dst, int64_t pstride) {
@@ -1072,7 +1072,8 @@ __global__ void __launch_bounds__(256, 3) slice_kernel(const __grid_constant__ O
                                                        const SplitInfo* info, int64_t kpad, int kt) {
     const int w = blockIdx.y < op.yb0 ? 0 : 1;
     const int by = w ? int(blockIdx.y - op.yb0) : int(blockIdx.y);
-    slice_rows<MODE, TX>(w, static_cast<const TX*>(op.X[w]), op.R[w], K, op.sr[w], op.sp[w], op.rexp[w], info, op.planes[w], op.rpad[w], kpad, by, kt);
+    slice_rows<MODE, TX>(w, static_cast<const TX*>(op.X[w]), op.R[w], K, op.sr[w], op.sp[w], op.rexp[w], info, op.planes[w],
+                         op.rpad[w], kpad, by, kt);
 }
 
 // ---- level / pair schedule ---------------------------------------------------------------------

@@ -46,9 +46,10 @@ __global__ void scale_kernel(int64_t rows, int64_t cols, V alpha, V* __restrict_
 //     T = L21 Y11,   Y21 = -Y22 T                              (s = 16, 32, ... nb / 2),
 // T being kept where the zeros above the diagonal go in the end (tri_zero_kernel).  The products skip
 // the zeros of Y11 and Y22, so the levels together take the nb^3 / 6 multiply-adds of a substitution,
-// and what bounds them is the FP64 pipe.  Substituting column by column was bound by its chain of
-// rows instead: 512 steps of a block-wide sum and two barriers, 1120 us for the four 512-row blocks of
-// a 2048-row triangle whatever the rest of the chip did; base and levels take 264 us there, against 143 us for their multiply-adds at the full FP64 rate.
+// and what bounds them is the FP64 pipe (94 % active in the last level, 87 in the one before).
+// Substituting column by column was bound by its chain of rows instead, 512 steps of a block-wide sum and
+// two barriers: 1120 us for the four 512-row blocks of a 2048-row triangle, now 284, of which 143 are the
+// multiply-adds at the full FP64 rate.
 template <typename V>
 struct TriArgs {
     const V* SA;
