@@ -1558,17 +1558,39 @@ __device__ __forceinline__ CrtWords<N> crt_load(const uint8_t* res, int64_t S, i
     return r;
 }
 
-// With k in segments: the sum of the residues b = r + 128 of column cc over the segments, reduced to
-// [0, p) and congruent to (sum of r) + 128, as the single segment's b is.
+// With k in segments: the sums of the residues b = r + 128 of the four columns over the segments, reduced to
+// [0, p) and congruent to (sum of r) + 128, as the single segment's b is.  A word of every segment (the
+// first one's is in r), its columns added in 16-bit halves, 255 values of at most 256 at a time.  Byte by
+// byte and column by column this took 132 us of a 1135 x 1557 x 1766 product in two segments.
 template <int N>
-__device__ __forceinline__ uint32_t crt_seg_sum(const uint8_t* res, int64_t S, int max_levels, int64_t off,
-                                                int nseg, int t, int cc, uint32_t p, uint32_t pinv32) {
-    uint32_t sum = 0;
-    for (int g = 0; g < nseg; ++g) {
-        const uint8_t* q = res + crt_plane(S, max_levels, g, t);
-        sum += t == 0 ? uint32_t(reinterpret_cast<const uint16_t*>(q)[off + cc]) : uint32_t(q[off + cc]);
+__device__ __forceinline__ void crt_seg_sums(const CrtWords<N>& r, const uint8_t* res, int64_t S, int max_levels,
+                                             int64_t off, int nseg, int t, uint32_t p, uint32_t pinv32,
+                                             uint32_t (&b)[4]) {
+    uint32_t s[4] = {0u, 0u, 0u, 0u};
+    uint32_t u = t == 0 ? r.w0[0] : r.w[t] & 0x00ff00ffu, v = t == 0 ? r.w0[1] : (r.w[t] >> 8) & 0x00ff00ffu;
+    for (int g = 1; g < nseg;) {
+        const int g1 = min(nseg, (g / 255 + 1) * 255);
+#pragma unroll 4
+        for (; g < g1; ++g) {
+            const uint8_t* q = res + crt_plane(S, max_levels, g, t);
+            if (t == 0) {
+                const uint2 z = *reinterpret_cast<const uint2*>(q + 2 * off);
+                u += z.x;
+                v += z.y;
+            } else {
+                const uint32_t w = *reinterpret_cast<const uint32_t*>(q + off);
+                u += w & 0x00ff00ffu;
+                v += (w >> 8) & 0x00ff00ffu;
+            }
+        }
+        s[0] += u & 0xffffu;
+        s[t == 0 ? 1 : 2] += u >> 16;
+        s[t == 0 ? 2 : 1] += v & 0xffffu;
+        s[3] += v >> 16;
+        u = v = 0u;
     }
-    return mod_small(sum + 128u * (p - 1u) * uint32_t(nseg - 1), p, pinv32);
+#pragma unroll
+    for (int cc = 0; cc < 4; ++cc) b[cc] = mod_small(s[cc] + 128u * (p - 1u) * uint32_t(nseg - 1), p, pinv32);
 }
 
 // The double W 2^(x) of the two's-complement integer W of LB 32-bit words (low word first), rounded to
@@ -1668,10 +1690,14 @@ __device__ __forceinline__ void crt_cols(const CrtWords<N>& r, const uint8_t* re
         const bool pair = Q.q > one;
         uint32_t x[4];
         if (nseg > 1) {
+            uint32_t b[4];
+            crt_seg_sums<N>(r, res, S, max_levels, off, nseg, Q.ia, Q.p, Q.pinv32, b);
 #pragma unroll
-            for (int cc = 0; cc < 4; ++cc) {
-                x[cc] = crt_seg_sum<N>(res, S, max_levels, off, nseg, Q.ia, cc, Q.p, Q.pinv32) * Q.A + Q.K;
-                if (pair) x[cc] += crt_seg_sum<N>(res, S, max_levels, off, nseg, Q.ib, cc, Q.q, Q.qinv32) * Q.B;
+            for (int cc = 0; cc < 4; ++cc) x[cc] = b[cc] * Q.A + Q.K;
+            if (pair) {
+                crt_seg_sums<N>(r, res, S, max_levels, off, nseg, Q.ib, Q.q, Q.qinv32, b);
+#pragma unroll
+                for (int cc = 0; cc < 4; ++cc) x[cc] += b[cc] * Q.B;
             }
         } else if (Q.ia == 0) {
 #pragma unroll

@@ -74,7 +74,7 @@ def cols(tmp_path_factory):
 
     body = (part("__device__ __forceinline__ uint32_t mod_small(", "// A modulus' constants") +
             part("__host__ __device__ __forceinline__ int64_t crt_plane(", "// With k in segments") +
-            part("template <int N>\n__device__ __forceinline__ uint32_t crt_seg_sum(", "// The double W 2^(x)") +
+            part("// With k in segments: ", "// The double W 2^(x)") +
             part("template <int LB>\n__device__ __noinline__ double words_to_double_any", "// Residue (CRT) reconstruction of four") +
             part("template <int N>\n__device__ __forceinline__ void crt_cols(", "template <typename TC>\nstruct CrtCombine"))
     cases = "".join(f"case {n}: crt_cols<{n}>(crt_load<{n}>(res, S, 0, 0), res, S, 0, nseg, levels, scale, 0, fj, v); break;\n"
@@ -153,7 +153,7 @@ def test_single_group_residues_one_past_the_symmetric_range(cols, n):
         assert cols(n, [res]) == [float(t) for t in four]
 
 
-@pytest.mark.parametrize("nseg", [2, 3, 38, 76])
+@pytest.mark.parametrize("nseg", [2, 3, 38, 76, 254, 255, 256, 700])
 @pytest.mark.parametrize("n", [2, 5, 12, 13, 15])
 def test_segments(cols, n, nseg):
     g = _gen()
