@@ -378,27 +378,32 @@ __host__ __device__ constexpr int max_shape() { return sizeof(T) == 8 ? 3 : 4; }
 template <typename T>
 __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 2 : 3)
 grouped_kernel(const DevProblem* __restrict__ probs, const DevTile* __restrict__ tiles, int ntiles,
-               int* __restrict__ counter) {
+               int* __restrict__ counter, int num_sms) {
     const int lane = threadIdx.x & 31;
     // the warps' staging regions (dynamic shared memory of kStageBytes or kDStageBytes per block)
     extern __shared__ __align__(16) float stage_smem[];
     float* sw = stage_smem + (threadIdx.x >> 5) * (2 * kStageBuf);
     (void)sw;
-    // The tickets run two tiles ahead and the tile descriptions one: the ticket after next is taken and
-    // the next tile's description read while this tile is worked on, so neither round trip precedes a
-    // tile (small tiles are a few hundred clocks of multiply-adds).
-    int t = 0, next = 0;
-    if (lane == 0) {
-        t = atomicAdd(counter, 1);
-        next = atomicAdd(counter, 1);
-    }
-    t = __shfl_sync(0xffffffffu, t, 0);
+    // A warp's first tile is fixed, the tiles being dealt out over the blocks before a block gets its second
+    // one (and over the quarters of an SM: the blocks of its next round start two warps on); further ones
+    // are tickets.  While there are plenty, the next tile's ticket is taken a tile ahead and its description
+    // read while this tile is worked on, so that neither round trip precedes a tile (small tiles are a few
+    // hundred clocks of multiply-adds).  Over the last three tiles a warp a ticket is taken when it is
+    // needed: one in hand would keep its tile waiting behind a long one while other warps have nothing to
+    // do (28 products of 64^3 FP64, 224 tiles for as many warps: 165 us with every warp taking two).  The
+    // shuffle tells the compiler that the lanes agree on t: a tile's description then lives in uniform
+    // registers, without which the kernel spills 64 bytes and 10,000 FP32 products take 420 us.
+    const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0);
+    int t = ((warp + int(blockIdx.x) / num_sms * 2) & 7) * int(gridDim.x) + int(blockIdx.x);
     if (t >= ntiles) return;
+    auto plenty = [&](int ticket) { return ticket < ntiles - 24 * int(gridDim.x); };
+    auto take = [&] { return lane == 0 ? 8 * int(gridDim.x) + atomicAdd(counter, 1) : 0; };
     DevTile tl = tiles[t];
+    int taken = plenty(t) ? take() : -1;
     while (true) {
-        t = __shfl_sync(0xffffffffu, next, 0);
-        if (lane == 0) next = atomicAdd(counter, 1);
-        const DevTile tn = tiles[min(t, ntiles - 1)];
+        t = __shfl_sync(0xffffffffu, taken, 0);  // the next tile's, -1 for none in hand
+        DevTile tn = tiles[min(unsigned(t), unsigned(ntiles - 1))];
+        taken = t >= 0 && plenty(t) ? take() : -1;
         const DevProblem p = probs[tl.prob];
         if constexpr (sizeof(T) == 4) {
             warp_tile_staged(p, tl.tm, tl.tn, lane, sw);
@@ -407,6 +412,10 @@ grouped_kernel(const DevProblem* __restrict__ probs, const DevTile* __restrict__
             const int rows = min(p.tr, p.m - i0), cols = min(p.tc, p.n - j0);
             double* sd = reinterpret_cast<double*>(stage_smem) + (threadIdx.x >> 5) * (2 * kDStage);
             warp_tile_flat(p, i0, j0, rows, cols, lane, sd);
+        }
+        if (t < 0) {
+            t = __shfl_sync(0xffffffffu, take(), 0);
+            tn = tiles[min(t, ntiles - 1)];
         }
         if (t >= ntiles) return;
         tl = tn;
@@ -644,13 +653,14 @@ int grouped_smem() {
     return bytes;
 }
 
-// Persistent grid for `ntiles` warp tiles: every SM's resident blocks, or fewer for a short list.
+// Persistent grid for `ntiles` warp tiles: every SM's resident blocks, or a block a tile for a short list,
+// which spreads it over the SMs and their quarters.
 template <typename T>
 int grouped_grid(int64_t ntiles, int num_sms) {
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, grouped_kernel<T>, 256, grouped_smem<T>());
     per_sm = std::max(per_sm, 1);
-    return int(std::max<int64_t>(1, std::min<int64_t>(int64_t(num_sms) * per_sm, (ntiles + 7) / 8)));
+    return int(std::max<int64_t>(1, std::min<int64_t>(int64_t(num_sms) * per_sm, ntiles)));
 }
 
 template <typename T>
@@ -695,7 +705,7 @@ int plan_create(const gb300_gemm_problem* probs, int64_t count, int force_shape,
         cudaMemsetAsync(p->d_counter, 0, sizeof(int), p->cap_stream);
         if (p->ntiles > 0)
             grouped_kernel<T><<<p->grid, 256, grouped_smem<T>(), p->cap_stream>>>(p->d_probs, p->d_tiles,
-                                                                              int(p->ntiles), p->d_counter);
+                                                                              int(p->ntiles), p->d_counter, r.num_sms);
         e = cudaStreamEndCapture(p->cap_stream, &p->graph);
     }
     if (e == cudaSuccess) e = cudaGraphInstantiate(&p->exec, p->graph, 0);
@@ -984,7 +994,7 @@ int grouped_lane_launch(GroupedLane* l, const gb300_gemm_problem* probs, int64_t
         const int grid = grouped_grid<double>(int64_t(l->ht.size()), runtime().num_sms);
         grouped_kernel<double><<<grid, 256, grouped_smem<double>(), l->stream>>>(reinterpret_cast<const DevProblem*>(d),
                                                             reinterpret_cast<const DevTile*>(d + off_t),
-                                                            int(l->ht.size()), l->d_counter);
+                                                            int(l->ht.size()), l->d_counter, runtime().num_sms);
         count_launches(1);
         e = cudaGetLastError();
     }
