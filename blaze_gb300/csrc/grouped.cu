@@ -487,11 +487,12 @@ double padded_outputs(int m, int n, int s, bool flat) {
            double(c.count - 1) * warp(lr, c.size) + warp(lr, lc);
 }
 
-int model_shape(int m, int n, int nshapes, bool flat, int k = 1, double tile_w = -1.0) {
+int model_shape(int m, int n, int nshapes, bool flat, int k = 1, double tile_w = -1.0, int max_outputs = 1 << 20) {
     int best = 0;
     double best_cost = 1e300;
     for (int s = 0; s < nshapes; ++s) {
         const double tr = shape_rows(s), tc = shape_cols(s);
+        if (tr * tc > max_outputs) continue;
         const double padded = padded_outputs(m, n, s, flat);
         const double tiles = std::ceil(m / tr) * std::ceil(n / tc);
         // a small per-tile overhead favours fewer, larger tiles when the padding is equal
@@ -518,7 +519,7 @@ void tune_defaults() {
     g_tune_init = true;
 }
 
-int pick_shape(int dtype_idx, int m, int n, int k, int mode_override = -1) {
+int pick_shape(int dtype_idx, int m, int n, int k, int mode_override = -1, int max_outputs = 1 << 20) {
     std::lock_guard<std::mutex> lock(g_tune_mu);
     tune_defaults();
     const int nshapes = dtype_idx == 0 ? max_shape<double>() + 1 : max_shape<float>() + 1;
@@ -539,8 +540,14 @@ int pick_shape(int dtype_idx, int m, int n, int k, int mode_override = -1) {
             }
             return best;
         }
-        default: return model_shape(m, n, nshapes, dtype_idx == 0, k, g_tune.tile_w[dtype_idx]);
+        default: return model_shape(m, n, nshapes, dtype_idx == 0, k, g_tune.tile_w[dtype_idx], max_outputs);
     }
+}
+
+// Whether plans pick shapes by the model.
+bool uses_model(int dtype_idx, int mode_override) {
+    std::lock_guard<std::mutex> lock(g_tune_mu);
+    return (mode_override >= 0 ? mode_override : g_tune.mode[dtype_idx]) == kPickModel;
 }
 
 }  // namespace
@@ -573,13 +580,17 @@ void plan_free(GroupedPlan* p) {
     delete p;
 }
 
-// The device problem table and the flat tile list of a batch (longest tiles first).  Each
-// product's shape depends only on its own (m, n, k) and the tuning state, so a product gets the same
-// tiles — and the same result bits — whatever else is in the batch.
+// The device problem table and the flat tile list of a batch (longest tiles first).  Every output sums its
+// k range in order whatever tile it is in, so a product gets the same result bits whatever else is in
+// the batch.
+//
+// Shapes come from the product's own (m, n, k) and the tuning state.  A list that does not fill the chip
+// waits for its longest tile, which one warp works on alone: where the model picks the shapes, such a
+// batch takes the smallest tiles that leave two of them or fewer on a quarter of an SM.
 template <typename T>
 int build_tables(const gb300_gemm_problem* probs, int64_t count, int force_shape, int policy,
                  std::vector<DevProblem>& hp, std::vector<DevTile>& ht, double& useful, double& padded,
-                 std::string* err) {
+                 std::string* err, int max_outputs = 1 << 20) {
     const int didx = sizeof(T) == 8 ? 0 : 1;
     hp.clear();
     ht.clear();
@@ -616,7 +627,7 @@ int build_tables(const gb300_gemm_problem* probs, int64_t count, int force_shape
         d.beta = x.beta;
         if (d.m == 0 || d.n == 0) continue;
         if (d.k == 0 || x.alpha == 0.0) d.k = 0;  // C = beta*C through the same kernel
-        d.shape = force_shape >= 0 ? force_shape : pick_shape(didx, d.m, d.n, d.k, policy);
+        d.shape = force_shape >= 0 ? force_shape : pick_shape(didx, d.m, d.n, d.k, policy, max_outputs);
         d.tr = shape_rows(d.shape);
         d.tc = shape_cols(d.shape);
         if (sizeof(T) == 8) {
@@ -630,6 +641,19 @@ int build_tables(const gb300_gemm_problem* probs, int64_t count, int force_shape
             for (int b = 0; b < nt; ++b) ht.push_back(DevTile{pid, a, b, 0});
         useful += 2.0 * d.m * d.n * d.k;
         padded += 2.0 * padded_outputs(d.m, d.n, d.shape, sizeof(T) == 8) * d.k;
+    }
+    const size_t few = size_t(runtime().num_sms) * 8;
+    if (force_shape < 0 && max_outputs == 1 << 20 && !ht.empty() && ht.size() <= few && uses_model(didx, policy)) {
+        for (int cap : {64, 256, 512}) {
+            size_t tiles = 0;
+            for (const DevProblem& d : hp) {
+                const int sh = pick_shape(didx, d.m, d.n, d.k, policy, cap);
+                tiles += size_t((int64_t(d.m) + shape_rows(sh) - 1) / shape_rows(sh)) *
+                         size_t((int64_t(d.n) + shape_cols(sh) - 1) / shape_cols(sh));
+            }
+            if (tiles <= few)
+                return build_tables<T>(probs, count, force_shape, policy, hp, ht, useful, padded, err, cap);
+        }
     }
     // longest first: tiles ordered by their k times tile area (descending)
     std::stable_sort(ht.begin(), ht.end(), [&](const DevTile& a, const DevTile& b) {
