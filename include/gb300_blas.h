@@ -157,12 +157,14 @@ void gb300_grouped_plan_destroy(gb300_grouped_plan* plan);
 int gb300_dgemm_grouped(const gb300_gemm_problem* problems, int64_t count, void* stream);
 int gb300_sgemm_grouped(const gb300_gemm_problem* problems, int64_t count, void* stream);
 /* Autotuner: time every warp-tile shape on synthetic batches of each size class (m, n bucketed by
- * powers of two up to 256, k in three ranges) and keep the fastest per class.  effort >= 1 scales
- * the batch size.  Tables persist through save/load ("gb300-grouped-tune v1" text files). */
+ * powers of two up to 256, k in three ranges), and keep the measured choice where it is faster than
+ * the default on a mixed batch.  effort >= 1 scales the batch size.  Tables persist through save/load
+ * ("gb300-grouped-tune v1" / "v2" text files; costs measured on other kernels are not used). */
 int gb300_grouped_autotune(int elem_bytes, int effort);
 int gb300_grouped_tuning_save(const char* path);
 int gb300_grouped_tuning_load(const char* path);
-/* Shape index the planner uses for a product, with its warp-tile rows and columns. */
+/* Shape index the planner uses for a product in a list that fills the GPU (short lists take smaller
+ * ones), with its largest tile's rows and columns. */
 int gb300_grouped_shape_for(int elem_bytes, int64_t m, int64_t n, int64_t k, int* rows, int* cols);
 
 /* ---- serving: continuous batching of product requests ---------------------------------------
