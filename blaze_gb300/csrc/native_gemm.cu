@@ -631,13 +631,17 @@ NativePlan native_plan(int64_t m, int64_t n, int64_t k, int elem_bytes, int num_
     const Small f64[] = {{16, 1.97, 128.0}, {8, 1.7, 48.0}};
     const Small f32[] = {{32, 40.0, 32.0}, {16, 18.0, 24.0}, {8, 10.0, 24.0}};
     const Small* forms = elem_bytes == 8 ? f64 : f32;
+    // A small tile takes at least the splits of the large ones: an output summed over more steps in one
+    // chain has a larger rounding error (4096 x 64 x 4096 FP64 in one chain 3.3e-17 normwise, in the large
+    // tiles' nine 1.1e-17).
+    const int least = best.splits;
     for (int f = 0; f < (elem_bytes == 8 ? 2 : 3); ++f) {
         const Small& t = forms[f];
         const double tiles = ceil_div(m, t.tile) * ceil_div(n, t.tile);
         if (tiles > 2147483647.0) continue;  // gridDim.x
         const int max_splits = int(std::min<double>(double(num_sms) / tiles, double(k / 128)));
-        for (int splits : {1, max_splits}) {
-            if (splits < 1) continue;
+        for (int splits : {1, max_splits, least}) {
+            if (splits < least) continue;
             const double per_sm = waves(tiles * splits);
             const double step = std::max(per_sm * t.tile * t.tile / t.rate, t.latency);
             const double clk = ceil_div(k, splits) * step + 3000.0 + (splits > 1 ? kReduceClk : 0.0);

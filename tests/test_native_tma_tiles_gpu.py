@@ -16,13 +16,13 @@ SMS = 152
 
 # element bytes, m, n, k, tile columns, k splits (row-major logical sizes)
 SHAPES = [
-    (8, 417, 43, 20003, 64, 76), (8, 109, 195, 20003, 128, 76), (8, 43, 417, 20003, 256, 76),
+    (8, 253, 55, 40001, 64, 152), (8, 115, 113, 40001, 128, 152), (8, 55, 253, 40001, 256, 152),
     (8, 38900, 59, 131, 64, 1), (8, 371, 19259, 67, 128, 1), (8, 59, 38900, 131, 256, 1),
-    (4, 1627, 5, 8203, 64, 16), (4, 195, 371, 4101, 128, 8), (4, 5, 1627, 8203, 256, 16),
+    (4, 229, 43, 40001, 64, 78), (4, 69, 161, 40001, 128, 76), (4, 43, 229, 40001, 256, 78),
     (4, 38900, 59, 131, 64, 1), (4, 1021, 1531, 203, 128, 1), (4, 59, 38900, 131, 256, 1),
 ]
-# allocation-free products whose split sums fill most of the 16 MiB scratch
-NOALLOC = [(240, 224, 12000, 128, 38), (464, 48, 20000, 64, 76), (48, 464, 20000, 256, 76)]
+# allocation-free products whose split sums fill most of the 16 MiB scratch, and their tiles (0: the large ones)
+NOALLOC = [(240, 224, 12000, 16, 38), (464, 48, 20000, 16, 76), (48, 464, 20000, 16, 76), (114, 114, 40000, 0, 152)]
 
 HOST = r"""
 #include <algorithm>
@@ -37,13 +37,15 @@ int main(int argc, char** argv) {
     for (int i = 1; i + 3 < argc; i += 4) {
         const long e = atol(argv[i]), m = atol(argv[i + 1]), n = atol(argv[i + 2]), k = atol(argv[i + 3]);
         const NativePlan p = native_plan(m, n, k, int(e), 152, false);
-        std::printf("%d %d %d\n", p.tile, native_tile_n(m, n), p.splits);
+        std::printf("%d %d %d %d\n", p.tile, native_tile_n(m, n), p.splits, native_choose_splits(m, n, k, int(e), 152));
     }
 }
 """
 
 
-def test_the_plan_picks_these_tiles(tmp_path):
+@pytest.fixture(scope="module")
+def host_plan(tmp_path_factory):
+    """Plans of (element bytes, m, n, k): (small tile or 0, large tiles' columns, splits, large tiles' splits)."""
     gxx = shutil.which("g++")
     if not gxx:
         pytest.skip("no host C++ compiler")
@@ -51,12 +53,30 @@ def test_the_plan_picks_these_tiles(tmp_path):
         src = f.read()
     line = lambda start: src[src.index(start):src.index("\n", src.index(start)) + 1]  # noqa: E731
     plan = src[src.index("int native_choose_splits("):src.index("template <typename T>\ncudaError_t native_gemm(const Gemm& g, const NativePlan& plan")]
-    (tmp_path / "p.cpp").write_text(HOST + line("constexpr int PANEL_BYTES") + line("int native_tile_n(") + plan + MAIN)
-    subprocess.run([gxx, "-std=c++17", "-o", str(tmp_path / "p"), str(tmp_path / "p.cpp")], check=True)
+    d = tmp_path_factory.mktemp("plan")
+    (d / "p.cpp").write_text(HOST + line("constexpr int PANEL_BYTES") + line("int native_tile_n(") + plan + MAIN)
+    subprocess.run([gxx, "-std=c++17", "-o", str(d / "p"), str(d / "p.cpp")], check=True)
+
+    def run(cases):
+        out = subprocess.run([str(d / "p"), *[str(x) for c in cases for x in c[:4]]], check=True, capture_output=True, text=True)
+        return [tuple(int(x) for x in l.split()) for l in out.stdout.splitlines()]
+
+    return run
+
+
+def test_the_plan_picks_these_tiles(host_plan):
     cases = SHAPES + [(8, *c) for c in NOALLOC]
-    out = subprocess.run([str(tmp_path / "p"), *[str(x) for c in cases for x in c[:4]]], check=True, capture_output=True, text=True)
-    got = [tuple(int(x) for x in l.split()) for l in out.stdout.splitlines()]
-    assert got == [(0, c[4], c[5]) for c in cases]
+    tiles = [(0, c[4], c[5]) for c in SHAPES] + [(c[3], None, c[4]) for c in NOALLOC]
+    got = [p[:3] for p in host_plan(cases)]
+    assert [(a, b if w[1] else None, c) for (a, b, c), w in zip(got, tiles)] == tiles
+
+
+def test_small_tiles_sum_no_longer_chains(host_plan):
+    # a plan in small tiles splits k at least as far as the large tiles do for the same product
+    cases = [(e, m, n, k) for e in (8, 4) for m in (1, 60, 100, 512, 1024, 4096) for n in (1, 48, 64, 200, 512, 4096)
+             for k in (100, 600, 1600, 6000, 8192, 20003, 100000)]
+    for case, (tile, _, splits, large) in zip(cases, host_plan(cases)):
+        assert splits >= large, (case, tile, splits, large)
 
 
 def _stored(torch, x, trans, pad):
@@ -97,8 +117,8 @@ def test_every_tile_width_and_transposition(elem, m, n, k, bn, splits, ta, tb):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("m,n,k,bn,splits", NOALLOC)
-def test_noalloc_products_that_use_the_scratch(m, n, k, bn, splits):
+@pytest.mark.parametrize("m,n,k,tile,splits", NOALLOC)
+def test_noalloc_products_that_use_the_scratch(m, n, k, tile, splits):
     torch = pytest.importorskip("torch")
     assert G.device_info()[0] == SMS
     assert splits * m * n * 8 <= (16 << 20) - 256
