@@ -627,9 +627,11 @@ NativePlan native_plan(int64_t m, int64_t n, int64_t k, int elem_bytes, int num_
     // 96^3 393 -> 10.5 us (about 7 of them the launches), 256^3 1030 -> 36, 512^3 1032 -> 233,
     // 1024^3 2055 -> 1733, 2048^3 16362 -> 13776.
     // Float: 128^3 25.8 -> 7.6 us, 256^3 38.5 -> 12.2, 512^3 64.7 -> 27.6, 768^3 94.3 -> 70.5; from
-    // 1024^3 on the large tiles stay ahead (28.7 TFLOP/s there, 36.6 at 2048^3).
+    // 1024^3 on the large tiles stay ahead (28.7 TFLOP/s there, 36.6 at 2048^3).  32-wide tiles at 40
+    // multiply-adds a clock would take 1024 x 256 x 2048 and 512 x 512 x 2048 too: 102 us a call, 81 in
+    // the large tiles.
     const Small f64[] = {{16, 1.97, 128.0}, {8, 1.7, 48.0}};
-    const Small f32[] = {{32, 40.0, 32.0}, {16, 18.0, 24.0}, {8, 10.0, 24.0}};
+    const Small f32[] = {{32, 27.0, 32.0}, {16, 18.0, 24.0}, {8, 10.0, 24.0}};
     const Small* forms = elem_bytes == 8 ? f64 : f32;
     // A small tile takes at least the splits of the large ones: an output summed over more steps in one
     // chain has a larger rounding error (4096 x 64 x 4096 FP64 in one chain 3.3e-17 normwise, in the large

@@ -137,3 +137,12 @@ def test_noalloc_products_that_use_the_scratch(m, n, k, tile, splits):
         assert torch.equal(c1, c2)  # the same plan
         err = float((c1 - A @ B).norm())
         assert err <= 2 * k * 2.0 ** -53 * float(A.norm()) * float(B.norm())
+
+
+def test_float_products_of_full_large_tiles_stay_in_them(host_plan):
+    # sizes that a 32-wide tile's rate of 40 multiply-adds a clock gave to the small tiles, which took longer
+    cases = [(4, 1024, 256, 2048), (4, 512, 512, 2048), (4, 1024, 512, 1024), (4, 1024, 1024, 512)]
+    assert [p[0] for p in host_plan(cases)] == [0] * len(cases)
+    # and sizes whose small tiles are faster
+    cases = [(4, 512, 512, 512), (4, 768, 768, 768), (4, 300, 300, 2000), (4, 2000, 100, 1500), (4, 256, 256, 256)]
+    assert all(p[0] != 0 for p in host_plan(cases))
