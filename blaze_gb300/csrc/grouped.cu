@@ -385,7 +385,7 @@ grouped_kernel(const DevProblem* __restrict__ probs, const DevTile* __restrict__
     float* sw = stage_smem + (threadIdx.x >> 5) * (2 * kStageBuf);
     (void)sw;
     // A warp's first tile is fixed, the tiles being dealt out over the blocks before a block gets its second
-    // one (and over the quarters of an SM: the blocks of its next round start two warps on); further ones
+    // one (and over the quarters of an SM: an SM's next block starts two warps on); further ones
     // are tickets.  While there are plenty, the next tile's ticket is taken a tile ahead and its description
     // read while this tile is worked on, so that neither round trip precedes a tile (small tiles are a few
     // hundred clocks of multiply-adds).  Over the last three tiles a warp a ticket is taken when it is

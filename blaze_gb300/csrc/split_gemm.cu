@@ -1848,11 +1848,13 @@ dim3 crt_combine_grid(int64_t m, int64_t n, int num_sms) {
     return dim3(unsigned(x), unsigned(y));
 }
 
+// Launched the plain way, so that its pointers can be __restrict__: as a dependent launch without, the next
+// row's loads waited for this row's stores (8192 x 8192 x 64 in six slices 1.79 ms a call, 1.60 so).
 template <typename TC>
-__global__ void __launch_bounds__(128, 8) combine_kernel(const int32_t* levels, int nseg, int max_levels, int64_t mpad,
-                               int64_t npad, int mode, const SplitInfo* info, const int* eA, const int* eB, int64_t m,
-                               int64_t n, double alpha, double beta, TC* C, int64_t ldc) {
-    griddep_wait();
+__global__ void __launch_bounds__(128, 8)
+combine_kernel(const int32_t* __restrict__ levels, int nseg, int max_levels, int64_t mpad, int64_t npad, int mode,
+               const SplitInfo* __restrict__ info, const int* __restrict__ eA, const int* __restrict__ eB, int64_t m,
+               int64_t n, double alpha, double beta, TC* __restrict__ C, int64_t ldc) {
     const int64_t j0 = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) * COMBINE_COLS;
     if (j0 >= n) return;
     const int64_t plane = mpad * npad;
@@ -1900,7 +1902,12 @@ __global__ void __launch_bounds__(128, 8) combine_kernel(const int32_t* levels, 
     for (int c = 0; c < COMBINE_COLS; ++c) {
         const int64_t j = j0 + c;
         if (j >= n) break;
-        crow[j] = plain ? TC(v[c]) : scaled(v[c], alpha, beta, crow + j);
+        if (plain) {
+            crow[j] = TC(v[c]);
+        } else {
+            const double x = alpha * v[c];
+            crow[j] = TC(beta == 0.0 ? x : fma(beta, double(crow[j]), x));
+        }
     }
     }
 }
@@ -2392,8 +2399,8 @@ int tensor_product(const Gemm& g, const SplitRequest& req, const LaunchCtl& ctl,
         } else {
             const int64_t colgroups = (n + COMBINE_COLS - 1) / COMBINE_COLS;
             dim3 cgrid(unsigned((colgroups + 127) / 128), unsigned(std::min<int64_t>(m, 65535)));
-            launch_dependent(combine_kernel<T>, cgrid, dim3(128), 0, st, lv, nseg, max_levels, mpad, npad, mode, info, eA,
-                             eB, m, n, g.alpha, g.beta, static_cast<T*>(g.C), g.ldc);
+            combine_kernel<T><<<cgrid, 128, 0, st>>>(lv, nseg, max_levels, mpad, npad, mode, info, eA, eB, m, n, g.alpha,
+                                                     g.beta, static_cast<T*>(g.C), g.ldc);
         }
     }
     count_launches(2);
